@@ -52,13 +52,13 @@ struct esm_ctx {
     bool has_state = false, has_scores = false;
     int move_wpb = 1;           // k_move block shape: warps per block (1, 2 or 4)
     int max_warps = 0;          // k_move warps launched per move: the resident limit or a tuned count
-    // the cooperative walk of the separable moves (k_move_sep): moves with at least sep_min units
-    // (0: off), its grid and where its per-warp walk buffers live
-    int sep_min = ESM_SEP_MIN_DEFAULT, sep_max_warps = 0, sep_in_smem = 1;
+    // the block walk of the separable moves (k_move_sep): moves with at least sep_min units (0: all),
+    // its grid (0 blocks: not used), shared memory and the buffer of its long sorts
+    int sep_min = ESM_SEP_MIN_DEFAULT, sep_blocks = 0, sep_region = 0, sep_tmp_warp = 0;
+    char *d_sep_tmp = nullptr;
     int sl_nunits = 0;  // eligible units of the last long-range storage sweep (its move log)
     int device = -1;                   // the device the context was created on
     double *score_scratch = nullptr;   // device address of the static score scratch on that device
-    char *d_sep_slab = nullptr;
     int warps_cap[3] = {0, 0, 0};  // the resident limit per block shape (1, 2, 4 warps per block)
     int nsm = 0;
     esm::DevModel<float> Mf;
@@ -495,22 +495,11 @@ int alloc_state(esm_ctx *c) {
     }
     if ((rc = dalloc(c, &q, per * wscr))) return rc;
     c->d_scratch = q;
-    // the cooperative walk: resident warps of k_move_sep and, when two walk regions and the
-    // descriptor do not fit a block's shared memory, one global region per warp (at most 1 GB)
-    {
-        int in_smem = 1;
-        int wps = esm::sep_warps_per_sm<real>(M, &in_smem);
-        size_t reg = esm::sep_region_bytes<real>(M);
-        size_t sw = (size_t)nsm * wps;
-        if (!in_smem) sw = std::max<size_t>(64, std::min(sw, ((size_t)1 << 30) / reg));
-        c->sep_max_warps = (int)(sw & ~(size_t)1);
-        c->sep_in_smem = in_smem;
-        if (!in_smem) {
-            char *sl;
-            if ((rc = dalloc(c, &sl, reg * (size_t)c->sep_max_warps))) return rc;
-            c->d_sep_slab = sl;
-        }
-    }
+    // the block walk of the separable moves
+    c->sep_region = esm::sep_region_bytes<real>(M);
+    c->sep_blocks = esm::sep_blocks<real>(M, nsm);
+    c->sep_tmp_warp = esm::sep_tmp_bytes<real>(M);
+    if ((rc = dalloc(c, &c->d_sep_tmp, (size_t)4 * c->sep_tmp_warp * c->sep_blocks))) return rc;
     // the move descriptors of a class pass
     char *dp;
     if ((rc = dalloc(c, &dp, esm::linemove_smem_per_warp<real>(M) * (size_t)(M.natoms + M.nextra)))) return rc;
@@ -609,7 +598,7 @@ __global__ void k_set_word(uint32_t *p, uint32_t v) { *p = v; }
 
 int class_pass_launch(esm_ctx *c, int cls, int limit) {
     int ns = c->class_len[cls];
-    esm::SepLaunch sep{c->sep_min, c->sep_max_warps, c->sep_in_smem, c->d_sep_slab};
+    esm::SepLaunch sep{c->sep_min, c->sep_blocks, c->sep_region, c->nsm, c->sep_tmp_warp, c->d_sep_tmp};
     esm::WaveLaunch wave{c->move_schedule == ESM_MOVES_PER_CLASS, c->d_wave_done, c->d_wave_err, c->wave_items};
     if (c->precision == 64)
         CK(esm::launch_class_pass<double>(c->Md, c->d_steps[cls], ns, c->d_sweep, cls, limit, (double *)c->d_scratch,
@@ -1681,7 +1670,7 @@ int esm_set_sep_walk(esm_ctx *c, int32_t min_units) {
 int esm_sep_walk(const esm_ctx *c, int32_t *min_units, int32_t *warps) {
     if (!c) return ESM_EINVAL;
     if (min_units) *min_units = c->sep_min;
-    if (warps) *warps = c->sep_max_warps;
+    if (warps) *warps = 4 * c->sep_blocks;
     return ESM_OK;
 }
 

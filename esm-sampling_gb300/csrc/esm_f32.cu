@@ -22,8 +22,9 @@ template cudaError_t launch_class_pass<float>(const DevModel<float> &, const int
                                               unsigned long long *, char *, unsigned int *, const SepLaunch &,
                                               const WaveLaunch &,
                                               cudaStream_t);
-template size_t sep_region_bytes<float>(const DevModel<float> &);
-template int sep_warps_per_sm<float>(const DevModel<float> &, int *);
+template int sep_region_bytes<float>(const DevModel<float> &);
+template int sep_tmp_bytes<float>(const DevModel<float> &);
+template int sep_blocks<float>(const DevModel<float> &, int);
 template int linemove_blocks_per_sm<float>(const DevModel<float> &, int);
 template cudaError_t launch_batch_passes<float>(const BatchModel<float> *, const BatchLaunch &, const uint32_t *,
                                                 cudaStream_t);

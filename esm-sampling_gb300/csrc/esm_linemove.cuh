@@ -10,13 +10,12 @@ template <class real>
 size_t linemove_scratch_reals(const DevModel<real> &M);  // per warp
 template <class real>
 size_t linemove_smem_per_warp(const DevModel<real> &M);  // bytes of one move descriptor
-// the cooperative walk of the separable moves: moves whose units are storage units at distinct nodes
-// and nothing else, with at least min_units units (0: none, k_move walks every move), run in
-// k_move_sep on max_warps warps, their walk buffers in shared memory (in_smem) or in per-warp slabs
-// of `slab` (sep_region_bytes each)
+// the block walk of the separable moves (k_move_sep): moves whose units are storage units at distinct
+// nodes and nothing else, with at least min_units units (0: all of them), on `blocks` blocks (0: none,
+// k_move walks every move) with `region` bytes of shared memory each and tmp_warp bytes of tmp a warp
 struct SepLaunch {
-    int min_units, max_warps, in_smem;
-    char *slab;
+    int min_units, blocks, region, nsm, tmp_warp;
+    char *tmp;
 };
 // the whole class pass in one k_move_wave launch (on = 1; not with the cooperative walk): done
 // holds the moves completed per work item (max_items), err is set when a bounded wait runs out
@@ -27,9 +26,11 @@ struct WaveLaunch {
     size_t max_items;
 };
 template <class real>
-size_t sep_region_bytes(const DevModel<real> &M);
+int sep_region_bytes(const DevModel<real> &M);
 template <class real>
-int sep_warps_per_sm(const DevModel<real> &M, int *in_smem);
+int sep_tmp_bytes(const DevModel<real> &M);
+template <class real>
+int sep_blocks(const DevModel<real> &M, int nsm);
 // one colour class: the descriptors of its moves into descs ((natoms + nextra) descriptors), then
 // per move one k_move launch (and one k_move_sep launch; the kernel that does not take the move
 // returns at once); the sweep index is read on the device from *sweep (graph-capturable)

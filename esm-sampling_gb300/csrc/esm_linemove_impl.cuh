@@ -746,14 +746,20 @@ struct Lane {
 
     // A min-heap of the units with a pending event, keyed by sgn * (event time): the next event of
     // the walk is at the top, and passing it costs log2(units) steps instead of a scan of all units.
+    // In the FP64 build events of one time come in unit order, as the block walk takes them (their
+    // slopes sum to other last bits in another order; the FP32 slopes' double sums are the same).
+    __device__ inline static bool heap_less(real k, real u, real ko, real uo) {
+        if constexpr (sizeof(real) == 8) return k < ko || (k == ko && u < uo);
+        return k < ko;
+    }
     __device__ inline void heap_up(int i) const {
         real k = S(LL.hk, i), u = S(LL.hu, i);
         while (i > 0) {
             int p = (i - 1) >> 1;
-            real kp = S(LL.hk, p);
-            if (!(k < kp)) break;
+            real kp = S(LL.hk, p), up = S(LL.hu, p);
+            if (!heap_less(k, u, kp, up)) break;
             S(LL.hk, i) = kp;
-            S(LL.hu, i) = S(LL.hu, p);
+            S(LL.hu, i) = up;
             i = p;
         }
         S(LL.hk, i) = k;
@@ -765,17 +771,18 @@ struct Lane {
             int l = 2 * i + 1;
             if (l >= n) break;
             int m = l;
-            real km = S(LL.hk, l);
+            real km = S(LL.hk, l), um = S(LL.hu, l);
             if (l + 1 < n) {
-                real kr = S(LL.hk, l + 1);
-                if (kr < km) {
+                real kr = S(LL.hk, l + 1), ur = S(LL.hu, l + 1);
+                if (heap_less(kr, ur, km, um)) {
                     m = l + 1;
                     km = kr;
+                    um = ur;
                 }
             }
-            if (!(km < k)) break;
+            if (!heap_less(km, um, k, u)) break;
             S(LL.hk, i) = km;
-            S(LL.hu, i) = S(LL.hu, m);
+            S(LL.hu, i) = um;
             i = m;
         }
         S(LL.hk, i) = k;
@@ -1691,6 +1698,10 @@ __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
     __shared__ Desc<real> sd;
     __shared__ LaneLayout sLL;
     int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    {  // not a valid move, or one that k_move_sep walks: nothing to do (grid-uniform)
+        const Desc<real> g = carve_desc<real>((char *)(descs + (size_t)mi * stride), M, M.natoms + M.nextra);
+        if (g.hdr[12] < 0 || sep_move<real>(g, sepmin)) return;
+    }
     {  // the block's warps share one copy of the descriptor
         const int4 *src = (const int4 *)(descs + (size_t)mi * stride);
         int4 *dst = (int4 *)smem;
@@ -1707,8 +1718,6 @@ __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
     Desc<real> &d = sd;
     const LaneLayout &LL = sLL;
     int fi = d.hdr[12];
-    if (fi < 0) return;  // not a valid move: nothing to do (grid-uniform)
-    if (sep_move<real>(d, sepmin)) return;  // k_move_sep walks it (grid-uniform)
     // per-lane scratch: a local array (cached in L1, written back) when the layout fits it, else
     // the lane's column of this warp's slab in global memory
     real local[ESM_LANE_LOCAL];
@@ -1914,25 +1923,28 @@ int linemove_blocks_per_sm(const DevModel<real> &M, int wpb) {
     return nb * wpb;
 }
 
-// The cooperative walk of the separable moves (k_move_sep, two-warp blocks): its per-warp region,
-// and whether two regions and the descriptor fit in a block's shared memory (else global slabs).
+// The block walk of the separable moves (k_move_sep): the shared memory of its batches (0: a task of
+// the largest move would not fit, k_move walks every move), the buffer of its long sorts per warp and the
+// resident blocks of the device's nsm multiprocessors. 50 KB a block: four per SM.
 template <class real>
-size_t sep_region_bytes(const DevModel<real> &M) {
-    return (size_t)sep_layout<real>(M.maxstu, M.maxpts).total;
+int sep_region_bytes(const DevModel<real> &M) {
+    int need = sep_unit_bytes<real>(M.maxstu) + 2 * sep_list_bytes<real>(M.maxstu, M.maxpts, SEP_SOLE);
+    if (need > 200 * 1024 || sep_entries(M.maxstu, M.maxpts, SEP_SOLE) > 0x7fff) return 0;
+    return need > 50 * 1024 ? (need + 127) & ~127 : 50 * 1024;
 }
-
 template <class real>
-int sep_warps_per_sm(const DevModel<real> &M, int *in_smem) {
-    size_t stride = linemove_smem_per_warp(M);
-    size_t per = sep_region_bytes(M);
-    size_t smem = stride + 2 * per;
-    *in_smem = smem <= 200 * 1024;
-    if (!*in_smem) smem = stride;
-    cudaFuncSetAttribute(k_move_sep<real, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    int nb = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_move_sep<real, 2>, 64, smem);
+int sep_tmp_bytes(const DevModel<real> &M) {
+    int n = sep_events(M.maxstu, M.maxpts, SEP_BATCH);
+    return n > sep_regs<real>() ? ((int)sizeof(double) * n + 15) & ~15 : 0;
+}
+template <class real>
+int sep_blocks(const DevModel<real> &M, int nsm) {
+    int region = sep_region_bytes(M), nb = 0;
+    if (region == 0) return 0;
+    cudaFuncSetAttribute(k_move_sep<real>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_move_sep<real>, 32 * ESM_SEP_WARPS, region);
     if (e != cudaSuccess || nb < 1) nb = 1;
-    return 2 * nb;
+    return nsm * nb;
 }
 
 template <class real>
@@ -1966,11 +1978,10 @@ cudaError_t launch_class_pass(const DevModel<real> &M, const int *steps, int nst
                                                       scratch, stats, counters, wave.done, wave.err);
         return cudaGetLastError();
     }
-    int sepmin = sep.min_units;
+    // (min_units 0: every separable move goes to the block walk)
+    int sepmin = sep.blocks > 0 ? (sep.min_units > 0 ? sep.min_units : 1) : 0;
     int ntask = nsteps * M.R;
-    int swarps = ntask < sep.max_warps ? ntask : sep.max_warps;
-    int sblocks = (swarps + 1) / 2;
-    size_t ssmem = stride + (sep.in_smem ? 2 * sep_region_bytes(M) : 0);
+    int sblocks = ntask < sep.blocks ? ntask : sep.blocks;
     for (int mi = 0; mi < nrun; ++mi) {
         if (wpb == 4)
             k_move<real, 4><<<blocks, 128, stride, s>>>(M, steps, nsteps, ntile, wpt, sweep, mi, descs, stride, scratch,
@@ -1983,8 +1994,9 @@ cudaError_t launch_class_pass(const DevModel<real> &M, const int *steps, int nst
                                                       stats, counters + mi, sepmin);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         if (sepmin > 0 && sblocks > 0) {
-            k_move_sep<real, 2><<<sblocks, 64, ssmem, s>>>(M, steps, nsteps, sweep, mi, descs, stride, sepmin,
-                                                          sep.in_smem, sep.slab, stats, counters + mi);
+            k_move_sep<real><<<sblocks, 32 * ESM_SEP_WARPS, sep.region, s>>>(M, steps, nsteps, sweep, mi, descs, stride,
+                                                                            sepmin, sep.region, sep.nsm, sep.tmp,
+                                                                            sep.tmp_warp, stats, counters + mi);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
     }

@@ -1,5 +1,6 @@
-// Warp-cooperative walk of the separable storage moves (the state-of-charge atoms of a storage field:
-// storage units at distinct nodes and nothing else), one (step, replica) task per warp.
+// The walk of the separable storage moves (the state-of-charge atoms of a storage field: storage
+// units at distinct nodes and nothing else) by blocks of warps, a batch of (step, replica) tasks at
+// a time.
 //
 // The line potential of such a move is a sum of one-dimensional piecewise-linear unit functions,
 // each with at most ten kinks in a walking direction: its clamps (0 and 1 of the state of charge,
@@ -8,13 +9,26 @@
 // the union of those points in walking order, stops at the first clamp where the potential stands
 // more than maxnats above its minimum, and takes ray steps once every clamp is behind.
 //
-// Here the lanes own the units. The walk goes window by window, a window ending at the nearest clamp
-// still ahead: every lane generates the events of its units up to the window end (the same per-unit
-// piece arithmetic as the per-lane walk), the window's events are compacted in unit order and sorted
-// in shared memory (bitonic, by time, ties by unit and sequence), and the potential at every event
-// follows from three warp scans over the sorted events (slope before the event, potential, running
-// minimum). Points, segment masses and the categorical draw (sample_line!, :1501) stay in shared
-// memory, so the walk keeps no per-lane scratch and runs without divergence between tasks.
+// A list holds one direction of one task's walk. Its work splits into parts of different width:
+//   1. events, one lane per (list, unit): the unit's pieces up to the window end, the nearest clamp
+//      of the list (98 % of the walks of a production chain stop there);
+//   2. order, one warp per list (bitonic, in shared memory) or, for a short list, its scan lane;
+//   3. scan, one lane per list: the summed slope, the potential and the stop test, event by event
+//      in double, in the order of the one-lane walk, so that every sum has the same bits;
+//   4. segment masses, one warp per task (a lane per segment);
+//   5. draw, one lane per task: the sums over the segments are again taken in order;
+//   6. commit, one lane per (task, unit).
+// A list that its window does not end gets the next clamp's window (every event made again: 2 % of
+// the lists at 40 nodes), at last one without an end, in which the ray steps follow.
+//
+// Why this split: the one-lane walk (Lane::walk_sep) runs a heap of units per lane; its lanes sit
+// in different units and pieces, and its unit and heap state, several KB a lane, goes through L2.
+// Here the events, which are nearly all of the arithmetic, are made by lanes in step, with the
+// unit in registers, and the lists stay in shared memory. What bounds it now: the latency of the
+// events' dependent arithmetic and of the scan, at 16 warps per SM (four blocks by registers and by
+// shared memory). Measured for one move at T = 2920, 64 replicas (93440 tasks), FP32, one-lane walk
+// and block walk: 40 units 16.4 and 3.7 ms, 20 units 5.7 and 2.1 ms, 10 units 2.1 and 1.3 ms, 7 units
+// 1.4 and 0.7 ms; an operation sweep at 40 nodes, T = 8760, 64 replicas 1.47 and 0.91 s.
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>
@@ -24,608 +38,949 @@
 
 namespace esm {
 
-// events one unit can produce in one window (clamps, six storage thresholds, two node-balance roots)
-#define ESM_SEP_EVMAX 12
+#define ESM_SEP_WARPS 4           // warps of a block
+#define ESM_SEP_LISTS 128         // lists of a batch at most: one scan thread each
+#define ESM_SEP_EV 12             // events of one unit in one direction, at most (ten by the unit's shape)
+#define ESM_SEP_SHORT 8           // lists up to this length are sorted by their scan lane
+// Moves up to this many units keep what the round-off scales and the ray steps need (18 bytes an entry
+// in FP32, and room for ray points). Larger moves do without (14 bytes): of their draws 0.3 % (7 units)
+// to 0.01 % (40 units) need the scales and run again, alone; of those of 2 units 27 % would.
+#define ESM_SEP_FULL 4
 
-// per-unit fields of the walk state (shared memory, field-major: field f of unit q at f * nu + q)
-enum {
-    SF_UT = 0,   // time of the unit's next event (+-inf: none)
-    SF_UK,       // its kind: 1 clamp, 0 other, -1 none
-    SF_USL,      // the unit's slope up to that event
-    SF_UE,       // events of the current piece (3)
-    SF_UN = SF_UE + 3,
-    SF_UH,       // how the piece ends: 1 clamp, 2 threshold, 0 not at all
-    SF_UI,       // next event of the piece
-    SF_UFE,      // potential at the piece end (or at a probe beyond the piece start)
-    SF_UFN,      // potential at the next event
-    SF_USW,      // node balances at the piece end (step tau, step tau - 1)
-    SF_USA,
-    SF_E0,       // state of charge at tau, tau + 1, tau - 1 and the node balances at tau, tau - 1
-    SF_E1,
-    SF_EM,
-    SF_S0W,
-    SF_S0A,
-    SF_CL0,      // the clamps still ahead, in walking order, and their count
-    SF_CL1,
-    SF_NCL,
-    SF_N
+// The FP32 potential of a unit decides which way a draw on an almost flat segment goes, so the block
+// walk gives every value the rounding that the one-lane walk (Lane::unit_val, Lane::commit) gives it:
+// the contractions of the FP32 build are written out here (fma_rn; in the FP64 build, which has none,
+// a product and a sum) instead of left to the compiler, which chooses them per function.
+__device__ inline float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ inline double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ inline float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ inline double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ inline float sub_rn(float a, float b) { return __fsub_rn(a, b); }
+__device__ inline double sub_rn(double a, double b) { return __dsub_rn(a, b); }
+__device__ inline float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ inline double fma_rn(double a, double b, double c) { return __dadd_rn(__dmul_rn(a, b), c); }
+
+// FP32 to FP64 and back (to nearest even) with integer instructions where the value is normal: a
+// conversion, like every FP64 instruction, holds a scheduler's FP64 unit for 64 cycles whatever the
+// number of active lanes (measured; 16 to 19 cycles per SM), and the scan lanes convert at every event.
+// (the other values in calls of their own, so that they are not converted on every lane)
+static __device__ __noinline__ double sep_widen_any(float x) { return (double)x; }
+static __device__ __noinline__ float sep_narrow_any(double x) { return (float)x; }
+__device__ __forceinline__ double sep_widen(float x) {
+    unsigned u = __float_as_uint(x), m = u & 0x7fffffffu;
+    if (m != 0 && m - 0x00800000u >= 0x7f000000u) return sep_widen_any(x);
+    unsigned h = m == 0 ? 0u : (m >> 3) + 0x38000000u;
+    return __hiloint2double((int)((u & 0x80000000u) | h), (int)(u << 29));
+}
+__device__ inline double sep_widen(double x) { return x; }
+__device__ __forceinline__ float sep_narrow(double x, float) {
+    unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x), m = h & 0x7fffffffu;
+    if (m - 0x38100000u >= 0x0fd00000u) return (m | l) == 0 ? __uint_as_float(h) : sep_narrow_any(x);
+    unsigned f = ((m - 0x38000000u) << 3) | (l >> 29);
+    unsigned rem = l & 0x1fffffffu;
+    f += rem > 0x10000000u || (rem == 0x10000000u && (f & 1u));
+    return __uint_as_float((h & 0x80000000u) | f);
+}
+__device__ inline double sep_narrow(double x, double) { return x; }
+// a float at least |x| (of FP32 size) and no more than 2^-19 above it
+__device__ __forceinline__ float sep_above(double x) {
+    unsigned m = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    return __uint_as_float(m < 0x38000000u ? 8u : ((m - 0x38000000u) << 3) + 8u);
+}
+
+// The draw inside a segment (sample_line!, src/local.jl:1501; a function of its own, so that its
+// contractions depend on nothing around it).
+template <class real>
+__device__ __noinline__ real sep_pick(real p0, real p1, real g, real L, real uoff, real flat) {
+    return (g >= 0 || fabs(g * L) < flat) ? p0 + Lane<real>::trexp_offset(uoff, g, L, flat)
+                                          : p1 - Lane<real>::trexp_offset(uoff, -g, L, flat);
+}
+
+// How a list is laid out: the entries of a batch's list, those of a small move's, and those of a task
+// that runs alone, with room for the events beyond the last clamp (two a unit) and for every ray point.
+enum { SEP_BATCH = 0, SEP_SMALL = 1, SEP_SOLE = 2 };
+__host__ __device__ inline int sep_kind(int nu, bool alone) { return alone ? SEP_SOLE : nu <= ESM_SEP_FULL ? SEP_SMALL : SEP_BATCH; }
+__host__ __device__ inline int sep_events(int nu, int maxpts, int kind) {
+    int e = ESM_SEP_EV * nu;
+    return (e < maxpts ? e : maxpts) + (kind == SEP_BATCH ? 1 : 2 * nu);
+}
+__host__ __device__ inline int sep_entries(int nu, int maxpts, int kind) {
+    int more = kind == SEP_BATCH ? 0 : 2 * nu + (kind == SEP_SMALL ? 8 : 84);
+    return (sep_events(nu, maxpts, kind) + more + 1) & ~1;
+}
+// The longest list that is sorted in registers; a longer one takes a buffer in global memory.
+template <class real>
+__host__ __device__ constexpr int sep_regs() {
+    return sizeof(real) == 4 ? 256 : 128;
+}
+// Shared memory of one list (SepList).
+template <class real>
+__host__ __device__ inline int sep_list_bytes(int nu, int maxpts, int kind) {
+    int n = sep_entries(nu, maxpts, kind);
+    return (((int)sizeof(real) * ((kind == SEP_BATCH ? 3 : 4) * n + nu) + (int)sizeof(real) / 2 * n) + 15) & ~15;
+}
+// shared memory of the move's units
+template <class real>
+__host__ __device__ inline int sep_unit_bytes(int nu) {
+    return ((2 * (int)sizeof(int) + 7 * (int)sizeof(real)) * nu + 15) & ~15;
+}
+
+template <class real>
+struct SepUnits {  // the move's storage units (shared memory)
+    int *j, *n;
+    real *a, *k, *h, *qt, *ein, *eout, *mc;
+    __device__ SepUnits(char *p, int nu) {
+        a = (real *)p;
+        k = a + nu;
+        h = k + nu;
+        qt = h + nu;
+        ein = qt + nu;
+        eout = ein + nu;
+        mc = eout + nu;
+        j = (int *)(mc + nu);
+        n = j + nu;
+    }
 };
 
-struct SepLayout {
-    int nu, maxpts, ev, wb;  // unit capacity, point cap per direction, event slots, sort capacity (power of 2)
-    int o_us, o_skey, o_wkey, o_wpay, o_wdsl, o_wdab, o_wcl, o_ucnt, o_pts, o_lm, total;  // byte offsets, bytes
+// One direction of one task (shared memory). An event comes with its key (sgn * t), its slot and the
+// unit's slopes before and after it (x, y of its pair). In order, an entry of a batch's list has the key,
+// negative for a clamp, and the change of the summed slope in double over x and y; the scan leaves the
+// potential in x, the segment masses go to y. The other lists keep the pairs by slot; the scan leaves the
+// potential and its round-off scale in x and y, the masses have an array.
+template <class real>
+struct SepPair {
+    real x, y;
+};
+// a slot with the event's clamp flag (bit 15); in the FP64 build, whose sums have other last bits in
+// another order, also the unit (bits 16 ..), by which events of one time are ordered
+template <class real>
+struct SepSlot {
+    using type = unsigned short;
+};
+template <>
+struct SepSlot<double> {
+    using type = unsigned int;
+};
+template <class real>
+struct SepList {
+    using slot_t = typename SepSlot<real>::type;
+    SepPair<real> *pair;
+    real *key, *sl, *m;
+    slot_t *slot;
+    __device__ __forceinline__ SepList(char *p, int n, int nu, bool full) {
+        pair = (SepPair<real> *)p;
+        key = (real *)(pair + n);
+        sl = key + n;
+        m = sl + nu;
+        slot = (slot_t *)(full ? m + n : m);
+    }
+};
+template <class real>
+__device__ __forceinline__ void sep_put(SepPair<real> &p, double v) {
+    if constexpr (sizeof(real) == 4)
+        *(double *)&p = v;
+    else
+        p.x = v;
+}
+template <class real>
+__device__ __forceinline__ double sep_get(const SepPair<real> &p) {
+    if constexpr (sizeof(real) == 4)
+        return *(const double *)&p;
+    else
+        return p.x;
+}
+
+enum { SEP_OPEN = 2, SEP_PROPER = 1, SEP_IMPROPER = 0, SEP_GUARD = -1, SEP_ALONE = -2 };
+
+// One storage term of a unit (its step tau or its step tau - 1) at the start: d0, its piece, the
+// linear coefficients there and its parts.
+template <class real>
+struct SepTerm {
+    real d0, si, sr, sp, inj, run, pen;
+    int piece;
+};
+// A unit in the walk: its constants and its two terms.
+template <class real>
+struct SepUnit {
+    real a, k, h, ein, eout, qt, e0, s0w, s0a;
+    real A, P, X;  // cost per unit of running part, penalty part and box excess
+    SepTerm<real> w, t;
+
+    // soc_parts at d, whose charging part pc = d / ein the caller has
+    __device__ __forceinline__ void parts(real d, real pc, real *inj, real *run, real *pen) const {
+        real x = mul_rn(-d, eout), m = fmin(x, real(1)), y = sub_rn(x, real(1));
+        bool up = d >= 0;
+        real c = ein > 0 ? pc : real(0);
+        *inj = up ? c : -m;
+        *run = up ? c : m;
+        real pu = add_rn(c > 1 ? sub_rn(c, real(1)) : real(0), ein <= 0 ? d : real(0));
+        real pd = (qt <= 0 && y > 0) ? y : real(0);
+        *pen = up ? pu : pd;
+    }
+    __device__ __forceinline__ int piece(real d, real pc) const {
+        return d >= 0 ? ((ein > 0 && pc > 1) ? 1 : 0) : (mul_rn(-d, eout) >= 1 ? 3 : 2);
+    }
+    __device__ __forceinline__ void start(SepTerm<real> &T, real d0) const {
+        T.d0 = d0;
+        real pc = d0 / ein;
+        T.piece = piece(d0, pc);
+        real r = real(1) / ein;
+        T.si = T.piece == 0 ? (ein > 0 ? r : real(0)) : T.piece == 1 ? r : T.piece == 2 ? eout : real(0);
+        T.sr = T.piece <= 1 ? T.si : T.piece == 2 ? -eout : real(0);
+        T.sp = T.piece == 0 ? (ein <= 0 ? real(1) : real(0))
+               : T.piece == 1 ? T.si
+               : T.piece == 2 ? real(0)
+                              : (qt <= 0 ? -eout : real(0));
+        parts(d0, pc, &T.inj, &T.run, &T.pen);
+    }
+    // soc_diff of a term whose d0 changes by dd and whose box excess changes by dex; *dj the injection change
+    __device__ __forceinline__ real soc(const SepTerm<real> &T, real dd, real dex, real *dj) const {
+        real dn = add_rn(T.d0, dd);
+        real pc = dn / ein;
+        bool same = piece(dn, pc) == T.piece;
+        real inj, run, pen;
+        parts(dn, pc, &inj, &run, &pen);
+        real dinj = same ? mul_rn(T.si, dd) : sub_rn(inj, T.inj);
+        real drun = same ? mul_rn(T.sr, dd) : sub_rn(run, T.run);
+        real dpen = same ? mul_rn(T.sp, dd) : sub_rn(pen, T.pen);
+        *dj = mul_rn(k, dinj);
+        return fma_rn(X, dex, fma_rn(A, drun, mul_rn(P, dpen)));
+    }
+    // the unit of slot q from its table and state
+    __device__ __forceinline__ void load(const DevModel<real> &M, const SepUnits<real> &U, int q, real e0_, real e1c,
+                                         real emc) {
+        a = U.a[q];
+        k = U.k[q];
+        h = U.h[q];
+        qt = U.qt[q];
+        ein = U.ein[q];
+        eout = U.eout[q];
+        e0 = e0_;
+        real wt = add_rn(k, M.kappa0), dt = M.dt, cv = M.c_viol;
+        A = mul_rn(mul_rn(dt, U.mc[q]), k);
+        P = mul_rn(mul_rn(cv, dt), wt);
+        X = mul_rn(mul_rn(cv, wt), h);
+        real ec = clampr<real>(e0, 0, 1);
+        start(w, sub_rn(mul_rn(h, sub_rn(e1c, ec)) / dt, qt));
+        start(t, sub_rn(mul_rn(h, sub_rn(ec, emc)) / dt, qt));
+    }
+    // the cost and injection changes of step tau and step tau - 1 when the state of charge moves by x
+    __device__ __forceinline__ void move(const DevModel<real> &M, real x, real *cw, real *ca, real *djw,
+                                         real *dja) const {
+        // clamp_diff
+        real y1 = add_rn(e0, x);
+        real c0 = clampr<real>(e0, 0, 1), c1 = clampr<real>(y1, 0, 1);
+        bool in = e0 > 0 && e0 < 1 && y1 > 0 && y1 < 1, above = e0 >= 1 && y1 >= 1, below = e0 <= 0 && y1 <= 0;
+        real dc = in ? x : (above || below) ? real(0) : sub_rn(c1, c0);
+        real dex = in ? real(0) : above ? x : below ? -x : sub_rn(fabs(sub_rn(y1, c1)), fabs(sub_rn(e0, c0)));
+        real dd = mul_rn(h, dc) / M.dt;
+        *cw = soc(w, -dd, dex, djw);
+        *ca = soc(t, dd, real(0), dja);
+    }
+    __device__ __forceinline__ static real phi(real S0, real dS, real cs, real cd) {  // phibal_diff
+        real S1 = add_rn(S0, dS);
+        real lin = S0 > 0 ? mul_rn(cs, dS) : mul_rn(-cd, dS);
+        real far = fma_rn(S1 > 0 ? cs : -cd, S1, -mul_rn(S0 > 0 ? cs : -cd, S0));
+        return (S0 > 0 && S1 > 0) || (S0 < 0 && S1 < 0) ? lin : far;
+    }
+    // beta * (cost change) at t, with the two node balances (Lane::unit_val)
+    __device__ __forceinline__ real val(const DevModel<real> &M, real tt, real *Sw, real *Sa) const {
+        real cw, ca, djw, dja;
+        move(M, mul_rn(tt, a), &cw, &ca, &djw, &dja);
+        *Sw = add_rn(s0w, djw);
+        *Sa = add_rn(s0a, dja);
+        real pw = phi(s0w, djw, M.c_shed, M.c_dump), pa = phi(s0a, dja, M.c_shed, M.c_dump);
+        return mul_rn(M.beta_v, fma_rn(M.dt, pa, add_rn(fma_rn(M.dt, pw, cw), ca)));
+    }
 };
 
 template <class real>
-__host__ __device__ inline SepLayout sep_layout(int nu, int maxpts) {
-    SepLayout L;
-    L.nu = nu < 1 ? 1 : nu;
-    L.maxpts = maxpts;
-    L.ev = L.nu * ESM_SEP_EVMAX;
-    int wb = 2;
-    while (wb < L.ev) wb <<= 1;
-    L.wb = wb;
-    int o = 0;
-    auto take = [&](int bytes) {
-        o = (o + 15) & ~15;
-        int r = o;
-        o += bytes;
-        return r;
-    };
-    L.o_us = take((int)sizeof(real) * SF_N * L.nu);
-    L.o_skey = take((int)sizeof(real) * L.ev);
-    L.o_wkey = take((int)sizeof(real) * wb);
-    L.o_wpay = take((int)sizeof(int) * wb);
-    L.o_wdsl = take((int)sizeof(double) * L.ev);
-    L.o_wdab = take((int)sizeof(float) * L.ev);
-    L.o_wcl = take(L.ev);
-    L.o_ucnt = take((int)sizeof(int) * L.nu);
-    L.o_pts = take((int)sizeof(real) * 6 * maxpts);
-    L.o_lm = take((int)sizeof(real) * (2 * maxpts + 1));
-    L.total = (o + 127) & ~127;
-    return L;
+__device__ __forceinline__ bool sep_root(real a, real b, real lo, real hi, real sgn, real *x) {
+    if ((a < 0) != (b < 0) && a != b) {
+        real xx = lo + (hi - lo) * a / (a - b);
+        if (sgn * (xx - lo) > 0 && sgn * (hi - xx) > 0) {
+            *x = xx;
+            return true;
+        }
+    }
+    return false;
 }
 
+// The block's shared state of a batch.
 template <class real>
-__device__ inline real warp_min(real v) {
-    for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-template <class real>
-__device__ inline real warp_max(real v) {
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-template <class T>
-__device__ inline T warp_sum(T v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-template <class T>
-__device__ inline T warp_incl_sum(T v, int lane) {
-    for (int o = 1; o < 32; o <<= 1) {
-        T x = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += x;
-    }
-    return v;
-}
-__device__ inline double warp_incl_min(double v, int lane) {
-    for (int o = 1; o < 32; o <<= 1) {
-        double x = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v = fmin(v, x);
-    }
-    return v;
-}
+struct SepBlock {
+    real W[ESM_SEP_LISTS];       // window end (sgn * t; infinite: none)
+    int n[ESM_SEP_LISTS];        // events of the list
+    int before[ESM_SEP_LISTS];   // those before the window end
+    int ncl[ESM_SEP_LISTS];      // clamps ahead of the start
+    int st[ESM_SEP_LISTS];       // SEP_*
+    int np[ESM_SEP_LISTS];       // points
+    int ray[ESM_SEP_LISTS];      // first point of the ray phase, whose points follow the events
+    float ab[ESM_SEP_LISTS];     // the summed magnitudes of the units' slopes (an upper bound, FP32)
+    real t[ESM_SEP_LISTS / 2];   // the task's draw
+    int alone[ESM_SEP_LISTS / 2];
+    int nalone, batch;
+};
 
 template <class real>
 struct SepWalk {
     const DevModel<real> &M;
-    const Desc<real> &d;
-    const SepLayout &SL;
-    char *base;  // this warp's region (shared memory, or its slab of global memory)
-    int lane, nu;
-    int tau, taum, tau1, rep;
+    const SepUnits<real> &U;
+    SepBlock<real> &B;
+    char *lists;
+    int nu, maxe, maxent, lbytes;  // units, events and entries per list, bytes of a list
+    bool full, alone;              // the pairs by slot (not SEP_BATCH); SEP_SOLE
+    int lane;
 
-    __device__ SepWalk(const DevModel<real> &M_, const Desc<real> &d_, const SepLayout &SL_, char *base_, int lane_)
-        : M(M_), d(d_), SL(SL_), base(base_), lane(lane_) {
-        nu = d.hdr[1];
+    __device__ __forceinline__ SepList<real> list(int l) const {
+        return SepList<real>(lists + (size_t)l * lbytes, maxent, nu, full);
+    }
+    __device__ __forceinline__ size_t ix(int x, int t, int rep) const { return sidx(x, t, rep, M.T, M.R); }
+
+    // The window end of list l, of which this lane holds the units q0, q0 + qstep, ...: the nearest
+    // clamp beyond `after` (sgn * t), over the lanes of the list (those nl apart); and the count of
+    // the clamps ahead of the start.
+    __device__ __forceinline__ real next_clamp(int q0, int qstep, int nl, int tau, int rep, real sgn, real after,
+                                               int *ncl) const {
+        real best = real(INFINITY);
+        int cnt = 0;
+        for (int q = q0; q < nu; q += qstep) {
+            real a = U.a[q], e0 = M.e[ix(U.j[q], tau, rep)];
+            real c0 = (real(0) - e0) / a, c1 = (real(1) - e0) / a;
+            if (isfinite(c0) && sgn * c0 > 0) {
+                ++cnt;
+                if (sgn * c0 > after) best = fmin(best, sgn * c0);
+            }
+            if (isfinite(c1) && sgn * c1 > 0) {
+                ++cnt;
+                if (sgn * c1 > after) best = fmin(best, sgn * c1);
+            }
+        }
+        for (int o = nl; o < 32; o <<= 1) {
+            best = fmin(best, __shfl_xor_sync(0xffffffffu, best, o));
+            cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+        }
+        *ncl = cnt;
+        return best;
     }
 
-    __device__ inline real &U(int f, int q) const { return ((real *)(base + SL.o_us))[f * SL.nu + q]; }
-    __device__ inline size_t ix(int x, int t) const { return sidx(x, t, rep, M.T, M.R); }
+    // The events of a warp's nl lists (a power of two; this lane's list is l, its units q0, q0 +
+    // qstep, ...) up to the window end Wk, appended to the lists in lane order, and every unit's
+    // slope at the start; *before the events before the window end. Each round takes one unit per lane through its pieces (unit_piece and
+    // unit_next of the one-lane walk): an iteration has one evaluation and gives at most one event,
+    // the previous one, whose outgoing slope the evaluation tells. Returns the list's event count.
+    __device__ __forceinline__ int events(int l, bool on, int q0, int qstep, int nl, int tau, int taum, int tau1,
+                                          int rep, real sgn, real Wk, int *before) const {
+        // what a lane evaluates next: the end of the piece at t, a node-balance root inside it, its
+        // end again (known), the slope beyond the last root; or it hands out its last event; or nothing
+        enum { PIECE, ROOT, END, TAIL, FLUSH, DONE };
+        const real INF = real(INFINITY);
+        SepList<real> A = list(l);
+        unsigned mine = 0;  // the lanes of this list
+        for (int i = lane & (nl - 1); i < 32; i += nl) mine |= 1u << i;
+        unsigned below = mine & ((1u << lane) - 1u);
+        int cnt = 0, last = 0;
+        int rounds = (nu + qstep - 1) / qstep;
+        for (int rd = 0; rd < rounds; ++rd) {
+            int q = q0 + rd * qstep;
+            int st = on && q < nu ? PIECE : DONE;
+            SepUnit<real> u{};
+            real ck[8];  // the unit's clamps (0, 1) and thresholds as sgn * t (infinite: none)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) ck[i] = INF;
+            if (st == PIECE) {
+                int j = U.j[q], n = U.n[q];
+                real e0 = M.e[ix(j, tau, rep)], e1 = M.e[ix(j, tau1, rep)], em = M.e[ix(j, taum, rep)];
+                u.s0w = M.r[ix(n, tau, rep)];
+                u.s0a = M.r[ix(n, taum, rep)];
+                real e1c = clampr<real>(e1, 0, 1), emc = clampr<real>(em, 0, 1);
+                u.load(M, U, q, e0, e1c, emc);
+                real h = u.h, qt = u.qt, dt = M.dt;
+                auto cand = [&](real x) -> real {
+                    real tc = x / u.a;
+                    return isfinite(tc) ? sgn * tc : INF;
+                };
+                ck[0] = cand(real(0) - e0);
+                ck[1] = cand(real(1) - e0);
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    real th = i == 0 ? real(0) : i == 1 ? u.ein : real(-1) / u.eout;
+                    if (i == 1 && !(u.ein > 0)) continue;
+                    if (i == 2 && !(u.eout > 0)) continue;
+                    real xw = e1c - e0 - (th + qt) * dt / h;
+                    if (e0 + xw >= 0 && e0 + xw <= 1) ck[2 + 2 * i] = cand(xw);
+                    real xa = emc - e0 + (th + qt) * dt / h;
+                    if (e0 + xa >= 0 && e0 + xa <= 1) ck[3 + 2 * i] = cand(xa);
+                }
+            }
+            real t = 0, f = 0, sw0 = u.s0w, sa0 = u.s0a;            // the position; the balances at its piece's start
+            real tE = 0, fE = 0, swE = 0, saE = 0, r0 = 0, r1 = 0;  // the piece's end and roots
+            int nr = 0;
+            bool have = false, prim = false, first = true;
+            bool pend = false, pcl = false;  // the event at the position, not yet handed out
+            real psl = 0;                    // the slope up to it
+            while (__any_sync(0xffffffffu, st != DONE)) {
+                bool emit = false, xcl = false, flush = st == FLUSH;
+                real xt = 0, xlo = 0, xhi = 0;
+                if (flush) {
+                    emit = true;
+                    xt = t;
+                    xlo = xhi = psl;
+                    xcl = pcl;
+                    st = DONE;
+                } else if (st != DONE) {
+                    real te;
+                    if (st == PIECE) {
+                        real tk = sgn * t, best = INF;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            if (ck[i] > tk) best = fmin(best, ck[i]);
+                        have = best < INF;
+                        prim = best == ck[0] || best == ck[1];
+                        tE = have ? sgn * best : t + sgn * fmax(real(1), fabs(t));
+                        te = tE;
+                    } else {
+                        te = st == ROOT ? r0 : st == END ? tE : t + sgn * fmax(real(1), fabs(t));
+                    }
+                    real v = fE, Sw = swE, Sa = saE;
+                    if (st != END) v = u.val(M, te, &Sw, &Sa);
+                    bool ev = true;     // an event at te (else only the slope to infinity)
+                    bool known = true;  // the slope up to te
+                    bool cl = false;
+                    if (st == PIECE) {
+                        fE = v;
+                        swE = Sw;
+                        saE = Sa;
+                        nr = 0;
+                        real x;
+                        bool hit;
+                        if (have) {
+                            hit = sep_root<real>(sw0, Sw, t, tE, sgn, &x);
+                        } else {  // linear to infinity: a crossing anywhere ahead
+                            x = t + (tE - t) * sw0 / (sw0 - Sw);
+                            hit = sw0 != Sw && isfinite(x) && sgn * (x - t) > 0;
+                        }
+                        if (hit) {
+                            r0 = x;
+                            nr = 1;
+                        }
+                        if (have) {
+                            hit = sep_root<real>(sa0, Sa, t, tE, sgn, &x);
+                        } else {
+                            x = t + (tE - t) * sa0 / (sa0 - Sa);
+                            hit = sa0 != Sa && isfinite(x) && sgn * (x - t) > 0;
+                        }
+                        if (hit) {
+                            r1 = x;
+                            if (nr == 0) {
+                                r0 = x;
+                            } else if (sgn * (r1 - r0) < 0) {
+                                r1 = r0;
+                                r0 = x;
+                            }
+                            ++nr;
+                        }
+                        if (nr > 0) {
+                            st = ROOT;
+                            known = false;
+                        } else if (have) {
+                            cl = prim;
+                            sw0 = Sw;
+                            sa0 = Sa;
+                        } else {
+                            ev = false;
+                        }
+                    } else if (st == ROOT) {
+                        r0 = r1;
+                        --nr;
+                        st = nr > 0 ? ROOT : have ? END : TAIL;
+                    } else if (st == END) {
+                        cl = prim;
+                        sw0 = swE;
+                        sa0 = saE;
+                        st = PIECE;
+                    } else {
+                        ev = false;
+                    }
+                    if (known) {
+                        real sl = te != t ? (v - f) / (te - t) : real(0);
+                        if (first) A.sl[q] = sl;
+                        first = false;
+                        emit = pend;
+                        xt = t;
+                        xlo = psl;
+                        xhi = sl;
+                        xcl = pcl;
+                        t = te;
+                        f = v;
+                        psl = sl;
+                        pcl = cl;
+                        pend = ev && sgn * te <= Wk;
+                        if (!pend) st = DONE;
+                        else if (sgn * te == Wk) st = FLUSH;
+                    }
+                }
+                unsigned em = __ballot_sync(0xffffffffu, emit);
+                if (em == 0) continue;
+                if (emit) {
+                    int p = cnt + __popc(em & below);
+                    if (p < maxe) {
+                        A.key[p] = sgn * xt;
+                        A.pair[p] = SepPair<real>{xlo, xhi};
+                        A.slot[p] = (typename SepList<real>::slot_t)(((unsigned)q << 16) | p | (xcl ? 0x8000 : 0));
+                    }
+                }
+                cnt += __popc(em & mine);
+                if (flush) ++last;
+            }
+        }
+        for (int o = nl; o < 32; o <<= 1) last += __shfl_xor_sync(0xffffffffu, last, o);
+        *before = cnt - last;
+        return cnt;
+    }
 
-    // the task's unit values (state of charge at three steps, node balances at two)
-    __device__ void load_units() const {
-        for (int q = lane; q < nu; q += 32) {
-            int j = d.si[q];
-            U(SF_E0, q) = M.e[ix(j, tau)];
-            U(SF_E1, q) = M.e[ix(j, tau1)];
-            U(SF_EM, q) = M.e[ix(j, taum)];
-            U(SF_S0W, q) = M.r[ix(d.nds[d.spos[q]], tau)];
-            U(SF_S0A, q) = M.r[ix(d.nda[d.sposa[q]], taum)];
+    // The entries of a list in order, the pairs of a batch's list with them.
+    __device__ __forceinline__ static real signed_key(real k, unsigned p) { return (p & 0x8000u) ? -k : k; }
+    __device__ __forceinline__ static double slope_change(const SepPair<real> &p) {
+        return sep_widen(p.y) - sep_widen(p.x);
+    }
+    // The first n <= 32 E entries of a list in order, by the warp, E consecutive entries a lane in
+    // registers: a bitonic network whose comparisons all point upward (each merge starts with mirrored
+    // pairs); strides below E stay in the lane.
+    // (FP32 entries of one time keep the order that the network gives them, the same in every run.)
+    __device__ __forceinline__ static bool after(real ka, unsigned pa, real kb, unsigned pb) {
+        if constexpr (sizeof(real) == 8) return ka > kb || (ka == kb && pa > pb);
+        return ka > kb;
+    }
+    template <int E>
+    __device__ __forceinline__ void sort_regs(const SepList<real> &A, int n) const {
+        real k[E];
+        unsigned p[E];
+#pragma unroll
+        for (int r = 0; r < E; ++r) {
+            int i = lane * E + r;
+            k[r] = i < n ? A.key[i] : real(INFINITY);
+            p[r] = i < n ? A.slot[i] : 0xffffffffu;
+        }
+#pragma unroll
+        for (int lk = 1; (1 << lk) <= 32 * E; ++lk) {
+#pragma unroll
+            for (int lj = lk - 1; lj >= 0; --lj) {
+                const int kk = 1 << lk, j = 1 << lj;
+                const bool mirror = lj == lk - 1;
+                if (j < E) {
+#pragma unroll
+                    for (int r = 0; r < E; ++r) {
+                        const int o = mirror ? r ^ ((kk - 1) & (E - 1)) : r ^ j;
+                        if (o > r) {
+                            bool sw = after(k[r], p[r], k[o], p[o]);
+                            real a = sw ? k[o] : k[r], b = sw ? k[r] : k[o];
+                            unsigned pa = sw ? p[o] : p[r], pb = sw ? p[r] : p[o];
+                            k[r] = a;
+                            k[o] = b;
+                            p[r] = pa;
+                            p[o] = pb;
+                        }
+                    }
+                } else {
+                    const int x = mirror ? (kk - 1) / E : j / E;
+                    bool low = (lane & (j / E)) == 0;
+                    real ok[E];
+                    unsigned op[E];
+#pragma unroll
+                    for (int r = 0; r < E; ++r) {
+                        ok[r] = __shfl_xor_sync(0xffffffffu, k[mirror ? E - 1 - r : r], x);
+                        op[r] = __shfl_xor_sync(0xffffffffu, p[mirror ? E - 1 - r : r], x);
+                    }
+#pragma unroll
+                    for (int r = 0; r < E; ++r) {
+                        if constexpr (sizeof(real) == 8) {
+                            bool sw = low ? after(k[r], p[r], ok[r], op[r]) : after(ok[r], op[r], k[r], p[r]);
+                            k[r] = sw ? ok[r] : k[r];
+                            p[r] = sw ? op[r] : p[r];
+                        } else {
+                            real nk = low ? fmin(k[r], ok[r]) : fmax(k[r], ok[r]);
+                            p[r] = nk == k[r] ? p[r] : op[r];  // (equal keys: each lane keeps its own)
+                            k[r] = nk;
+                        }
+                    }
+                }
+            }
+        }
+        double ds[E];
+        if (!full)
+#pragma unroll
+            for (int r = 0; r < E; ++r)
+                if (lane * E + r < n) ds[r] = slope_change(A.pair[p[r] & 0x7fffu]);
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < E; ++r) {
+            int i = lane * E + r;
+            if (i < n) {
+                A.key[i] = full ? k[r] : signed_key(k[r], p[r]);
+                A.slot[i] = (typename SepList<real>::slot_t)p[r];
+                if (!full) sep_put<real>(A.pair[i], ds[r]);
+            }
         }
         __syncwarp();
     }
-
-    // beta * (cost change) of unit q at t, with its two node balances (the per-lane walk's unit_val
-    // on the cached values: the same arithmetic, so the same events)
-    __device__ __noinline__ real unit_val(int q, real t, real *Sw, real *Sa) const {
-        int j = d.si[q];
-        real x = t * d.sa[q];
-        real k = M.kc_s[j], w = k + M.kappa0, dt = M.dt, cv = M.c_viol;
-        real djw, dw, dja, da;
-        real cw = soc_diff<real>(M.s_hours[j], M.s_qt[j], M.s_etain[j], M.s_etaout[j], M.s_mc[j], k, w, dt, cv,
-                                 U(SF_E0, q), U(SF_E1, q), x, real(0), &djw, &dw);
-        real ca = soc_diff<real>(M.s_hours[j], M.s_qt[j], M.s_etain[j], M.s_etaout[j], M.s_mc[j], k, w, dt, cv,
-                                 U(SF_EM, q), U(SF_E0, q), real(0), x, &dja, &da);
-        real S0w = U(SF_S0W, q), S0a = U(SF_S0A, q);
-        *Sw = S0w + djw;
-        *Sa = S0a + dja;
-        real bw = dt * phibal_diff<real>(S0w, djw, M.c_shed, M.c_dump);
-        real ba = dt * phibal_diff<real>(S0a, dja, M.c_shed, M.c_dump);
-        return M.beta_v * (cw + bw + ca + ba);
-    }
-
-    __device__ inline static bool root_of(real a, real b, real lo, real hi, real sgn, real *x) {
-        if ((a < 0) != (b < 0) && a != b) {
-            real xx = lo + (hi - lo) * a / (a - b);
-            if (sgn * (xx - lo) > 0 && sgn * (hi - xx) > 0) {
-                *x = xx;
-                return true;
-            }
-        }
-        return false;
-    }
-
-    // the piece of unit q starting at t0 (node balances Sw0, Sa0 there): its end and the node-balance
-    // roots inside it, as the per-lane walk's unit_piece
-    __device__ __noinline__ void unit_piece(int q, real t0, real sgn, real Sw0, real Sa0) const {
-        int j = d.si[q];
-        real a = d.sa[q];
-        real e0 = U(SF_E0, q);
-        real e1c = clampr<real>(U(SF_E1, q), 0, 1), emc = clampr<real>(U(SF_EM, q), 0, 1);
-        real h = M.s_hours[j], qt = M.s_qt[j], ein = M.s_etain[j], eout = M.s_etaout[j], dt = M.dt;
-        bool have = false, prim = false;
-        real ts = 0;
-        auto cand = [&](real x, bool p) {
-            real tc = x / a;
-            if (!isfinite(tc) || !(sgn * (tc - t0) > 0)) return;
-            if (!have || sgn * (tc - ts) < 0) {
-                ts = tc;
-                prim = p;
-                have = true;
-            }
-        };
-        cand(real(0) - e0, true);
-        cand(real(1) - e0, true);
-        real th[3];
-        int nth = 0;
-        th[nth++] = 0;
-        if (ein > 0) th[nth++] = ein;
-        if (eout > 0) th[nth++] = real(-1) / eout;
-        for (int i = 0; i < nth; ++i) {
-            real xw = e1c - e0 - (th[i] + qt) * dt / h;
-            if (e0 + xw >= 0 && e0 + xw <= 1) cand(xw, false);
-            real xa = emc - e0 + (th[i] + qt) * dt / h;
-            if (e0 + xa >= 0 && e0 + xa <= 1) cand(xa, false);
-        }
-        real tpb = have ? ts : t0 + sgn * fmax(real(1), fabs(t0));
-        real Sw1, Sa1;
-        U(SF_UFE, q) = unit_val(q, tpb, &Sw1, &Sa1);
-        U(SF_USW, q) = Sw1;
-        U(SF_USA, q) = Sa1;
-        real r[2];
-        int nr = 0;
-        real pa[2] = {Sw0, Sa0}, pb[2] = {Sw1, Sa1};
-        for (int i = 0; i < 2; ++i) {
-            real x;
-            if (have) {
-                if (root_of(pa[i], pb[i], t0, tpb, sgn, &x)) r[nr++] = x;
-            } else if (pa[i] != pb[i]) {
-                x = t0 + (tpb - t0) * pa[i] / (pa[i] - pb[i]);
-                if (isfinite(x) && sgn * (x - t0) > 0) r[nr++] = x;
-            }
-        }
-        if (nr == 2 && sgn * (r[1] - r[0]) < 0) {
-            real x = r[0];
-            r[0] = r[1];
-            r[1] = x;
-        }
-        int n = 0;
-        for (int i = 0; i < nr; ++i) U(SF_UE + n++, q) = r[i];
-        if (have) U(SF_UE + n++, q) = ts;
-        U(SF_UN, q) = real(n);
-        U(SF_UH, q) = have ? (prim ? real(1) : real(2)) : real(0);
-        U(SF_UI, q) = real(0);
-    }
-
-    // the next event of unit q after its position t (potential f there), as the per-lane unit_next
-    __device__ __noinline__ void unit_next(int q, real t, real f, real sgn) const {
-        int i = (int)U(SF_UI, q), n = (int)U(SF_UN, q), hk = (int)U(SF_UH, q);
-        real Sw, Sa, tn, fn;
-        if (i < n) {
-            tn = U(SF_UE + i, q);
-            bool end = i == n - 1 && hk != 0;
-            fn = end ? U(SF_UFE, q) : unit_val(q, tn, &Sw, &Sa);
-            U(SF_UT, q) = tn;
-            U(SF_UK, q) = end ? (hk == 1 ? real(1) : real(0)) : real(0);
-            U(SF_UFN, q) = fn;
-            U(SF_USL, q) = tn != t ? (fn - f) / (tn - t) : real(0);
-        } else {
-            real tp = t + sgn * fmax(real(1), fabs(t));
-            fn = unit_val(q, tp, &Sw, &Sa);
-            U(SF_UT, q) = real(INFINITY) * sgn;
-            U(SF_UK, q) = real(-1);
-            U(SF_USL, q) = (fn - f) / (tp - t);
-        }
-    }
-
-    __device__ void unit_pass(int q, real t, real sgn) const {
-        int i = (int)U(SF_UI, q), n = (int)U(SF_UN, q), hk = (int)U(SF_UH, q);
-        real f = U(SF_UFN, q);
-        if (i == n - 1 && hk != 0)
-            unit_piece(q, t, sgn, U(SF_USW, q), U(SF_USA, q));
-        else
-            U(SF_UI, q) = real(i + 1);
-        unit_next(q, t, f, sgn);
-    }
-
-    // sort n (key, payload) pairs ascending by key, then payload (bitonic, padded to a power of 2)
-    __device__ void sort_window(real *key, int *pay, int n) const {
-        int n2 = 2;
+    // the same in shared memory, for lists of any length; tmp: n doubles
+    __device__ __noinline__ void sort_mem(const SepList<real> &A, int n, double *tmp) const {
+        int n2 = 32;
         while (n2 < n) n2 <<= 1;
-        for (int i = n + lane; i < n2; i += 32) {
-            key[i] = real(INFINITY);
-            pay[i] = 0x7fffffff;
-        }
-        __syncwarp();
-        for (int k = 2; k <= n2; k <<= 1)
+        for (int k = 2; k <= n2; k <<= 1) {
             for (int j = k >> 1; j > 0; j >>= 1) {
+                bool mirror = j == (k >> 1);
                 for (int i = lane; i < (n2 >> 1); i += 32) {
                     int lo = ((i & ~(j - 1)) << 1) | (i & (j - 1));
-                    int hi = lo + j;
-                    real ka = key[lo], kb = key[hi];
-                    int pa = pay[lo], pb = pay[hi];
-                    bool up = (lo & k) == 0;
-                    bool gt = ka > kb || (ka == kb && pa > pb);
-                    if (gt == up) {
-                        key[lo] = kb;
-                        key[hi] = ka;
-                        pay[lo] = pb;
-                        pay[hi] = pa;
+                    int hi = mirror ? lo ^ (k - 1) : lo + j;
+                    if (hi < n) {
+                        real ka = A.key[lo], kb = A.key[hi];
+                        auto pa = A.slot[lo], pb = A.slot[hi];
+                        if (after(ka, pa, kb, pb)) {
+                            A.key[lo] = kb;
+                            A.key[hi] = ka;
+                            A.slot[lo] = pb;
+                            A.slot[hi] = pa;
+                        }
                     }
                 }
                 __syncwarp();
             }
+        }
+        if (full) return;
+        for (int i = lane; i < n; i += 32) {
+            unsigned p = A.slot[i];
+            tmp[i] = slope_change(A.pair[p & 0x7fffu]);
+            A.key[i] = signed_key(A.key[i], p);
+        }
+        __syncwarp();
+        for (int i = lane; i < n; i += 32) sep_put<real>(A.pair[i], tmp[i]);
+        __syncwarp();
+    }
+    __device__ __forceinline__ void sort(const SepList<real> &A, int n, double *tmp) const {
+        if (n <= 32)
+            sort_regs<1>(A, n);
+        else if (n <= 64)
+            sort_regs<2>(A, n);
+        else if (n <= 128)
+            sort_regs<4>(A, n);
+        else if (n <= sep_regs<real>())
+            sort_regs<sep_regs<real>() / 32>(A, n);
+        else
+            sort_mem(A, n, tmp);
+    }
+    // a short list, by one lane
+    __device__ __forceinline__ void sort_short(const SepList<real> &A, int n) const {
+        for (int i = 0; i < n; ++i) {
+            real k = A.key[i];
+            unsigned p = A.slot[i];
+            SepPair<real> v = A.pair[i];
+            if (!full) {
+                double ds = slope_change(v);
+                sep_put<real>(v, ds);
+                if (p & 0x8000u) k = -k;
+            }
+            int j = i - 1;
+            for (; j >= 0 && after(fabs(A.key[j]), A.slot[j], fabs(k), p); --j) {
+                A.key[j + 1] = A.key[j];
+                A.slot[j + 1] = A.slot[j];
+                if (!full) A.pair[j + 1] = A.pair[j];
+            }
+            A.key[j + 1] = k;
+            A.slot[j + 1] = (typename SepList<real>::slot_t)p;
+            if (!full) A.pair[j + 1] = v;
+        }
     }
 
-    // One direction of walk! (src/local.jl:1294) for the separable move. Returns 1 proper, 0 improper
-    // (ray steps exhausted), -1 when the points exceed the cap or a unit its event slots (a guard
-    // event). The points, their potentials and (FP32) round-off scales go to P, C, Z; *np their count.
-    __device__ __noinline__ int walk(real sgn, real *P, real *C, real *Z, int *np) const {
-        real *skey = (real *)(base + SL.o_skey);
-        real *wkey = (real *)(base + SL.o_wkey);
-        int *wpay = (int *)(base + SL.o_wpay);
-        double *wdsl = (double *)(base + SL.o_wdsl);
-        float *wdab = (float *)(base + SL.o_wdab);
-        unsigned char *wcl = (unsigned char *)(base + SL.o_wcl);
-        int *ucnt = (int *)(base + SL.o_ucnt);
+    // One direction of walk! over list l of a batch, whose window ends at a clamp: the potential at
+    // every event and the stop test at the clamps. Sets the list's state: SEP_OPEN when the window
+    // does not end it.
+    __device__ __forceinline__ void scan(int l, real sgn) const {
+        SepList<real> A = list(l);
+        int n = B.n[l], ncl = B.ncl[l];
+        if (n > maxe) {  // more events before the window end than points; else many at the end itself
+            B.st[l] = B.before[l] >= M.maxpts ? SEP_GUARD : SEP_ALONE;
+            return;
+        }
+        if (n <= ESM_SEP_SHORT) sort_short(A, n);
+        double b = 0, c = 0, cmin = 0;
+        float abf = 0;
+        real kcur = 0, fmn = 0;
+        for (int q = 0; q < nu; ++q) {
+            real x = A.sl[q];
+            b += sep_widen(x);
+            abf += fabsf((float)x);
+        }
+        const double maxnats = (double)M.maxnats;
+        const int last = n < M.maxpts ? n : M.maxpts;
+        int i = 0, st = SEP_OPEN;
+        real k = A.key[0];
+        double ds = sep_get<real>(A.pair[0]);
+        for (; i < last; ++i) {
+            real k0 = k;
+            double d0 = ds;
+            if (i + 1 < n) {  // (the next entry while this one's sums are formed)
+                k = A.key[i + 1];
+                ds = sep_get<real>(A.pair[i + 1]);
+            }
+            real ka = fabs(k0);
+            c += b * sep_widen(sgn * (ka - kcur));
+            kcur = ka;
+            real cf = sep_narrow(c, real(0));
+            A.pair[i].x = cf;
+            if (cf < fmn || (cf == fmn && c < cmin)) {  // (the rounding keeps the order)
+                fmn = cf;
+                cmin = c;
+            }
+            b += d0;
+            abf += sep_above(d0);
+            if (k0 < 0) {
+                --ncl;
+                if (c - cmin > maxnats) {
+                    st = SEP_PROPER;
+                    break;
+                }
+            }
+        }
+        if (st == SEP_OPEN && i < n) st = SEP_GUARD;  // more points than the cap
+        B.np[l] = i + 1;
+        B.ab[l] = abf;
+        B.st[l] = st;
+    }
+
+    // The same for any window, with the ray steps after the last clamp and the round-off scale of every
+    // point. SEP_ALONE when the list has not the room.
+    __device__ __forceinline__ void scan_full(int l, real sgn) const {
         const real INF = real(INFINITY);
-        const int maxpts = SL.maxpts;
-        double Bl = 0, Al = 0;
-        int ncll = 0;
-        for (int q = lane; q < nu; q += 32) {
-            real a = d.sa[q], e0 = U(SF_E0, q);
-            real c0 = (real(0) - e0) / a, c1 = (real(1) - e0) / a;
-            bool h0 = isfinite(c0) && sgn * c0 > 0, h1 = isfinite(c1) && sgn * c1 > 0;
-            real f0 = h0 ? c0 : c1, f1 = c1;
-            if (h0 && h1 && sgn * (c1 - c0) < 0) {
-                f0 = c1;
-                f1 = c0;
-            }
-            U(SF_CL0, q) = (h0 || h1) ? f0 : INF * sgn;
-            U(SF_CL1, q) = (h0 && h1) ? f1 : INF * sgn;
-            U(SF_NCL, q) = real((int)h0 + (int)h1);
-            ncll += (int)h0 + (int)h1;
-            unit_piece(q, real(0), sgn, U(SF_S0W, q), U(SF_S0A, q));
-            unit_next(q, real(0), real(0), sgn);
-            Bl += (double)U(SF_USL, q);
-            Al += fabs((double)U(SF_USL, q));
+        SepList<real> A = list(l);
+        int n = B.n[l], ncl = B.ncl[l];
+        bool inf = !(B.W[l] < INF);
+        if (n > maxe) {
+            B.st[l] = B.before[l] >= M.maxpts || alone ? SEP_GUARD : SEP_ALONE;
+            return;
         }
-        double B = warp_sum(Bl), absB = warp_sum(Al);
-        int ncl = warp_sum(ncll);
-        int npts = 0;
-        double c = 0, cmin = 0;
+        if (n <= ESM_SEP_SHORT) sort_short(A, n);
+        double b = 0, ab = 0, c = 0, cmin = 0;
+        for (int q = 0; q < nu; ++q) {
+            double x = sep_widen(A.sl[q]);
+            b += x;
+            ab += fabs(x);
+        }
+        const double maxnats = (double)M.maxnats;
+        const int maxpts = M.maxpts;
         real tcur = 0;
-        bool over = false;
-        while (ncl > 0) {
-            // the window ends at the nearest clamp ahead
-            real wl = INF;
-            for (int q = lane; q < nu; q += 32)
-                if (U(SF_NCL, q) > 0) wl = fmin(wl, sgn * U(SF_CL0, q));
-            wl = warp_min(wl);
-            if (!(wl < INF)) break;  // (no clamp left where the count expects one: ray steps)
-            real W = sgn * wl;
-            int ncw = 0;
-            for (int q = lane; q < nu; q += 32) {
-                int cq = 0;
-                while (true) {
-                    real tq = U(SF_UT, q);
-                    if (!isfinite(tq) || !(sgn * tq <= sgn * W)) break;
-                    if (cq >= ESM_SEP_EVMAX) {
-                        over = true;
-                        break;
-                    }
-                    bool clamp = U(SF_UK, q) == real(1);
-                    real old = U(SF_USL, q);
-                    unit_pass(q, tq, sgn);
-                    real nw = U(SF_USL, q);
-                    int slot = q * ESM_SEP_EVMAX + cq;
-                    skey[slot] = sgn * tq;
-                    wdsl[slot] = (double)nw - (double)old;
-                    wdab[slot] = (float)fmax(0.0, fabs((double)nw) - fabs((double)old));
-                    wcl[slot] = clamp ? 1 : 0;
-                    if (clamp) {
-                        ++ncw;
-                        U(SF_CL0, q) = U(SF_CL1, q);
-                        U(SF_CL1, q) = INF * sgn;
-                        U(SF_NCL, q) -= real(1);
-                    }
-                    ++cq;
-                }
-                ucnt[q] = cq;
-            }
-            if (__any_sync(0xffffffffu, over)) return -1;
-            __syncwarp();
-            // compaction in unit order
-            int n = 0;
-            for (int q0 = 0; q0 < nu; q0 += 32) {
-                int q = q0 + lane;
-                int cq = q < nu ? ucnt[q] : 0;
-                int incl = warp_incl_sum(cq, lane);
-                int pos = n + incl - cq;
-                for (int s = 0; s < cq; ++s) {
-                    wkey[pos + s] = skey[q * ESM_SEP_EVMAX + s];
-                    wpay[pos + s] = q * ESM_SEP_EVMAX + s;
-                }
-                n += __shfl_sync(0xffffffffu, incl, 31);
-            }
-            __syncwarp();
-            sort_window(wkey, wpay, n);
-            ncl -= warp_sum(ncw);
-            // the potential along the window's events
-            int npw = npts;
-            for (int b0 = 0; b0 < n; b0 += 32) {
-                int i = b0 + lane;
-                bool v = i < n;
-                real ti = v ? sgn * wkey[i] : tcur;
-                real tp = i == 0 ? tcur : sgn * wkey[(v ? i : n) - 1];
-                int slot = v ? wpay[i] : 0;
-                double ds = v ? wdsl[slot] : 0.0;
-                double da = v ? (double)wdab[slot] : 0.0;
-                bool cl = v && wcl[slot];
-                double dsi = warp_incl_sum(ds, lane);
-                double Bx = B + (dsi - ds);  // the summed slope before the event
-                double inc = v ? Bx * (double)(ti - tp) : 0.0;
-                double ci = c + warp_incl_sum(inc, lane);
-                double cmi = fmin(cmin, warp_incl_min(v ? ci : 1e300, lane));
-                double dai = warp_incl_sum(da, lane);
-                double Ax = absB + (dai - da);
-                bool stop = cl && (ci - cmi > (double)M.maxnats);
-                unsigned sb = __ballot_sync(0xffffffffu, stop);
-                int last = sb ? __ffs(sb) - 1 : 31;
-                bool gd = false;
-                if (v && lane <= last) {
-                    int k = npw + i;
-                    if (k >= maxpts) {
-                        gd = true;
-                    } else {
-                        P[k] = ti;
-                        C[k] = (real)ci;
-                        if constexpr (sizeof(real) == 4) Z[k] = real(4.8e-7) * (real)(fabs(ci) + Ax * fabs((double)ti));
-                    }
-                }
-                if (__any_sync(0xffffffffu, gd)) return -1;
-                int lv = min(last, n - 1 - b0);
-                B = __shfl_sync(0xffffffffu, Bx + ds, lv);
-                c = __shfl_sync(0xffffffffu, ci, lv);
-                cmin = __shfl_sync(0xffffffffu, cmi, lv);
-                absB = __shfl_sync(0xffffffffu, Ax + da, lv);
-                tcur = __shfl_sync(0xffffffffu, ti, lv);
-                if (sb) {
-                    __syncwarp();
-                    *np = npw + b0 + lv + 1;
-                    return 1;
-                }
-            }
-            npts = npw + n;
-            __syncwarp();
-        }
-        // ray steps once every clamp is behind (every unit then sits outside its box, so no events
-        // are expected; any left are taken in order)
-        real delta = 0;
-        int nx = 0;
+        int i = 0, np = 0, ray = 0x7fffffff, st = SEP_OPEN;
+        auto advance = [&](real t) {
+            c += b * sep_widen((real)(t - tcur));
+            tcur = t;
+        };
+        auto pass = [&](const SepPair<real> &v) {  // an event's slopes
+            b += slope_change(v);
+            ab = fmax(ab, ab + fabs(sep_widen(v.y)) - fabs(sep_widen(v.x)));
+        };
         auto point = [&](real t) -> bool {
-            if (npts >= maxpts) return false;
-            if (lane == 0) {
-                P[npts] = t;
-                C[npts] = (real)c;
-                if constexpr (sizeof(real) == 4) Z[npts] = real(4.8e-7) * (real)(fabs(c) + absB * fabs((double)t));
+            int e = np < ray ? np : n + np - ray;
+            if (np >= maxpts || e >= maxent) {
+                st = np >= maxpts || alone ? SEP_GUARD : SEP_ALONE;
+                return false;
             }
-            ++npts;
+            if (e >= n) {
+                A.key[e] = sgn * t;
+                A.slot[e] = (typename SepList<real>::slot_t)e;
+            }
+            SepPair<real> v;
+            v.x = sep_narrow(c, real(0));
+            v.y = 0;
+            if constexpr (sizeof(real) == 4)
+                v.y = real(4.8e-7) * sep_narrow(fabs(c) + ab * fabs(sep_widen(t)), real(0));
+            A.pair[A.slot[e] & 0x7fffu] = v;
             cmin = fmin(cmin, c);
+            ++np;
             return true;
         };
-        // the unit with the nearest pending event: (time, owner lane, unit) -- warp-uniform
-        auto nearest = [&](real *tS, int *qS) {
-            real best = INF;
-            int bq = 0x7fffffff;
-            for (int q = lane; q < nu; q += 32) {
-                real tq = U(SF_UT, q);
-                if (isfinite(tq) && (sgn * tq < best || (sgn * tq == best && q < bq))) {
-                    best = sgn * tq;
-                    bq = q;
+        while (st == SEP_OPEN && ncl > 0 && i < n) {
+            unsigned p = A.slot[i];
+            SepPair<real> v = A.pair[p & 0x7fffu];
+            advance(sgn * A.key[i]);
+            if (!point(tcur)) break;
+            pass(v);
+            if (p & 0x8000u) {
+                --ncl;
+                if (c - cmin > maxnats) st = SEP_PROPER;
+            }
+            ++i;
+        }
+        if (st == SEP_OPEN && inf) {  // (no event left before the clamps the count expects: as behind them)
+            ray = np;
+            real delta = 0;
+            int nx = 0;
+            while (st == SEP_OPEN) {
+                double sl = (double)sgn * b;
+                if (sl > 0)
+                    delta = fmin(real(2) * M.maxnats / (real)sl, real(1e3) * fmax(fabs(tcur), real(1e-3)));
+                else
+                    delta = delta == 0 ? fmax(fabs(tcur), real(1e-6)) : real(2) * delta;
+                real target = tcur + sgn * delta;
+                if (++nx > 80) {
+                    st = SEP_IMPROPER;
+                    break;
                 }
-            }
-            for (int o = 16; o > 0; o >>= 1) {
-                real ob = __shfl_xor_sync(0xffffffffu, best, o);
-                int oq = __shfl_xor_sync(0xffffffffu, bq, o);
-                if (ob < best || (ob == best && oq < bq)) {
-                    best = ob;
-                    bq = oq;
+                bool ok = true;
+                while (ok && i < n) {  // the events before the target
+                    real t = sgn * A.key[i];
+                    if (!(sgn * (target - t) > 0)) break;
+                    SepPair<real> v = A.pair[A.slot[i] & 0x7fffu];
+                    advance(t);
+                    ok = point(t);
+                    if (ok) pass(v);
+                    ++i;
                 }
+                if (ok) {
+                    advance(target);
+                    ok = point(target);
+                }
+                if (!ok) break;
+                while (i < n && sgn * A.key[i] == target) pass(A.pair[A.slot[i++] & 0x7fffu]);
+                if (c - cmin > maxnats) st = SEP_PROPER;
             }
-            *tS = sgn * best;
-            *qS = bq;
-        };
-        auto pass = [&](int qS, real tS) {
-            double ds = 0, da = 0;
-            if ((qS & 31) == lane) {
-                real old = U(SF_USL, qS);
-                unit_pass(qS, tS, sgn);
-                real nw = U(SF_USL, qS);
-                ds = (double)nw - (double)old;
-                da = fmax(0.0, fabs((double)nw) - fabs((double)old));
+        }
+        B.np[l] = np;
+        B.ray[l] = ray;
+        B.st[l] = st;
+    }
+
+    // The points of a list, and the segments: segment k ends at point k and starts at point k - 1 (at
+    // 0 for k = 0).
+    struct Points {
+        SepList<real> A;
+        int ray, n;
+        bool full;
+        __device__ __forceinline__ int entry(int k) const { return k < ray ? k : n + k - ray; }
+        __device__ __forceinline__ real key(int k) const { return k < 0 ? real(0) : fabs(A.key[entry(k)]); }
+        __device__ __forceinline__ int at(int k) const { return full ? A.slot[entry(k)] & 0x7fff : k; }
+        __device__ __forceinline__ real c(int k) const { return k < 0 ? real(0) : A.pair[at(k)].x; }
+        __device__ __forceinline__ real z(int k) const { return k < 0 ? real(0) : A.pair[at(k)].y; }
+        __device__ __forceinline__ real &m(int k) const { return full ? A.m[entry(k)] : A.pair[k].y; }
+    };
+    __device__ __forceinline__ Points points(int l) const {
+        return Points{list(l), full ? B.ray[l] : 0x7fffffff, B.n[l], full};
+    }
+
+    // the masses of the segments of task k relative to the largest (sample_line!, src/local.jl:1501), by
+    // the warp
+    __device__ __forceinline__ void masses(int k) const {
+        real mx = -INFINITY;
+#pragma unroll 1
+        for (int side = 0; side < 2; ++side) {
+            Points pt = points(2 * k + side);
+            int np = B.np[2 * k + side];
+            for (int j = lane; j < np; j += 32) {
+                real L = pt.key(j) - pt.key(j - 1), c0 = pt.c(j - 1), c1 = pt.c(j);
+                real lm = L > 0 ? -fmin(c0, c1) + Lane<real>::logseg(L, fabs(c1 - c0)) : real(-INFINITY);
+                pt.m(j) = lm;
+                mx = fmax(mx, lm);
             }
-            B += __shfl_sync(0xffffffffu, ds, qS & 31);
-            absB += __shfl_sync(0xffffffffu, da, qS & 31);
-        };
-        __syncwarp();
-        while (true) {
-            double sl = (double)sgn * B;
-            if (sl > 0)
-                delta = fmin(real(2) * M.maxnats / (real)sl, real(1e3) * fmax(fabs(tcur), real(1e-3)));
-            else
-                delta = delta == 0 ? fmax(fabs(tcur), real(1e-6)) : real(2) * delta;
-            real target = tcur + sgn * delta;
-            if (++nx > 80) {
-                __syncwarp();
-                *np = npts;
-                return 0;
-            }
-            while (true) {
-                real tS;
-                int qS;
-                nearest(&tS, &qS);
-                if (!isfinite(tS) || !(sgn * (target - tS) > 0)) break;
-                c += B * (double)(tS - tcur);
-                tcur = tS;
-                if (!point(tS)) return -1;
-                pass(qS, tS);
-            }
-            c += B * (double)(target - tcur);
-            tcur = target;
-            if (!point(target)) return -1;
-            while (true) {
-                real tS;
-                int qS;
-                nearest(&tS, &qS);
-                if (!(isfinite(tS) && tS == target)) break;
-                pass(qS, target);
-            }
-            if (c - cmin > (double)M.maxnats) {
-                __syncwarp();
-                *np = npts;
-                return 1;
+        }
+        for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+#pragma unroll 1
+        for (int side = 0; side < 2; ++side) {
+            Points pt = points(2 * k + side);
+            int np = B.np[2 * k + side];
+            for (int j = lane; j < np; j += 32) {
+                real &x = pt.m(j);
+                x = exp(x - mx);
             }
         }
     }
 
-    // sample_line! (src/local.jl:1501) over both walks; *guard when a walk overflowed (t = 0)
-    __device__ __noinline__ real sample_line(real ucat, real uoff, bool *guard) const {
-        const int mp = SL.maxpts;
-        real *pts = (real *)(base + SL.o_pts);
-        real *pr = pts, *cr = pts + mp, *zr = pts + 2 * mp, *pl = pts + 3 * mp, *cl = pts + 4 * mp, *zl = pts + 5 * mp;
-        real *lm = (real *)(base + SL.o_lm);
-        *guard = false;
-        int nr = 0, nl = 0;
-        int w = walk(real(1), pr, cr, zr, &nr);
-        if (w < 0) {
-            *guard = true;
-            return 0;
-        }
-        if (w == 0) return 0;
-        w = walk(real(-1), pl, cl, zl, &nl);
-        if (w < 0) {
-            *guard = true;
-            return 0;
-        }
-        if (w == 0) return 0;
-        __syncwarp();
-        auto Pm = [&](int i) -> real { return i < nl ? pl[nl - 1 - i] : (i == nl ? real(0) : pr[i - nl - 1]); };
-        auto Cm = [&](int i) -> real { return i < nl ? cl[nl - 1 - i] : (i == nl ? real(0) : cr[i - nl - 1]); };
-        auto Zm = [&](int i) -> real { return i < nl ? zl[nl - 1 - i] : (i == nl ? real(0) : zr[i - nl - 1]); };
-        int nseg = nl + nr;
-        real mx = -INFINITY;
-        for (int j = lane; j < nseg; j += 32) {
-            real p0 = Pm(j), p1 = Pm(j + 1), c0 = Cm(j), c1 = Cm(j + 1);
-            real L = p1 - p0;
-            real v = L > 0 ? -fmin(c0, c1) + Lane<real>::logseg(L, fabs(c1 - c0)) : real(-INFINITY);
-            lm[j] = v;
-            mx = fmax(mx, v);
-        }
-        mx = warp_max(mx);
-        real totl = 0;
-        for (int j = lane; j < nseg; j += 32) {
-            real x = exp(lm[j] - mx);
-            lm[j] = x;
-            totl += x;
-        }
-        real tot = warp_sum(totl);
-        __syncwarp();
+    // the draw over the segments of task k; the sums in segment order: the left walk's from its last
+    // point inward, then the right walk's. *again: the round-off scales decide, which a batch has not.
+    __device__ __forceinline__ real draw(int k, real ucat, real uoff, bool *again) const {
+        const Points R = points(2 * k), Lf = points(2 * k + 1);
+        const int nr = B.np[2 * k], nl = B.np[2 * k + 1];
+        real tot = 0;
+#pragma unroll 8
+        for (int j = nl - 1; j >= 0; --j) tot += Lf.m(j);
+#pragma unroll 8
+        for (int j = 0; j < nr; ++j) tot += R.m(j);
         real u = ucat * tot, acc = 0;
-        int jj = nseg - 1;
-        for (int b0 = 0; b0 < nseg; b0 += 32) {
-            int j = b0 + lane;
-            real x = j < nseg ? lm[j] : real(0);
-            real inc = acc + warp_incl_sum(x, lane);
-            unsigned bb = __ballot_sync(0xffffffffu, j < nseg && u <= inc);
-            if (bb) {
-                jj = b0 + __ffs(bb) - 1;
-                break;
+        // eight sums, then the test of each: the first segment whose sum reaches u (the last, if none)
+        auto find = [&](const Points &pt, int n, bool down) -> int {
+            for (int j0 = 0; j0 < n; j0 += 8) {
+                real s[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    int j = j0 + i;
+                    s[i] = j < n ? acc + pt.m(down ? n - 1 - j : j) : acc;
+                    acc = s[i];
+                }
+                if (!(u <= acc)) continue;
+                int x = -1;
+#pragma unroll
+                for (int i = 7; i >= 0; --i)
+                    if (j0 + i < n && u <= s[i]) x = j0 + i;
+                if (x >= 0) return x;
             }
-            acc = __shfl_sync(0xffffffffu, inc, 31);
+            return -1;
+        };
+        // the segment starts at merged point m0 (0: the start, -k the left walk's, k the right walk's)
+        int m0 = find(Lf, nl, true);
+        if (m0 >= 0) {
+            m0 -= nl;
+        } else {
+            m0 = find(R, nr, false);
+            if (m0 < 0) m0 = nr - 1;
         }
-        real p0 = Pm(jj), p1 = Pm(jj + 1);
+        auto P = [&](int m) -> real { return m < 0 ? -Lf.key(-m - 1) : R.key(m - 1); };
+        auto C = [&](int m) -> real { return m < 0 ? Lf.c(-m - 1) : R.c(m - 1); };
+        real p0 = P(m0), p1 = P(m0 + 1), c0 = C(m0), c1 = C(m0 + 1);
         real L = p1 - p0;
-        real g = (Cm(jj + 1) - Cm(jj)) / L;
+        real g = (c1 - c0) / L;
         real flat = Lane<real>::flat_nats;
         if constexpr (sizeof(real) == 4) {
-            auto slope = [&](int j) -> real {
-                if (j < 0 || j >= nseg) return 0;
-                real Lj = Pm(j + 1) - Pm(j);
-                return Lj > 0 ? fabs((Cm(j + 1) - Cm(j)) / Lj) : real(0);
+            auto slope = [&](int m) -> real {
+                if (m < -nl || m >= nr) return 0;
+                real Lm = P(m + 1) - P(m);
+                return Lm > 0 ? fabs((C(m + 1) - C(m)) / Lm) : real(0);
             };
-            real gl = slope(jj - 1), gm = slope(jj), gr = slope(jj + 1);
-            real z0 = Zm(jj) + real(2.4e-7) * fabs(p0) * fmax(gl, gm);
-            real z1 = Zm(jj + 1) + real(2.4e-7) * fabs(p1) * fmax(gm, gr);
-            flat = fmax(flat, z0 + z1);
+            real gl = slope(m0 - 1), gm = slope(m0), gr = slope(m0 + 1);
+            if (full) {
+                auto Z = [&](int m) -> real { return m < 0 ? Lf.z(-m - 1) : R.z(m - 1); };
+                real z0 = Z(m0) + real(2.4e-7) * fabs(p0) * fmax(gl, gm);
+                real z1 = Z(m0 + 1) + real(2.4e-7) * fabs(p1) * fmax(gm, gr);
+                flat = fmax(flat, z0 + z1);
+            } else {
+                // an upper bound of the two scales: where it leaves no doubt they are not needed
+                real a0 = B.ab[2 * k + (m0 < 0)], a1 = B.ab[2 * k + (m0 + 1 < 0)];
+                real most = real(4.9e-7) * (fabs(c0) + a0 * fabs(p0) + fabs(c1) + a1 * fabs(p1)) +
+                            real(2.5e-7) * (fabs(p0) * fmax(gl, gm) + fabs(p1) * fmax(gm, gr));
+                if (!(fabs(g * L) > most && fabs(g * L) > flat)) {
+                    *again = true;
+                    return 0;
+                }
+            }
         }
-        real t = (g >= 0 || fabs(g * L) < flat) ? p0 + Lane<real>::trexp_offset(uoff, g, L, flat)
-                                                : p1 - Lane<real>::trexp_offset(uoff, -g, L, flat);
-        __syncwarp();
-        return t;
+        return sep_pick<real>(p0, p1, g, L, uoff, flat);
     }
 
-    // commit (apply_step!, src/local.jl:2507): every unit's state of charge and its node balances
-    __device__ void commit(real t) const {
-        for (int q = lane; q < nu; q += 32) {
-            int j = d.si[q];
-            real x = t * d.sa[q];
-            real k = M.kc_s[j], w = k + M.kappa0;
-            real djw, dw, dja, da;
-            soc_diff<real>(M.s_hours[j], M.s_qt[j], M.s_etain[j], M.s_etaout[j], M.s_mc[j], k, w, M.dt, M.c_viol,
-                           U(SF_E0, q), U(SF_E1, q), x, real(0), &djw, &dw);
-            soc_diff<real>(M.s_hours[j], M.s_qt[j], M.s_etain[j], M.s_etaout[j], M.s_mc[j], k, w, M.dt, M.c_viol,
-                           U(SF_EM, q), U(SF_E0, q), real(0), x, &dja, &da);
-            M.r[ix(d.nda[d.sposa[q]], taum)] += dja;
-            M.e[ix(j, tau)] += x;
-            M.r[ix(d.nds[d.spos[q]], tau)] += djw;
-        }
+    // the commit of unit q of a task at t (apply_step!, src/local.jl:2507): its state of charge and
+    // its two node balances
+    __device__ __forceinline__ void commit(int q, real t, int tau, int taum, int tau1, int rep) const {
+        int j = U.j[q], n = U.n[q];
+        real *pe = &M.e[ix(j, tau, rep)];
+        SepUnit<real> u{};
+        u.load(M, U, q, *pe, clampr<real>(M.e[ix(j, tau1, rep)], 0, 1), clampr<real>(M.e[ix(j, taum, rep)], 0, 1));
+        real cw, ca, djw, dja;
+        u.move(M, mul_rn(t, u.a), &cw, &ca, &djw, &dja);
+        real *pa = &M.r[ix(n, taum, rep)], *pw = &M.r[ix(n, tau, rep)];
+        *pa = add_rn(*pa, dja);
+        *pw = add_rn(*pw, djw);
+        *pe = fma_rn(t, u.a, u.e0);
     }
 };
 
-// Whether move descriptor d is separable with at least sepmin units (the cooperative walk's moves).
+// Whether move descriptor d is separable with at least sepmin units (the moves of k_move_sep).
 template <class real>
 __device__ inline bool sep_move(const Desc<real> &d, int sepmin) {
     const int *h = d.hdr;
@@ -635,73 +990,188 @@ __device__ inline bool sep_move(const Desc<real> &d, int sepmin) {
 }
 
 // Move mi of the class for every (step, replica) task when it is a separable move with at least
-// sepmin units (else nothing: k_move runs it): one task per warp, taken from the per-move counter.
-// The warps' walk buffers sit in dynamic shared memory after the descriptor (sep_smem = 1) or in
-// per-warp slabs of gslab.
-template <class real, int WPB>
-__global__ void __launch_bounds__(32 * WPB)
+// sepmin units (else nothing: k_move runs it). A block takes batches of tasks from the per-move
+// counter: as many as its shared memory (region bytes) holds lists for, but no more than share the
+// tasks over the grid. A task whose walk passes every clamp, or whose draw needs the round-off scales
+// of its points, runs again, alone, with room for both. tmp: tmp_warp bytes a warp (sort_mem).
+template <class real>
+__global__ void __launch_bounds__(32 * ESM_SEP_WARPS, 4)
     k_move_sep(const __grid_constant__ DevModel<real> M, const int *steps, int nsteps, const uint32_t *sweep_p, int mi,
-               const char *descs, size_t stride, int sepmin, int sep_smem, char *gslab, unsigned long long *stats,
-               unsigned int *next_item) {
+               const char *descs, size_t stride, int sepmin, int region, int nsm, char *tmp, int tmp_warp,
+               unsigned long long *stats, unsigned int *next_item) {
     extern __shared__ __align__(16) char smem[];
-    __shared__ Desc<real> sd;
-    __shared__ SepLayout sSL;
-    int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    if (threadIdx.x == 0) {
-        // the header first: most moves are not this kernel's
-        Desc<real> g = carve_desc<real>((char *)(descs + (size_t)mi * stride), M, M.natoms + M.nextra);
-        sd.hdr = g.hdr;
+    __shared__ SepBlock<real> B;
+    const Desc<real> d = carve_desc<real>((char *)(descs + (size_t)mi * stride), M, M.natoms + M.nextra);
+    if (!sep_move<real>(d, sepmin)) return;  // grid-uniform
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int nu = d.hdr[1], T = M.T;
+    const int ntask = nsteps * M.R;
+    SepUnits<real> U(smem, nu);
+    for (int q = threadIdx.x; q < nu; q += 32 * ESM_SEP_WARPS) {
+        int j = d.si[q];
+        U.j[q] = j;
+        U.n[q] = M.s_bus[j];
+        U.a[q] = d.sa[q];
+        U.k[q] = M.kc_s[j];
+        U.h[q] = M.s_hours[j];
+        U.qt[q] = M.s_qt[j];
+        U.ein[q] = M.s_etain[j];
+        U.eout[q] = M.s_etaout[j];
+        U.mc[q] = M.s_mc[j];
     }
-    __syncthreads();
-    if (!sep_move<real>(sd, sepmin)) return;  // grid-uniform
-    __syncthreads();
-    {
-        const int4 *src = (const int4 *)(descs + (size_t)mi * stride);
-        int4 *dst = (int4 *)smem;
-        for (size_t i = threadIdx.x; i < stride / 16; i += 32 * WPB) dst[i] = src[i];
-    }
-    if (threadIdx.x == 0) {
-        sd = carve_desc<real>(smem, M, M.natoms + M.nextra);
-        sSL = sep_layout<real>(M.maxstu, M.maxpts);
-    }
-    __syncthreads();
-    const Desc<real> &d = sd;
-    const SepLayout &SL = sSL;
-    char *wbase = sep_smem ? smem + stride + (size_t)wib * SL.total
-                           : gslab + ((size_t)blockIdx.x * WPB + wib) * (size_t)SL.total;
-    SepWalk<real> W(M, d, SL, wbase, lane);
-    uint32_t sweep = *sweep_p;
-    unsigned long long tried = 0, moved = 0, guards = 0;
-    int ntask = nsteps * M.R;
-    int T = M.T;
+    const int ub = sep_unit_bytes<real>(nu);
+    // tasks of a batch: nw warps of nt tasks (a power of two)
+    int fit = (region - ub) / (2 * sep_list_bytes<real>(nu, M.maxpts, sep_kind(nu, false)));
+    int share = (ntask + gridDim.x - 1) / gridDim.x;
+    if (fit > share) fit = share;
+    const int nw_batch = fit < ESM_SEP_WARPS ? fit : ESM_SEP_WARPS;
+    int nt_batch = 1;
+    while (nt_batch < 16 && 2 * nt_batch * ESM_SEP_WARPS <= fit) nt_batch <<= 1;
+    tmp += ((size_t)blockIdx.x * ESM_SEP_WARPS + wib) * tmp_warp;
+    const uint32_t sweep = *sweep_p;
+    unsigned int tried = 0, moved = 0, guards = 0;
+    // the list of this thread's scan: the blocks of an SM start at different warps, whose FP64 units
+    // are those of different schedulers
+    const int sl = (threadIdx.x + 32 * (blockIdx.x / nsm)) & (32 * ESM_SEP_WARPS - 1);
+    if (threadIdx.x == 0) B.nalone = 0;
     while (true) {
-        unsigned int it = 0;
-        if (lane == 0) it = atomicAdd(next_item, 1u);
-        int task = (int)__shfl_sync(0xffffffffu, it, 0);
-        if (task >= ntask) break;
-        int q = task / M.R;
-        W.rep = task % M.R;
-        W.tau = steps[q];
-        W.taum = (W.tau - 1 + T) % T;
-        W.tau1 = (W.tau + 1) % T;
-        W.load_units();
-        double uc, uo;
-        uniform2(M.seed, ESM_TAG_LANE, 2 * (uint32_t)mi, (uint32_t)W.tau, (uint32_t)W.rep, sweep, &uc, &uo);
-        bool guard;
-        real t = W.sample_line(unit_uniform<real>(uc), unit_uniform<real>(uo), &guard);
-        if (guard) ++guards;
-        if (t != 0) W.commit(t);
-        if (M.mlog && W.rep < M.mlog_nrep && lane == 0)
-            M.mlog[((size_t)mi * nsteps + q) * M.mlog_nrep + W.rep] = (double)t;
-        ++tried;
-        if (t != 0) ++moved;
+        __syncthreads();
+        const bool alone = B.nalone > 0;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (alone)
+                B.batch = B.alone[--B.nalone];
+            else
+                B.batch = (int)atomicAdd(next_item, 1u);
+        }
+        __syncthreads();
+        const int nw = alone ? 1 : nw_batch, nt = alone ? 1 : nt_batch;
+        const int tb = nw * nt;  // tasks of the batch
+        const int task0 = alone ? B.batch : B.batch * tb;
+        if (task0 >= ntask) break;
+        const int kind = sep_kind(nu, alone);
+        const bool full = kind != SEP_BATCH;
+        SepWalk<real> S{M, U, B, smem + ub, nu, sep_events(nu, M.maxpts, kind), sep_entries(nu, M.maxpts, kind),
+                        sep_list_bytes<real>(nu, M.maxpts, kind), full, alone, lane};
+        // this lane's list in the event part: list l (task l / 2, direction l % 2)
+        const int nl = 2 * nt;
+        const int l = wib * nl + (lane & (nl - 1));
+        const int q0 = lane / nl, qstep = 32 / nl;
+        const real sgn = (l & 1) ? real(-1) : real(1);
+        const int task = task0 + (l >> 1);
+        const bool mine = wib < nw && (l >> 1) < tb && task < ntask;
+        int rep = 0, tau = 0, taum = 0, tau1 = 0;
+        if (mine) {
+            rep = task % M.R;
+            tau = steps[task / M.R];
+            taum = (tau - 1 + T) % T;
+            tau1 = (tau + 1) % T;
+        }
+        if (wib < nw) {
+            int ncl;
+            real W = S.next_clamp(mine ? q0 : nu, qstep, nl, tau, rep, sgn, real(0), &ncl);
+            if (lane < nl) {
+                B.W[l] = W;
+                B.ncl[l] = ncl;
+                B.st[l] = !mine ? SEP_IMPROPER : (full || W < real(INFINITY)) ? SEP_OPEN : SEP_ALONE;
+            }
+        }
         __syncwarp();
+        bool open = true;
+        while (open) {
+            if (wib < nw) {
+                bool on = mine && B.st[l] == SEP_OPEN;
+                if (__any_sync(0xffffffffu, on)) {
+                    int before;
+                    int n = S.events(l, on, q0, qstep, nl, tau, taum, tau1, rep, sgn, B.W[l], &before);
+                    if (on && lane < nl) {
+                        B.n[l] = n;
+                        B.before[l] = before;
+                    }
+                    __syncwarp();
+                    unsigned todo = __ballot_sync(0xffffffffu, on && lane < nl && n > ESM_SEP_SHORT && n <= S.maxe);
+                    while (todo) {
+                        int x = __ffs(todo) - 1;
+                        todo &= todo - 1;
+                        S.sort(S.list(wib * nl + x), __shfl_sync(0xffffffffu, n, x),
+                               (double *)tmp);
+                    }
+                }
+            }
+            __syncthreads();
+            bool again = false;
+            if (sl < 2 * tb && B.st[sl] == SEP_OPEN) {
+                real dir = (sl & 1) ? real(-1) : real(1);
+                if (full)
+                    S.scan_full(sl, dir);
+                else
+                    S.scan(sl, dir);
+                again = B.st[sl] == SEP_OPEN;
+            }
+            open = __syncthreads_or(again);
+            if (open && wib < nw) {  // the open lists' windows end at the next clamp
+                bool on = mine && B.st[l] == SEP_OPEN;
+                int ncl;
+                real W = S.next_clamp(on ? q0 : nu, qstep, nl, tau, rep, sgn, B.W[l], &ncl);
+                __syncwarp();
+                if (on && lane < nl) {
+                    B.W[l] = W;
+                    if (!full && !(W < real(INFINITY))) B.st[l] = SEP_ALONE;
+                }
+                __syncwarp();
+            }
+        }
+        if (wib < nw)
+            for (int k = wib * nt; k < (wib + 1) * nt; ++k)
+                if (B.st[2 * k] == SEP_PROPER && B.st[2 * k + 1] == SEP_PROPER) S.masses(k);
+        __syncthreads();
+        if (sl < tb) {
+            int k = sl, tk = task0 + k;
+            real t = 0;
+            if (tk < ntask) {
+                int r = tk % M.R, qs = tk / M.R, ts = steps[qs];
+                int a = B.st[2 * k], b = B.st[2 * k + 1];
+                // the right walk's outcome counts first, as in the one-lane walk
+                int w = a != SEP_PROPER ? a : b;
+                bool again = w == SEP_ALONE;
+                if (w == SEP_PROPER) {
+                    double uc, uo;
+                    uniform2(M.seed, ESM_TAG_LANE, 2 * (uint32_t)mi, (uint32_t)ts, (uint32_t)r, sweep, &uc, &uo);
+                    t = S.draw(k, unit_uniform<real>(uc), unit_uniform<real>(uo), &again);
+                }
+                if (again) {
+                    B.alone[atomicAdd(&B.nalone, 1)] = tk;
+                } else {
+                    ++tried;
+                    if (w == SEP_GUARD) ++guards;
+                    if (t != 0) ++moved;
+                    if (M.mlog && r < M.mlog_nrep) M.mlog[((size_t)mi * nsteps + qs) * M.mlog_nrep + r] = (double)t;
+                }
+            }
+            B.t[k] = t;
+        }
+        __syncthreads();
+        if (wib < nw) {  // lanes: the warp's tasks, then its units
+            int k = wib * nt + (lane & (nt - 1)), tk = task0 + k;
+            if (k < tb && tk < ntask) {
+                real t = B.t[k];
+                if (t != 0) {
+                    int r = tk % M.R, ts = steps[tk / M.R];
+                    for (int q = lane / nt; q < nu; q += 32 / nt) S.commit(q, t, ts, (ts - 1 + T) % T, (ts + 1) % T, r);
+                }
+            }
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        tried += __shfl_xor_sync(0xffffffffu, tried, o);
+        moved += __shfl_xor_sync(0xffffffffu, moved, o);
+        guards += __shfl_xor_sync(0xffffffffu, guards, o);
     }
     if (lane == 0) {
         int fi = ESM_NFAM;  // atoms
-        if (tried) atomicAdd(&stats[2 * fi], tried);
-        if (moved) atomicAdd(&stats[2 * fi + 1], moved);
-        if (guards) atomicAdd(&stats[2 * (ESM_NFAM + 1)], guards);
+        if (tried) atomicAdd(&stats[2 * fi], (unsigned long long)tried);
+        if (moved) atomicAdd(&stats[2 * fi + 1], (unsigned long long)moved);
+        if (guards) atomicAdd(&stats[2 * (ESM_NFAM + 1)], (unsigned long long)guards);
     }
 }
 

@@ -282,14 +282,15 @@ int esm_move_grid(const esm_ctx *ctx, int32_t *warps_per_block, int32_t *warps_p
 int esm_set_move_log(esm_ctx *ctx, int32_t nreps);
 int esm_move_log(esm_ctx *ctx, int32_t cls, double *out);
 
-/* The cooperative walk of the separable moves. A move whose terms are storage units at distinct
-   nodes and nothing else (the state-of-charge atoms, walk!, src/local.jl:1294, on a potential that
-   is a sum of per-unit functions) with at least min_units units runs one (step, replica) task per
-   warp: the lanes generate the units' breakpoints, a window's breakpoints are sorted in shared memory
-   and the potential follows from warp scans. Smaller and other moves keep one task per lane (k_move).
-   min_units 0 switches it off. Same draws and the same points as the per-lane walk, up to the
-   order of floating-point sums. esm_set_sep_walk drops the captured class graphs; esm_sep_walk
-   reads the setting and the kernel's warps. No reference counterpart. */
+/* The block walk of the separable moves. A move whose terms are storage units at distinct nodes and
+   nothing else (the state-of-charge atoms, walk!, src/local.jl:1294, on a potential that is a sum of
+   per-unit functions) with at least min_units units is walked by blocks of warps, a batch of (step,
+   replica) tasks at a time: lanes make the units' breakpoints, the breakpoints of a window are sorted
+   in shared memory, and the sums over them are taken in order. Smaller and other moves keep one task
+   per lane (k_move). min_units 0 (the default): every separable move that fits a block's shared memory.
+   The same draws and points as the one-lane walk, to the last bit. esm_set_sep_walk drops the
+   captured class graphs; esm_sep_walk reads the setting and the kernel's warps. No reference
+   counterpart. */
 #define ESM_SEP_MIN_DEFAULT 0
 int esm_set_sep_walk(esm_ctx *ctx, int32_t min_units);
 int esm_sep_walk(const esm_ctx *ctx, int32_t *min_units, int32_t *warps);
@@ -301,7 +302,7 @@ int esm_sep_walk(const esm_ctx *ctx, int32_t *min_units, int32_t *warps);
    independent, so a task's moves and their results are the same: bit-identical states), without
    the idle tail each per-move launch ends with; each of its waits for an item's previous move is
    bounded, and one that runs out makes the next esm_sync or statistics read return ESM_ETIMEOUT.
-   Not combined with the cooperative walk (esm_set_sep_walk > 0 keeps the per-move launches). No
+   It walks every move one task per lane; esm_set_sep_walk > 0 keeps the per-move launches. No
    reference counterpart. */
 enum { ESM_MOVES_PER_MOVE = 0, ESM_MOVES_PER_CLASS = 1 };
 int esm_set_move_schedule(esm_ctx *ctx, int32_t schedule);
