@@ -56,6 +56,7 @@ struct esm_ctx {
     // its grid (0 blocks: not used), shared memory and the buffer of its long sorts
     int sep_min = ESM_SEP_MIN_DEFAULT, sep_blocks = 0, sep_region = 0, sep_tmp_warp = 0;
     char *d_sep_tmp = nullptr;
+    int walk_blocks = 0, walk_region = 0;  // k_move_walk
     int sl_nunits = 0;  // eligible units of the last long-range storage sweep (its move log)
     int device = -1;                   // the device the context was created on
     double *score_scratch = nullptr;   // device address of the static score scratch on that device
@@ -500,6 +501,9 @@ int alloc_state(esm_ctx *c) {
     c->sep_blocks = esm::sep_blocks<real>(M, nsm);
     c->sep_tmp_warp = esm::sep_tmp_bytes<real>(M);
     if ((rc = dalloc(c, &c->d_sep_tmp, (size_t)4 * c->sep_tmp_warp * c->sep_blocks))) return rc;
+    c->walk_region = 48 * 1024;
+    c->walk_blocks = esm::walk_blocks<real>(M, nsm, c->walk_region, (int)wscr);
+    if (c->walk_blocks == 0) c->walk_region = 0;
     // the move descriptors of a class pass
     char *dp;
     if ((rc = dalloc(c, &dp, esm::linemove_smem_per_warp<real>(M) * (size_t)(M.natoms + M.nextra)))) return rc;
@@ -598,7 +602,8 @@ __global__ void k_set_word(uint32_t *p, uint32_t v) { *p = v; }
 
 int class_pass_launch(esm_ctx *c, int cls, int limit) {
     int ns = c->class_len[cls];
-    esm::SepLaunch sep{c->sep_min, c->sep_blocks, c->sep_region, c->nsm, c->sep_tmp_warp, c->d_sep_tmp};
+    esm::SepLaunch sep{c->sep_min, c->sep_blocks, c->sep_region, c->nsm, c->sep_tmp_warp, c->d_sep_tmp,
+                       c->walk_blocks, c->walk_region};
     esm::WaveLaunch wave{c->move_schedule == ESM_MOVES_PER_CLASS, c->d_wave_done, c->d_wave_err, c->wave_items};
     if (c->precision == 64)
         CK(esm::launch_class_pass<double>(c->Md, c->d_steps[cls], ns, c->d_sweep, cls, limit, (double *)c->d_scratch,

@@ -16,6 +16,7 @@ size_t linemove_smem_per_warp(const DevModel<real> &M);  // bytes of one move de
 struct SepLaunch {
     int min_units, blocks, region, nsm, tmp_warp;
     char *tmp;
+    int walk_blocks, walk_region;  // k_move_walk: blocks and shared memory (0: not used)
 };
 // the whole class pass in one k_move_wave launch (on = 1; not with the cooperative walk): done
 // holds the moves completed per work item (max_items), err is set when a bounded wait runs out
@@ -29,6 +30,8 @@ template <class real>
 int sep_region_bytes(const DevModel<real> &M);
 template <class real>
 int sep_tmp_bytes(const DevModel<real> &M);
+template <class real>
+int walk_blocks(const DevModel<real> &M, int nsm, int region, int max_warps);
 template <class real>
 int sep_blocks(const DevModel<real> &M, int nsm);
 // one colour class: the descriptors of its moves into descs ((natoms + nextra) descriptors), then

@@ -1592,6 +1592,7 @@ __device__ __noinline__ void lane_kinks(const Lane<real> &Ln) {
 }  // namespace esm
 
 #include "esm_sepwalk.cuh"
+#include "esm_walk.cuh"
 
 namespace esm {
 
@@ -1693,14 +1694,15 @@ template <class real, int WPB>
 __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
     k_move(const __grid_constant__ DevModel<real> M, const int *steps, int nsteps, int ntile, int wpt,
            const uint32_t *sweep_p, int mi, const char *descs, size_t stride, real *scratch,
-           unsigned long long *stats, unsigned int *next_item, int sepmin) {
+           unsigned long long *stats, unsigned int *next_item, int sepmin, int walk_region) {
     extern __shared__ __align__(16) char smem[];
     __shared__ Desc<real> sd;
     __shared__ LaneLayout sLL;
     int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    {  // not a valid move, or one that k_move_sep walks: nothing to do (grid-uniform)
+    {  // not a valid move, or one that k_move_sep or k_move_walk walks: nothing to do (grid-uniform)
         const Desc<real> g = carve_desc<real>((char *)(descs + (size_t)mi * stride), M, M.natoms + M.nextra);
-        if (g.hdr[12] < 0 || sep_move<real>(g, sepmin)) return;
+        WalkLayout w;
+        if (g.hdr[12] < 0 || sep_move<real>(g, sepmin) || walk_move<real>(g, walk_region, &w)) return;
     }
     {  // the block's warps share one copy of the descriptor
         const int4 *src = (const int4 *)(descs + (size_t)mi * stride);
@@ -1947,6 +1949,22 @@ int sep_blocks(const DevModel<real> &M, int nsm) {
     return nsm * nb;
 }
 
+// The walk of the other moves (k_move_walk): 48 KB of shared memory a block, four blocks per SM, no more
+// than the scratch has warps for (max_warps) where the points need it.
+template <class real>
+int walk_blocks(const DevModel<real> &M, int nsm, int region, int max_warps) {
+    int nb = 0;
+    cudaFuncSetAttribute(k_move_walk<real>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_move_walk<real>, 32 * ESM_WALK_WARPS, region);
+    if (e != cudaSuccess || nb < 1) nb = 1;
+    nb *= nsm;
+    if (M.maxpts > ESM_WALK_PTS) {  // points in the scratch slabs, where there are such
+        if (linemove_scratch_reals(M) == 0) return 0;
+        if (nb * ESM_WALK_WARPS > max_warps) nb = max_warps / ESM_WALK_WARPS;
+    }
+    return nb;
+}
+
 template <class real>
 cudaError_t launch_class_pass(const DevModel<real> &M, const int *steps, int nsteps, const uint32_t *sweep, int cls,
                               int limit, real *scratch, int wpb, int max_warps, unsigned long long *stats,
@@ -1982,17 +2000,25 @@ cudaError_t launch_class_pass(const DevModel<real> &M, const int *steps, int nst
     int sepmin = sep.blocks > 0 ? (sep.min_units > 0 ? sep.min_units : 1) : 0;
     int ntask = nsteps * M.R;
     int sblocks = ntask < sep.blocks ? ntask : sep.blocks;
+    int wblocks = (ntask + 15) / 16;
+    if (wblocks > sep.walk_blocks) wblocks = sep.walk_blocks;
     for (int mi = 0; mi < nrun; ++mi) {
         if (wpb == 4)
             k_move<real, 4><<<blocks, 128, stride, s>>>(M, steps, nsteps, ntile, wpt, sweep, mi, descs, stride, scratch,
-                                                       stats, counters + mi, sepmin);
+                                                       stats, counters + mi, sepmin, sep.walk_region);
         else if (wpb == 2)
             k_move<real, 2><<<blocks, 64, stride, s>>>(M, steps, nsteps, ntile, wpt, sweep, mi, descs, stride, scratch,
-                                                      stats, counters + mi, sepmin);
+                                                      stats, counters + mi, sepmin, sep.walk_region);
         else
             k_move<real, 1><<<blocks, 32, stride, s>>>(M, steps, nsteps, ntile, wpt, sweep, mi, descs, stride, scratch,
-                                                      stats, counters + mi, sepmin);
+                                                      stats, counters + mi, sepmin, sep.walk_region);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if (sep.walk_region > 0 && wblocks > 0) {
+            k_move_walk<real><<<wblocks, 32 * ESM_WALK_WARPS, sep.walk_region, s>>>(
+                M, steps, nsteps, sweep, mi, descs, stride, sepmin, sep.walk_region, scratch,
+                linemove_scratch_reals(M), stats, counters + mi);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        }
         if (sepmin > 0 && sblocks > 0) {
             k_move_sep<real><<<sblocks, 32 * ESM_SEP_WARPS, sep.region, s>>>(M, steps, nsteps, sweep, mi, descs, stride,
                                                                             sepmin, sep.region, sep.nsm, sep.tmp,

@@ -205,6 +205,7 @@ struct SepUnit {
     real a, k, h, ein, eout, qt, e0, s0w, s0a;
     real A, P, X;  // cost per unit of running part, penalty part and box excess
     SepTerm<real> w, t;
+    int pos, posa;  // the unit's node slots at tau and tau - 1 (LineWalk)
 
     // soc_parts at d, whose charging part pc = d / ein the caller has
     __device__ __forceinline__ void parts(real d, real pc, real *inj, real *run, real *pen) const {
@@ -233,9 +234,11 @@ struct SepUnit {
                               : (qt <= 0 ? -eout : real(0));
         parts(d0, pc, &T.inj, &T.run, &T.pen);
     }
-    // soc_diff of a term whose d0 changes by dd and whose box excess changes by dex; *dj the injection change
-    __device__ __forceinline__ real soc(const SepTerm<real> &T, real dd, real dex, real *dj) const {
+    // soc_diff of a term whose d0 changes by dd and whose box excess changes by dex; *di the injection
+    // change per unit capacity, *d1 the new d
+    __device__ __forceinline__ real cost(const SepTerm<real> &T, real dd, real dex, real *di, real *d1) const {
         real dn = add_rn(T.d0, dd);
+        *d1 = dn;
         real pc = dn / ein;
         bool same = piece(dn, pc) == T.piece;
         real inj, run, pen;
@@ -243,21 +246,31 @@ struct SepUnit {
         real dinj = same ? mul_rn(T.si, dd) : sub_rn(inj, T.inj);
         real drun = same ? mul_rn(T.sr, dd) : sub_rn(run, T.run);
         real dpen = same ? mul_rn(T.sp, dd) : sub_rn(pen, T.pen);
-        *dj = mul_rn(k, dinj);
+        *di = dinj;
         return fma_rn(X, dex, fma_rn(A, drun, mul_rn(P, dpen)));
+    }
+    __device__ __forceinline__ real soc(const SepTerm<real> &T, real dd, real dex, real *dj) const {
+        real di, d1;
+        real c = cost(T, dd, dex, &di, &d1);
+        *dj = mul_rn(k, di);
+        return c;
     }
     // the unit of slot q from its table and state
     __device__ __forceinline__ void load(const DevModel<real> &M, const SepUnits<real> &U, int q, real e0_, real e1c,
                                          real emc) {
-        a = U.a[q];
-        k = U.k[q];
-        h = U.h[q];
-        qt = U.qt[q];
-        ein = U.ein[q];
-        eout = U.eout[q];
+        load(M, U.k[q], U.h[q], U.qt[q], U.ein[q], U.eout[q], U.mc[q], U.a[q], e0_, e1c, emc);
+    }
+    __device__ __forceinline__ void load(const DevModel<real> &M, real k_, real h_, real qt_, real ein_, real eout_,
+                                         real mc, real a_, real e0_, real e1c, real emc) {
+        a = a_;
+        k = k_;
+        h = h_;
+        qt = qt_;
+        ein = ein_;
+        eout = eout_;
         e0 = e0_;
         real wt = add_rn(k, M.kappa0), dt = M.dt, cv = M.c_viol;
-        A = mul_rn(mul_rn(dt, U.mc[q]), k);
+        A = mul_rn(mul_rn(dt, mc), k);
         P = mul_rn(mul_rn(cv, dt), wt);
         X = mul_rn(mul_rn(cv, wt), h);
         real ec = clampr<real>(e0, 0, 1);
