@@ -602,7 +602,7 @@ __global__ void k_set_word(uint32_t *p, uint32_t v) { *p = v; }
 
 int class_pass_launch(esm_ctx *c, int cls, int limit) {
     int ns = c->class_len[cls];
-    esm::SepLaunch sep{c->sep_min, c->sep_blocks, c->sep_region, c->nsm, c->sep_tmp_warp, c->d_sep_tmp,
+    esm::SepLaunch sep{c->sep_min, c->sep_blocks, c->sep_region, c->sep_tmp_warp, c->d_sep_tmp,
                        c->walk_blocks, c->walk_region};
     esm::WaveLaunch wave{c->move_schedule == ESM_MOVES_PER_CLASS, c->d_wave_done, c->d_wave_err, c->wave_items};
     if (c->precision == 64)

@@ -14,7 +14,7 @@ size_t linemove_smem_per_warp(const DevModel<real> &M);  // bytes of one move de
 // nodes and nothing else, with at least min_units units (0: all of them), on `blocks` blocks (0: none,
 // k_move walks every move) with `region` bytes of shared memory each and tmp_warp bytes of tmp a warp
 struct SepLaunch {
-    int min_units, blocks, region, nsm, tmp_warp;
+    int min_units, blocks, region, tmp_warp;
     char *tmp;
     int walk_blocks, walk_region;  // k_move_walk: blocks and shared memory (0: not used)
 };

@@ -2021,7 +2021,7 @@ cudaError_t launch_class_pass(const DevModel<real> &M, const int *steps, int nst
         }
         if (sepmin > 0 && sblocks > 0) {
             k_move_sep<real><<<sblocks, 32 * ESM_SEP_WARPS, sep.region, s>>>(M, steps, nsteps, sweep, mi, descs, stride,
-                                                                            sepmin, sep.region, sep.nsm, sep.tmp,
+                                                                            sepmin, sep.region, sep.tmp,
                                                                             sep.tmp_warp, stats, counters + mi);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }

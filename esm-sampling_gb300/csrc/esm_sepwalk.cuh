@@ -82,6 +82,15 @@ __device__ __forceinline__ float sep_narrow(double x, float) {
     return __uint_as_float((h & 0x80000000u) | f);
 }
 __device__ inline double sep_narrow(double x, double) { return x; }
+// the sums over a list, in double in both builds
+template <class real>
+__device__ __forceinline__ double sep_fma(double a, double b, double c) {
+    return sizeof(real) == 4 ? __fma_rn(a, b, c) : __dadd_rn(__dmul_rn(a, b), c);
+}
+// the double of a high word in integer order (and a low word of zeros)
+__device__ __forceinline__ double sep_word(int w) {
+    return __hiloint2double(w ^ ((w >> 31) & 0x7fffffff), w < 0 ? -1 : 0);
+}
 // a float at least |x| (of FP32 size) and no more than 2^-19 above it
 __device__ __forceinline__ float sep_above(double x) {
     unsigned m = (unsigned)__double2hiint(x) & 0x7fffffffu;
@@ -145,7 +154,7 @@ struct SepUnits {  // the move's storage units (shared memory)
 // One direction of one task (shared memory). An event comes with its key (sgn * t), its slot and the
 // unit's slopes before and after it (x, y of its pair). In order, an entry of a batch's list has the key,
 // negative for a clamp, and the change of the summed slope in double over x and y; the scan leaves the
-// potential in x, the segment masses go to y. The other lists keep the pairs by slot; the scan leaves the
+// potential there, which masses() rounds into x, and the segment masses go to y. The other lists keep the pairs by slot; the scan leaves the
 // potential and its round-off scale in x and y, the masses have an array.
 template <class real>
 struct SepPair {
@@ -711,15 +720,14 @@ struct SepWalk {
     // does not end it.
     __device__ __forceinline__ void scan(int l, real sgn) const {
         SepList<real> A = list(l);
-        int n = B.n[l], ncl = B.ncl[l];
+        int n = B.n[l];
         if (n > maxe) {  // more events before the window end than points; else many at the end itself
             B.st[l] = B.before[l] >= M.maxpts ? SEP_GUARD : SEP_ALONE;
             return;
         }
         if (n <= ESM_SEP_SHORT) sort_short(A, n);
-        double b = 0, c = 0, cmin = 0;
+        double b = 0, c = 0;
         float abf = 0;
-        real kcur = 0, fmn = 0;
         for (int q = 0; q < nu; ++q) {
             real x = A.sl[q];
             b += sep_widen(x);
@@ -727,37 +735,51 @@ struct SepWalk {
         }
         const double maxnats = (double)M.maxnats;
         const int last = n < M.maxpts ? n : M.maxpts;
-        int i = 0, st = SEP_OPEN;
-        real k = A.key[0];
-        double ds = sep_get<real>(A.pair[0]);
-        for (; i < last; ++i) {
-            real k0 = k;
-            double d0 = ds;
-            if (i + 1 < n) {  // (the next entry while this one's sums are formed)
-                k = A.key[i + 1];
-                ds = sep_get<real>(A.pair[i + 1]);
-            }
-            real ka = fabs(k0);
-            c += b * sep_widen(sgn * (ka - kcur));
-            kcur = ka;
-            real cf = sep_narrow(c, real(0));
-            A.pair[i].x = cf;
-            if (cf < fmn || (cf == fmn && c < cmin)) {  // (the rounding keeps the order)
-                fmn = cf;
-                cmin = c;
-            }
-            b += d0;
-            abf += sep_above(d0);
-            if (k0 < 0) {
-                --ncl;
-                if (c - cmin > maxnats) {
+        int i = 0, st = SEP_OPEN, low = 0;  // the high word of the least potential so far (ordered as an integer)
+        // Two FP64 instructions an event, 64 cycles each, up to the next clamp: the potentials are kept in
+        // double (masses() rounds them), the minimum by its high word, and the stop test stands outside the
+        // loop (395 cycles an event with the rounding and the exact minimum in it, 635 with the test too).
+        real kn = A.key[0];
+        double dn = sep_get<real>(A.pair[0]);
+        real kc = 0;
+        while (i < last) {
+            bool clamp = false;
+#pragma unroll 2
+            do {
+                const real ka = fabs(kn);
+                const double wn = sep_widen(sgn * (ka - kc));
+                clamp = kn < 0;
+                kc = ka;
+                c = sep_fma<real>(b, wn, c);
+                b += dn;
+                abf += sep_above(dn);
+                if (i + 1 < last) {
+                    kn = A.key[i + 1];
+                    dn = sep_get<real>(A.pair[i + 1]);
+                }
+                sep_put<real>(A.pair[i], c);
+                const int h = __double2hiint(c);
+                low = min(low, h ^ ((h >> 31) & 0x7fffffff));
+                ++i;
+            } while (!clamp && i < last);
+            if (clamp) {
+                // the least potential lies between this word and the next: where that does not decide, it
+                // is taken from the potentials
+                const double m0 = sep_word(low), m1 = sep_word(low + 1);
+                bool stop = c - m1 > maxnats;
+                if (!stop && c - m0 > maxnats) {
+                    double cmin = 0;
+                    for (int j = 0; j < i; ++j) cmin = fmin(cmin, sep_get<real>(A.pair[j]));
+                    stop = c - cmin > maxnats;
+                }
+                if (stop) {
                     st = SEP_PROPER;
                     break;
                 }
             }
         }
         if (st == SEP_OPEN && i < n) st = SEP_GUARD;  // more points than the cap
-        B.np[l] = i + 1;
+        B.np[l] = i;
         B.ab[l] = abf;
         B.st[l] = st;
     }
@@ -785,7 +807,7 @@ struct SepWalk {
         real tcur = 0;
         int i = 0, np = 0, ray = 0x7fffffff, st = SEP_OPEN;
         auto advance = [&](real t) {
-            c += b * sep_widen((real)(t - tcur));
+            c = sep_fma<real>(b, sep_widen((real)(t - tcur)), c);
             tcur = t;
         };
         auto pass = [&](const SepPair<real> &v) {  // an event's slopes
@@ -806,7 +828,7 @@ struct SepWalk {
             v.x = sep_narrow(c, real(0));
             v.y = 0;
             if constexpr (sizeof(real) == 4)
-                v.y = real(4.8e-7) * sep_narrow(fabs(c) + ab * fabs(sep_widen(t)), real(0));
+                v.y = real(4.8e-7) * sep_narrow(sep_fma<real>(ab, fabs(sep_widen(t)), fabs(c)), real(0));
             A.pair[A.slot[e] & 0x7fffu] = v;
             cmin = fmin(cmin, c);
             ++np;
@@ -880,27 +902,30 @@ struct SepWalk {
         return Points{list(l), full ? B.ray[l] : 0x7fffffff, B.n[l], full};
     }
 
-    // the masses of the segments of task k relative to the largest (sample_line!, src/local.jl:1501), by
-    // the warp
-    __device__ __forceinline__ void masses(int k) const {
-        real mx = -INFINITY;
-#pragma unroll 1
-        for (int side = 0; side < 2; ++side) {
-            Points pt = points(2 * k + side);
-            int np = B.np[2 * k + side];
-            for (int j = lane; j < np; j += 32) {
+    // the masses of the segments of tasks k0 .. k0 + nt - 1 relative to each task's largest (sample_line!,
+    // src/local.jl:1501), by the warp: G lanes a list, two lists a task
+    template <int G>
+    __device__ __forceinline__ void masses(int k0, int nt) const {
+        const int side = (lane / G) & 1, j0 = lane & (G - 1);
+        for (int k = k0 + lane / (2 * G); k - lane / (2 * G) < k0 + nt; k += 16 / G) {
+            bool on = k < k0 + nt && B.st[2 * k] == SEP_PROPER && B.st[2 * k + 1] == SEP_PROPER;
+            const int l = on ? 2 * k + side : 0;
+            Points pt = points(l);
+            int np = on ? B.np[l] : 0;
+            real mx = -INFINITY;
+            if (!full) {  // the potentials of the scan, rounded
+                for (int j = j0; j < np; j += G) pt.A.pair[j].x = sep_narrow(sep_get<real>(pt.A.pair[j]), real(0));
+                __syncwarp();
+            }
+            for (int j = j0; j < np; j += G) {
                 real L = pt.key(j) - pt.key(j - 1), c0 = pt.c(j - 1), c1 = pt.c(j);
                 real lm = L > 0 ? -fmin(c0, c1) + Lane<real>::logseg(L, fabs(c1 - c0)) : real(-INFINITY);
                 pt.m(j) = lm;
                 mx = fmax(mx, lm);
             }
-        }
-        for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-#pragma unroll 1
-        for (int side = 0; side < 2; ++side) {
-            Points pt = points(2 * k + side);
-            int np = B.np[2 * k + side];
-            for (int j = lane; j < np; j += 32) {
+#pragma unroll
+            for (int o = G; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            for (int j = j0; j < np; j += G) {
                 real &x = pt.m(j);
                 x = exp(x - mx);
             }
@@ -912,22 +937,26 @@ struct SepWalk {
     __device__ __forceinline__ real draw(int k, real ucat, real uoff, bool *again) const {
         const Points R = points(2 * k), Lf = points(2 * k + 1);
         const int nr = B.np[2 * k], nl = B.np[2 * k + 1];
+        // masses j of a list, in its order: eight loads, then the sums one after the other
         real tot = 0;
-#pragma unroll 8
-        for (int j = nl - 1; j >= 0; --j) tot += Lf.m(j);
-#pragma unroll 8
-        for (int j = 0; j < nr; ++j) tot += R.m(j);
-        real u = ucat * tot, acc = 0;
-        // eight sums, then the test of each: the first segment whose sum reaches u (the last, if none)
-        auto find = [&](const Points &pt, int n, bool down) -> int {
+        auto total = [&](int n, auto &&at) {
             for (int j0 = 0; j0 < n; j0 += 8) {
                 real s[8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    int j = j0 + i;
-                    s[i] = j < n ? acc + pt.m(down ? n - 1 - j : j) : acc;
-                    acc = s[i];
-                }
+                for (int i = 0; i < 8; ++i) s[i] = j0 + i < n ? at(j0 + i) : real(0);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) tot += s[i];
+            }
+        };
+        real u = 0, acc = 0;
+        // the first segment whose sum reaches u, -1 if none
+        auto find = [&](int n, auto &&at) -> int {
+            for (int j0 = 0; j0 < n; j0 += 8) {
+                real s[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) s[i] = j0 + i < n ? at(j0 + i) : real(0);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) s[i] = acc = acc + s[i];
                 if (!(u <= acc)) continue;
                 int x = -1;
 #pragma unroll
@@ -937,14 +966,26 @@ struct SepWalk {
             }
             return -1;
         };
-        // the segment starts at merged point m0 (0: the start, -k the left walk's, k the right walk's)
-        int m0 = find(Lf, nl, true);
-        if (m0 >= 0) {
-            m0 -= nl;
+        int m0, mr = -1;
+        if (full) {
+            total(nl, [&](int j) { return Lf.m(nl - 1 - j); });
+            total(nr, [&](int j) { return R.m(j); });
+            u = ucat * tot;
+            m0 = find(nl, [&](int j) { return Lf.m(nl - 1 - j); });
+            if (m0 < 0) mr = find(nr, [&](int j) { return R.m(j); });
         } else {
-            m0 = find(R, nr, false);
-            if (m0 < 0) m0 = nr - 1;
+            const SepPair<real> *pl = Lf.A.pair + (nl - 1), *pr = R.A.pair;
+            total(nl, [&](int j) { return pl[-j].y; });
+            total(nr, [&](int j) { return pr[j].y; });
+            u = ucat * tot;
+            m0 = find(nl, [&](int j) { return pl[-j].y; });
+            if (m0 < 0) mr = find(nr, [&](int j) { return pr[j].y; });
         }
+        // the segment starts at merged point m0 (0: the start, -k the left walk's, k the right walk's)
+        if (m0 >= 0)
+            m0 -= nl;
+        else
+            m0 = mr >= 0 ? mr : nr - 1;
         auto P = [&](int m) -> real { return m < 0 ? -Lf.key(-m - 1) : R.key(m - 1); };
         auto C = [&](int m) -> real { return m < 0 ? Lf.c(-m - 1) : R.c(m - 1); };
         real p0 = P(m0), p1 = P(m0 + 1), c0 = C(m0), c1 = C(m0 + 1);
@@ -1010,7 +1051,7 @@ __device__ inline bool sep_move(const Desc<real> &d, int sepmin) {
 template <class real>
 __global__ void __launch_bounds__(32 * ESM_SEP_WARPS, 4)
     k_move_sep(const __grid_constant__ DevModel<real> M, const int *steps, int nsteps, const uint32_t *sweep_p, int mi,
-               const char *descs, size_t stride, int sepmin, int region, int nsm, char *tmp, int tmp_warp,
+               const char *descs, size_t stride, int sepmin, int region, char *tmp, int tmp_warp,
                unsigned long long *stats, unsigned int *next_item) {
     extern __shared__ __align__(16) char smem[];
     __shared__ SepBlock<real> B;
@@ -1043,10 +1084,16 @@ __global__ void __launch_bounds__(32 * ESM_SEP_WARPS, 4)
     tmp += ((size_t)blockIdx.x * ESM_SEP_WARPS + wib) * tmp_warp;
     const uint32_t sweep = *sweep_p;
     unsigned int tried = 0, moved = 0, guards = 0;
-    // the list of this thread's scan: the blocks of an SM start at different warps, whose FP64 units
-    // are those of different schedulers
-    const int sl = (threadIdx.x + 32 * (blockIdx.x / nsm)) & (32 * ESM_SEP_WARPS - 1);
-    if (threadIdx.x == 0) B.nalone = 0;
+    // the list of this thread's scan: the blocks of an SM start at different warps (by the warp slots
+    // they sit in), so that their FP64 instructions go to different schedulers' units
+    if (threadIdx.x == 0) {
+        unsigned w;
+        asm volatile("mov.u32 %0, %%warpid;" : "=r"(w));
+        B.nalone = 0;
+        B.batch = (int)(w / ESM_SEP_WARPS);
+    }
+    __syncthreads();
+    const int sl = (threadIdx.x + 32 * B.batch) & (32 * ESM_SEP_WARPS - 1);
     while (true) {
         __syncthreads();
         const bool alone = B.nalone > 0;
@@ -1135,8 +1182,10 @@ __global__ void __launch_bounds__(32 * ESM_SEP_WARPS, 4)
             }
         }
         if (wib < nw)
-            for (int k = wib * nt; k < (wib + 1) * nt; ++k)
-                if (B.st[2 * k] == SEP_PROPER && B.st[2 * k + 1] == SEP_PROPER) S.masses(k);
+            if (nu <= ESM_SEP_FULL)
+                S.template masses<8>(wib * nt, nt);
+            else
+                S.template masses<16>(wib * nt, nt);
         __syncthreads();
         if (sl < tb) {
             int k = sl, tk = task0 + k;
