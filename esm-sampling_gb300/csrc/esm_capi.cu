@@ -52,11 +52,10 @@ struct esm_ctx {
     bool has_state = false, has_scores = false;
     int move_wpb = 1;           // k_move block shape: warps per block (1, 2 or 4)
     int max_warps = 0;          // k_move warps launched per move: the resident limit or a tuned count
-    // the block walk of the separable moves (k_move_sep): moves with at least sep_min units (0: all),
-    // its grid (0 blocks: not used), shared memory and the buffer of its long sorts
-    int sep_min = ESM_SEP_MIN_DEFAULT, sep_blocks = 0, sep_region = 0, sep_tmp_warp = 0;
+    // the moves walked by blocks (k_move_blocks): separable moves with at least sep_min units (0: all);
+    // the grid (0: not used), its shared memory, that of either kind of move, the buffer of long sorts
+    int sep_min = ESM_SEP_MIN_DEFAULT, mblocks = 0, mblocks_smem = 0, sep_region = 0, walk_region = 0, sep_tmp_warp = 0;
     char *d_sep_tmp = nullptr;
-    int walk_blocks = 0, walk_region = 0;  // k_move_walk
     int sl_nunits = 0;  // eligible units of the last long-range storage sweep (its move log)
     int device = -1;                   // the device the context was created on
     double *score_scratch = nullptr;   // device address of the static score scratch on that device
@@ -496,14 +495,13 @@ int alloc_state(esm_ctx *c) {
     }
     if ((rc = dalloc(c, &q, per * wscr))) return rc;
     c->d_scratch = q;
-    // the block walk of the separable moves
+    // the moves walked by blocks
     c->sep_region = esm::sep_region_bytes<real>(M);
-    c->sep_blocks = esm::sep_blocks<real>(M, nsm);
+    c->walk_region = esm::walk_region_bytes<real>(M);
+    c->mblocks_smem = std::max(c->sep_region, c->walk_region);
+    if (c->mblocks_smem > 0) c->mblocks = esm::move_blocks<real>(M, nsm, c->mblocks_smem, (int)wscr);
     c->sep_tmp_warp = esm::sep_tmp_bytes<real>(M);
-    if ((rc = dalloc(c, &c->d_sep_tmp, (size_t)4 * c->sep_tmp_warp * c->sep_blocks))) return rc;
-    c->walk_region = 48 * 1024;
-    c->walk_blocks = esm::walk_blocks<real>(M, nsm, c->walk_region, (int)wscr);
-    if (c->walk_blocks == 0) c->walk_region = 0;
+    if ((rc = dalloc(c, &c->d_sep_tmp, (size_t)4 * c->sep_tmp_warp * c->mblocks))) return rc;
     // the move descriptors of a class pass
     char *dp;
     if ((rc = dalloc(c, &dp, esm::linemove_smem_per_warp<real>(M) * (size_t)(M.natoms + M.nextra)))) return rc;
@@ -602,8 +600,8 @@ __global__ void k_set_word(uint32_t *p, uint32_t v) { *p = v; }
 
 int class_pass_launch(esm_ctx *c, int cls, int limit) {
     int ns = c->class_len[cls];
-    esm::SepLaunch sep{c->sep_min, c->sep_blocks, c->sep_region, c->sep_tmp_warp, c->d_sep_tmp,
-                       c->walk_blocks, c->walk_region};
+    esm::SepLaunch sep{c->sep_min, c->mblocks, c->mblocks_smem, c->sep_region, c->sep_tmp_warp, c->walk_region,
+                       c->d_sep_tmp};
     esm::WaveLaunch wave{c->move_schedule == ESM_MOVES_PER_CLASS, c->d_wave_done, c->d_wave_err, c->wave_items};
     if (c->precision == 64)
         CK(esm::launch_class_pass<double>(c->Md, c->d_steps[cls], ns, c->d_sweep, cls, limit, (double *)c->d_scratch,
@@ -640,7 +638,7 @@ int class_pass_any(esm_ctx *c, uint32_t sweep, int cls, int limit = 0) {
     CK(cudaGetLastError());
     int nmoves = c->precision == 64 ? c->Md.natoms + c->Md.nextra : c->Mf.natoms + c->Mf.nextra;
     int nrun = limit > 0 && limit < nmoves ? limit : nmoves;
-    c->launches += 2 + nrun;
+    c->launches += 2 + (c->mblocks > 0 ? 2 : 1) * nrun;
     if (limit > 0) return class_pass_launch(c, cls, limit);
     if (!c->graph[cls]) {
         cudaGraph_t g = nullptr;
@@ -1675,7 +1673,7 @@ int esm_set_sep_walk(esm_ctx *c, int32_t min_units) {
 int esm_sep_walk(const esm_ctx *c, int32_t *min_units, int32_t *warps) {
     if (!c) return ESM_EINVAL;
     if (min_units) *min_units = c->sep_min;
-    if (warps) *warps = 4 * c->sep_blocks;
+    if (warps) *warps = 4 * c->mblocks;
     return ESM_OK;
 }
 
@@ -1891,6 +1889,10 @@ int batch_setup(esm_batch *b) {
         m.descs = c->d_descs;
         m.stride = esm::linemove_smem_per_warp<real>(m.M);
         m.stats = c->d_stats;
+        m.sep_on = c->sep_region > 0 ? 1 : 0;
+        m.walk_region = c->walk_region;
+        b->bl.region = std::max(b->bl.region, std::max(c->sep_region, c->walk_region));
+        b->bl.tmp_warp = std::max(b->bl.tmp_warp, c->sep_tmp_warp);
         maxstride = std::max(maxstride, m.stride);
         maxlane = std::max(maxlane, esm::linemove_scratch_reals<real>(m.M));
         b->bl.maxpass = std::max(b->bl.maxpass, c->ncls);
@@ -1922,9 +1924,16 @@ int batch_setup(esm_batch *b) {
         b->bl.scratch = q;
         b->scratch_warps = (int)w;
     }
+    // the moves walked by blocks, on no more blocks than the slabs have warps for
+    if (b->bl.region > 0) {
+        b->bl.bblocks = b->nsm * esm::batch_blocks_per_sm<real>(b->bl.region);
+        if (maxlane > 0) b->bl.bblocks = std::min(b->bl.bblocks, b->scratch_warps / 4);
+        if ((rc = balloc(b, &b->bl.tmp, (size_t)4 * b->bl.tmp_warp * b->bl.bblocks))) return rc;
+    }
     if ((rc = balloc(b, &b->bl.pass_cls, (size_t)b->bl.maxpass * n))) return rc;
+    if ((rc = balloc(b, &b->bl.choff, (size_t)b->bl.maxpass * (n + 1)))) return rc;
     if ((rc = balloc(b, &b->bl.off, (size_t)b->bl.maxpass * (n + 1)))) return rc;
-    if ((rc = balloc(b, &b->bl.counters, (size_t)b->bl.maxpass * b->bl.maxmoves))) return rc;
+    if ((rc = balloc(b, &b->bl.counters, 2 * (size_t)b->bl.maxpass * b->bl.maxmoves))) return rc;
     if ((rc = balloc(b, &b->d_sweep, 1))) return rc;
     return ESM_OK;
 }
@@ -1960,7 +1969,7 @@ int batch_sweep(esm_batch *b, uint32_t sweep) {
         BCK(e);
     }
     BCK(cudaGraphLaunch(b->graph, b->stream));
-    b->launches += 1 + b->n + b->bl.maxpass * (1 + b->bl.maxmoves);
+    b->launches += 1 + b->n + b->bl.maxpass * (1 + (b->bl.bblocks > 0 ? 2 : 1) * b->bl.maxmoves);
     return ESM_OK;
 }
 

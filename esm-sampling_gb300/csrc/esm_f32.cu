@@ -24,8 +24,9 @@ template cudaError_t launch_class_pass<float>(const DevModel<float> &, const int
                                               cudaStream_t);
 template int sep_region_bytes<float>(const DevModel<float> &);
 template int sep_tmp_bytes<float>(const DevModel<float> &);
-template int walk_blocks<float>(const DevModel<float> &, int, int, int);
-template int sep_blocks<float>(const DevModel<float> &, int);
+template int walk_region_bytes<float>(const DevModel<float> &);
+template int move_blocks<float>(const DevModel<float> &, int, int, int);
+template int batch_blocks_per_sm<float>(int);
 template int linemove_blocks_per_sm<float>(const DevModel<float> &, int);
 template cudaError_t launch_batch_passes<float>(const BatchModel<float> *, const BatchLaunch &, const uint32_t *,
                                                 cudaStream_t);

@@ -30,8 +30,9 @@ template cudaError_t launch_class_pass<double>(const DevModel<double> &, const i
                                               cudaStream_t);
 template int sep_region_bytes<double>(const DevModel<double> &);
 template int sep_tmp_bytes<double>(const DevModel<double> &);
-template int walk_blocks<double>(const DevModel<double> &, int, int, int);
-template int sep_blocks<double>(const DevModel<double> &, int);
+template int walk_region_bytes<double>(const DevModel<double> &);
+template int move_blocks<double>(const DevModel<double> &, int, int, int);
+template int batch_blocks_per_sm<double>(int);
 template int linemove_blocks_per_sm<double>(const DevModel<double> &, int);
 template cudaError_t launch_batch_passes<double>(const BatchModel<double> *, const BatchLaunch &, const uint32_t *,
                                                 cudaStream_t);

@@ -10,13 +10,12 @@ template <class real>
 size_t linemove_scratch_reals(const DevModel<real> &M);  // per warp
 template <class real>
 size_t linemove_smem_per_warp(const DevModel<real> &M);  // bytes of one move descriptor
-// the block walk of the separable moves (k_move_sep): moves whose units are storage units at distinct
-// nodes and nothing else, with at least min_units units (0: all of them), on `blocks` blocks (0: none,
-// k_move walks every move) with `region` bytes of shared memory each and tmp_warp bytes of tmp a warp
+// the moves walked by blocks (k_move_blocks) on `blocks` blocks (0: none, k_move walks every move) with
+// smem bytes of shared memory: the separable moves of at least min_units units (0: all) with `region`
+// bytes (0: none) and tmp_warp bytes of tmp a warp, and the other moves with walk_region bytes (0: none)
 struct SepLaunch {
-    int min_units, blocks, region, tmp_warp;
+    int min_units, blocks, smem, region, tmp_warp, walk_region;
     char *tmp;
-    int walk_blocks, walk_region;  // k_move_walk: blocks and shared memory (0: not used)
 };
 // the whole class pass in one k_move_wave launch (on = 1; not with the cooperative walk): done
 // holds the moves completed per work item (max_items), err is set when a bounded wait runs out
@@ -31,9 +30,9 @@ int sep_region_bytes(const DevModel<real> &M);
 template <class real>
 int sep_tmp_bytes(const DevModel<real> &M);
 template <class real>
-int walk_blocks(const DevModel<real> &M, int nsm, int region, int max_warps);
+int walk_region_bytes(const DevModel<real> &M);
 template <class real>
-int sep_blocks(const DevModel<real> &M, int nsm);
+int move_blocks(const DevModel<real> &M, int nsm, int smem, int max_warps);
 // one colour class: the descriptors of its moves into descs ((natoms + nextra) descriptors), then
 // per move one k_move launch (and one k_move_sep launch; the kernel that does not take the move
 // returns at once); the sweep index is read on the device from *sweep (graph-capturable)
@@ -58,6 +57,7 @@ struct BatchModel {
     char *descs;                // its descriptor buffer: nmoves descriptors of stride bytes
     size_t stride;
     unsigned long long *stats;  // its move counts, laid out as a context's
+    int sep_on, walk_region;    // as in its own passes: separable moves from this many units; walk_run's bytes
 };
 struct BatchLaunch {
     int nm;                  // models
@@ -71,7 +71,10 @@ struct BatchLaunch {
     size_t scratch_per_warp; // reals of one warp's slab (0: no model needs one)
     int *pass_cls;           // device [maxpass * nm]: the class model b runs in pass p (-1: none)
     unsigned int *off;       // device [maxpass * (nm + 1)]: the item prefix over the models of pass p
-    unsigned int *counters;  // device [maxpass * maxmoves]: the item counters of the launches
+    unsigned int *choff;     // device [maxpass * (nm + 1)]: the chunk prefix (k_move_blocks_batch)
+    unsigned int *counters;  // device [2 * maxpass * maxmoves]: the item and chunk counters of the launches
+    int bblocks, region, tmp_warp;  // k_move_blocks_batch: blocks (0: not used), shared memory, sort buffer
+    char *tmp;
 };
 // the passes of one sweep of every model of the batch (the sweep index read from *sweep on the
 // device, graph-capturable); the caching rebuild at the sweep start is the caller's
@@ -81,6 +84,8 @@ cudaError_t launch_batch_passes(const BatchModel<real> *bm, const BatchLaunch &b
 // resident k_move_batch warps per SM with blocks of wpb (1 or 2) warps; sets the kernels' limits
 template <class real>
 int batch_warps_per_sm(int wpb);
+template <class real>
+int batch_blocks_per_sm(int region);
 
 // ---- storage multiscale sweep (esm_plateau.cuh)
 #define ESM_PLAT_MAXU 32  // units of one plateau move (a cell-class aggregate)

@@ -1699,7 +1699,7 @@ __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
     __shared__ Desc<real> sd;
     __shared__ LaneLayout sLL;
     int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    {  // not a valid move, or one that k_move_sep or k_move_walk walks: nothing to do (grid-uniform)
+    {  // not a valid move, or one that k_move_blocks walks: nothing to do (grid-uniform)
         const Desc<real> g = carve_desc<real>((char *)(descs + (size_t)mi * stride), M, M.natoms + M.nextra);
         WalkLayout w;
         if (g.hdr[12] < 0 || sep_move<real>(g, sepmin) || walk_move<real>(g, walk_region, &w)) return;
@@ -1758,6 +1758,67 @@ __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
         if (moved) atomicAdd(&stats[2 * fi + 1], moved);
         if (guards) atomicAdd(&stats[2 * (ESM_NFAM + 1)], guards);
     }
+}
+
+// ---------------------------------------------------------------------------------------------
+// the moves walked by blocks (esm_sepwalk.cuh, esm_walk.cuh)
+// ---------------------------------------------------------------------------------------------
+// add a block's counts to the class totals
+__device__ __forceinline__ void block_counts(unsigned long long *stats, int fi, unsigned int tried, unsigned int moved,
+                                             unsigned int guards) {
+    for (int o = 16; o > 0; o >>= 1) {
+        tried += __shfl_xor_sync(0xffffffffu, tried, o);
+        moved += __shfl_xor_sync(0xffffffffu, moved, o);
+        guards += __shfl_xor_sync(0xffffffffu, guards, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (tried) atomicAdd(&stats[2 * fi], (unsigned long long)tried);
+        if (moved) atomicAdd(&stats[2 * fi + 1], (unsigned long long)moved);
+        if (guards) atomicAdd(&stats[2 * (ESM_NFAM + 1)], (unsigned long long)guards);
+    }
+}
+// the warp at which a block's scans start: the blocks of an SM take different ones (by the warp slots
+// they sit in), so that their FP64 instructions go to different schedulers' units
+__device__ __forceinline__ int scan_warp(int *slot) {
+    if (threadIdx.x == 0) {
+        unsigned w;
+        asm volatile("mov.u32 %0, %%warpid;" : "=r"(w));
+        *slot = (int)(w / ESM_SEP_WARPS);
+    }
+    __syncthreads();
+    int r = *slot;
+    __syncthreads();
+    return r;
+}
+
+// Move mi of the class for every (step, replica) task when sep_run (a separable move of at least sepmin
+// units; sepmin 0: none) or walk_run walks it (else nothing: k_move does).
+template <class real>
+__global__ void __launch_bounds__(32 * ESM_SEP_WARPS, 4)
+    k_move_blocks(const __grid_constant__ DevModel<real> M, const int *steps, int nsteps, const uint32_t *sweep_p,
+                  int mi, const char *descs, size_t stride, int sepmin, int region, int walk_region, char *tmp,
+                  int tmp_warp, real *scratch, size_t scratch_per_warp, unsigned long long *stats,
+                  unsigned int *next_item) {
+    extern __shared__ __align__(16) char smem[];
+    __shared__ SepBlock<real> B;
+    __shared__ WalkLayout sW;
+    const Desc<real> d = carve_desc<real>((char *)(descs + (size_t)mi * stride), M, M.natoms + M.nextra);
+    const int ntask = nsteps * M.R, wib = threadIdx.x >> 5;
+    unsigned int tried = 0, moved = 0, guards = 0;
+    if (sep_move<real>(d, sepmin)) {
+        sep_run<real>(M, d, B, smem, region, (ntask + gridDim.x - 1) / gridDim.x, scan_warp(&B.batch),
+                      tmp + ((size_t)blockIdx.x * ESM_SEP_WARPS + wib) * tmp_warp, steps, nsteps, *sweep_p, mi, ntask,
+                      tried, moved, guards, [&](int n) { return (int)atomicAdd(next_item, 1u) * n; });
+    } else {
+        WalkLayout w;
+        if (!walk_move<real>(d, walk_region, &w)) return;  // (grid-uniform)
+        if (threadIdx.x == 0) sW = w;
+        __syncthreads();
+        walk_run<real>(M, d, sW, smem, walk_region,
+                       scratch + ((size_t)blockIdx.x * ESM_WALK_WARPS + wib) * scratch_per_warp, steps, nsteps, *sweep_p,
+                       mi, ntask, tried, moved, guards, [&](int) { return (int)atomicAdd(next_item, 1u) * 16; });
+    }
+    block_counts(stats, d.hdr[12], tried, moved, guards);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1925,9 +1986,9 @@ int linemove_blocks_per_sm(const DevModel<real> &M, int wpb) {
     return nb * wpb;
 }
 
-// The block walk of the separable moves (k_move_sep): the shared memory of its batches (0: a task of
-// the largest move would not fit, k_move walks every move), the buffer of its long sorts per warp and the
-// resident blocks of the device's nsm multiprocessors. 50 KB a block: four per SM.
+// The walk of the separable moves (sep_run): the shared memory of its batches (0: a task of the largest
+// move would not fit, and the one-lane walk takes them) and the buffer of its long sorts per warp. 50 KB a
+// block: four per SM.
 template <class real>
 int sep_region_bytes(const DevModel<real> &M) {
     int need = sep_unit_bytes<real>(M.maxstu) + 2 * sep_list_bytes<real>(M.maxstu, M.maxpts, SEP_SOLE);
@@ -1939,29 +2000,22 @@ int sep_tmp_bytes(const DevModel<real> &M) {
     int n = sep_events(M.maxstu, M.maxpts, SEP_BATCH);
     return n > sep_regs<real>() ? ((int)sizeof(double) * n + 15) & ~15 : 0;
 }
+// The walks of the other moves take 48 KB a block; 0 where their points would need scratch slabs that the
+// model has not.
 template <class real>
-int sep_blocks(const DevModel<real> &M, int nsm) {
-    int region = sep_region_bytes(M), nb = 0;
-    if (region == 0) return 0;
-    cudaFuncSetAttribute(k_move_sep<real>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_move_sep<real>, 32 * ESM_SEP_WARPS, region);
-    if (e != cudaSuccess || nb < 1) nb = 1;
-    return nsm * nb;
+int walk_region_bytes(const DevModel<real> &M) {
+    return M.maxpts > ESM_WALK_PTS && linemove_scratch_reals(M) == 0 ? 0 : 48 * 1024;
 }
-
-// The walk of the other moves (k_move_walk): 48 KB of shared memory a block, four blocks per SM, no more
-// than the scratch has warps for (max_warps) where the points need it.
+// Resident blocks of k_move_blocks on nsm multiprocessors, no more than the scratch has warps for
+// (max_warps) where points go there.
 template <class real>
-int walk_blocks(const DevModel<real> &M, int nsm, int region, int max_warps) {
+int move_blocks(const DevModel<real> &M, int nsm, int smem, int max_warps) {
     int nb = 0;
-    cudaFuncSetAttribute(k_move_walk<real>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_move_walk<real>, 32 * ESM_WALK_WARPS, region);
+    cudaFuncSetAttribute(k_move_blocks<real>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_move_blocks<real>, 32 * ESM_SEP_WARPS, smem);
     if (e != cudaSuccess || nb < 1) nb = 1;
     nb *= nsm;
-    if (M.maxpts > ESM_WALK_PTS) {  // points in the scratch slabs, where there are such
-        if (linemove_scratch_reals(M) == 0) return 0;
-        if (nb * ESM_WALK_WARPS > max_warps) nb = max_warps / ESM_WALK_WARPS;
-    }
+    if (M.maxpts > ESM_WALK_PTS && nb * ESM_WALK_WARPS > max_warps) nb = max_warps / ESM_WALK_WARPS;
     return nb;
 }
 
@@ -1997,11 +2051,9 @@ cudaError_t launch_class_pass(const DevModel<real> &M, const int *steps, int nst
         return cudaGetLastError();
     }
     // (min_units 0: every separable move goes to the block walk)
-    int sepmin = sep.blocks > 0 ? (sep.min_units > 0 ? sep.min_units : 1) : 0;
+    int sepmin = sep.region > 0 ? (sep.min_units > 0 ? sep.min_units : 1) : 0;
     int ntask = nsteps * M.R;
-    int sblocks = ntask < sep.blocks ? ntask : sep.blocks;
-    int wblocks = (ntask + 15) / 16;
-    if (wblocks > sep.walk_blocks) wblocks = sep.walk_blocks;
+    int bblocks = ntask < sep.blocks ? ntask : sep.blocks;
     for (int mi = 0; mi < nrun; ++mi) {
         if (wpb == 4)
             k_move<real, 4><<<blocks, 128, stride, s>>>(M, steps, nsteps, ntile, wpt, sweep, mi, descs, stride, scratch,
@@ -2013,16 +2065,10 @@ cudaError_t launch_class_pass(const DevModel<real> &M, const int *steps, int nst
             k_move<real, 1><<<blocks, 32, stride, s>>>(M, steps, nsteps, ntile, wpt, sweep, mi, descs, stride, scratch,
                                                       stats, counters + mi, sepmin, sep.walk_region);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        if (sep.walk_region > 0 && wblocks > 0) {
-            k_move_walk<real><<<wblocks, 32 * ESM_WALK_WARPS, sep.walk_region, s>>>(
-                M, steps, nsteps, sweep, mi, descs, stride, sepmin, sep.walk_region, scratch,
-                linemove_scratch_reals(M), stats, counters + mi);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        }
-        if (sepmin > 0 && sblocks > 0) {
-            k_move_sep<real><<<sblocks, 32 * ESM_SEP_WARPS, sep.region, s>>>(M, steps, nsteps, sweep, mi, descs, stride,
-                                                                            sepmin, sep.region, sep.tmp,
-                                                                            sep.tmp_warp, stats, counters + mi);
+        if (sep.blocks > 0) {
+            k_move_blocks<real><<<bblocks, 32 * ESM_SEP_WARPS, sep.smem, s>>>(
+                M, steps, nsteps, sweep, mi, descs, stride, sepmin, sep.region, sep.walk_region, sep.tmp, sep.tmp_warp,
+                scratch, linemove_scratch_reals(M), stats, counters + mi);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
     }
@@ -2032,13 +2078,14 @@ cudaError_t launch_class_pass(const DevModel<real> &M, const int *steps, int nst
 // ---------------------------------------------------------------------------------------------
 // a batch of models
 // ---------------------------------------------------------------------------------------------
+#define ESM_CHUNK 64  // tasks that a block of k_move_blocks_batch takes at a time
 // Pass p of every model of a batch: block b builds the descriptors of the class that model b runs
 // in pass p of the sweep (its own class order, class_order_of), exactly as k_prep_moves does for
 // the model alone; block 0 also writes every model's class of the pass and the pass's item prefix
 // over the models (items: the model's tiles of its class x the warps of a tile).
 template <class real>
 __global__ void __launch_bounds__(32) k_prep_batch(const BatchModel<real> *bm, int nm, const uint32_t *sweep_p, int p,
-                                                   int *pass_cls, unsigned int *off) {
+                                                   int *pass_cls, unsigned int *off, unsigned int *choff) {
     extern __shared__ __align__(16) char smem[];
     __shared__ Desc<real> sd;
     int b = blockIdx.x, lane = threadIdx.x;
@@ -2047,8 +2094,9 @@ __global__ void __launch_bounds__(32) k_prep_batch(const BatchModel<real> *bm, i
     int order[3], ncls;
     class_order_of(B.M.seed, B.M.T, sweep, order, &ncls);
     if (b == 0 && lane == 0) {
-        unsigned int acc = 0;
+        unsigned int acc = 0, chunks = 0;
         off[0] = 0;
+        choff[0] = 0;
         for (int q = 0; q < nm; ++q) {
             const BatchModel<real> &Q = bm[q];
             int oq[3], nq;
@@ -2059,8 +2107,10 @@ __global__ void __launch_bounds__(32) k_prep_batch(const BatchModel<real> *bm, i
                 int ntile = (Q.nsteps[c] + Q.M.span - 1) / Q.M.span;
                 int wpt = (Q.M.span * Q.M.R + 31) / 32;
                 acc += (unsigned int)(ntile * wpt);
+                chunks += (unsigned int)((Q.nsteps[c] * Q.M.R + ESM_CHUNK - 1) / ESM_CHUNK);
             }
             off[q + 1] = acc;
+            choff[q + 1] = chunks;
         }
     }
     if (p >= ncls || B.nsteps[order[p]] == 0) return;
@@ -2075,6 +2125,85 @@ __global__ void __launch_bounds__(32) k_prep_batch(const BatchModel<real> *bm, i
 // adding its counts so far to the previous model's statistics. Each task then runs exactly the
 // arithmetic of k_move (move_task), so a model's state after a batch pass is the state its own
 // class pass gives. The cooperative walk of separable moves is not used in a batch.
+// Move mi of the current pass for the models whose move sep_run or walk_run walks: blocks take chunks of
+// ESM_CHUNK tasks of one model from the launch's counter (choff: the chunk prefix over the models).
+template <class real>
+__global__ void __launch_bounds__(32 * ESM_SEP_WARPS, 4)
+    k_move_blocks_batch(const BatchModel<real> *bm, int nact, const int *pass_cls, const unsigned int *choff,
+                        const uint32_t *sweep_p, int mi, int region, char *tmp, int tmp_warp, real *scratch,
+                        size_t scratch_per_warp, unsigned int *next_chunk) {
+    extern __shared__ __align__(16) char smem[];
+    __shared__ SepBlock<real> B;
+    __shared__ DevModel<real> M;
+    __shared__ WalkLayout sW;
+    __shared__ unsigned int sit;
+    const int wib = threadIdx.x >> 5;
+    const int rot = scan_warp(&B.batch);
+    const uint32_t sweep = *sweep_p;
+    const unsigned int total = choff[nact];
+    tmp += ((size_t)blockIdx.x * ESM_SEP_WARPS + wib) * tmp_warp;
+    scratch += ((size_t)blockIdx.x * ESM_WALK_WARPS + wib) * scratch_per_warp;
+    int cur = -1, fi = -1, nsteps = 0;
+    const int *steps = nullptr;
+    unsigned int tried = 0, moved = 0, guards = 0;
+    while (true) {
+        __syncthreads();
+        if (threadIdx.x == 0) sit = atomicAdd(next_chunk, 1u);
+        __syncthreads();
+        const unsigned int it = sit;
+        const bool done = it >= total;
+        int b = cur;
+        if (!done) {  // the last model whose prefix is <= it
+            int lo = 0, hi = nact - 1;
+            while (lo < hi) {
+                int mid = (lo + hi + 1) >> 1;
+                if (choff[mid] <= it)
+                    lo = mid;
+                else
+                    hi = mid - 1;
+            }
+            b = lo;
+        }
+        if (done || b != cur) {  // block-uniform
+            if (cur >= 0 && fi >= 0) block_counts(bm[cur].stats, fi, tried, moved, guards);
+            tried = moved = guards = 0;
+            if (done) break;
+            const unsigned int *src = (const unsigned int *)&bm[b].M;
+            for (int i = threadIdx.x; i < (int)(sizeof(DevModel<real>) / 4); i += blockDim.x) ((unsigned int *)&M)[i] = src[i];
+            cur = b;
+            int cls = pass_cls[b];
+            nsteps = cls >= 0 ? bm[b].nsteps[cls] : 0;
+            steps = cls >= 0 ? bm[b].steps[cls] : nullptr;
+            __syncthreads();
+        }
+        const Desc<real> d = carve_desc<real>(bm[b].descs + (size_t)mi * bm[b].stride, M, bm[b].nmoves);
+        fi = d.hdr[12];
+        const int t0 = (int)(it - choff[b]) * ESM_CHUNK;
+        const int end = min(nsteps * M.R, t0 + ESM_CHUNK);
+        if (sep_move<real>(d, bm[b].sep_on)) {
+            int at = t0;
+            sep_run<real>(M, d, B, smem, region, ESM_CHUNK, rot, tmp, steps, nsteps, sweep, mi, end, tried, moved, guards,
+                          [&](int n) {
+                              int x = at;
+                              at += n;
+                              return x;
+                          });
+        } else {
+            WalkLayout w;
+            if (!walk_move<real>(d, bm[b].walk_region, &w)) continue;  // (block-uniform)
+            if (threadIdx.x == 0) sW = w;
+            __syncthreads();
+            int at = t0 + 16 * wib;
+            walk_run<real>(M, d, sW, smem, bm[b].walk_region, scratch, steps, nsteps, sweep, mi, end, tried, moved, guards,
+                           [&](int n) {
+                               int x = at;
+                               at += 16 * n;
+                               return x;
+                           });
+        }
+    }
+}
+
 template <class real, int WPB>
 __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
     k_move_batch(const BatchModel<real> *bm, int nact, const int *pass_cls, const unsigned int *off,
@@ -2132,6 +2261,8 @@ __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
             __syncwarp();
             cur = b;
             fi = sd[wib].hdr[12];
+            WalkLayout w;  // (k_move_blocks_batch's moves: nothing to do)
+            if (fi >= 0 && (sep_move<real>(sd[wib], bm[b].sep_on) || walk_move<real>(sd[wib], bm[b].walk_region, &w))) fi = -1;
             cls = pass_cls[b];
             nsteps = cls >= 0 ? bm[b].nsteps[cls] : 0;
             steps = cls >= 0 ? bm[b].steps[cls] : nullptr;
@@ -2158,6 +2289,15 @@ __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
     }
 }
 
+// resident blocks of k_move_blocks_batch per SM with `region` bytes of shared memory
+template <class real>
+int batch_blocks_per_sm(int region) {
+    int nb = 0;
+    cudaFuncSetAttribute(k_move_blocks_batch<real>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_move_blocks_batch<real>, 32 * ESM_SEP_WARPS, region);
+    return e != cudaSuccess || nb < 1 ? 1 : nb;
+}
+
 template <class real>
 int batch_warps_per_sm(int wpb) {
     int nb = 0;
@@ -2174,13 +2314,14 @@ int batch_warps_per_sm(int wpb) {
 template <class real>
 cudaError_t launch_batch_passes(const BatchModel<real> *bm, const BatchLaunch &bl, const uint32_t *sweep,
                                 cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(bl.counters, 0, sizeof(unsigned int) * bl.maxpass * bl.maxmoves, s);
+    cudaError_t e = cudaMemsetAsync(bl.counters, 0, sizeof(unsigned int) * 2 * bl.maxpass * bl.maxmoves, s);
     if (e != cudaSuccess) return e;
     int blocks = (bl.warps + bl.wpb - 1) / bl.wpb;
     for (int p = 0; p < bl.npass; ++p) {
         int *pc = bl.pass_cls + (size_t)p * bl.nm;
         unsigned int *off = bl.off + (size_t)p * (bl.nm + 1);
-        k_prep_batch<real><<<bl.nm, 32, bl.prep_smem, s>>>(bm, bl.nm, sweep, p, pc, off);
+        unsigned int *choff = bl.choff + (size_t)p * (bl.nm + 1);
+        k_prep_batch<real><<<bl.nm, 32, bl.prep_smem, s>>>(bm, bl.nm, sweep, p, pc, off, choff);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         for (int mi = 0; mi < bl.nmove; ++mi) {
             unsigned int *ctr = bl.counters + (size_t)p * bl.maxmoves + mi;
@@ -2191,6 +2332,12 @@ cudaError_t launch_batch_passes(const BatchModel<real> *bm, const BatchLaunch &b
                 k_move_batch<real, 1><<<blocks, 32, 0, s>>>(bm, bl.nact[mi], pc, off, sweep, mi, (real *)bl.scratch,
                                                            bl.scratch_per_warp, ctr);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            if (bl.bblocks > 0) {
+                k_move_blocks_batch<real><<<bl.bblocks, 32 * ESM_SEP_WARPS, bl.region, s>>>(
+                    bm, bl.nact[mi], pc, choff, sweep, mi, bl.region, bl.tmp, bl.tmp_warp, (real *)bl.scratch,
+                    bl.scratch_per_warp, ctr + (size_t)bl.maxpass * bl.maxmoves);
+                if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            }
         }
     }
     return cudaSuccess;

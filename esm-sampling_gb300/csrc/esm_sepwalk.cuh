@@ -1034,7 +1034,7 @@ struct SepWalk {
     }
 };
 
-// Whether move descriptor d is separable with at least sepmin units (the moves of k_move_sep).
+// Whether move descriptor d is separable with at least sepmin units (the moves of sep_run).
 template <class real>
 __device__ inline bool sep_move(const Desc<real> &d, int sepmin) {
     const int *h = d.hdr;
@@ -1043,23 +1043,18 @@ __device__ inline bool sep_move(const Desc<real> &d, int sepmin) {
     return sepmin > 0 && h[12] >= 0 && sep && h[1] >= sepmin;
 }
 
-// Move mi of the class for every (step, replica) task when it is a separable move with at least
-// sepmin units (else nothing: k_move runs it). A block takes batches of tasks from the per-move
-// counter: as many as its shared memory (region bytes) holds lists for, but no more than share the
-// tasks over the grid. A task whose walk passes every clamp, or whose draw needs the round-off scales
-// of its points, runs again, alone, with room for both. tmp: tmp_warp bytes a warp (sort_mem).
-template <class real>
-__global__ void __launch_bounds__(32 * ESM_SEP_WARPS, 4)
-    k_move_sep(const __grid_constant__ DevModel<real> M, const int *steps, int nsteps, const uint32_t *sweep_p, int mi,
-               const char *descs, size_t stride, int sepmin, int region, char *tmp, int tmp_warp,
-               unsigned long long *stats, unsigned int *next_item) {
-    extern __shared__ __align__(16) char smem[];
-    __shared__ SepBlock<real> B;
-    const Desc<real> d = carve_desc<real>((char *)(descs + (size_t)mi * stride), M, M.natoms + M.nextra);
-    if (!sep_move<real>(d, sepmin)) return;  // grid-uniform
+// The walks of separable move mi of one model over a block's tasks, in batches of as many as its shared
+// memory (region bytes at smem) holds lists for, but no more than `share`; next(n), called by thread 0,
+// gives the first task of a batch of n (none from `end` on). A task whose walk passes every clamp, or
+// whose draw needs the round-off scales of its points, runs again, alone, with room for both. rot: the
+// warp that the scans start at; tmp: the warp's buffer for long sorts.
+template <class real, class Next>
+__device__ __forceinline__ void sep_run(const DevModel<real> &M, const Desc<real> &d, SepBlock<real> &B, char *smem,
+                                        int region, int share, int rot, char *tmp, const int *steps, int nsteps,
+                                        uint32_t sweep, int mi, int end, unsigned int &tried, unsigned int &moved,
+                                        unsigned int &guards, Next next) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int nu = d.hdr[1], T = M.T;
-    const int ntask = nsteps * M.R;
     SepUnits<real> U(smem, nu);
     for (int q = threadIdx.x; q < nu; q += 32 * ESM_SEP_WARPS) {
         int j = d.si[q];
@@ -1076,24 +1071,12 @@ __global__ void __launch_bounds__(32 * ESM_SEP_WARPS, 4)
     const int ub = sep_unit_bytes<real>(nu);
     // tasks of a batch: nw warps of nt tasks (a power of two)
     int fit = (region - ub) / (2 * sep_list_bytes<real>(nu, M.maxpts, sep_kind(nu, false)));
-    int share = (ntask + gridDim.x - 1) / gridDim.x;
     if (fit > share) fit = share;
     const int nw_batch = fit < ESM_SEP_WARPS ? fit : ESM_SEP_WARPS;
     int nt_batch = 1;
     while (nt_batch < 16 && 2 * nt_batch * ESM_SEP_WARPS <= fit) nt_batch <<= 1;
-    tmp += ((size_t)blockIdx.x * ESM_SEP_WARPS + wib) * tmp_warp;
-    const uint32_t sweep = *sweep_p;
-    unsigned int tried = 0, moved = 0, guards = 0;
-    // the list of this thread's scan: the blocks of an SM start at different warps (by the warp slots
-    // they sit in), so that their FP64 instructions go to different schedulers' units
-    if (threadIdx.x == 0) {
-        unsigned w;
-        asm volatile("mov.u32 %0, %%warpid;" : "=r"(w));
-        B.nalone = 0;
-        B.batch = (int)(w / ESM_SEP_WARPS);
-    }
-    __syncthreads();
-    const int sl = (threadIdx.x + 32 * B.batch) & (32 * ESM_SEP_WARPS - 1);
+    const int sl = (threadIdx.x + 32 * rot) & (32 * ESM_SEP_WARPS - 1);  // the list of this thread's scan
+    if (threadIdx.x == 0) B.nalone = 0;
     while (true) {
         __syncthreads();
         const bool alone = B.nalone > 0;
@@ -1102,12 +1085,12 @@ __global__ void __launch_bounds__(32 * ESM_SEP_WARPS, 4)
             if (alone)
                 B.batch = B.alone[--B.nalone];
             else
-                B.batch = (int)atomicAdd(next_item, 1u);
+                B.batch = next(nw_batch * nt_batch);
         }
         __syncthreads();
         const int nw = alone ? 1 : nw_batch, nt = alone ? 1 : nt_batch;
         const int tb = nw * nt;  // tasks of the batch
-        const int task0 = alone ? B.batch : B.batch * tb;
+        const int task0 = B.batch, ntask = alone ? task0 + 1 : end;
         if (task0 >= ntask) break;
         const int kind = sep_kind(nu, alone);
         const bool full = kind != SEP_BATCH;
@@ -1223,17 +1206,6 @@ __global__ void __launch_bounds__(32 * ESM_SEP_WARPS, 4)
                 }
             }
         }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        tried += __shfl_xor_sync(0xffffffffu, tried, o);
-        moved += __shfl_xor_sync(0xffffffffu, moved, o);
-        guards += __shfl_xor_sync(0xffffffffu, guards, o);
-    }
-    if (lane == 0) {
-        int fi = ESM_NFAM;  // atoms
-        if (tried) atomicAdd(&stats[2 * fi], (unsigned long long)tried);
-        if (moved) atomicAdd(&stats[2 * fi + 1], (unsigned long long)moved);
-        if (guards) atomicAdd(&stats[2 * (ESM_NFAM + 1)], (unsigned long long)guards);
     }
 }
 

@@ -463,26 +463,14 @@ __device__ inline bool walk_move(const Desc<real> &d, int region, WalkLayout *w)
     return walk_const_bytes<real>(*w) + walk_warp_bytes<real>(*w) <= region;
 }
 
-// Move mi of the class for every (step, replica) task when its walk is this file's (else nothing). A
-// warp takes items of 16 tasks from the per-move counter; the block runs as many warps as its shared
-// memory (region bytes) holds.
-template <class real>
-__global__ void __launch_bounds__(32 * ESM_WALK_WARPS, 4)
-    k_move_walk(const __grid_constant__ DevModel<real> M, const int *steps, int nsteps, const uint32_t *sweep_p, int mi,
-                const char *descs, size_t stride, int sepmin, int region, real *scratch, size_t scratch_per_warp,
-                unsigned long long *stats, unsigned int *next_item) {
-    extern __shared__ __align__(16) char smem[];
-    __shared__ WalkLayout sW;
-    const Desc<real> d = carve_desc<real>((char *)(descs + (size_t)mi * stride), M, M.natoms + M.nextra);
-    if (sep_move<real>(d, sepmin)) return;  // k_move_sep's (grid-uniform)
-    {
-        WalkLayout w;
-        if (!walk_move<real>(d, region, &w)) return;  // k_move's (grid-uniform)
-        if (threadIdx.x == 0) sW = w;
-    }
-    __syncthreads();
-    const WalkLayout &W = sW;
-    const int fi = d.hdr[12];
+// The walks of move mi of one model by the warps of a block, as many as its shared memory (region bytes
+// at smem) holds; next(n), called by lane 0 of each of the n warps, gives the first of its next 16 tasks (none from `end`
+// on). scratch: the warp's slab for the points where the cap exceeds the local arrays.
+template <class real, class Next>
+__device__ __forceinline__ void walk_run(const DevModel<real> &M, const Desc<real> &d, const WalkLayout &W, char *smem,
+                                         int region, real *scratch, const int *steps, int nsteps, uint32_t sweep, int mi,
+                                         int end, unsigned int &tried, unsigned int &moved, unsigned int &guards,
+                                         Next next) {
     real *K = (real *)smem;
     const int n = W.ng + W.nga;
     for (int q = threadIdx.x; q < n; q += blockDim.x) {
@@ -504,26 +492,25 @@ __global__ void __launch_bounds__(32 * ESM_WALK_WARPS, 4)
     __syncthreads();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int cb = walk_const_bytes<real>(W), wb = walk_warp_bytes<real>(W);
-    if (wib >= (region - cb) / wb) return;
+    const int nw = (region - cb) / wb;
+    if (wib >= nw) return;
     real *tv = (real *)(smem + cb + (size_t)wib * wb), *lv = tv + 16 * W.task;
     tv += lane >> 1;
     lv += lane;
     real local[4 * ESM_WALK_PTS];
     const bool loc = M.maxpts <= ESM_WALK_PTS;
-    real *pts = loc ? local : scratch + ((size_t)blockIdx.x * ESM_WALK_WARPS + wib) * scratch_per_warp + lane;
+    real *pts = loc ? local : scratch + lane;
     SepUnit<real> u{};
     LineWalk<real> S{M, W, K, tv, lv, pts, loc ? 1 : 32, loc ? ESM_WALK_PTS : M.maxpts, u};
-    const uint32_t sweep = *sweep_p;
     const bool left = lane & 1;
-    const int T = M.T, ntask = nsteps * M.R, nitems = (ntask + 15) / 16;
-    unsigned int tried = 0, moved = 0, guards = 0;
+    const int T = M.T;
     while (true) {
-        unsigned int it = 0;
-        if (lane == 0) it = atomicAdd(next_item, 1u);
-        int item = (int)__shfl_sync(0xffffffffu, it, 0);
-        if (item >= nitems) break;
-        const int task = item * 16 + (lane >> 1);
-        const bool on = task < ntask;
+        int task0 = 0;
+        if (lane == 0) task0 = next(nw);
+        task0 = __shfl_sync(0xffffffffu, task0, 0);
+        if (task0 >= end) break;
+        const int task = task0 + (lane >> 1);
+        const bool on = task < end;
         int rep = 0, tau = 0, qs = 0;
         if (on) {
             rep = task % M.R;
@@ -599,16 +586,6 @@ __global__ void __launch_bounds__(32 * ESM_WALK_WARPS, 4)
             if (w < 0) ++guards;
             if (t != 0) ++moved;
         }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        tried += __shfl_xor_sync(0xffffffffu, tried, o);
-        moved += __shfl_xor_sync(0xffffffffu, moved, o);
-        guards += __shfl_xor_sync(0xffffffffu, guards, o);
-    }
-    if (lane == 0) {
-        if (tried) atomicAdd(&stats[2 * fi], (unsigned long long)tried);
-        if (moved) atomicAdd(&stats[2 * fi + 1], (unsigned long long)moved);
-        if (guards) atomicAdd(&stats[2 * (ESM_NFAM + 1)], (unsigned long long)guards);
     }
 }
 
