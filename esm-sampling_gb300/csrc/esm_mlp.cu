@@ -132,59 +132,120 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(GemmArgs g) {
             }
 }
 
-// delta of a hidden layer: d_z = d_a * SiLU'(z)
-__global__ void k_silu_back(int n, const float *z, const float *da, float *dz, __nv_bfloat16 *dzb) {
+// element c of a BF16 row of cols elements padded to ld (the deltas' buffer serves layers of different
+// widths, so the pads are written with the row's last element)
+__device__ inline void put_row(__nv_bfloat16 *row, int c, int cols, int ld, float v) {
+    row[c] = __float2bfloat16(v);
+    if (c == cols - 1)
+        for (int p = cols; p < ld; ++p) row[p] = __float2bfloat16(0.f);
+}
+
+// delta of a hidden layer: d_z = d_a * SiLU'(z) (the BF16 copy's rows padded to ld)
+__global__ void k_silu_back(int n, int cols, int ld, const float *z, const float *da, float *dz, __nv_bfloat16 *dzb) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float s = 1.f / (1.f + expf(-z[i]));
     float v = da[i] * (s * (1.f + z[i] * (1.f - s)));
     dz[i] = v;
-    dzb[i] = __float2bfloat16(v);
+    put_row(dzb + (size_t)(i / cols) * ld, i % cols, cols, ld, v);
 }
 
-// output delta of the mean-squared loss: d = (y - t) / B (masked columns beyond d_out are zero);
-// per-row squared error accumulated into loss
-__global__ void k_loss(int B, int dout, const float *y, const float *t, float *d, __nv_bfloat16 *db, double *loss) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B * dout) return;
-    float e = y[i] - t[i];
-    d[i] = e / (float)B;
-    db[i] = __float2bfloat16(e / (float)B);
-    atomicAdd(loss, 0.5 * (double)e * (double)e / (double)B);
-}
-
-// column sums (bias gradient): out[n] = sum_m d[m, n]
-__global__ void k_colsum(int M, int N, const float *d, float *out) {
-    int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    float s = 0.f;
-    for (int m = 0; m < M; ++m) s += d[(long long)m * N + n];
-    out[n] = s;
-}
-
-// Adam (Kingma and Ba 2015) on FP32 master weights; refresh the BF16 copy and its transpose
-__global__ void k_adam(int n, int rows, int cols, float *w, float *m, float *v, const float *g, float lr, float b1,
-                       float b2, float eps, float c1, float c2, __nv_bfloat16 *wb, __nv_bfloat16 *wt) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float gi = g[i];
-    float mi = b1 * m[i] + (1.f - b1) * gi;
-    float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    w[i] = wi;
-    if (wb) wb[i] = __float2bfloat16(wi);
-    if (wt) {
-        int r = i / cols, c = i % cols;
-        wt[(long long)c * rows + r] = __float2bfloat16(wi);
+// output delta of the mean-squared loss: d = (y - t) / B; every block's squared error into part (summed by
+// k_loss_sum; one atomic per element took 2 ms at 1024 x 1357)
+#define LOSS_BLOCKS 304
+__global__ void __launch_bounds__(256) k_loss(int B, int dout, int ldb, const float *y, const float *t, float *d,
+                                              __nv_bfloat16 *db, double *part) {
+    double s = 0;
+    const int n = B * dout;
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+        float e = y[i] - t[i];
+        float v = e / (float)B;
+        d[i] = v;
+        put_row(db + (size_t)(i / dout) * ldb, i % dout, dout, ldb, v);
+        s += 0.5 * (double)e * (double)e / (double)B;
     }
-    (void)rows;
+    __shared__ double ws[8];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < 8; ++i) s += ws[i];
+        part[blockIdx.x] = s;
+    }
+}
+__global__ void __launch_bounds__(32) k_loss_sum(int n, const double *part, double *loss) {
+    double s = 0;
+    for (int i = threadIdx.x; i < n; i += 32) s += part[i];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) *loss = s;
 }
 
-__global__ void k_to_bf16(int n, const float *x, __nv_bfloat16 *y) {
+// column sums (bias gradient): out[n] = sum_m d[m, n]. A block sums 32 columns, thread (x, y) the rows y, y +
+// 32, ..., then the 32 partial sums in order (one thread per column, row after row, took 57 to 71 us at 1024
+// rows).
+__global__ void __launch_bounds__(1024) k_colsum(int M, int N, const float *d, float *out) {
+    __shared__ float ps[32][33];
+    int n = blockIdx.x * 32 + threadIdx.x;
+    float s = 0.f;
+    if (n < N)
+#pragma unroll 4
+        for (int m = threadIdx.y; m < M; m += 32) s += d[(size_t)m * N + n];
+    ps[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.y == 0 && n < N) {
+        float t = 0.f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) t += ps[i][threadIdx.x];
+        out[n] = t;
+    }
+}
+
+// Adam (Kingma and Ba 2015) on FP32 master weights; refresh the BF16 copy and its transpose (rows padded to
+// ldb, ldt), a 32 x 32 tile per block so that both are written along their rows
+__device__ inline float adam_step(float gi, float *w, float *m, float *v, float lr, float b1, float b2, float eps,
+                                  float c1, float c2) {
+    float mi = b1 * *m + (1.f - b1) * gi;
+    float vi = b2 * *v + (1.f - b2) * gi * gi;
+    *m = mi;
+    *v = vi;
+    float wi = *w - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    *w = wi;
+    return wi;
+}
+__global__ void __launch_bounds__(256) k_adam(int rows, int cols, float *w, float *m, float *v, const float *g, float lr,
+                                              float b1, float b2, float eps, float c1, float c2, __nv_bfloat16 *wb,
+                                              int ldb, __nv_bfloat16 *wt, int ldt) {
+    __shared__ __nv_bfloat16 tile[32][33];
+    const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32, x = threadIdx.x, y0 = threadIdx.y;
+#pragma unroll
+    for (int y = y0; y < 32; y += 8) {
+        int r = r0 + y, c = c0 + x;
+        if (r < rows && c < cols) {
+            size_t i = (size_t)r * cols + c;
+            float wi = adam_step(g[i], w + i, m + i, v + i, lr, b1, b2, eps, c1, c2);
+            __nv_bfloat16 h = __float2bfloat16(wi);
+            wb[(size_t)r * ldb + c] = h;
+            tile[y][x] = h;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int y = y0; y < 32; y += 8) {
+        int c = c0 + y, r = r0 + x;
+        if (r < rows && c < cols) wt[(size_t)c * ldt + r] = tile[x][y];
+    }
+}
+// the biases of a layer
+__global__ void k_adam_bias(int n, float *w, float *m, float *v, const float *g, float lr, float b1, float b2, float eps,
+                            float c1, float c2) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) y[i] = __float2bfloat16(x[i]);
+    if (i < n) adam_step(g[i], w + i, m + i, v + i, lr, b1, b2, eps, c1, c2);
+}
+
+// x [rows, cols] to BF16 with rows padded to ld
+__global__ void k_to_bf16(int n, int cols, int ld, const float *x, __nv_bfloat16 *y) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) y[(size_t)(i / cols) * ld + i % cols] = __float2bfloat16(x[i]);
 }
 
 }  // namespace
@@ -201,13 +262,14 @@ struct esm_mlp {
     int64_t launches = 0, steps = 0;
     float lr = 1e-3f, b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     vector<float *> W, b, mW, vW, mb, vb, gW, gb;  // FP32 master, Adam moments, gradients
-    vector<__nv_bfloat16 *> Wb, Wt;               // BF16 copies [out, in] and transposed [in, out]
+    vector<__nv_bfloat16 *> Wb, Wt;               // BF16 copies [out, in] and transposed [in, out]; as every BF16
+                                                  // matrix, rows padded to 8 elements (ld8), pads zero
     vector<float *> Z;                             // pre-activations per layer [B, d_{l+1}]
     vector<__nv_bfloat16 *> Ab;                    // activations BF16 per layer [B, d_l] (Ab[0] = input)
     float *dA = nullptr, *dZ = nullptr, *target = nullptr;
     __nv_bfloat16 *dZb = nullptr;
     float *xin = nullptr;
-    double *loss = nullptr;
+    double *loss = nullptr, *loss_part = nullptr;
     vector<void *> allocs;
     int gemm_kind = 1;                             // 1: tcgen05 (k_gemm_tc), 0: mma.sync (k_gemm_bf16)
     __nv_bfloat16 *tA = nullptr, *tB = nullptr;    // K-major copies of the weight-gradient operands
@@ -215,6 +277,8 @@ struct esm_mlp {
 };
 
 namespace {
+
+inline int ld8(int d) { return (d + 7) & ~7; }
 
 int mfail(esm_mlp *c, int code, const char *fmt, ...) {
     char buf[512];
@@ -269,11 +333,11 @@ int gemm_tc(esm_mlp *c, const GemmArgs &g, const __nv_bfloat16 *A, int lda, cons
     return ESM_OK;
 }
 
-// K-major copy of a BF16 operand given by strides: out[r*ld + k] = X(r, k), X(r, k) at X[r*sr + k*sk]
+// K-major copy of a BF16 operand given by strides: out[r*ld8(K) + k] = X(r, k), X(r, k) at X[r*sr + k*sk]
 // with sr == 1 (the row index fastest: a transpose of the row-major [k, r] matrix)
 int kmajor(esm_mlp *c, const __nv_bfloat16 *X, int rows, int K, long long sk, __nv_bfloat16 *out) {
     dim3 grid((rows + 31) / 32, (K + 31) / 32), block(32, 8);
-    tc::k_transpose_bf16<<<grid, block, 0, c->stream>>>(K, rows, X, (int)sk, out, K);
+    tc::k_transpose_bf16<<<grid, block, 0, c->stream>>>(K, rows, X, (int)sk, out, ld8(K));
     c->launches += 1;
     MK(cudaGetLastError());
     return ESM_OK;
@@ -290,13 +354,13 @@ int gemm(esm_mlp *c, GemmArgs g) {
             if (g.sam != 1) return mfail(c, ESM_EINVAL, "GEMM operand A with neither stride 1");
             if ((rc = kmajor(c, g.A, g.M, g.K, g.sak, c->tA))) return rc;
             A = c->tA;
-            lda = g.K;
+            lda = ld8(g.K);
         }
         if (!bk) {
             if (g.sbn != 1) return mfail(c, ESM_EINVAL, "GEMM operand B with neither stride 1");
             if ((rc = kmajor(c, g.B, g.N, g.K, g.sbk, c->tB))) return rc;
             B = c->tB;
-            ldb = g.K;
+            ldb = ld8(g.K);
         }
         return gemm_tc(c, g, A, lda, B, ldb);
     }
@@ -305,6 +369,14 @@ int gemm(esm_mlp *c, GemmArgs g) {
     c->launches += 1;
     MK(cudaGetLastError());
     return ESM_OK;
+}
+
+// an Adam pass over the weights of layer l
+void adam_weights(esm_mlp *c, int l, float lr, float b1, float b2, float eps, float c1, float c2) {
+    int rows = c->dims[l + 1], cols = c->dims[l];
+    dim3 grid((cols + 31) / 32, (rows + 31) / 32), block(32, 8);
+    k_adam<<<grid, block, 0, c->stream>>>(rows, cols, c->W[l], c->mW[l], c->vW[l], c->gW[l], lr, b1, b2, eps, c1, c2,
+                                          c->Wb[l], ld8(cols), c->Wt[l], ld8(rows));
 }
 
 // a wait of the tensor-core GEMM ran out: the stream's results are not to be used
@@ -327,17 +399,17 @@ int forward(esm_mlp *c, int B) {
         g.N = dout;
         g.K = din;
         g.A = c->Ab[l];
-        g.sam = din;
+        g.sam = ld8(din);
         g.sak = 1;
         g.B = c->Wb[l];  // B(k, n) = W[n, k]
         g.sbk = 1;
-        g.sbn = din;
+        g.sbn = ld8(din);
         g.C = c->Z[l];
         g.ldc = dout;
         g.bias = c->b[l];
         g.silu = hidden ? 1 : 0;
         g.Cb = hidden ? c->Ab[l + 1] : nullptr;
-        g.ldcb = dout;
+        g.ldcb = ld8(dout);
         int rc = gemm(c, g);
         if (rc) return rc;
     }
@@ -381,20 +453,21 @@ int esm_mlp_create(int32_t nlayers, const int32_t *dims, int32_t batch_max, uint
             if ((rc = malloc_(c, p, nw))) return rc;
         for (float **p : {&c->b[l], &c->mb[l], &c->vb[l], &c->gb[l]})
             if ((rc = malloc_(c, p, nb))) return rc;
-        if ((rc = malloc_(c, &c->Wb[l], nw))) return rc;
-        if ((rc = malloc_(c, &c->Wt[l], nw))) return rc;
+        if ((rc = malloc_(c, &c->Wb[l], (size_t)c->dims[l + 1] * ld8(c->dims[l])))) return rc;
+        if ((rc = malloc_(c, &c->Wt[l], (size_t)c->dims[l] * ld8(c->dims[l + 1])))) return rc;
         if ((rc = malloc_(c, &c->Z[l], (size_t)batch_max * c->dims[l + 1]))) return rc;
     }
     for (int l = 0; l <= nlayers; ++l)
-        if ((rc = malloc_(c, &c->Ab[l], (size_t)batch_max * c->dims[l]))) return rc;
+        if ((rc = malloc_(c, &c->Ab[l], (size_t)batch_max * ld8(c->dims[l])))) return rc;
     if ((rc = malloc_(c, &c->dA, (size_t)batch_max * dmax))) return rc;
     if ((rc = malloc_(c, &c->dZ, (size_t)batch_max * dmax))) return rc;
-    if ((rc = malloc_(c, &c->dZb, (size_t)batch_max * dmax))) return rc;
+    if ((rc = malloc_(c, &c->dZb, (size_t)batch_max * ld8(dmax)))) return rc;
     if ((rc = malloc_(c, &c->target, (size_t)batch_max * c->dims[nlayers]))) return rc;
     if ((rc = malloc_(c, &c->xin, (size_t)batch_max * c->dims[0]))) return rc;
     if ((rc = malloc_(c, &c->loss, 1))) return rc;
-    if ((rc = malloc_(c, &c->tA, (size_t)batch_max * dmax))) return rc;
-    if ((rc = malloc_(c, &c->tB, (size_t)batch_max * dmax))) return rc;
+    if ((rc = malloc_(c, &c->loss_part, LOSS_BLOCKS))) return rc;
+    if ((rc = malloc_(c, &c->tA, (size_t)ld8(batch_max) * dmax))) return rc;
+    if ((rc = malloc_(c, &c->tB, (size_t)ld8(batch_max) * dmax))) return rc;
     if ((rc = malloc_(c, &c->tc_err, 1))) return rc;
     MK(cudaFuncSetAttribute(tc::k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
     // He-style initialisation from a fixed LCG stream (host), zero biases
@@ -436,9 +509,7 @@ int esm_mlp_set_layer(esm_mlp *c, int32_t l, const float *w, const float *bias) 
         MK(cudaMemcpyAsync(c->W[l], w, sizeof(float) * nw, cudaMemcpyHostToDevice, c->stream));
         // BF16 copy and transpose through a zero-rate Adam pass (lr 0 leaves the weights unchanged)
         MK(cudaMemsetAsync(c->gW[l], 0, sizeof(float) * nw, c->stream));
-        k_adam<<<(unsigned)((nw + 255) / 256), 256, 0, c->stream>>>((int)nw, rows, cols, c->W[l], c->mW[l], c->vW[l],
-                                                                     c->gW[l], 0.f, 0.f, 0.f, 1.f, 1.f, 1.f,
-                                                                     c->Wb[l], c->Wt[l]);
+        adam_weights(c, l, 0.f, 0.f, 0.f, 1.f, 1.f, 1.f);
         MK(cudaGetLastError());
         c->launches += 1;
     }
@@ -460,7 +531,7 @@ int esm_mlp_forward(esm_mlp *c, int32_t B, const float *x, float *y) {
     if (!c || !x || B < 1 || B > c->Bmax) return c ? mfail(c, ESM_EINVAL, "batch %d out of range", B) : ESM_EINVAL;
     int din = c->dims[0], dout = c->dims[c->nl];
     MK(cudaMemcpyAsync(c->xin, x, sizeof(float) * B * din, cudaMemcpyHostToDevice, c->stream));
-    k_to_bf16<<<(B * din + 255) / 256, 256, 0, c->stream>>>(B * din, c->xin, c->Ab[0]);
+    k_to_bf16<<<(B * din + 255) / 256, 256, 0, c->stream>>>(B * din, din, ld8(din), c->xin, c->Ab[0]);
     MK(cudaGetLastError());
     c->launches += 1;
     int rc = forward(c, B);
@@ -479,12 +550,14 @@ int esm_mlp_train_step(esm_mlp *c, int32_t B, const float *x, const float *targe
     int nl = c->nl, din = c->dims[0], dout = c->dims[nl];
     MK(cudaMemcpyAsync(c->xin, x, sizeof(float) * B * din, cudaMemcpyHostToDevice, c->stream));
     MK(cudaMemcpyAsync(c->target, target, sizeof(float) * B * dout, cudaMemcpyHostToDevice, c->stream));
-    MK(cudaMemsetAsync(c->loss, 0, sizeof(double), c->stream));
-    k_to_bf16<<<(B * din + 255) / 256, 256, 0, c->stream>>>(B * din, c->xin, c->Ab[0]);
+    k_to_bf16<<<(B * din + 255) / 256, 256, 0, c->stream>>>(B * din, din, ld8(din), c->xin, c->Ab[0]);
     int rc = forward(c, B);
     if (rc) return rc;
-    k_loss<<<(B * dout + 255) / 256, 256, 0, c->stream>>>(B, dout, c->Z[nl - 1], c->target, c->dZ, c->dZb, c->loss);
-    c->launches += 2;
+    int lb = (B * dout + 255) / 256;
+    if (lb > LOSS_BLOCKS) lb = LOSS_BLOCKS;
+    k_loss<<<lb, 256, 0, c->stream>>>(B, dout, ld8(dout), c->Z[nl - 1], c->target, c->dZ, c->dZb, c->loss_part);
+    k_loss_sum<<<1, 32, 0, c->stream>>>(lb, c->loss_part, c->loss);
+    c->launches += 3;
     MK(cudaGetLastError());
     for (int l = nl - 1; l >= 0; --l) {
         int di = c->dims[l], dn = c->dims[l + 1];
@@ -495,14 +568,14 @@ int esm_mlp_train_step(esm_mlp *c, int32_t B, const float *x, const float *targe
         g.K = B;
         g.A = c->dZb;
         g.sam = 1;
-        g.sak = dn;
+        g.sak = ld8(dn);
         g.B = c->Ab[l];
-        g.sbk = di;
+        g.sbk = ld8(di);
         g.sbn = 1;
         g.C = c->gW[l];
         g.ldc = di;
         if ((rc = gemm(c, g))) return rc;
-        k_colsum<<<(dn + 127) / 128, 128, 0, c->stream>>>(B, dn, c->dZ, c->gb[l]);
+        k_colsum<<<(dn + 31) / 32, dim3(32, 32), 0, c->stream>>>(B, dn, c->dZ, c->gb[l]);
         c->launches += 1;
         if (l > 0) {
             // dA[b, k] = sum_n dZ[b, n] W[n, k]
@@ -511,40 +584,39 @@ int esm_mlp_train_step(esm_mlp *c, int32_t B, const float *x, const float *targe
             h.N = di;
             h.K = dn;
             h.A = c->dZb;
-            h.sam = dn;
+            h.sam = ld8(dn);
             h.sak = 1;
             h.B = c->Wt[l];  // B(k=n, n=k): Wt[k, n] = W[n, k]
             h.sbk = 1;
-            h.sbn = dn;
+            h.sbn = ld8(dn);
             h.C = c->dA;
             h.ldc = di;
             if ((rc = gemm(c, h))) return rc;
-            k_silu_back<<<(B * di + 255) / 256, 256, 0, c->stream>>>(B * di, c->Z[l - 1], c->dA, c->dZ, c->dZb);
+            k_silu_back<<<(B * di + 255) / 256, 256, 0, c->stream>>>(B * di, di, ld8(di), c->Z[l - 1], c->dA, c->dZ, c->dZb);
             c->launches += 1;
             MK(cudaGetLastError());
-        }
-        // the deltas of layer l are consumed: dZ now holds the layer below (computed above)
-        if (grads_out) {
-            size_t off = 0;
-            for (int q = 0; q < l; ++q) off += (size_t)c->dims[q] * c->dims[q + 1] + c->dims[q + 1];
-            MK(cudaMemcpyAsync(grads_out + off, c->gW[l], sizeof(float) * dn * di, cudaMemcpyDeviceToHost, c->stream));
-            MK(cudaMemcpyAsync(grads_out + off + (size_t)dn * di, c->gb[l], sizeof(float) * dn, cudaMemcpyDeviceToHost,
-                               c->stream));
         }
     }
     c->steps += 1;
     float c1 = 1.f - powf(c->b1, (float)c->steps), c2 = 1.f - powf(c->b2, (float)c->steps);
     for (int l = 0; l < nl; ++l) {
-        int rows = c->dims[l + 1], cols = c->dims[l];
-        int nw = rows * cols;
-        k_adam<<<(nw + 255) / 256, 256, 0, c->stream>>>(nw, rows, cols, c->W[l], c->mW[l], c->vW[l], c->gW[l], lr,
-                                                         c->b1, c->b2, c->eps, c1, c2, c->Wb[l], c->Wt[l]);
-        k_adam<<<(rows + 255) / 256, 256, 0, c->stream>>>(rows, 1, rows, c->b[l], c->mb[l], c->vb[l], c->gb[l], lr,
-                                                           c->b1, c->b2, c->eps, c1, c2, nullptr, nullptr);
+        int rows = c->dims[l + 1];
+        adam_weights(c, l, lr, c->b1, c->b2, c->eps, c1, c2);
+        k_adam_bias<<<(rows + 255) / 256, 256, 0, c->stream>>>(rows, c->b[l], c->mb[l], c->vb[l], c->gb[l], lr, c->b1,
+                                                               c->b2, c->eps, c1, c2);
         c->launches += 2;
     }
     MK(cudaGetLastError());
     double L = 0;
+    if (grads_out) {  // (a copy to pageable memory waits for the stream: after every launch of the step)
+        size_t off = 0;
+        for (int l = 0; l < nl; ++l) {
+            size_t nw = (size_t)c->dims[l] * c->dims[l + 1], nb = c->dims[l + 1];
+            MK(cudaMemcpyAsync(grads_out + off, c->gW[l], sizeof(float) * nw, cudaMemcpyDeviceToHost, c->stream));
+            MK(cudaMemcpyAsync(grads_out + off + nw, c->gb[l], sizeof(float) * nb, cudaMemcpyDeviceToHost, c->stream));
+            off += nw + nb;
+        }
+    }
     MK(cudaMemcpyAsync(&L, c->loss, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     MK(cudaStreamSynchronize(c->stream));
     if (loss_out) *loss_out = L;

@@ -4,12 +4,14 @@
 // One CTA of 4 warps per 128 x 64 tile of C. Operands are staged through shared memory in the
 // canonical no-swizzle K-major layout of tcgen05 (core matrices of 8 rows x 16 bytes; along K the
 // core matrices of a row group are 128 bytes apart (the leading-dimension offset), row groups 1024
-// bytes apart (the stride-dimension offset)), two stages deep: while the tensor core multiplies
-// stage s, the threads load stage s + 1 from global memory into registers. One elected thread issues
-// tcgen05.mma (M = 128, N = 64, K = 16, kind::f16, BF16 x BF16 -> FP32) and commits each stage to an
-// mbarrier that releases the stage's shared memory. The epilogue reads the accumulator with
-// tcgen05.ld (32 lanes x 32 bits, each warp its 32 rows), adds the bias, applies SiLU and writes
-// FP32 and BF16 outputs. Every mbarrier wait is bounded: on time-out the kernel sets *err, frees its
+// bytes apart (the stride-dimension offset)) by 16-byte asynchronous copies, TC_STAGES deep: three tiles
+// are on their way while the tensor core multiplies one. (With one tile ahead, through registers, every
+// 64 columns of K waited for memory: 1024 x 1024 x 1024 took 75 us.) Rows are padded to 8 elements, so
+// every copy is aligned, and the pads are zero. One elected thread issues tcgen05.mma (M = 128, N = 64,
+// K = 16, kind::f16, BF16 x BF16 -> FP32) and commits each stage to an mbarrier that releases the
+// stage's shared memory. The epilogue reads the accumulator with tcgen05.ld (32 lanes x 32 bits, each
+// warp its 32 rows), adds the bias, applies SiLU and writes FP32 and BF16 outputs, 16 bytes at a time
+// where the rows allow. Every mbarrier wait is bounded: on time-out the kernel sets *err, frees its
 // tensor memory and returns.
 #pragma once
 #include <cuda_bf16.h>
@@ -23,14 +25,15 @@ namespace tc {
 #define TC_BK 64
 #define TC_STAGE_A (TC_BM * TC_BK * 2)  // bytes of one A stage
 #define TC_STAGE_B (TC_BN * TC_BK * 2)
-#define TC_SMEM (2 * (TC_STAGE_A + TC_STAGE_B) + 1024)
+#define TC_STAGES 4
+#define TC_SMEM (TC_STAGES * (TC_STAGE_A + TC_STAGE_B) + 1024)
 #define TC_WAIT_LIMIT (1 << 24)
 
 struct GemmTC {
     int M, N, K;
-    const __nv_bfloat16 *A;  // A(m, k) at A[m*lda + k]
-    int lda;
-    const __nv_bfloat16 *B;  // B(n, k) at B[n*ldb + k]
+    const __nv_bfloat16 *A;  // A(m, k) at A[m*lda + k]; 16-byte aligned, lda a multiple of 8, zeros from K to
+    int lda;                 // the next multiple of 8
+    const __nv_bfloat16 *B;  // B(n, k) at B[n*ldb + k], likewise
     int ldb;
     float *C;  // C(m, n) at C[m*ldc + n] (may be null)
     int ldc;
@@ -77,24 +80,18 @@ __device__ inline bool mbar_wait(uint32_t bar, uint32_t parity) {
 // offset in the canonical layout
 __device__ inline uint32_t tile_off(int row, int kc) { return (uint32_t)((row >> 3) * 1024 + kc * 128 + (row & 7) * 16); }
 
-__device__ inline uint4 load_chunk(const __nv_bfloat16 *X, int ld, int rows, int K, int r, int k) {
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (r >= rows || k >= K) return v;
-    const __nv_bfloat16 *p = X + (size_t)r * ld + k;
-    if (k + 8 <= K && ((ld & 7) == 0) && ((((uintptr_t)p) & 15) == 0)) return *(const uint4 *)p;
-    __nv_bfloat16 t[8];
-    for (int i = 0; i < 8; ++i) t[i] = (k + i < K) ? p[i] : __float2bfloat16(0.f);
-    return *(const uint4 *)t;
+// 16 bytes from global to shared memory, zeros when not `valid`
+__device__ inline void copy_chunk(uint32_t dst, const void *src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 
 __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTC g) {
     extern __shared__ uint8_t smraw[];
-    __shared__ __align__(8) uint64_t mbar[2];
+    __shared__ __align__(8) uint64_t mbar[TC_STAGES];
     __shared__ uint32_t tmem_s;
     __shared__ int bad_s;
     uint8_t *sm = (uint8_t *)(((uintptr_t)smraw + 1023) & ~(uintptr_t)1023);
-    uint8_t *sA[2] = {sm, sm + TC_STAGE_A};
-    uint8_t *sB[2] = {sm + 2 * TC_STAGE_A, sm + 2 * TC_STAGE_A + TC_STAGE_B};
+    const uint32_t sA = smem_u32(sm), sB = sA + TC_STAGES * TC_STAGE_A;
     int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int m0 = blockIdx.y * TC_BM, n0 = blockIdx.x * TC_BN;
     if (warp == 0) {
@@ -105,8 +102,8 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTC g) {
     }
     if (tid == 0) {
         bad_s = 0;
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[0])) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[1])) : "memory");
+        for (int s = 0; s < TC_STAGES; ++s)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[s])) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -115,50 +112,40 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTC g) {
     uint32_t tmem = tmem_s;
     const uint32_t idesc = idesc_bf16(TC_BM, TC_BN);
     int nk = (g.K + TC_BK - 1) / TC_BK;
-    uint32_t phase[2] = {0, 0};
-    uint4 ra[8], rb[4];
-    auto fetch = [&](int t) {  // tile t into registers: A 1024 chunks, B 512 chunks over 128 threads
-        int k0 = t * TC_BK;
+    auto load = [&](int t) {  // tile t into its stage: A 1024 chunks, B 512 chunks over 128 threads
+        const int s = t % TC_STAGES, k0 = t * TC_BK;
+#pragma unroll
         for (int i = 0; i < 8; ++i) {
-            int c = tid + i * 128, r = c >> 3, kc = c & 7;
-            ra[i] = load_chunk(g.A, g.lda, g.M, g.K, m0 + r, k0 + kc * 8);
+            int c = tid + i * 128, r = m0 + (c >> 3), k = k0 + (c & 7) * 8;
+            bool v = r < g.M && k < g.K;
+            copy_chunk(sA + s * TC_STAGE_A + tile_off(c >> 3, c & 7), v ? g.A + (size_t)r * g.lda + k : g.A, v);
         }
+#pragma unroll
         for (int i = 0; i < 4; ++i) {
-            int c = tid + i * 128, r = c >> 3, kc = c & 7;
-            rb[i] = load_chunk(g.B, g.ldb, g.N, g.K, n0 + r, k0 + kc * 8);
+            int c = tid + i * 128, r = n0 + (c >> 3), k = k0 + (c & 7) * 8;
+            bool v = r < g.N && k < g.K;
+            copy_chunk(sB + s * TC_STAGE_B + tile_off(c >> 3, c & 7), v ? g.B + (size_t)r * g.ldb + k : g.B, v);
         }
-    };
-    auto store = [&](int s) {
-        for (int i = 0; i < 8; ++i) {
-            int c = tid + i * 128, r = c >> 3, kc = c & 7;
-            *(uint4 *)(sA[s] + tile_off(r, kc)) = ra[i];
-        }
-        for (int i = 0; i < 4; ++i) {
-            int c = tid + i * 128, r = c >> 3, kc = c & 7;
-            *(uint4 *)(sB[s] + tile_off(r, kc)) = rb[i];
-        }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     };
     bool ok = true;
-    if (nk > 0) fetch(0);
-    for (int t = 0; t < nk && ok; ++t) {
-        int s = t & 1;
-        if (t >= 2) {  // the stage's previous multiplications (tile t - 2) must have read it
-            if (!mbar_wait(smem_u32(&mbar[s]), phase[s])) ok = false;
-            phase[s] ^= 1;
-        }
+    // (a group is committed for every tile of the loop, empty ones too, so that the count stands for tiles)
+    for (int t = 0; t < TC_STAGES - 1; ++t) {
+        if (t < nk) load(t);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int t = 0; t < nk; ++t) {
+        const int s = t % TC_STAGES;
+        asm volatile("cp.async.wait_group %0;" ::"n"(TC_STAGES - 2) : "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         if (__syncthreads_or(!ok)) {
             ok = false;
             break;
         }
-        store(s);
-        __syncthreads();
         if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint32_t a0 = smem_u32(sA[s]), b0 = smem_u32(sB[s]);
             for (int kk = 0; kk < TC_BK / 16; ++kk) {
-                uint64_t ad = sdesc(a0 + kk * 256, 128, 1024);
-                uint64_t bd = sdesc(b0 + kk * 256, 128, 1024);
+                uint64_t ad = sdesc(sA + s * TC_STAGE_A + kk * 256, 128, 1024);
+                uint64_t bd = sdesc(sB + s * TC_STAGE_B + kk * 256, 128, 1024);
                 uint32_t acc = (t > 0 || kk > 0) ? 1u : 0u;
                 asm volatile(
                     "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(
@@ -170,16 +157,15 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTC g) {
                              smem_u32(&mbar[s]))
                          : "memory");
         }
-        if (t + 1 < nk) fetch(t + 1);
+        // the stage of tile t - 1 takes tile t + TC_STAGES - 1 once its multiplications have read it
+        const int nt = t + TC_STAGES - 1;
+        if (t >= 1 && !mbar_wait(smem_u32(&mbar[(t - 1) % TC_STAGES]), (uint32_t)(((t - 1) / TC_STAGES) & 1))) ok = false;
+        if (ok && nt < nk) load(nt);
+        asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    // the last stages' multiplications: their commits complete the accumulator
-    if (ok) {
-        for (int t = nk - 2 < 0 ? 0 : nk - 2; t < nk; ++t) {
-            int s = t & 1;
-            if (!mbar_wait(smem_u32(&mbar[s]), phase[s])) ok = false;
-            phase[s] ^= 1;
-        }
-    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    // the last tile's multiplications complete the accumulator (every wait of a stage before it was made)
+    if (ok && nk > 0 && !mbar_wait(smem_u32(&mbar[(nk - 1) % TC_STAGES]), (uint32_t)(((nk - 1) / TC_STAGES) & 1))) ok = false;
     if (!ok) bad_s = 1;
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -195,24 +181,39 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTC g) {
                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                 : "r"(taddr));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (row < g.M)
-                for (int j = 0; j < 16; ++j) {
-                    int n = n0 + cc + j;
-                    if (n >= g.N) break;
-                    float v = __uint_as_float(r[j]);
-                    if (g.bias) v += g.bias[n];
-                    if (g.C) {
-                        float *cp = g.C + (size_t)row * g.ldc + n;
-                        if (g.accumulate)
-                            *cp += v;
-                        else
-                            *cp = v;
-                    }
-                    if (g.Cb) {
-                        float o = g.silu ? v / (1.f + expf(-v)) : v;
-                        g.Cb[(size_t)row * g.ldcb + n] = __float2bfloat16(o);
-                    }
+            if (row >= g.M) continue;
+            const int n1 = n0 + cc;
+            float v[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                v[j] = __uint_as_float(r[j]);
+                if (g.bias && n1 + j < g.N) v[j] += g.bias[n1 + j];
+            }
+            if (g.C) {
+                float *cp = g.C + (size_t)row * g.ldc + n1;
+                if (n1 + 16 <= g.N && (g.ldc & 3) == 0 && !g.accumulate) {
+#pragma unroll
+                    for (int j = 0; j < 16; j += 4) *(float4 *)(cp + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (n1 + j < g.N) cp[j] = g.accumulate ? cp[j] + v[j] : v[j];
                 }
+            }
+            if (g.Cb) {
+                __align__(16) __nv_bfloat16 o[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) o[j] = __float2bfloat16(g.silu ? v[j] / (1.f + expf(-v[j])) : v[j]);
+                __nv_bfloat16 *bp = g.Cb + (size_t)row * g.ldcb + n1;
+                if (n1 + 16 <= g.N && (g.ldcb & 7) == 0) {
+                    *(uint4 *)bp = *(const uint4 *)o;
+                    *(uint4 *)(bp + 8) = *(const uint4 *)(o + 8);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (n1 + j < g.N) bp[j] = o[j];
+                }
+            }
         }
     }
     if (bad_s && tid == 0 && g.err) atomicExch(g.err, 1);
@@ -222,7 +223,8 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTC g) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TC_BN) : "memory");
 }
 
-// B[n, k] (K-major) from a row-major [k, n] BF16 matrix: out[n*ldo + k] = in[k*ldi + n]
+// B[n, k] (K-major) from a row-major [k, n] BF16 matrix: out[n*ldo + k] = in[k*ldi + n], and zeros in out
+// from `rows` up to the next multiple of 8
 __global__ void k_transpose_bf16(int rows, int cols, const __nv_bfloat16 *in, int ldi, __nv_bfloat16 *out, int ldo) {
     __shared__ __nv_bfloat16 tile[32][33];
     int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
@@ -233,7 +235,7 @@ __global__ void k_transpose_bf16(int rows, int cols, const __nv_bfloat16 *in, in
     __syncthreads();
     for (int i = threadIdx.y; i < 32; i += blockDim.y) {
         int c = c0 + i, r = r0 + threadIdx.x;
-        if (c < cols && r < rows) out[(size_t)c * ldo + r] = tile[threadIdx.x][i];
+        if (c < cols && r < ((rows + 7) & ~7)) out[(size_t)c * ldo + r] = tile[threadIdx.x][i];
     }
 }
 
