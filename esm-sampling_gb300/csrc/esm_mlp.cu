@@ -274,6 +274,7 @@ struct esm_mlp {
     int gemm_kind = 1;                             // 1: tcgen05 (k_gemm_tc), 0: mma.sync (k_gemm_bf16)
     __nv_bfloat16 *tA = nullptr, *tB = nullptr;    // K-major copies of the weight-gradient operands
     int *tc_err = nullptr;                         // set by k_gemm_tc when a wait ran out
+    double *host = nullptr;                        // pinned: the loss, then the error flag
 };
 
 namespace {
@@ -379,13 +380,14 @@ void adam_weights(esm_mlp *c, int l, float lr, float b1, float b2, float eps, fl
                                           c->Wb[l], ld8(cols), c->Wt[l], ld8(rows));
 }
 
-// a wait of the tensor-core GEMM ran out: the stream's results are not to be used
+// A wait of the tensor-core GEMM ran out: the stream's results are not to be used. The flag is copied to
+// pinned memory with the call's other results and read after the call's one synchronisation.
+int tc_flag(esm_mlp *c) {
+    MK(cudaMemcpyAsync(c->host + 1, c->tc_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    return ESM_OK;
+}
 int tc_check(esm_mlp *c) {
-    if (c->gemm_kind != 1) return ESM_OK;
-    int e = 0;
-    MK(cudaMemcpyAsync(&e, c->tc_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    MK(cudaStreamSynchronize(c->stream));
-    if (e) return mfail(c, ESM_ETIMEOUT, "a tensor-core GEMM wait ran out");
+    if (c->gemm_kind == 1 && *(const int *)(c->host + 1)) return mfail(c, ESM_ETIMEOUT, "a tensor-core GEMM wait ran out");
     return ESM_OK;
 }
 
@@ -469,6 +471,7 @@ int esm_mlp_create(int32_t nlayers, const int32_t *dims, int32_t batch_max, uint
     if ((rc = malloc_(c, &c->tA, (size_t)ld8(batch_max) * dmax))) return rc;
     if ((rc = malloc_(c, &c->tB, (size_t)ld8(batch_max) * dmax))) return rc;
     if ((rc = malloc_(c, &c->tc_err, 1))) return rc;
+    MK(cudaMallocHost((void **)&c->host, 2 * sizeof(double)));
     MK(cudaFuncSetAttribute(tc::k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
     // He-style initialisation from a fixed LCG stream (host), zero biases
     uint64_t st = seed * 6364136223846793005ull + 1442695040888963407ull;
@@ -494,6 +497,7 @@ int esm_mlp_destroy(esm_mlp *c) {
     if (!c) return ESM_OK;
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (void *p : c->allocs) cudaFree(p);
+    if (c->host) cudaFreeHost(c->host);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return ESM_OK;
@@ -535,7 +539,7 @@ int esm_mlp_forward(esm_mlp *c, int32_t B, const float *x, float *y) {
     MK(cudaGetLastError());
     c->launches += 1;
     int rc = forward(c, B);
-    if (rc) return rc;
+    if (rc || (rc = tc_flag(c))) return rc;
     if (y) MK(cudaMemcpyAsync(y, c->Z[c->nl - 1], sizeof(float) * B * dout, cudaMemcpyDeviceToHost, c->stream));
     MK(cudaStreamSynchronize(c->stream));
     return tc_check(c);
@@ -607,7 +611,8 @@ int esm_mlp_train_step(esm_mlp *c, int32_t B, const float *x, const float *targe
         c->launches += 2;
     }
     MK(cudaGetLastError());
-    double L = 0;
+    if ((rc = tc_flag(c))) return rc;
+    MK(cudaMemcpyAsync(c->host, c->loss, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     if (grads_out) {  // (a copy to pageable memory waits for the stream: after every launch of the step)
         size_t off = 0;
         for (int l = 0; l < nl; ++l) {
@@ -617,9 +622,8 @@ int esm_mlp_train_step(esm_mlp *c, int32_t B, const float *x, const float *targe
             off += nw + nb;
         }
     }
-    MK(cudaMemcpyAsync(&L, c->loss, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     MK(cudaStreamSynchronize(c->stream));
-    if (loss_out) *loss_out = L;
+    if (loss_out) *loss_out = *c->host;
     return tc_check(c);
 }
 
