@@ -1350,6 +1350,7 @@ int esm_weather_step(esm_ctx *c, const int32_t *moved, const double *theta, cons
         c->launches += 1;
     }
     if (anyw) {  // regime window, then z rebuilt from its innovations at the new regimes
+        CK(cudaMemcpyAsync(c->d_reg2, c->d_reg, sizeof(int32_t) * c->T * R, cudaMemcpyDeviceToDevice, c->stream));
         esm::k_regime_window<<<(R + 63) / 64, 64, 0, c->stream>>>(c->T, R, c->nreg, c->d_Ptr, c->d_pi0, c->d_moved,
                                                                   c->d_window, c->d_wstart, c->d_reg, c->d_reg2,
                                                                   c->d_wbeta, c->seed, (uint32_t)it);

@@ -25,12 +25,11 @@ __device__ inline real avail_map(real x) {  // logistic availability map (builde
 // ---------------------------------------------------------------------------------------------
 template <class real>
 __global__ void k_rebuild(DevModel<real> M) {
-    size_t TR = (size_t)M.T * M.R;
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)M.N * TR) return;
-    int n = (int)(i / TR);
-    size_t tr = i % TR;
-    int t = (int)(tr / M.R), rep = (int)(tr % M.R);
+    const unsigned tr = blockIdx.x * blockDim.x + threadIdx.x;  // (step, replica) of node blockIdx.y
+    if (tr >= (unsigned)M.T * M.R) return;
+    const int n = blockIdx.y;
+    const size_t i = (size_t)n * M.T * M.R + tr;
+    const int t = (int)(tr / (unsigned)M.R), rep = (int)(tr - (unsigned)t * M.R);
     int T = M.T, R = M.R;
     real x = wraw(M, n, t, rep);
     real r = x > 0 ? x : real(0);
@@ -594,10 +593,10 @@ __global__ void k_score_finish(DevModel<real> M, const double *k_raw, const doub
 template <class real>
 __global__ void k_follow_disp(DevModel<real> M, const int *disp, const double *kold, const double *knew,
                               const double *u_lo, const double *u_hi) {
-    size_t TR = (size_t)M.T * M.R;
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)M.D * TR) return;
-    int j = (int)(i / TR);
+    const unsigned tr = blockIdx.x * blockDim.x + threadIdx.x;
+    if (tr >= (unsigned)M.T * M.R) return;
+    const int j = blockIdx.y;
+    const size_t i = (size_t)j * M.T * M.R + tr;
     int u = disp[j];
     double kc0 = fmin(fmax(kold[u], u_lo[u]), u_hi[u]), kc1 = fmin(fmax(knew[u], u_lo[u]), u_hi[u]);
     double sc = kc0 == kc1 ? 1.0 : kc0 / kc1;  // kc_ratio (src/local.jl:2119)
@@ -612,12 +611,11 @@ __global__ void k_follow_disp(DevModel<real> M, const int *disp, const double *k
 template <class real>
 __global__ void k_kop(DevModel<real> M, const double *kold, const double *k1v, const double *u_lo,
                       const double *u_hi, double kmin) {
-    size_t TR = (size_t)M.T * M.R;
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)M.N * TR) return;
-    int n = (int)(i / TR);
-    size_t tr = i % TR;
-    int t = (int)(tr / M.R), rep = (int)(tr % M.R);
+    const unsigned tr = blockIdx.x * blockDim.x + threadIdx.x;  // (step, replica) of node blockIdx.y
+    if (tr >= (unsigned)M.T * M.R) return;
+    const int n = blockIdx.y;
+    const size_t i = (size_t)n * M.T * M.R + tr;
+    const int t = (int)(tr / (unsigned)M.R), rep = (int)(tr - (unsigned)t * M.R);
     int T = M.T, R = M.R;
     for (int p = M.nu_ptr[n]; p < M.nu_ptr[n + 1]; ++p) {
         int u = M.nu_unit[p], j = M.u_loc[u];
@@ -697,14 +695,14 @@ __global__ void k_set_kc(int K, const double *k_raw, const double *u_lo, const d
 
 #ifdef ESM_COMMON_KERNELS
 
-// regime_window (src/replicas.jl:131-163), one thread per replica; a is 1-based; beta scratch [R*K*T]
+// regime_window (src/replicas.jl:131-163), one thread per replica; a is 1-based; beta scratch [R*K*T];
+// reg2 holds a copy of reg and takes the window's regimes
 __global__ void k_regime_window(int T, int R, int K, const double *Ptr, const double *pi0, const int *moved,
                                 const int *window, const int *wstart, const int *reg, int *reg2, double *beta,
                                 uint64_t seed, uint32_t it) {
     int rep = blockIdx.x * blockDim.x + threadIdx.x;
     if (rep >= R) return;
-    for (int t = 0; t < T; ++t) reg2[(size_t)t * R + rep] = reg[(size_t)t * R + rep];
-    if (!moved[rep] || window[rep] <= 0) return;
+    if (!moved[rep] || window[rep] <= 0) return;  // (reg2 is a copy of reg)
     int a = min(T, max(1, wstart[rep]));
     int b = min(T, a + window[rep] - 1);
     int B = b - a + 1;
@@ -798,10 +796,15 @@ __global__ void k_kop_capacity(int K, const int *u_kind, const double *kold, con
 // ---------------------------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------------------------
+// one thread per (step, replica) of each of n rows (nodes or units): the row is the block's, so that the
+// tables a thread walks are uniform, and no thread divides 64-bit indices
+template <class real>
+inline dim3 row_grid(const DevModel<real> &M, int n) {
+    return dim3((unsigned)(((size_t)M.T * M.R + 255) / 256), n);
+}
 template <class real>
 cudaError_t launch_rebuild(const DevModel<real> &M, cudaStream_t s) {
-    size_t n = (size_t)M.N * M.T * M.R;
-    k_rebuild<real><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(M);
+    k_rebuild<real><<<row_grid(M, M.N), 256, 0, s>>>(M);
     return cudaGetLastError();
 }
 
@@ -810,13 +813,18 @@ cudaError_t launch_rebuild(const DevModel<real> &M, cudaStream_t s) {
 // final sums) would not fit the static score scratch of 2^20 doubles, so that both score entry
 // points sum in the same order
 // step chunks of the score pass: 64 steps a chunk, fewer chunks where the partials (values and
-// bounds) and the sums would not fit 2^20 doubles (the static scratch)
+// bounds) and the sums would not fit 2^20 doubles (the static scratch). Two blocks of the pass are resident
+// per SM, 304 in all: a grid of a little more runs a second wave nearly empty, so it takes the fewer chunks
+// that fill whole waves (40 nodes, T = 8760, 64 replicas: 30 chunks of 10 blocks and not 33).
 __host__ inline int score_chunks(int T, int R, int K, int N) {
     int ng = (N + ESM_SCORE_NSLOT - 1) / ESM_SCORE_NSLOT;
     long long room = (1LL << 20) - 2LL * R * (K + 8);
     long long nmax = room > 0 ? room / (2LL * R * (K + 5 * ng)) : 0;
     int n = (T + 63) / 64;
     if (nmax >= 1 && n > nmax) n = (int)nmax;
+    const int per = ng * ((R + 31) / 32), wave = 304;  // blocks of a chunk
+    int waves = (int)((long long)n * per / wave);
+    if (waves >= 1 && waves <= 4 && (long long)waves * wave >= per) n = (int)((long long)waves * wave / per);
     return n < 1 ? 1 : n;
 }
 __host__ inline size_t score_partial_doubles(int T, int R, int K, int N) {
@@ -878,16 +886,14 @@ cudaError_t launch_score_finish(const DevModel<real> &M, const double *k_raw, co
 template <class real>
 cudaError_t launch_follow_disp(const DevModel<real> &M, const int *disp, const double *kold, const double *knew,
                                const double *lo, const double *hi, cudaStream_t s) {
-    size_t n = (size_t)M.D * M.T * M.R;
-    k_follow_disp<real><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(M, disp, kold, knew, lo, hi);
+    if (M.D > 0) k_follow_disp<real><<<row_grid(M, M.D), 256, 0, s>>>(M, disp, kold, knew, lo, hi);
     return cudaGetLastError();
 }
 
 template <class real>
 cudaError_t launch_kop(const DevModel<real> &M, const double *kold, const double *k1, const double *lo,
                        const double *hi, double kmin, cudaStream_t s) {
-    size_t n = (size_t)M.N * M.T * M.R;
-    k_kop<real><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(M, kold, k1, lo, hi, kmin);
+    k_kop<real><<<row_grid(M, M.N), 256, 0, s>>>(M, kold, k1, lo, hi, kmin);
     return cudaGetLastError();
 }
 
@@ -913,14 +919,6 @@ static __global__ void k_season(int T, double *season) {
 }
 
 template <class real>
-__device__ inline double var_mean(const DevModel<real> &M, const double *phi, const double *mu, const double *season,
-                                  int k, int i, double zprev, int t) {
-    double cs = season[2 * t], sn = season[2 * t + 1];
-    const double *m3 = mu + ((size_t)k * M.n0 + i) * 3;
-    return phi[(size_t)k * M.n0 + i] * zprev + 1.0 * m3[0] + cs * m3[1] + sn * m3[2];
-}
-
-template <class real>
 __device__ inline double weather_normal(uint64_t seed, uint32_t j, uint32_t rep, uint32_t it) {
     double u0, u1;
     uniform2(seed, ESM_TAG_WTH, j >> 1, 0, rep, it, &u0, &u1);
@@ -929,46 +927,119 @@ __device__ inline double weather_normal(uint64_t seed, uint32_t j, uint32_t rep,
     return (double)((j & 1) ? rr * sin(a) : rr * cos(a));
 }
 
-// one pass over series i of replica rep: innovations at regA, rotation by theta (> 0), rebuilt at regB
+// FP64 a b + c: contracted in the FP32 build, as its FP64 expressions are, and not in the FP64 build
 template <class real>
-__global__ void k_weather_z(DevModel<real> M, const double *phi, const double *mu, const double *season,
-                            const double *sig, const double *sig0, const int *moved, const double *theta, const int *regA,
-                            const int *regB, const double *xi, uint64_t seed, uint32_t it, int use_theta) {
-    int rep = blockIdx.y * blockDim.x + threadIdx.x;
-    int i = blockIdx.x;
-    if (rep >= M.R || i >= M.n0) return;
-    if (!moved[rep]) return;
-    double th = use_theta ? theta[rep] : 0.0;
-    if (use_theta && !(th > 0)) return;
-    double ct = cos(th), st = sin(th);
-    double zpo = 0, zpn = 0;
-    int T = M.T, R = M.R;
-    for (int t = 0; t < T; ++t) {
-        size_t zi = sidx(i, t, rep, T, R);
-        double zo = (double)M.z[zi];
-        int ka = regA[(size_t)t * R + rep], kb = regB[(size_t)t * R + rep];
-        double e = t == 0 ? zo / sig0[i] : (zo - var_mean(M, phi, mu, season, ka, i, zpo, t)) / sig[(size_t)ka * M.n0 + i];
-        if (use_theta) {
-            double x = xi ? xi[(size_t)rep * M.n0 * T + (size_t)t * M.n0 + i]
-                          : weather_normal<real>(seed, (uint32_t)((size_t)t * M.n0 + i), (uint32_t)rep, it);
-            e = ct * e + st * x;
+__device__ inline double wfma(double a, double b, double c) {
+    return sizeof(real) == 4 ? __fma_rn(a, b, c) : __dadd_rn(__dmul_rn(a, b), c);
+}
+
+// One pass over series i: innovations at regA, rotation by theta (> 0), rebuilt at regB. A block takes one
+// series and 32 replicas (the lanes). The innovations need only the old anomalies, so they are formed for
+// ESM_WEATHER_CHUNK steps at a time by seven warps, while warp 0 runs the recursion of the chunk before:
+// two to four dependent FP64 operations a step. (One thread per series and replica ran all of it in step
+// order, some 40 FP64 instructions a step at 64 cycles each: 4.7 ms at T = 2920.)
+#define ESM_WEATHER_CHUNK 56
+#define ESM_WEATHER_REG 8   // regimes whose coefficients are kept in shared memory
+template <class real>
+__global__ void __launch_bounds__(256)
+    k_weather_z(DevModel<real> M, const double *phi, const double *mu, const double *season, const double *sig,
+                const double *sig0, const int *moved, const double *theta, const int *regA, const int *regB,
+                const double *xi, uint64_t seed, uint32_t it, int use_theta) {
+    __shared__ double se[2][ESM_WEATHER_CHUNK][32];       // the innovations
+    __shared__ double ss[2][ESM_WEATHER_CHUNK][2];        // the seasonal regressors
+    __shared__ unsigned short sk[2][ESM_WEATHER_CHUNK][32];  // the regimes
+    __shared__ double sl[2][32];                          // the old anomalies at the chunk's last step
+    __shared__ double sc[ESM_WEATHER_REG][5];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int i = blockIdx.x, rep = blockIdx.y * 32 + lane;
+    const int T = M.T, R = M.R, n0 = M.n0;
+    const bool small = M.nreg <= ESM_WEATHER_REG;
+    if (small)
+        for (int q = threadIdx.x; q < 5 * M.nreg; q += 256) {
+            int k = q / 5, f = q % 5;
+            sc[k][f] = f == 0 ? phi[(size_t)k * n0 + i] : f == 4 ? sig[(size_t)k * n0 + i] : mu[((size_t)k * n0 + i) * 3 + f - 1];
         }
-        double zn = t == 0 ? sig0[i] * e : var_mean(M, phi, mu, season, kb, i, zpn, t) + sig[(size_t)kb * M.n0 + i] * e;
-        M.z[zi] = (real)zn;
-        zpo = zo;
-        zpn = zn;
+    __syncthreads();
+    auto coef = [&](int k, int f) -> double {
+        return small ? sc[k][f] : f == 0 ? phi[(size_t)k * n0 + i] : f == 4 ? sig[(size_t)k * n0 + i] : mu[((size_t)k * n0 + i) * 3 + f - 1];
+    };
+    // var_mean of regime k at step t after z
+    auto mean = [&](int k, double z, double cs, double sn) -> double {
+        double m = wfma<real>(coef(k, 0), z, coef(k, 1)), a = coef(k, 2), b = coef(k, 3);
+        if (a != 0.0) m = wfma<real>(cs, a, m);
+        if (b != 0.0) m = wfma<real>(sn, b, m);
+        return m;
+    };
+    double th = 0;
+    bool on = rep < R && moved[rep];
+    if (on && use_theta) {
+        th = theta[rep];
+        on = th > 0;
+    }
+    double ct = 1, st = 0;
+    if (on) {
+        ct = cos(th);
+        st = sin(th);
+    }
+    const int nchunk = (T + ESM_WEATHER_CHUNK - 1) / ESM_WEATHER_CHUNK;
+    auto fill = [&](int c, int w0, int nw) {
+        const int t0 = c * ESM_WEATHER_CHUNK, t1 = min(T, t0 + ESM_WEATHER_CHUNK), b = c & 1;
+        for (int t = t0 + w - w0; t < t1; t += nw) {
+            const double cs = season[2 * t], sn = season[2 * t + 1];
+            if (lane == 0) {
+                ss[b][t - t0][0] = cs;
+                ss[b][t - t0][1] = sn;
+            }
+            if (!on) continue;
+            const double zo = (double)M.z[sidx(i, t, rep, T, R)];
+            const int ka = regA[(size_t)t * R + rep];
+            double e;
+            if (t == 0) {
+                e = zo / sig0[i];
+            } else {
+                double zp = t == t0 ? sl[b ^ 1][lane] : (double)M.z[sidx(i, t - 1, rep, T, R)];
+                e = (zo - mean(ka, zp, cs, sn)) / coef(ka, 4);
+            }
+            if (use_theta) {
+                double x = xi ? xi[(size_t)rep * n0 * T + (size_t)t * n0 + i]
+                              : weather_normal<real>(seed, (uint32_t)((size_t)t * n0 + i), (uint32_t)rep, it);
+                e = wfma<real>(ct, e, st * x);
+            }
+            se[b][t - t0][lane] = e;
+            sk[b][t - t0][lane] = (unsigned short)regB[(size_t)t * R + rep];
+            if (t == t1 - 1) sl[b][lane] = zo;
+        }
+    };
+    fill(0, 0, 8);
+    double z = 0;
+    for (int c = 0; c < nchunk; ++c) {
+        __syncthreads();
+        if (w > 0) {
+            if (c + 1 < nchunk) fill(c + 1, 1, 7);
+        } else if (on) {
+            const int t0 = c * ESM_WEATHER_CHUNK, t1 = min(T, t0 + ESM_WEATHER_CHUNK), b = c & 1;
+            for (int t = t0; t < t1; ++t) {
+                const double e = se[b][t - t0][lane];
+                if (t == 0) {
+                    z = sig0[i] * e;
+                } else {
+                    const int k = sk[b][t - t0][lane];
+                    z = wfma<real>(coef(k, 4), e, mean(k, z, ss[b][t - t0][0], ss[b][t - t0][1]));
+                }
+                M.z[sidx(i, t, rep, T, R)] = (real)z;
+            }
+        }
     }
 }
 
 // compensate_weather! (src/replicas.jl:207) per (node, step, replica) of the moved replicas
 template <class real>
 __global__ void k_compensate(DevModel<real> M, const int *moved, const real *r0) {
-    size_t TR = (size_t)M.T * M.R;
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)M.N * TR) return;
-    int n = (int)(i / TR);
-    size_t tr = i % TR;
-    int t = (int)(tr / M.R), rep = (int)(tr % M.R);
+    const unsigned tr = blockIdx.x * blockDim.x + threadIdx.x;  // (step, replica) of node blockIdx.y
+    if (tr >= (unsigned)M.T * M.R) return;
+    const int n = blockIdx.y;
+    const size_t i = (size_t)n * M.T * M.R + tr;
+    const int t = (int)(tr / (unsigned)M.R), rep = (int)(tr - (unsigned)t * M.R);
     if (!moved[rep]) return;
     real need = M.r[i] - r0[i];
     if (fabs(need) < real(1e-6)) return;
@@ -1001,17 +1072,15 @@ cudaError_t launch_weather_z(const DevModel<real> &M, const double *phi, const d
                              const double *sig, const double *sig0, const int *moved, const double *theta,
                              const int *regA, const int *regB, const double *xi, uint64_t seed, uint32_t it,
                              int use_theta, cudaStream_t s) {
-    int bx = M.R < 64 ? M.R : 64;
-    dim3 grid(M.n0, (M.R + bx - 1) / bx);
-    k_weather_z<real><<<grid, bx, 0, s>>>(M, phi, mu, season, sig, sig0, moved, theta, regA, regB, xi, seed, it,
+    dim3 grid(M.n0, (M.R + 31) / 32);
+    k_weather_z<real><<<grid, 256, 0, s>>>(M, phi, mu, season, sig, sig0, moved, theta, regA, regB, xi, seed, it,
                                           use_theta);
     return cudaGetLastError();
 }
 
 template <class real>
 cudaError_t launch_compensate(const DevModel<real> &M, const int *moved, const real *r0, cudaStream_t s) {
-    size_t n = (size_t)M.N * M.T * M.R;
-    k_compensate<real><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(M, moved, r0);
+    k_compensate<real><<<row_grid(M, M.N), 256, 0, s>>>(M, moved, r0);
     return cudaGetLastError();
 }
 
