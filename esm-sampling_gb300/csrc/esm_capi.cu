@@ -107,8 +107,9 @@ struct esm_ctx {
     double kappa_min = 1.0;
     int *d_sl_plan = nullptr;            // the long-range sweep's per-unit move lists
     esm_ctx *probe = nullptr;            // one-replica context of the lag probe (esm_opts.probe)
-    int sms_threads = 0;
-    size_t sms_per = 0;                  // reals of global scratch per storage-kernel thread (0: local arrays)
+    int sms_slots = 0;                   // tasks of the storage kernels at a time
+    size_t sms_per = 0;                  // reals of global scratch per such task
+    int maxd = 0;                        // most dispatchable units at a node
     void *d_sms_scratch = nullptr;
     int scratch_warps = 0;               // line-move warps the global scratch holds (0: no global scratch needed)
     unsigned long long *d_sms_stats = nullptr;
@@ -510,10 +511,6 @@ int alloc_state(esm_ctx *c) {
     if ((rc = dalloc(c, &ctr, (size_t)(M.natoms + M.nextra)))) return rc;
     c->d_item_ctr = ctr;
     if ((rc = dalloc(c, &c->d_sweep, 1))) return rc;
-    // storage sweeps: resident threads of their kernels; the global scratch they need when the lane
-    // layout exceeds the local arrays is allocated at their first use (sms_scratch)
-    c->sms_threads = esm::plateau_threads<real>(M);
-    c->sms_per = esm::plateau_scratch_reals<real>(M);
     if ((rc = dalloc(c, &c->d_sms_stats, 3))) return rc;
     return ESM_OK;
 }
@@ -734,6 +731,11 @@ int esm_create(const esm_model *m, const esm_opts *o, esm_ctx **out) {
     for (int n = 0; n < m->N; ++n)
         if (m->units_ptr[n + 1] - m->units_ptr[n] > ESM_PLAT_MAXK)
             return fail(c, ESM_EINVAL, "a node has more than %d dispatchable units", ESM_PLAT_MAXK);
+    for (int n = 0; n < m->N; ++n) c->maxd = std::max(c->maxd, m->units_ptr[n + 1] - m->units_ptr[n]);
+    // storage sweeps: the tasks at a time; their global scratch is allocated at their first use (sms_scratch)
+    c->sms_slots = c->precision == 64 ? esm::plateau_slots<double>(c->Md, c->maxd) : esm::plateau_slots<float>(c->Mf, c->maxd);
+    c->sms_per = c->precision == 64 ? esm::plateau_scratch_reals<double>(c->Md, c->maxd)
+                                    : esm::plateau_scratch_reals<float>(c->Mf, c->maxd);
     // classes
     c->ncls = c->T % 2 ? 3 : 2;
     c->class_len.assign(3, 0);
@@ -1012,18 +1014,18 @@ int sms_plan(const esm_ctx *c, uint32_t sweep, bool force, std::vector<esm::Plat
     return (int)out.size();
 }
 
-// the storage kernels' global scratch (layouts beyond the local arrays only), at their first use:
-// at most 256 MB, the grid capped to the threads it holds
+// the storage kernels' global scratch, at their first use: at most 256 MB, the grid capped to the
+// tasks it holds
 int sms_scratch(esm_ctx *c) {
-    if (c->sms_per == 0 || c->d_sms_scratch) return ESM_OK;
+    if (c->d_sms_scratch) return ESM_OK;
     size_t rb = c->precision == 64 ? sizeof(double) : sizeof(float);
     size_t fit = ((size_t)256 << 20) / (c->sms_per * rb);
-    int thr = (int)std::min((size_t)c->sms_threads, std::max((size_t)128, fit / 128 * 128));
+    int slots = (int)std::min((size_t)c->sms_slots, std::max((size_t)32, fit / 32 * 32));
     char *q;
-    int rc = dalloc(c, &q, c->sms_per * rb * (size_t)thr);
+    int rc = dalloc(c, &q, c->sms_per * rb * (size_t)slots);
     if (rc) return rc;
     c->d_sms_scratch = q;
-    c->sms_threads = thr;
+    c->sms_slots = slots;
     return ESM_OK;
 }
 
@@ -1040,10 +1042,10 @@ int sms_sweep_any(esm_ctx *c, uint32_t sweep, bool force, int max_passes = 0) {
     Span sp(c, ESM_KT_STORAGE);
     for (auto &mv : plan) {
         if (c->precision == 64)
-            CK(esm::launch_plateau<double>(c->Md, mv, sweep, (double *)c->d_sms_scratch, c->sms_threads,
+            CK(esm::launch_plateau<double>(c->Md, c->maxd, mv, sweep, (double *)c->d_sms_scratch, c->sms_slots,
                                            c->d_sms_stats, c->stream));
         else
-            CK(esm::launch_plateau<float>(c->Mf, mv, sweep, (float *)c->d_sms_scratch, c->sms_threads,
+            CK(esm::launch_plateau<float>(c->Mf, c->maxd, mv, sweep, (float *)c->d_sms_scratch, c->sms_slots,
                                           c->d_sms_stats, c->stream));
         c->launches += 1;
     }
@@ -1094,10 +1096,10 @@ int sl_sweep_any(esm_ctx *c, uint32_t sweep) {
     if (mlog) CK(cudaMemsetAsync(mlog, 0xff, sizeof(double) * nu * 5 * c->Md.mlog_nrep, c->stream));
     Span sp(c, ESM_KT_STORAGE);
     if (c->precision == 64)
-        CK(esm::launch_storage_long<double>(c->Md, c->d_sl_plan, nu, sweep, (double *)c->d_sms_scratch, c->sms_threads,
+        CK(esm::launch_storage_long<double>(c->Md, c->maxd, c->d_sl_plan, nu, sweep, (double *)c->d_sms_scratch, c->sms_slots,
                                             c->d_sms_stats, c->stream));
     else
-        CK(esm::launch_storage_long<float>(c->Mf, c->d_sl_plan, nu, sweep, (float *)c->d_sms_scratch, c->sms_threads,
+        CK(esm::launch_storage_long<float>(c->Mf, c->maxd, c->d_sl_plan, nu, sweep, (float *)c->d_sms_scratch, c->sms_slots,
                                            c->d_sms_stats, c->stream));
     c->launches += 1;
     return esm_sync(c, 600.0);  // (the host plan buffer is reused by the next call)

@@ -96,16 +96,17 @@ struct PlatMoves {
     int nu[8];                  // units per move
     int j[8][ESM_PLAT_MAXU];    // storage unit indices (into stor)
 };
+// maxd: the most dispatchable units at a node
 template <class real>
-int plateau_threads(const DevModel<real> &M);  // resident threads of k_plateau
+int plateau_slots(const DevModel<real> &M, int maxd);  // tasks that the storage kernels' global scratch holds
 template <class real>
-size_t plateau_scratch_reals(const DevModel<real> &M);  // global scratch per thread (0: local arrays)
+size_t plateau_scratch_reals(const DevModel<real> &M, int maxd);  // reals per such task
 template <class real>
-cudaError_t launch_plateau(const DevModel<real> &M, const PlatMoves &mv, uint32_t sweep, real *scratch, int threads,
-                           unsigned long long *stats, cudaStream_t s);
+cudaError_t launch_plateau(const DevModel<real> &M, int maxd, const PlatMoves &mv, uint32_t sweep, real *scratch,
+                           int slots, unsigned long long *stats, cudaStream_t s);
 // ---- long-range storage sweep: per unit [stor index, moves, (L, a) per move], at most 5 moves
 #define ESM_SL_STRIDE 12
 template <class real>
-cudaError_t launch_storage_long(const DevModel<real> &M, const int *plan, int nunits, uint32_t sweep, real *scratch,
-                                int threads, unsigned long long *stats, cudaStream_t s);
+cudaError_t launch_storage_long(const DevModel<real> &M, int maxd, const int *plan, int nunits, uint32_t sweep,
+                                real *scratch, int slots, unsigned long long *stats, cudaStream_t s);
 }  // namespace esm

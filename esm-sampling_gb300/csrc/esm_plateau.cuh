@@ -7,9 +7,14 @@
 // of logjac (:1871). Every step of the block has the units' storage terms and node balances.
 //
 // Mapping. The blocks of one length and parity are independent (they share no step); a class pass
-// is one launch in which every thread takes (block, replica) tasks, replica fastest (coalesced
-// state access), and runs the class's 8 moves in order. The move selections are state-independent
-// and drawn on the host from the class stream, as the local sweep's move list is.
+// is one launch in which tasks (block, replica), replica fastest (neighbouring state access), run
+// the class's 8 moves in order. The move selections are state-independent and drawn on the host
+// from the class stream, as the local sweep's move list is. Blocks below 32 steps take one thread
+// a task: thousands of tasks, whose walks go through one state machine so that the threads of a
+// warp evaluate together. Longer blocks and the long-range moves take one warp a task, with the
+// move's states, units and ends in shared memory: the lanes take one (unit, end), one interior step
+// or one segment each, the sums are formed in a fixed order, and what the walk decides every lane
+// decides alike. @MAP@
 //
 // Interior steps. At an interior step both state-of-charge values of a unit's storage term move by
 // t, so while every moved value stays strictly inside (0, 1) the term's cost, injection and
@@ -28,38 +33,54 @@
 namespace esm {
 
 #define ESM_PLAT_RB 256   // roots between two walk points (beyond: the move is left, a guard event)
-#define ESM_PLAT_LOCAL 4096  // reals of a thread's local scratch array; larger layouts use the global slab
 #define ESM_PLAT_NACT 8   // listed steps per unit whose state lies outside the box (more: the unit is evaluated whole)
+#define ESM_PLAT_LOCAL 4096  // reals of a thread's local array, if a task has one thread (larger layouts: the global slab)
+#define ESM_PLAT_PTS 48   // walk points per direction a warp's shared memory holds (beyond: the global slab)
+#define ESM_PLAT_ROOTS 32 // roots of either kind it holds (beyond: the global slab)
+#define ESM_PLAT_STAGE (100 << 10)  // a group's shared memory with the move's states in it (more: read from global memory)
 
-// per-lane scratch layout (reals)
+// a task's layout (reals): a thread's array or a warp's shared memory, and the warp's global slab for what
+// that does not hold
 struct PlatLayout {
-    int pr, cr, zr, pl, cl, zl, lm, ro, gro;
+    int K;                               // kinked units per node
+    int npt, nrt;                        // walk points per direction, roots of a kind
+    int pt;                              // [6 * npt] walk points: position, cost, round-off bound, to the right and left
+    int ro;                              // [2 * nrt] node-balance and storage roots; then the segment masses
+    int cnt;                             // two root counters (integers)
     int slo, shi;                        // [U] clamp-free interval of the moved states inside the box
     int na, act;                         // [U] count, [U * NACT] interior steps touching a state outside the box
-    int kv, kq, kg, kp, ke, knm, kph;    // [2U] compensation kink per (end, unit)
-    int ka;                              // [2U * MAXK] kinked coefficient per (end, unit, disp unit)
-    int dr;                              // [2U] node-balance change per (end, unit)
+    int par;                             // [U * 7] capacity, hours, inflow, efficiencies, marginal cost, node
+    int Di, Ai;                          // [U] interior sums
+    int kv, kq, kg, kp, ke, knm, kph;    // [2U] compensation kink per (unit, end)
+    int ka;                              // [2U * K * 5] per (unit, end, disp unit): kinked coefficient, state, unit data
+    int dr, r0;                          // [2U] node-balance change and value per (unit, end)
     int s3, p3;                          // [2U * 3] end storage secondaries, current / previous
     int sb, pb;                          // [2U] end node balances, current / previous
+    int w;                               // [2U * (K + 2)] an evaluation's terms, in the order of their sum
+    int ys, ny;                          // [U * ny] the states at the block's positions (ny 0: not staged)
     int total;
+    int gp, gr, gl, gtotal;              // global slab: points, roots, masses
 };
 
-__host__ __device__ inline PlatLayout plat_layout(int maxpts, int U) {
+// U units, K kinked units per node, ny staged positions; wide: of a warp
+__host__ __device__ inline PlatLayout plat_layout(int maxpts, int U, int K, int ny, bool wide) {
     PlatLayout L;
     int o = 0;
-    L.pr = o; o += maxpts;
-    L.cr = o; o += maxpts;
-    L.zr = o; o += maxpts;
-    L.pl = o; o += maxpts;
-    L.cl = o; o += maxpts;
-    L.zl = o; o += maxpts;
-    L.lm = o; o += 2 * maxpts + 1;
-    L.ro = o; o += ESM_PLAT_RB;
-    L.gro = o; o += ESM_PLAT_RB;
+    L.K = K;
+    L.npt = wide && maxpts > ESM_PLAT_PTS ? ESM_PLAT_PTS : maxpts;
+    L.nrt = wide ? ESM_PLAT_ROOTS : ESM_PLAT_RB > maxpts + 1 ? ESM_PLAT_RB : maxpts + 1;
+    L.ny = ny;
+    L.w = o; o += 2 * U * (K + 2);  // (first: also read as doubles)
+    L.pt = o; o += 6 * L.npt;
+    L.ro = o; o += 2 * L.nrt;
+    L.cnt = o; o += 2;
     L.slo = o; o += U;
     L.shi = o; o += U;
     L.na = o; o += U;
     L.act = o; o += U * ESM_PLAT_NACT;
+    L.par = o; o += 7 * U;
+    L.Di = o; o += U;
+    L.Ai = o; o += U;
     L.kv = o; o += 2 * U;
     L.kq = o; o += 2 * U;
     L.kg = o; o += 2 * U;
@@ -67,60 +88,81 @@ __host__ __device__ inline PlatLayout plat_layout(int maxpts, int U) {
     L.ke = o; o += 2 * U;
     L.knm = o; o += 2 * U;
     L.kph = o; o += 2 * U;
-    L.ka = o; o += 2 * U * ESM_PLAT_MAXK;
+    L.ka = o; o += 2 * U * K * 5;
     L.dr = o; o += 2 * U;
+    L.r0 = o; o += 2 * U;
     L.s3 = o; o += 6 * U;
     L.p3 = o; o += 6 * U;
     L.sb = o; o += 2 * U;
     L.pb = o; o += 2 * U;
-    L.total = o;
+    L.ys = o; o += U * ny;
+    L.total = (o + 3) & ~3;
+    L.gp = 0;
+    L.gr = 6 * maxpts;
+    L.gl = L.gr + 2 * ESM_PLAT_RB;
+    L.gtotal = (L.gl + 2 * maxpts + 1 + 3) & ~3;
     return L;
 }
 
-// COOP: the 32 lanes of a warp run one task together. Every lane runs the walk on its own copy of
-// the scratch (identical contents), and the loops over the block's steps -- the clamp-free interval,
-// the interior terms outside it, the breakpoint scan, the commit -- are split over the lanes and
-// combined by reductions that every lane receives from lane 0, so the control flow stays uniform.
-template <class real, bool COOP = false>
+// One move at a time of a task of G lanes (1 or 32). The (unit, end) pair i = 2 u + s belongs to lane
+// i % G, which alone writes and reads its entries; what the walk needs of them goes through sums,
+// minima and the root buffers that every lane of the task receives.
+template <class real, int G>
 struct PLane {
     const DevModel<real> &M;
     const PlatLayout &LL;
-    real *slab;
-    int sstride;
+    real *sm, *gm;  // the task's layout, the warp's global slab
+    int sstride;    // between reals of a thread's layout in global memory (else 1)
+    int lane;       // within the task
+    bool on = true; // the thread has a task (G 1: the threads of a warp walk together)
     int L, b0, rep, U;
     bool lvl = false;  // the level move of the long-range sweep: every instant of the year rises, no end steps
+    bool dup = false;  // two units at one node
     const int *uj;  // the move's storage units
     mutable real nzs = 0;
-    int lane = 0;
-    static constexpr int NL = COOP ? 32 : 1;
+
+    __device__ PLane(const DevModel<real> &M_, const PlatLayout &LL_, real *sm_, int sstride_, real *gm_)
+        : M(M_), LL(LL_), sm(sm_), gm(gm_), sstride(sstride_), lane(G == 1 ? 0 : threadIdx.x & 31) {}
+    __device__ inline void sync() const {
+        if constexpr (G == 32) __syncwarp();
+    }
+    __device__ inline real bcast(real v, int l) const { return G == 1 ? v : __shfl_sync(0xffffffffu, v, l); }
     __device__ inline real wsum(real v) const {
-        if constexpr (COOP) {
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            return __shfl_sync(0xffffffffu, v, 0);
-        }
-        return v;
+        for (int o = G / 2; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        return bcast(v, 0);
     }
     __device__ inline real wmin(real v) const {
-        if constexpr (COOP) {
-            for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-            return __shfl_sync(0xffffffffu, v, 0);
-        }
+        for (int o = G / 2; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
         return v;
     }
     __device__ inline real wmax(real v) const {
-        if constexpr (COOP) {
-            for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-            return __shfl_sync(0xffffffffu, v, 0);
-        }
+        for (int o = G / 2; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
         return v;
     }
 
-    __device__ PLane(const DevModel<real> &M_, const PlatLayout &LL_, real *slab_, int sstride_)
-        : M(M_), LL(LL_), slab(slab_), sstride(sstride_) {}
-
-    __device__ inline real &S(int off, int i) const { return slab[(size_t)(off + i) * sstride]; }
+    __device__ inline real &S(int off, int i) const {
+        return G == 32 ? sm[off + i] : sm[(size_t)(off + i) * sstride];
+    }
+    // walk point i of array a (0 position, 1 cost, 2 round-off bound to the right; 3, 4, 5 to the left)
+    __device__ inline real &pt(int a, int i) const {
+        return G == 1 || i < LL.npt ? S(LL.pt, a * LL.npt + i) : gm[LL.gp + a * M.maxpts + i];
+    }
+    // root i of kind h (0 node balances, 1 storage); mass j
+    __device__ inline real &rt(int h, int i) const {
+        return G == 1 || i < LL.nrt ? S(LL.ro, h * LL.nrt + i) : gm[LL.gr + h * ESM_PLAT_RB + i];
+    }
+    __device__ inline real &lm(int j) const { return G == 1 || j < 2 * LL.nrt ? S(LL.ro, j) : gm[LL.gl + j]; }
+    __device__ inline int &cnt(int h) const { return reinterpret_cast<int *>(sm + LL.cnt)[h]; }
     __device__ inline size_t ix(int x, int t) const { return sidx(x, t, rep, M.T, M.R); }
-    __device__ inline int node(int u) const { return M.s_bus[uj[u]]; }
+    // unit data: 0 capacity, 1 hours, 2 inflow, 3 and 4 efficiencies, 5 marginal cost (a thread's task reads
+    // the model, at the same address as its warp's others)
+    __device__ inline real par(int u, int k) const {
+        if constexpr (G == 32) return S(LL.par, 7 * u + k);
+        const int j = uj[u];
+        const real *const f[6] = {M.kc_s, M.s_hours, M.s_qt, M.s_etain, M.s_etaout, M.s_mc};
+        return f[k][j];
+    }
+    __device__ inline int node(int u) const { return G == 32 ? (int)S(LL.par, 7 * u + 6) : M.s_bus[uj[u]]; }
     // block positions: step b0 + q, cyclic (the long-range plateaus wrap); the interior terms (both
     // states raised) are q0() .. q0() + nq() - 1, the raised states q0() .. q0() + ns() - 1
     __device__ inline int cyc(int x) const { return x >= M.T ? x - M.T : x; }
@@ -129,79 +171,112 @@ struct PLane {
     __device__ inline int nq() const { return lvl ? M.T : L - 1; }
     __device__ inline int ns() const { return lvl ? M.T : L; }
     __device__ inline int tau_end(int s) const { return s == 0 ? stp(0) : stp(L); }
+    // the state of unit u at position q, and at the one after it
+    __device__ inline real Y(int u, int q) const { return G == 32 && LL.ny ? S(LL.ys, u * LL.ny + q) : M.e[ix(uj[u], stp(q))]; }
+    __device__ inline real Y1(int u, int q) const {
+        return G == 32 && LL.ny ? S(LL.ys, u * LL.ny + (lvl && q + 1 == M.T ? 0 : q + 1)) : M.e[ix(uj[u], cyc(stp(q) + 1))];
+    }
     // an interior term whose two states stay strictly inside (0, 1) at t is exactly unchanged
     __device__ inline bool quiet(int u, int q, real t) const {
-        int tau = stp(q);
-        real y0 = M.e[ix(uj[u], tau)], y1 = M.e[ix(uj[u], cyc(tau + 1))];
+        real y0 = Y(u, q), y1 = Y1(u, q);
         return y0 > 0 && y0 < 1 && y1 > 0 && y1 < 1 && y0 + t > 0 && y0 + t < 1 && y1 + t > 0 && y1 + t < 1;
     }
     __device__ inline bool inside(int u, real t) const { return t > S(LL.slo, u) && t < S(LL.shi, u); }
 
+    // the move's units and their states into shared memory
+    __device__ __noinline__ void load() {
+        sync();
+        if constexpr (G == 1) {
+            dup = true;  // (one lane: always in order)
+            return;
+        }
+        for (int u = lane; u < U; u += G) {
+            const int j = uj[u];
+            const real q[7] = {M.kc_s[j], M.s_hours[j], M.s_qt[j], M.s_etain[j], M.s_etaout[j], M.s_mc[j], real(M.s_bus[j])};
+            for (int k = 0; k < 7; ++k) S(LL.par, 7 * u + k) = q[k];
+        }
+        if (LL.ny) {
+            const int np = lvl ? M.T : L + 2;
+            for (int u = 0; u < U; ++u)
+                for (int q = lane; q < np; q += G) S(LL.ys, u * LL.ny + q) = M.e[ix(uj[u], cyc(stp(q)))];
+        }
+        sync();
+        bool d = false;
+        for (int u = lane; u < U; u += G)
+            for (int v = 0; v < u; ++v) d = d || node(v) == node(u);
+        dup = __any_sync(0xffffffffu, d);
+    }
+
     // storage term of unit u at block step q (0..L): the change of its cost; *dj the injection
     // change, *d1 the new d (src/energy.jl:448 soc_cost in difference form)
     __device__ __noinline__ real sterm(int u, int q, real t, real *dj, real *d1) const {
-        int j = uj[u];
-        int tau = stp(q);
-        real k = M.kc_s[j];
-        return soc_diff<real>(M.s_hours[j], M.s_qt[j], M.s_etain[j], M.s_etaout[j], M.s_mc[j], k, k + M.kappa0, M.dt,
-                              M.c_viol, M.e[ix(j, tau)], M.e[ix(j, cyc(tau + 1))], (lvl || q >= 1) ? t : real(0),
-                              (lvl || q + 1 <= L) ? t : real(0), dj, d1);
+        real k = par(u, 0);
+        return soc_diff<real>(par(u, 1), par(u, 2), par(u, 3), par(u, 4), par(u, 5), k, k + M.kappa0, M.dt, M.c_viol, Y(u, q), Y1(u, q),
+                              (lvl || q >= 1) ? t : real(0), (lvl || q + 1 <= L) ? t : real(0), dj, d1);
     }
     __device__ inline void sec3(int u, real d, real out[3]) const {
-        real ein = M.s_etain[uj[u]];
+        real ein = par(u, 3);
         out[0] = d;
         out[1] = ein > 0 ? d - ein : real(1);
-        out[2] = -d * M.s_etaout[uj[u]] - real(1);
+        out[2] = -d * par(u, 4) - real(1);
     }
 
-    // the compensation at the end steps (prorata! with soc_qadj), per (end, unit)
+    // the compensation at the end steps (prorata! with soc_qadj), per (unit, end)
     __device__ __noinline__ void kinks() const {
-        for (int s = 0; s < 2; ++s) {
-            int tau = tau_end(s), t1 = (tau + 1) % M.T;
-            for (int u = 0; u < U; ++u) {
-                int i = s * U + u, n = node(u), j = uj[u];
-                real ks = M.kc_s[j] * M.s_hours[j] / M.dt;
-                real g = s == 0 ? ks : -ks;
-                real Pm = 0, Qs = 0;
-                int nv = 0, c = 0;
-                for (int p = M.up[n]; p < M.up[n + 1] && c < ESM_PLAT_MAXK; ++p, ++c) {
+        for (int i = lane; i < 2 * U; i += G) {
+            const int u = i >> 1, s = i & 1;
+            int tau = tau_end(s);
+            int n = node(u);
+            real ks = par(u, 0) * par(u, 1) / M.dt;
+            real g = s == 0 ? ks : -ks;
+            real Pm = 0, Qs = 0;
+            int nv = 0, c = 0;
+            for (int p = M.up[n]; p < M.up[n + 1] && c < LL.K; ++p, ++c) {
+                int d = M.ua[p];
+                real kap = M.d_avail[d] * M.kc_d[d];
+                if (!(fabs(kap) >= M.kmin)) continue;
+                real om = M.g[ix(d, tau)];
+                Pm += kap * om;
+                Qs += kap * clampr<real>(om, 0, 1);
+                nv += 1;
+            }
+            bool valid = g != 0 && nv > 0 && !(fabs(Pm) < real(1e-6));
+            // soc_qadj: nominal minus actual injection of the unit at its node
+            real ye = Y(u, s == 0 ? 0 : L), ye1 = Y1(u, s == 0 ? 0 : L);
+            real ec = clampr<real>(ye, 0, 1), ec1 = clampr<real>(ye1, 0, 1);
+            real dd = par(u, 1) * (ec1 - ec) / M.dt - par(u, 2);
+            real pc = 0, mcx = 0;
+            if (dd >= 0)
+                pc = par(u, 3) > 0 ? dd / par(u, 3) : real(0);
+            else
+                mcx = fmin(-dd * par(u, 4), real(1));
+            real qadj = par(u, 0) * par(u, 1) * (ye1 - ye) / M.dt - par(u, 0) * (pc - mcx);
+            real r0 = M.r[ix(n, tau)];
+            real Q = r0 + Qs + qadj;
+            S(LL.r0, i) = r0;
+            S(LL.kv, i) = valid ? real(1) : real(0);
+            S(LL.kq, i) = Q;
+            S(LL.kg, i) = g;
+            S(LL.kp, i) = valid ? Pm : real(1);
+            S(LL.ke, i) = Pm - fmax(Q, real(0));
+            S(LL.knm, i) = real(nv - 1);
+            c = 0;
+            for (int p = M.up[n]; c < LL.K; ++p, ++c) {
+                const int ka = 5 * (i * LL.K + c);
+                real ak = 0;
+                if (p < M.up[n + 1]) {
                     int d = M.ua[p];
                     real kap = M.d_avail[d] * M.kc_d[d];
-                    if (!(fabs(kap) >= M.kmin)) continue;
-                    real om = M.g[ix(d, tau)];
-                    Pm += kap * om;
-                    Qs += kap * clampr<real>(om, 0, 1);
-                    nv += 1;
-                }
-                bool valid = g != 0 && nv > 0 && !(fabs(Pm) < real(1e-6));
-                // soc_qadj: nominal minus actual injection of the unit at its node
-                real ye = M.e[ix(j, tau)], ye1 = M.e[ix(j, t1)];
-                real ec = clampr<real>(ye, 0, 1), ec1 = clampr<real>(ye1, 0, 1);
-                real dd = M.s_hours[j] * (ec1 - ec) / M.dt - M.s_qt[j];
-                real pc = 0, mcx = 0;
-                if (dd >= 0)
-                    pc = M.s_etain[j] > 0 ? dd / M.s_etain[j] : real(0);
-                else
-                    mcx = fmin(-dd * M.s_etaout[j], real(1));
-                real qadj = M.kc_s[j] * M.s_hours[j] * (ye1 - ye) / M.dt - M.kc_s[j] * (pc - mcx);
-                real Q = M.r[ix(n, tau)] + Qs + qadj;
-                S(LL.kv, i) = valid ? real(1) : real(0);
-                S(LL.kq, i) = Q;
-                S(LL.kg, i) = g;
-                S(LL.kp, i) = valid ? Pm : real(1);
-                S(LL.ke, i) = Pm - fmax(Q, real(0));
-                S(LL.knm, i) = real(nv - 1);
-                c = 0;
-                for (int p = M.up[n]; p < M.up[n + 1] && c < ESM_PLAT_MAXK; ++p, ++c) {
-                    int d = M.ua[p];
-                    real kap = M.d_avail[d] * M.kc_d[d];
-                    real ak = 0;
                     if (valid && fabs(kap) >= M.kmin) {
                         real sigma = kap * M.g[ix(d, tau)] / Pm;
                         if (sigma != 0) ak = sigma / kap;
                     }
-                    S(LL.ka, i * ESM_PLAT_MAXK + c) = ak;
+                    S(LL.ka, ka + 1) = M.g[ix(d, tau)];
+                    S(LL.ka, ka + 2) = M.kc_d[d];
+                    S(LL.ka, ka + 3) = M.d_avail[d];
+                    S(LL.ka, ka + 4) = M.d_mc[d];
                 }
+                S(LL.ka, ka + 0) = ak;
             }
         }
     }
@@ -213,17 +288,18 @@ struct PLane {
     // steps gets an empty interval (evaluated whole).
     __device__ __noinline__ void intervals() const {
         for (int u = 0; u < U; ++u) {
-            int j = uj[u];
             real mn = 2, mx = -1;
             int na = 0;
             bool over = false;
             auto list = [&](int qt) {  // an interior term involving a state outside the box
                 for (int i = 0; i < na; ++i)
                     if (S(LL.act, u * ESM_PLAT_NACT + i) == real(qt)) return;
-                if (na < ESM_PLAT_NACT)
-                    S(LL.act, u * ESM_PLAT_NACT + na++) = real(qt);
-                else
+                if (na < ESM_PLAT_NACT) {
+                    S(LL.act, u * ESM_PLAT_NACT + na++) = real(qt);  // (every lane writes the same value)
+                    sync();
+                } else {
                     over = true;
+                }
             };
             auto out_state = [&](int q) {  // state q is the end value of term q - 1 and the start of term q
                 if (lvl) {
@@ -234,11 +310,11 @@ struct PLane {
                     if (q <= L - 1) list(q);
                 }
             };
-            for (int base = 0; base < ns(); base += NL) {
+            for (int base = 0; base < ns(); base += G) {
                 int p = base + lane, qo = -1;
                 if (p < ns()) {
                     int q = q0() + p;
-                    real y = M.e[ix(j, stp(q))];
+                    real y = Y(u, q);
                     if (y > 0 && y < 1) {
                         mn = fmin(mn, y);
                         mx = fmax(mx, y);
@@ -246,9 +322,10 @@ struct PLane {
                         qo = q;
                     }
                 }
-                if constexpr (COOP) {  // the states outside the box, in step order, listed on every lane
-                    unsigned bal = __ballot_sync(0xffffffffu, qo >= 0);
-                    while (bal) {
+                // the states outside the box, in step order, listed alike on every lane
+                if constexpr (G == 32) {
+                    unsigned bal = over ? 0u : __ballot_sync(0xffffffffu, qo >= 0);
+                    while (bal && !over) {
                         int l = __ffs(bal) - 1;
                         bal &= bal - 1;
                         out_state(__shfl_sync(0xffffffffu, qo, l));
@@ -260,95 +337,155 @@ struct PLane {
             mn = wmin(mn);
             mx = wmax(mx);
             bool ok = !over && mn <= mx;
-            if (!over && mn > mx) {  // every raised state outside the box: no interval, terms listed
-                S(LL.slo, u) = real(-INFINITY);
-                S(LL.shi, u) = real(INFINITY);
-            } else {
-                S(LL.slo, u) = ok ? -mn : real(0);
-                S(LL.shi, u) = ok ? real(1) - mx : real(0);
+            if (lane == 0) {
+                if (!over && mn > mx) {  // every raised state outside the box: no interval, terms listed
+                    S(LL.slo, u) = real(-INFINITY);
+                    S(LL.shi, u) = real(INFINITY);
+                } else {
+                    S(LL.slo, u) = ok ? -mn : real(0);
+                    S(LL.shi, u) = ok ? real(1) - mx : real(0);
+                }
+                S(LL.na, u) = real(over ? 0 : na);
             }
-            S(LL.na, u) = real(over ? 0 : na);
         }
+        sync();
     }
 
     // the interior step terms of unit u to evaluate at t: every one outside its interval, else the listed
-    __device__ inline int nterms(int u, real t) const { return inside(u, t) ? (int)S(LL.na, u) : nq(); }
-    __device__ inline int term_q(int u, real t, int i) const {
-        return inside(u, t) ? (int)S(LL.act, u * ESM_PLAT_NACT + i) : q0() + i;
+    __device__ inline int nterms(int u, bool in) const { return in ? (int)S(LL.na, u) : nq(); }
+    __device__ inline int term_q(int u, bool in, int i) const {
+        return in ? (int)S(LL.act, u * ESM_PLAT_NACT + i) : q0() + i;
+    }
+    // f(u, in, q) for the terms of all units, split over the lanes in the order of unit and step; the
+    // number of the terms of unit u and whether they are its listed ones from nt(u, &in)
+    template <class N, class F>
+    __device__ inline void each_term(N nt, F f) const {
+        int u = 0, i = lane;
+        while (u < U) {
+            bool in;
+            const int n = nt(u, &in);
+            if (i >= n) {
+                i -= n;
+                ++u;
+                continue;
+            }
+            f(u, in, term_q(u, in, i));
+            i += G;
+        }
     }
 
     // mv_eval! of the block (src/local.jl:1219): beta * DeltaC(t); the end steps' secondaries into
     // s3/sb (the interior ones are evaluated where they change, in collect)
     __device__ __noinline__ real eval(real t) const {
-        real dt = M.dt, cv = M.c_viol, k0 = M.kappa0;
+        const real dt = M.dt, cv = M.c_viol, k0 = M.kappa0;
         real D = 0, A = 0;
-        for (int i = 0; i < 2 * U; ++i) {
-            real Q = S(LL.kq, i);
-            S(LL.kph, i) = S(LL.kv, i) != 0 ? fmax(Q + S(LL.kg, i) * t, real(0)) - fmax(Q, real(0)) : real(0);
-            S(LL.dr, i) = 0;
-        }
-        for (int u = 0; u < U; ++u) {
-            int n = node(u);
-            for (int s = 0; s < (lvl ? 0 : 2); ++s) {  // end steps: storage term, kinked dispatch, node balance
-                int i = s * U + u, q = s == 0 ? 0 : L, tau = tau_end(s);
+        // interior steps of a unit: storage term and node balance; the listed terms in order, the terms of
+        // a unit outside its interval by lanes, each on to its next term that changes
+        auto inner = [&](int u) {
+            const bool in = inside(u, t);
+            const int nt = nterms(u, in);
+            real Di = 0, Ai = 0;
+            auto term = [&](int q, real *v, real *a) {
                 real dj, d1;
                 real cs = sterm(u, q, t, &dj, &d1);
-                D += cs;
-                A += fabs(cs);
-                real sc[3];
-                sec3(u, d1, sc);
-                for (int h = 0; h < 3; ++h) S(LL.s3, 3 * i + h) = sc[h];
-                real dr = dj;
-                real ph = S(LL.kph, i);
-                int c = 0;
-                for (int p = M.up[n]; p < M.up[n + 1] && c < ESM_PLAT_MAXK; ++p, ++c) {
-                    real ak = S(LL.ka, i * ESM_PLAT_MAXK + c);
-                    if (ak == 0) continue;
-                    int d = M.ua[p];
-                    real k = M.kc_d[d], Av = M.d_avail[d];
+                real cb = dt * phibal_diff<real>(M.r[ix(node(u), stp(q))], dj, M.c_shed, M.c_dump);
+                *v = cs + cb;
+                *a = fabs(cs) + fabs(cb);
+            };
+            if (G == 32 && in) {
+                real v = 0, a = 0;
+                if (lane < nt) term(term_q(u, true, lane), &v, &a);
+                for (int l = 0; l < nt; ++l) {
+                    Di += bcast(v, l);
+                    Ai += bcast(a, l);
+                }
+            } else {
+                int i = lane;
+                while (true) {
+                    while (i < nt && !in && quiet(u, q0() + i, t)) i += G;
+                    if (i >= nt) break;
+                    real v, a;
+                    term(term_q(u, in, i), &v, &a);
+                    Di += v;
+                    Ai += a;
+                    i += G;
+                }
+                if constexpr (G == 32) {
+                    sync();
+                    Di = wsum(Di);
+                    Ai = wsum(Ai);
+                }
+            }
+            if constexpr (G == 1) {
+                D += Di;
+                A += Ai;
+            } else if (lane == 0) {
+                S(LL.Di, u) = Di;
+                S(LL.Ai, u) = Ai;
+            }
+        };
+        sync();
+        for (int i = lane; i < (lvl ? 0 : 2 * U); i += G) {  // end steps: storage term, kinked dispatch, node balance
+            const int u = i >> 1, s = i & 1, q = s == 0 ? 0 : L;
+            const int w = i * (LL.K + 2);
+            auto add = [&](int h, real v) {  // a term of the sum
+                if constexpr (G == 32) {
+                    S(LL.w, w + h) = v;
+                } else {
+                    D += v;
+                    A += fabs(v);
+                }
+            };
+            real Q = S(LL.kq, i);
+            real ph = S(LL.kv, i) != 0 ? fmax(Q + S(LL.kg, i) * t, real(0)) - fmax(Q, real(0)) : real(0);
+            S(LL.kph, i) = ph;
+            real dj, d1;
+            add(0, sterm(u, q, t, &dj, &d1));
+            real sc[3];
+            sec3(u, d1, sc);
+            for (int h = 0; h < 3; ++h) S(LL.s3, 3 * i + h) = sc[h];
+            real dr = dj;
+            for (int c = 0; c < LL.K; ++c) {
+                const int ka = 5 * (i * LL.K + c);
+                real ak = S(LL.ka, ka), cg = 0;
+                if (ak != 0) {
+                    real k = S(LL.ka, ka + 2), Av = S(LL.ka, ka + 3);
                     real dyc, dex;
-                    clamp_diff<real>(M.g[ix(d, tau)], ak * ph, &dyc, &dex);
+                    clamp_diff<real>(S(LL.ka, ka + 1), ak * ph, &dyc, &dex);
                     real dp = Av * k * dyc;
-                    real cg = dt * M.d_mc[d] * dp + cv * dt * (k + k0) * dex;
-                    D += cg;
-                    A += fabs(cg);
+                    cg = dt * S(LL.ka, ka + 4) * dp + cv * dt * (k + k0) * dex;
                     dr -= dp;
                 }
-                S(LL.dr, i) = dr;
-                real r0 = M.r[ix(n, tau)];
-                real cb = dt * phibal_diff<real>(r0, dr, M.c_shed, M.c_dump);
-                D += cb;
-                A += fabs(cb);
-                S(LL.sb, i) = r0 + dr;
+                add(1 + c, cg);
             }
-            int nt = nterms(u, t);
-            bool in = inside(u, t);
-            real Di = 0, Ai = 0;
-            // interior steps: storage term and node balance (the listed ones on every lane; outside
-            // the interval every term, split over the lanes)
-            for (int i = in ? 0 : lane; i < nt; i += in ? 1 : NL) {
-                int q = term_q(u, t, i);
-                if (!in && quiet(u, q, t)) continue;
-                real dj, d1;
-                real cs = sterm(u, q, t, &dj, &d1);
-                real cb = dt * phibal_diff<real>(M.r[ix(n, stp(q))], dj, M.c_shed, M.c_dump);
-                Di += cs + cb;
-                Ai += fabs(cs) + fabs(cb);
+            S(LL.dr, i) = dr;
+            real r0 = S(LL.r0, i);
+            add(1 + LL.K, dt * phibal_diff<real>(r0, dr, M.c_shed, M.c_dump));
+            S(LL.sb, i) = r0 + dr;
+            if (G == 1 && s == 1) inner(u);
+        }
+        if constexpr (G == 32) {
+            for (int u = 0; u < U; ++u) inner(u);
+            sync();
+            for (int u = 0; u < U; ++u) {
+                const int w = 2 * u * (LL.K + 2);
+                for (int h = 0; h < (lvl ? 0 : 2 * (LL.K + 2)); ++h) {
+                    D += S(LL.w, w + h);
+                    A += fabs(S(LL.w, w + h));
+                }
+                D += S(LL.Di, u);
+                A += S(LL.Ai, u);
             }
-            if (!in) {
-                Di = wsum(Di);
-                Ai = wsum(Ai);
-            }
-            D += Di;
-            A += Ai;
         }
         if constexpr (sizeof(real) == 4) nzs = M.beta_v * A * real(4.8e-7);
         return M.beta_v * D;
     }
 
-    __device__ __noinline__ void save_prev() const {
-        for (int i = 0; i < 6 * U; ++i) S(LL.p3, i) = S(LL.s3, i);
-        for (int i = 0; i < 2 * U; ++i) S(LL.pb, i) = S(LL.sb, i);
+    __device__ inline void save_prev() const {
+        for (int i = lane; i < 2 * U; i += G) {
+            for (int h = 0; h < 3; ++h) S(LL.p3, 3 * i + h) = S(LL.s3, 3 * i + h);
+            S(LL.pb, i) = S(LL.sb, i);
+        }
     }
 
     __device__ static inline bool root_of(real a, real b, real lo, real hi, real sgn, real *x) {
@@ -361,94 +498,69 @@ struct PLane {
         }
         return false;
     }
-    __device__ inline bool add_root(int off, int *n, real x) const {
-        if (*n >= ESM_PLAT_RB) return false;
-        S(off, (*n)++) = x;
-        return true;
+    __device__ inline void add_root(int h, real x, int *n) const {  // n: a thread's counts
+        const int i = G == 1 ? n[h]++ : atomicAdd(&cnt(h), 1);
+        if (i < ESM_PLAT_RB) rt(h, i) = x;
     }
 
-    // sign changes of the secondaries between prev (at lo) and cur (at hi): storage ones into gro
-    // (when storage splitting applies), node balances into ro; interior steps of the units whose
-    // states leave their interval in [lo, hi]
-    __device__ __noinline__ bool collect(real lo, real hi, real sgn, bool want_stor, bool want_other, int *nro, int *ngro) const {
+    // sign changes of the secondaries between prev (at lo) and cur (at hi): storage ones (want_stor)
+    // and node balances into their buffers, in any order (they are sorted); interior steps of the
+    // units whose states leave their interval in [lo, hi]
+    __device__ __noinline__ void collect(real lo, real hi, real sgn, bool want_stor, int *nro, int *ngro) const {
+        int n[2] = {0, 0};
+        if constexpr (G == 32) {
+            sync();
+            if (lane < 2) cnt(lane) = 0;
+            sync();
+        }
         real x;
-        for (int i = 0; i < 2 * U; ++i) {
+        for (int i = lane; i < (lvl ? 0 : 2 * U); i += G) {
             if (want_stor)
                 for (int h = 0; h < 3; ++h)
-                    if (root_of(S(LL.p3, 3 * i + h), S(LL.s3, 3 * i + h), lo, hi, sgn, &x) && !add_root(LL.gro, ngro, x))
-                        return false;
-            if (want_other && root_of(S(LL.pb, i), S(LL.sb, i), lo, hi, sgn, &x) && !add_root(LL.ro, nro, x))
-                return false;
+                    if (root_of(S(LL.p3, 3 * i + h), S(LL.s3, 3 * i + h), lo, hi, sgn, &x)) add_root(1, x, n);
+            if (root_of(S(LL.pb, i), S(LL.sb, i), lo, hi, sgn, &x)) add_root(0, x, n);
         }
-        for (int u = 0; u < U; ++u) {
-            bool in = inside(u, lo) && inside(u, hi);
-            int n = node(u);
-            int nt = in ? (int)S(LL.na, u) : nq();
-            // the listed terms on every lane; outside the interval every term, split over the lanes in
-            // rounds of NL terms, whose roots every lane adds in term order
-            int step = in ? 1 : NL;
-            for (int base = 0; base < nt; base += step) {
-                int i = in ? base : base + lane;
-                real rg[3] = {0, 0, 0}, rr = 0;
-                int ng = 0;
-                bool hr = false;
-                if (i < nt) {
-                    int q = in ? (int)S(LL.act, u * ESM_PLAT_NACT + i) : q0() + i;
-                    if (in || !(quiet(u, q, lo) && quiet(u, q, hi))) {
-                        real dja, d1a, djb, d1b;
-                        sterm(u, q, lo, &dja, &d1a);
-                        sterm(u, q, hi, &djb, &d1b);
-                        if (want_stor) {
-                            real a3[3], b3[3];
-                            sec3(u, d1a, a3);
-                            sec3(u, d1b, b3);
-                            for (int h = 0; h < 3; ++h)
-                                if (root_of(a3[h], b3[h], lo, hi, sgn, &x)) rg[ng++] = x;
-                        }
-                        if (want_other) {
-                            real r0 = M.r[ix(n, stp(q))];
-                            if (root_of(r0 + dja, r0 + djb, lo, hi, sgn, &x)) {
-                                rr = x;
-                                hr = true;
-                            }
-                        }
-                    }
+        each_term(
+            [&](int u, bool *in) {
+                *in = inside(u, lo) && inside(u, hi);
+                return nterms(u, *in);
+            },
+            [&](int u, bool in, int q) {
+                if (!in && quiet(u, q, lo) && quiet(u, q, hi)) return;
+                real dja, d1a, djb, d1b;
+                sterm(u, q, lo, &dja, &d1a);
+                sterm(u, q, hi, &djb, &d1b);
+                if (want_stor) {
+                    real a3[3], b3[3];
+                    sec3(u, d1a, a3);
+                    sec3(u, d1b, b3);
+                    for (int h = 0; h < 3; ++h)
+                        if (root_of(a3[h], b3[h], lo, hi, sgn, &x)) add_root(1, x, n);
                 }
-                bool ok = true;
-                if (COOP && !in) {
-                    unsigned bal = __ballot_sync(0xffffffffu, ng > 0 || hr);
-                    while (bal) {
-                        int l = __ffs(bal) - 1;
-                        bal &= bal - 1;
-                        int nl = __shfl_sync(0xffffffffu, ng, l);
-                        for (int h = 0; h < 3; ++h) {
-                            real xs = __shfl_sync(0xffffffffu, rg[h], l);
-                            if (h < nl) ok = add_root(LL.gro, ngro, xs) && ok;
-                        }
-                        bool hl = __shfl_sync(0xffffffffu, hr, l);
-                        real xr = __shfl_sync(0xffffffffu, rr, l);
-                        if (hl) ok = add_root(LL.ro, nro, xr) && ok;
-                    }
-                } else {
-                    for (int h = 0; h < ng; ++h) ok = add_root(LL.gro, ngro, rg[h]) && ok;
-                    if (hr) ok = add_root(LL.ro, nro, rr) && ok;
-                }
-                if (!ok) return false;
-            }
+                real r0 = M.r[ix(node(u), stp(q))];
+                if (root_of(r0 + dja, r0 + djb, lo, hi, sgn, &x)) add_root(0, x, n);
+            });
+        if constexpr (G == 32) {
+            sync();
+            n[0] = cnt(0);
+            n[1] = cnt(1);
         }
-        return true;
+        *nro = n[0];
+        *ngro = n[1];
     }
 
-    __device__ __noinline__ void sort_buf(int off, int n, real sgn) const {
-        for (int i = 1; i < n; ++i) {
-            real x = S(off, i);
-            int j = i - 1;
-            while (j >= 0 && (sgn > 0 ? x < S(off, j) : x > S(off, j))) {
-                S(off, j + 1) = S(off, j);
-                --j;
+    __device__ __noinline__ void sort_buf(int h, int n, real sgn) const {
+        if (n > 1 && lane == 0)
+            for (int i = 1; i < n; ++i) {
+                real x = rt(h, i);
+                int j = i - 1;
+                while (j >= 0 && (sgn > 0 ? x < rt(h, j) : x > rt(h, j))) {
+                    rt(h, j + 1) = rt(h, j);
+                    --j;
+                }
+                rt(h, j + 1) = x;
             }
-            S(off, j + 1) = x;
-        }
+        sync();
     }
 
     // next primary breakpoint beyond tp (finalize! of every step, scanned): the kink points, the
@@ -465,16 +577,15 @@ struct PLane {
                 have = true;
             }
         };
-        for (int i = 0; i < (lvl ? 0 : 2 * U); ++i) {
+        for (int i = lane; i < (lvl ? 0 : 2 * U); i += G) {
             if (S(LL.kv, i) == 0) continue;
             real g = S(LL.kg, i), Q = S(LL.kq, i);
             consider(-Q / g);
-            int u = i % U, s = i / U, n = node(u), tau = tau_end(s);
-            int c = 0;
-            for (int p = M.up[n]; p < M.up[n + 1] && c < ESM_PLAT_MAXK; ++p, ++c) {
-                real ak = S(LL.ka, i * ESM_PLAT_MAXK + c);
+            for (int c = 0; c < LL.K; ++c) {
+                const int ka = 5 * (i * LL.K + c);
+                real ak = S(LL.ka, ka);
                 if (ak == 0) continue;
-                real y0 = M.g[ix(M.ua[p], tau)];
+                real y0 = S(LL.ka, ka + 1);
                 real offs[4] = {real(0), real(0), -ak * Q, ak * Q};
                 real sls[4] = {ak * g, real(0), real(0), ak * g};
                 for (int h = 0; h < 4; ++h) {
@@ -484,44 +595,41 @@ struct PLane {
                 }
             }
         }
-        for (int u = 0; u < U; ++u) {
-            int j = uj[u];
-            if (tp > S(LL.slo, u) && tp < S(LL.shi, u) && S(LL.slo, u) < S(LL.shi, u)) {
-                // the nearest clamp of the states inside the box, then the clamps of the states
-                // outside it (each a state of a listed term)
-                consider(sgn > 0 ? S(LL.shi, u) : S(LL.slo, u));
-                int na = (int)S(LL.na, u);
-                for (int i = 0; i < na; ++i) {
-                    int q = (int)S(LL.act, u * ESM_PLAT_NACT + i);
-                    for (int h = 0; h < 2; ++h) {
-                        real y0 = M.e[ix(j, cyc(stp(q) + h))];
-                        if (y0 > 0 && y0 < 1) continue;
-                        consider(real(0) - y0);
-                        consider(real(1) - y0);
-                    }
+        // a unit inside its interval: the nearest clamp of the states inside the box, then the clamps of
+        // the states outside it (each a state of a listed term); another: the clamps of all its states
+        auto in_box = [&](int u) { return tp > S(LL.slo, u) && tp < S(LL.shi, u) && S(LL.slo, u) < S(LL.shi, u); };
+        for (int u = lane; u < U; u += G) {
+            if (!in_box(u)) continue;
+            consider(sgn > 0 ? S(LL.shi, u) : S(LL.slo, u));
+            int na = (int)S(LL.na, u);
+            for (int i = 0; i < na; ++i) {
+                int q = (int)S(LL.act, u * ESM_PLAT_NACT + i);
+                for (int h = 0; h < 2; ++h) {
+                    real y0 = h == 0 ? Y(u, q) : Y1(u, q);
+                    if (y0 > 0 && y0 < 1) continue;
+                    consider(real(0) - y0);
+                    consider(real(1) - y0);
                 }
+            }
+        }
+        int u = 0, i = lane;
+        while (u < U) {
+            const int n = in_box(u) ? 0 : ns();
+            if (i >= n) {
+                i -= n;
+                ++u;
                 continue;
             }
-            for (int p = lane; p < ns(); p += NL) {
-                real y0 = M.e[ix(j, stp(q0() + p))];
-                consider(real(0) - y0);
-                consider(real(1) - y0);
-            }
+            real y0 = Y(u, q0() + i);
+            consider(real(0) - y0);
+            consider(real(1) - y0);
+            i += G;
         }
-        if constexpr (COOP) {  // the nearest candidate over the lanes (a sign flip is exact)
-            real key = wmin(have ? sgn * best : real(INFINITY));
-            have = key < real(INFINITY);
-            best = have ? sgn * key : real(0);
-        }
-        *out = best;
+        sync();
+        real key = wmin(have ? sgn * best : real(INFINITY));  // the nearest over the lanes (a sign flip is exact)
+        have = key < real(INFINITY);
+        *out = have ? sgn * key : real(0);
         return have;
-    }
-
-    __device__ inline void push(int pofs, int cofs, int *np, real x, real c, real z) const {
-        S(pofs, *np) = x;
-        S(cofs, *np) = c;
-        if constexpr (sizeof(real) == 4) S(pofs == LL.pr ? LL.zr : LL.zl, *np) = z;
-        ++*np;
     }
 
     // walk! (src/local.jl:1294) with storage splitting, to the right and then to the left; 1 both proper, 0
@@ -529,8 +637,10 @@ struct PLane {
     // iteration evaluates the move once, at whatever point the walk needs next, so the threads of a warp,
     // whose walks differ in length and in roots, stay together over the evaluation; the secondaries at a
     // point are saved before the roots of its segment are evaluated, so that none is evaluated again only to
-    // restore them. Two storage sweeps of 40
-    // nodes, T=2920, 16 replicas: 193 ms with the evaluation called from nine places of two walks, 151 ms so.
+    // restore them. The roots of both kinds come from one pass over the segment; those of the node balances
+    // are taken again, piece by piece, only where the segment has storage roots. Two storage
+    // sweeps of 40 nodes, T=2920, 16 replicas: 193 ms with the evaluation called from nine places of two
+    // walks, 64 ms so.
     __device__ __noinline__ int walks(int *nr, int *nl) const {
         // the point evaluated next: 0; a breakpoint (chosen first); the slope probe of a ray step; the
         // segment's end; a storage root; the segment's end again; a node-balance root
@@ -547,7 +657,13 @@ struct PLane {
                 st = DONE;
                 return false;
             }
-            push(sgn > 0 ? LL.pr : LL.pl, sgn > 0 ? LL.cr : LL.cl, &np, x, v, z);
+            if (lane == 0) {
+                const int a = sgn > 0 ? 0 : 3;
+                pt(a, np) = x;
+                pt(a + 1, np) = v;
+                if constexpr (sizeof(real) == 4) pt(a + 2, np) = z;
+            }
+            ++np;
             cmin = fmin(cmin, v);
             cprev = v;
             return true;
@@ -575,7 +691,8 @@ struct PLane {
             lo = xs;
             st = ++gi < ngro ? STAT : BACK;
         };
-        while (st != DONE) {
+        if (!on) st = DONE;
+        while (G == 1 ? __any_sync(0xffffffffu, st != DONE) : st != DONE) {
             real te = 0;
             if (st == NEXT) {
                 if (next_bp(tp, sgn, &t)) {
@@ -589,12 +706,15 @@ struct PLane {
             } else if (st == END || st == BACK) {
                 te = t;
             } else if (st == STAT) {
-                te = S(LL.gro, gi);
+                te = rt(1, gi);
             } else if (st == ROOT) {
-                te = S(LL.ro, ri);
+                te = rt(0, ri);
             }
-            const real v = eval(te), z = nzs;
-            bool piece = false;
+            __syncwarp();
+            real v = 0;
+            if (st != DONE) v = eval(te);
+            const real z = nzs;
+            __syncwarp();
             if (st == START) {
                 save_prev();
                 st = NEXT;
@@ -617,52 +737,48 @@ struct PLane {
                     else
                         station();
                 }
-            } else {
+            } else if (st != DONE) {
+                // the piece lo .. te: its roots (of a segment's first pass: of both kinds)
+                int ng = 0;
                 if (st == END) {
                     c = v;
                     zc = z;
                     lo = tp;
-                    nro = ngro = gi = 0;
-                    if (!collect(tp, t, sgn, true, false, &nro, &ngro)) {
-                        rc = -1;
-                        st = DONE;
-                    } else if (ngro > 0) {
-                        sort_buf(LL.gro, ngro, sgn);
-                        st = STAT;
-                    } else {
-                        after = END;
-                        piece = true;
-                    }
-                } else if (st == STAT) {
+                    gi = 0;
+                }
+                collect(lo, te, sgn, st == END, &nro, &ng);
+                ri = 0;
+                if (st == END) ngro = ng;
+                if (st == STAT) {
                     xs = te;
                     cs = v;
                     zs = z;
-                    after = STAT;
-                    piece = true;
-                } else {
-                    after = END;
-                    piece = true;
                 }
-                if (piece) {  // the node-balance roots of the piece lo .. te
-                    int ng = 0;
-                    nro = ri = 0;
-                    if (!collect(lo, te, sgn, false, true, &nro, &ng)) {
+                after = st == STAT ? STAT : END;
+                if (st == END && ngro > 0) {
+                    sort_buf(1, min(ngro, ESM_PLAT_RB), sgn);
+                    st = STAT;
+                    if (ngro > ESM_PLAT_RB) {
                         rc = -1;
                         st = DONE;
+                    }
+                } else if (nro > ESM_PLAT_RB) {
+                    rc = -1;
+                    st = DONE;
+                } else {
+                    save_prev();
+                    if (nro > 0) {
+                        sort_buf(0, nro, sgn);
+                        st = ROOT;
+                    } else if (after == END) {
+                        finish();
                     } else {
-                        save_prev();
-                        if (nro > 0) {
-                            sort_buf(LL.ro, nro, sgn);
-                            st = ROOT;
-                        } else if (after == END) {
-                            finish();
-                        } else {
-                            station();
-                        }
+                        station();
                     }
                 }
             }
         }
+        sync();
         return rc;
     }
 
@@ -678,37 +794,42 @@ struct PLane {
         return Ls + log1p(-u * (-expm1(x))) / (-g);
     }
     __device__ inline real P(int i, int nl) const {
-        return i < nl ? S(LL.pl, nl - 1 - i) : (i == nl ? real(0) : S(LL.pr, i - nl - 1));
+        return i < nl ? pt(3, nl - 1 - i) : (i == nl ? real(0) : pt(0, i - nl - 1));
     }
     __device__ inline real Cc(int i, int nl) const {
-        return i < nl ? S(LL.cl, nl - 1 - i) : (i == nl ? real(0) : S(LL.cr, i - nl - 1));
+        return i < nl ? pt(4, nl - 1 - i) : (i == nl ? real(0) : pt(1, i - nl - 1));
     }
     __device__ inline real Zz(int i, int nl) const {
-        return i < nl ? S(LL.zl, nl - 1 - i) : (i == nl ? real(0) : S(LL.zr, i - nl - 1));
+        return i < nl ? pt(5, nl - 1 - i) : (i == nl ? real(0) : pt(2, i - nl - 1));
     }
 
-    // sample_line! (src/local.jl:1501), as Lane::sample_line
+    // sample_line! (src/local.jl:1501), as Lane::sample_line: the segments' masses split over the lanes,
+    // added in order
     __device__ __noinline__ real sample_line(real ucat, real uoff, bool *guard) const {
         *guard = false;
         int nr = 0, nl = 0;
         int w = walks(&nr, &nl);
         if (w < 0) *guard = true;
-        if (w <= 0) return 0;
+        if (w <= 0 || !on) return 0;
         int nseg = nl + nr;
         real mx = -INFINITY;
-        for (int j = 0; j < nseg; ++j) {
+        for (int j = lane; j < nseg; j += G) {
             real p0 = P(j, nl), p1 = P(j + 1, nl), c0 = Cc(j, nl), c1 = Cc(j + 1, nl);
             real Ls = p1 - p0;
-            real lm = Ls > 0 ? -fmin(c0, c1) + logseg(Ls, fabs(c1 - c0)) : real(-INFINITY);
-            S(LL.lm, j) = lm;
-            mx = fmax(mx, lm);
+            real m = Ls > 0 ? -fmin(c0, c1) + logseg(Ls, fabs(c1 - c0)) : real(-INFINITY);
+            lm(j) = m;
+            mx = fmax(mx, m);
         }
+        sync();
+        mx = wmax(mx);
+        for (int j = lane; j < nseg; j += G) lm(j) = exp(lm(j) - mx);
+        sync();
         real tot = 0;
-        for (int j = 0; j < nseg; ++j) tot += exp(S(LL.lm, j) - mx);
+        for (int j = 0; j < nseg; ++j) tot += lm(j);
         real u = ucat * tot, acc = 0;
         int jj = nseg - 1;
         for (int q = 0; q < nseg; ++q) {
-            acc += exp(S(LL.lm, q) - mx);
+            acc += lm(q);
             if (u <= acc) {
                 jj = q;
                 break;
@@ -735,86 +856,118 @@ struct PLane {
 
     // logjac (src/local.jl:1871) of the compensations, in FP64 in both builds (the log-acceptance
     // ratio is an FP64 quantity; its inputs are the build's values)
-    __device__ double logjac(real t, bool *any) const {
+    __device__ __noinline__ double logjac(real t, bool *any) const {
+        auto lg = [&](int i) -> double {
+            if (S(LL.kv, i) == 0) return 0.0;
+            double Q = S(LL.kq, i);
+            return log(fabs((fmax(Q + (double)S(LL.kg, i) * (double)t, 0.0) + (double)S(LL.ke, i)) /
+                            (double)S(LL.kp, i)));
+        };
+        double *lw = reinterpret_cast<double *>(sm + LL.w);
+        if constexpr (G == 32) {
+            sync();
+            for (int i = lane; i < (lvl ? 0 : 2 * U); i += G) lw[i] = lg(i);
+            sync();
+        }
         double lj = 0;
         *any = false;
-        for (int i = 0; i < (lvl ? 0 : 2 * U); ++i) {
-            if (S(LL.kv, i) == 0) continue;
-            *any = true;
-            double Q = S(LL.kq, i);
-            lj += (double)S(LL.knm, i) *
-                  log(fabs((fmax(Q + (double)S(LL.kg, i) * (double)t, 0.0) + (double)S(LL.ke, i)) / (double)S(LL.kp, i)));
-        }
+        for (int s = 0; s < (lvl ? 0 : 2); ++s)
+            for (int u = 0; u < U; ++u) {
+                const int i = 2 * u + s;
+                if (S(LL.kv, i) == 0) continue;
+                *any = true;
+                lj += (double)S(LL.knm, i) * (G == 32 ? lw[i] : lg(i));
+            }
         return lj;
     }
 
     // commit_block! (src/local.jl:2495): states of charge, kinked dispatch, node balances (each
-    // global write by one lane)
+    // global write by one lane; all by one, in order, where two units share a node)
     __device__ __noinline__ void commit(real t) const {
         eval(t);
-        for (int u = 0; u < U; ++u) {
-            int n = node(u);
-            for (int s = 0; s < (lvl ? 0 : 2); ++s) {  // end steps: the compensation and the node balance
-                if (lane != 0) break;
-                int i = s * U + u, tau = tau_end(s);
-                real ph = S(LL.kph, i);
-                int c = 0;
-                for (int p = M.up[n]; p < M.up[n + 1] && c < ESM_PLAT_MAXK; ++p, ++c) {
-                    real ak = S(LL.ka, i * ESM_PLAT_MAXK + c);
-                    if (ak != 0) M.g[ix(M.ua[p], tau)] += ak * ph;
+        sync();
+        auto end = [&](int i) {  // an end step: the compensation and the node balance
+            const int u = i >> 1, n = node(u), tau = tau_end(i & 1);
+            real ph = S(LL.kph, i);
+            int c = 0;
+            for (int p = M.up[n]; p < M.up[n + 1] && c < LL.K; ++p, ++c) {
+                real ak = S(LL.ka, 5 * (i * LL.K + c));
+                if (ak != 0) M.g[ix(M.ua[p], tau)] += ak * ph;
+            }
+            M.r[ix(n, tau)] += S(LL.dr, i);
+        };
+        auto inner = [&](int u, bool in, int q) {  // an interior step whose injection changes
+            if (!in && quiet(u, q, t)) return;
+            real dj, d1;
+            sterm(u, q, t, &dj, &d1);
+            M.r[ix(node(u), stp(q))] += dj;
+        };
+        if (dup) {
+            if (lane == 0)
+                for (int u = 0; u < U; ++u) {
+                    for (int s = 0; s < (lvl ? 0 : 2); ++s) end(2 * u + s);
+                    const bool in = inside(u, t);
+                    const int nt = nterms(u, in);
+                    for (int i = 0; i < nt; ++i) inner(u, in, term_q(u, in, i));
                 }
-                M.r[ix(n, tau)] += S(LL.dr, i);
-            }
-            int nt = nterms(u, t);  // interior steps whose injection changes
-            bool in = inside(u, t);
-            for (int i = lane; i < nt; i += NL) {
-                int q = term_q(u, t, i);
-                if (!in && quiet(u, q, t)) continue;
-                real dj, d1;
-                sterm(u, q, t, &dj, &d1);
-                M.r[ix(n, stp(q))] += dj;
-            }
+        } else {
+            for (int i = lane; i < (lvl ? 0 : 2 * U); i += G) end(i);
+            each_term(
+                [&](int u, bool *in) {
+                    *in = inside(u, t);
+                    return nterms(u, *in);
+                },
+                inner);
         }
-        for (int u = 0; u < U; ++u)
-            for (int p = lane; p < ns(); p += NL) M.e[ix(uj[u], stp(q0() + p))] += t;
-        if constexpr (COOP) __syncwarp();
+        sync();
+        for (int u = 0; u < U; ++u) {
+            for (int p = lane; p < ns(); p += G) M.e[ix(uj[u], stp(q0() + p))] += t;
+            if (dup) sync();
+        }
+        sync();
     }
 };
 
-// One class pass of the storage multiscale sweep: threads take (block, replica) tasks (replica
-// fastest) and run the class's moves in order. COOP: one warp per task (long blocks, whose moves
-// loop over up to 128 steps and whose passes have few tasks).
-template <class real, bool COOP>
-__global__ void __launch_bounds__(128, 8) k_plateau(const __grid_constant__ DevModel<real> M,
-                                                 const __grid_constant__ PlatMoves mv, uint32_t sweep,
-                                                 real *scratch, unsigned long long *stats) {
-    PlatLayout LL = plat_layout(M.maxpts, ESM_PLAT_MAXU);
-    real local[ESM_PLAT_LOCAL];
-    size_t gid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    size_t nthr = (size_t)gridDim.x * blockDim.x;
-    bool loc = LL.total <= ESM_PLAT_LOCAL;
-    real *slab = loc ? local : scratch + gid;
-    PLane<real, COOP> Ln(M, LL, slab, loc ? 1 : (int)nthr);
-    Ln.lane = COOP ? (int)(threadIdx.x & 31) : 0;
+// One class pass of the storage multiscale sweep: threads (G 1) or warps (G 32) take (block, replica)
+// tasks, replica fastest, and run the class's moves in order. Blocks of one warp: the tasks of the
+// middle lengths make fewer warps than the device has schedulers.
+template <class real, int G>
+__global__ void __launch_bounds__(32, 16) k_plateau(const __grid_constant__ DevModel<real> M,
+                                                    const __grid_constant__ PlatMoves mv,
+                                                    const __grid_constant__ PlatLayout LL, uint32_t sweep,
+                                                    real *scratch, unsigned long long *stats) {
+    extern __shared__ __align__(16) char plat_smem[];
+    real local[G == 1 ? ESM_PLAT_LOCAL : 1];
+    const size_t n = (size_t)gridDim.x * (32 / G);  // tasks at a time
+    const size_t slot = (size_t)blockIdx.x * (32 / G) + (G == 1 ? threadIdx.x : 0);
+    const bool loc = LL.total <= ESM_PLAT_LOCAL;
+    real *lay = G == 32 ? reinterpret_cast<real *>(plat_smem) : loc ? local : scratch + slot;
+    PLane<real, G> Ln(M, LL, lay, G == 32 || loc ? 1 : (int)n, scratch + (G == 32 ? slot * LL.gtotal : 0));
     Ln.L = mv.L;
     unsigned long long tried = 0, moved = 0, guards = 0;
-    size_t ntask = (size_t)mv.nb * M.R;
-    size_t t0 = COOP ? gid >> 5 : gid, ts = COOP ? nthr >> 5 : nthr;
-    for (size_t task = t0; task < ntask; task += ts) {
-        int k = (int)(task / M.R);
-        Ln.rep = (int)(task % M.R);
+    const size_t ntask = (size_t)mv.nb * M.R;
+    const size_t wbase = (size_t)blockIdx.x * (32 / G);
+    for (size_t base = wbase; base < ntask; base += n) {  // (the threads of a warp stay together)
+        const size_t task = base + (slot - wbase);
+        Ln.on = task < ntask;
+        int k = (int)((Ln.on ? task : base) / M.R);
+        Ln.rep = (int)((Ln.on ? task : base) % M.R);
         Ln.b0 = mv.o + (2 * k + mv.cls) * mv.L;
         for (int m = 0; m < 8; ++m) {
             Ln.U = mv.nu[m];
             Ln.uj = mv.j[m];
             if (Ln.U <= 0) continue;
-            Ln.intervals();
-            Ln.kinks();
+            if (Ln.on) {
+                Ln.load();
+                Ln.intervals();
+                Ln.kinks();
+            }
             uint32_t w0 = 2u * (8u * (uint32_t)mv.li + (uint32_t)m);
             double uc, uo, uj, un;
             uniform2(M.seed, ESM_TAG_SML, w0, (uint32_t)Ln.b0, (uint32_t)Ln.rep, sweep, &uc, &uo);
             bool guard;
             real t = Ln.sample_line(unit_uniform<real>(uc), unit_uniform<real>(uo), &guard);
+            if (!Ln.on) continue;
             if (guard) ++guards;
             if (t != 0) {
                 bool any;
@@ -836,26 +989,22 @@ __global__ void __launch_bounds__(128, 8) k_plateau(const __grid_constant__ DevM
     }
 }
 
-// The long-range storage sweep (storage_long_sweep!, src/storage_long.jl:245): threads take (unit,
+// The long-range storage sweep (storage_long_sweep!, src/storage_long.jl:245): warps take (unit,
 // replica) tasks and run the unit's moves in order -- the level move (every instant of the year
 // rises) and the long-range plateaus (prep_slong!, :77: one unit, the cyclic instants a+1 .. a+L,
 // compensation at steps a and a+L). plan: per unit [stor index, moves, (L, a) per move]; L = T is the
 // level move. The moves of different units touch different nodes (one unit per node and carrier).
+// A move's points each go over up to T states, from shared memory where a year of them fits
+// (ESM_PLAT_STAGE); each lane goes on to its next state that a bound is near, not the warp.
 template <class real>
-__global__ void __launch_bounds__(128, 8) k_storage_long(const __grid_constant__ DevModel<real> M, const int *plan,
-                                                        int nunits, uint32_t sweep, real *scratch,
-                                                        unsigned long long *stats) {
-    PlatLayout LL = plat_layout(M.maxpts, ESM_PLAT_MAXU);
-    real local[ESM_PLAT_LOCAL];
-    size_t gid = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    size_t nthr = (size_t)gridDim.x * blockDim.x;
-    bool loc = LL.total <= ESM_PLAT_LOCAL;
-    real *slab = loc ? local : scratch + gid;
-    PLane<real, true> Ln(M, LL, slab, loc ? 1 : (int)nthr);  // one warp per task
-    Ln.lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(32, 16) k_storage_long(const __grid_constant__ DevModel<real> M, const int *plan,
+                                                     const __grid_constant__ PlatLayout LL, int nunits, uint32_t sweep,
+                                                     real *scratch, unsigned long long *stats) {
+    extern __shared__ __align__(16) char plat_smem[];
+    PLane<real, 32> Ln(M, LL, reinterpret_cast<real *>(plat_smem), 1, scratch + (size_t)blockIdx.x * LL.gtotal);
     unsigned long long tried = 0, moved = 0, guards = 0;
-    size_t ntask = (size_t)nunits * M.R;
-    for (size_t task = gid >> 5; task < ntask; task += nthr >> 5) {
+    const size_t ntask = (size_t)nunits * M.R;
+    for (size_t task = blockIdx.x; task < ntask; task += gridDim.x) {
         const int *pu = plan + (task / M.R) * ESM_SL_STRIDE;
         Ln.rep = (int)(task % M.R);
         Ln.U = 1;
@@ -865,6 +1014,7 @@ __global__ void __launch_bounds__(128, 8) k_storage_long(const __grid_constant__
             Ln.lvl = L >= M.T;
             Ln.L = Ln.lvl ? M.T : L;
             Ln.b0 = Ln.lvl ? 0 : a;
+            Ln.load();
             Ln.intervals();
             if (!Ln.lvl) Ln.kinks();
             double uc, uo, uj, un;
@@ -895,41 +1045,52 @@ __global__ void __launch_bounds__(128, 8) k_storage_long(const __grid_constant__
     }
 }
 
-template <class real>
-cudaError_t launch_storage_long(const DevModel<real> &M, const int *plan, int nunits, uint32_t sweep, real *scratch,
-                                int threads, unsigned long long *stats, cudaStream_t s) {
-    size_t nthr = (size_t)nunits * M.R * 32;  // one warp per (unit, replica) task
-    int blocks = (int)(((size_t)threads < nthr ? (size_t)threads : nthr) + 127) / 128;
-    k_storage_long<real><<<blocks, 128, 0, s>>>(M, plan, nunits, sweep, scratch, stats);
-    return cudaGetLastError();
-}
+// the layout of a task of the multiscale sweep's pass: a thread for blocks below 32 steps, else a warp
+inline bool plat_wide(int L) { return L >= 32; }
 
-// threads of k_plateau resident on the device, and the global scratch it needs per thread (0: the
-// local array suffices)
+// tasks of the storage kernels that the global scratch holds at a time, and the reals of one: the warps'
+// slabs (32 warps an SM), or the threads' layouts if the largest is beyond their local arrays. The
+// kernels' shared memory limit is set here.
 template <class real>
-int plateau_threads(const DevModel<real> &M) {
-    int nb = 0, dev = 0, nsm = 0;
+int plateau_slots(const DevModel<real> &M, int maxd) {
+    int dev = 0, nsm = 1, lim = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_plateau<real, false>, 128, 0) != cudaSuccess || nb < 1)
-        nb = 4;
-    return nb * nsm * 128;
+    cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaFuncSetAttribute(k_plateau<real, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    cudaFuncSetAttribute(k_storage_long<real>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    return nsm * (plat_layout(M.maxpts, ESM_PLAT_MAXU, maxd, 0, false).total <= ESM_PLAT_LOCAL ? 32 : 512);
 }
 template <class real>
-size_t plateau_scratch_reals(const DevModel<real> &M) {
-    PlatLayout LL = plat_layout(M.maxpts, ESM_PLAT_MAXU);
-    return LL.total <= ESM_PLAT_LOCAL ? 0 : (size_t)LL.total;
+size_t plateau_scratch_reals(const DevModel<real> &M, int maxd) {
+    const PlatLayout a = plat_layout(M.maxpts, ESM_PLAT_MAXU, maxd, 0, false), b = plat_layout(M.maxpts, 1, 1, 0, true);
+    return a.total > ESM_PLAT_LOCAL && a.total > b.gtotal ? a.total : b.gtotal;
 }
 template <class real>
-cudaError_t launch_plateau(const DevModel<real> &M, const PlatMoves &mv, uint32_t sweep, real *scratch, int threads,
-                           unsigned long long *stats, cudaStream_t s) {
-    bool coop = mv.L >= 32;  // long blocks: one warp per task
-    size_t nthr = (size_t)mv.nb * M.R * (coop ? 32 : 1);
-    int blocks = (int)(((size_t)threads < nthr ? (size_t)threads : nthr) + 127) / 128;
-    if (coop)
-        k_plateau<real, true><<<blocks, 128, 0, s>>>(M, mv, sweep, scratch, stats);
-    else
-        k_plateau<real, false><<<blocks, 128, 0, s>>>(M, mv, sweep, scratch, stats);
+cudaError_t launch_storage_long(const DevModel<real> &M, int maxd, const int *plan, int nunits, uint32_t sweep,
+                                real *scratch, int slots, unsigned long long *stats, cudaStream_t s) {
+    PlatLayout LL = plat_layout(M.maxpts, 1, maxd, M.T + 1, true);
+    if (LL.total * sizeof(real) > ESM_PLAT_STAGE) LL = plat_layout(M.maxpts, 1, maxd, 0, true);
+    size_t ntask = (size_t)nunits * M.R;  // one warp per (unit, replica) task
+    int blocks = (int)(ntask < (size_t)slots ? ntask : (size_t)slots);
+    k_storage_long<real><<<blocks, 32, LL.total * sizeof(real), s>>>(M, plan, LL, nunits, sweep, scratch, stats);
+    return cudaGetLastError();
+}
+template <class real>
+cudaError_t launch_plateau(const DevModel<real> &M, int maxd, const PlatMoves &mv, uint32_t sweep, real *scratch,
+                           int slots, unsigned long long *stats, cudaStream_t s) {
+    int U = 1;
+    for (int m = 0; m < 8; ++m) U = mv.nu[m] > U ? mv.nu[m] : U;
+    size_t ntask = (size_t)mv.nb * M.R;
+    if (plat_wide(mv.L)) {
+        PlatLayout LL = plat_layout(M.maxpts, U, maxd, mv.L + 2, true);
+        int blocks = (int)(ntask < (size_t)slots ? ntask : (size_t)slots);
+        k_plateau<real, 32><<<blocks, 32, LL.total * sizeof(real), s>>>(M, mv, LL, sweep, scratch, stats);
+    } else {
+        PlatLayout LL = plat_layout(M.maxpts, U, maxd, 0, false);
+        size_t n = LL.total <= ESM_PLAT_LOCAL || ntask < (size_t)slots ? ntask : (size_t)slots;
+        k_plateau<real, 1><<<(int)((n + 31) / 32), 32, 0, s>>>(M, mv, LL, sweep, scratch, stats);
+    }
     return cudaGetLastError();
 }
 
