@@ -107,8 +107,7 @@ struct esm_ctx {
     double kappa_min = 1.0;
     int *d_sl_plan = nullptr;            // the long-range sweep's per-unit move lists
     esm_ctx *probe = nullptr;            // one-replica context of the lag probe (esm_opts.probe)
-    int sms_slots = 0;                   // tasks of the storage kernels at a time
-    size_t sms_per = 0;                  // reals of global scratch per such task
+    size_t sms_reals = 0, sms_least = 0; // reals of the storage kernels' global scratch, and the least they run with
     int maxd = 0;                        // most dispatchable units at a node
     void *d_sms_scratch = nullptr;
     int scratch_warps = 0;               // line-move warps the global scratch holds (0: no global scratch needed)
@@ -732,10 +731,9 @@ int esm_create(const esm_model *m, const esm_opts *o, esm_ctx **out) {
         if (m->units_ptr[n + 1] - m->units_ptr[n] > ESM_PLAT_MAXK)
             return fail(c, ESM_EINVAL, "a node has more than %d dispatchable units", ESM_PLAT_MAXK);
     for (int n = 0; n < m->N; ++n) c->maxd = std::max(c->maxd, m->units_ptr[n + 1] - m->units_ptr[n]);
-    // storage sweeps: the tasks at a time; their global scratch is allocated at their first use (sms_scratch)
-    c->sms_slots = c->precision == 64 ? esm::plateau_slots<double>(c->Md, c->maxd) : esm::plateau_slots<float>(c->Mf, c->maxd);
-    c->sms_per = c->precision == 64 ? esm::plateau_scratch_reals<double>(c->Md, c->maxd)
-                                    : esm::plateau_scratch_reals<float>(c->Mf, c->maxd);
+    // the storage sweeps' global scratch is allocated at their first use (sms_scratch)
+    c->sms_reals = c->precision == 64 ? esm::plateau_scratch_reals<double>(c->Md, c->maxd, &c->sms_least)
+                                      : esm::plateau_scratch_reals<float>(c->Mf, c->maxd, &c->sms_least);
     // classes
     c->ncls = c->T % 2 ? 3 : 2;
     c->class_len.assign(3, 0);
@@ -1014,18 +1012,17 @@ int sms_plan(const esm_ctx *c, uint32_t sweep, bool force, std::vector<esm::Plat
     return (int)out.size();
 }
 
-// the storage kernels' global scratch, at their first use: at most 256 MB, the grid capped to the
-// tasks it holds
+// the storage kernels' global scratch, at their first use: at most 256 MB (one task's, if that is
+// more), the grids capped to the tasks it holds
 int sms_scratch(esm_ctx *c) {
     if (c->d_sms_scratch) return ESM_OK;
     size_t rb = c->precision == 64 ? sizeof(double) : sizeof(float);
-    size_t fit = ((size_t)256 << 20) / (c->sms_per * rb);
-    int slots = (int)std::min((size_t)c->sms_slots, std::max((size_t)32, fit / 32 * 32));
+    size_t n = std::max(c->sms_least, std::min(c->sms_reals, ((size_t)256 << 20) / rb));
     char *q;
-    int rc = dalloc(c, &q, c->sms_per * rb * (size_t)slots);
+    int rc = dalloc(c, &q, n * rb);
     if (rc) return rc;
     c->d_sms_scratch = q;
-    c->sms_slots = slots;
+    c->sms_reals = n;
     return ESM_OK;
 }
 
@@ -1042,10 +1039,10 @@ int sms_sweep_any(esm_ctx *c, uint32_t sweep, bool force, int max_passes = 0) {
     Span sp(c, ESM_KT_STORAGE);
     for (auto &mv : plan) {
         if (c->precision == 64)
-            CK(esm::launch_plateau<double>(c->Md, c->maxd, mv, sweep, (double *)c->d_sms_scratch, c->sms_slots,
+            CK(esm::launch_plateau<double>(c->Md, c->maxd, mv, sweep, (double *)c->d_sms_scratch, c->sms_reals,
                                            c->d_sms_stats, c->stream));
         else
-            CK(esm::launch_plateau<float>(c->Mf, c->maxd, mv, sweep, (float *)c->d_sms_scratch, c->sms_slots,
+            CK(esm::launch_plateau<float>(c->Mf, c->maxd, mv, sweep, (float *)c->d_sms_scratch, c->sms_reals,
                                           c->d_sms_stats, c->stream));
         c->launches += 1;
     }
@@ -1096,10 +1093,10 @@ int sl_sweep_any(esm_ctx *c, uint32_t sweep) {
     if (mlog) CK(cudaMemsetAsync(mlog, 0xff, sizeof(double) * nu * 5 * c->Md.mlog_nrep, c->stream));
     Span sp(c, ESM_KT_STORAGE);
     if (c->precision == 64)
-        CK(esm::launch_storage_long<double>(c->Md, c->maxd, c->d_sl_plan, nu, sweep, (double *)c->d_sms_scratch, c->sms_slots,
+        CK(esm::launch_storage_long<double>(c->Md, c->maxd, c->d_sl_plan, nu, sweep, (double *)c->d_sms_scratch, c->sms_reals,
                                             c->d_sms_stats, c->stream));
     else
-        CK(esm::launch_storage_long<float>(c->Mf, c->maxd, c->d_sl_plan, nu, sweep, (float *)c->d_sms_scratch, c->sms_slots,
+        CK(esm::launch_storage_long<float>(c->Mf, c->maxd, c->d_sl_plan, nu, sweep, (float *)c->d_sms_scratch, c->sms_reals,
                                            c->d_sms_stats, c->stream));
     c->launches += 1;
     return esm_sync(c, 600.0);  // (the host plan buffer is reused by the next call)

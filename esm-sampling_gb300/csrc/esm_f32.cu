@@ -10,11 +10,10 @@ cudaError_t launch_scores_f32(const DevModel<float> &Mf, const DevModel<double> 
     return launch_scores_f32_t<0>(Mf, Md, partial, sums, s);
 }
 cudaError_t preload_scores_f32() { return preload_scores_f32_t<0>(); }
-template int plateau_slots<float>(const DevModel<float> &, int);
-template size_t plateau_scratch_reals<float>(const DevModel<float> &, int);
-template cudaError_t launch_plateau<float>(const DevModel<float> &, int, const PlatMoves &, uint32_t, float *, int,
+template size_t plateau_scratch_reals<float>(const DevModel<float> &, int, size_t *);
+template cudaError_t launch_plateau<float>(const DevModel<float> &, int, const PlatMoves &, uint32_t, float *, size_t,
                                         unsigned long long *, cudaStream_t);
-template cudaError_t launch_storage_long<float>(const DevModel<float> &, int, const int *, int, uint32_t, float *, int,
+template cudaError_t launch_storage_long<float>(const DevModel<float> &, int, const int *, int, uint32_t, float *, size_t,
                                              unsigned long long *, cudaStream_t);
 template size_t linemove_scratch_reals<float>(const DevModel<float> &);
 template size_t linemove_smem_per_warp<float>(const DevModel<float> &);

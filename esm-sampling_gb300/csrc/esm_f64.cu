@@ -16,11 +16,10 @@ cudaError_t preload_score_kernels() {
     if ((e = cudaFuncGetAttributes(&a, k_score_finish<double>)) != cudaSuccess) return e;
     return cudaFuncGetAttributes(&a, k_set_kc<double>);
 }
-template int plateau_slots<double>(const DevModel<double> &, int);
-template size_t plateau_scratch_reals<double>(const DevModel<double> &, int);
-template cudaError_t launch_plateau<double>(const DevModel<double> &, int, const PlatMoves &, uint32_t, double *, int,
+template size_t plateau_scratch_reals<double>(const DevModel<double> &, int, size_t *);
+template cudaError_t launch_plateau<double>(const DevModel<double> &, int, const PlatMoves &, uint32_t, double *, size_t,
                                         unsigned long long *, cudaStream_t);
-template cudaError_t launch_storage_long<double>(const DevModel<double> &, int, const int *, int, uint32_t, double *, int,
+template cudaError_t launch_storage_long<double>(const DevModel<double> &, int, const int *, int, uint32_t, double *, size_t,
                                              unsigned long long *, cudaStream_t);
 template size_t linemove_scratch_reals<double>(const DevModel<double> &);
 template size_t linemove_smem_per_warp<double>(const DevModel<double> &);

@@ -97,16 +97,15 @@ struct PlatMoves {
     int j[8][ESM_PLAT_MAXU];    // storage unit indices (into stor)
 };
 // maxd: the most dispatchable units at a node
+// reals of the storage kernels' global scratch (*least: with which they still run, a task at a time)
 template <class real>
-int plateau_slots(const DevModel<real> &M, int maxd);  // tasks that the storage kernels' global scratch holds
-template <class real>
-size_t plateau_scratch_reals(const DevModel<real> &M, int maxd);  // reals per such task
+size_t plateau_scratch_reals(const DevModel<real> &M, int maxd, size_t *least);
 template <class real>
 cudaError_t launch_plateau(const DevModel<real> &M, int maxd, const PlatMoves &mv, uint32_t sweep, real *scratch,
-                           int slots, unsigned long long *stats, cudaStream_t s);
+                           size_t reals, unsigned long long *stats, cudaStream_t s);
 // ---- long-range storage sweep: per unit [stor index, moves, (L, a) per move], at most 5 moves
 #define ESM_SL_STRIDE 12
 template <class real>
 cudaError_t launch_storage_long(const DevModel<real> &M, int maxd, const int *plan, int nunits, uint32_t sweep,
-                                real *scratch, int slots, unsigned long long *stats, cudaStream_t s);
+                                real *scratch, size_t reals, unsigned long long *stats, cudaStream_t s);
 }  // namespace esm

@@ -11,10 +11,14 @@
 // the class's 8 moves in order. The move selections are state-independent and drawn on the host
 // from the class stream, as the local sweep's move list is. Blocks below 32 steps take one thread
 // a task: thousands of tasks, whose walks go through one state machine so that the threads of a
-// warp evaluate together. Longer blocks and the long-range moves take one warp a task, with the
-// move's states, units and ends in shared memory: the lanes take one (unit, end), one interior step
-// or one segment each, the sums are formed in a fixed order, and what the walk decides every lane
-// decides alike. @MAP@
+// warp evaluate together. Longer blocks take one warp a task and the long-range moves one block of 8
+// warps, with the move's states, units and ends in shared memory: the threads take one (unit, end),
+// one interior step or one segment each, the sums are formed in a fixed order, and what the walk
+// decides every thread decides alike. Bound by the latency and the instructions of the evaluations'
+// chains, not by memory. 40 nodes, T=2920, 64 replicas, one pass: 27.7 -> 12.0 ms for blocks of 2 steps
+// and 14.9 -> 6.4 ms for 16 (threads that part at every root and come together late -> one evaluation
+// site that they reach together), 8.2 -> 3.6 ms for 64 (every lane of a warp doing all of the ends ->
+// shared).
 //
 // Interior steps. At an interior step both state-of-charge values of a unit's storage term move by
 // t, so while every moved value stays strictly inside (0, 1) the term's cost, injection and
@@ -37,7 +41,8 @@ namespace esm {
 #define ESM_PLAT_LOCAL 4096  // reals of a thread's local array, if a task has one thread (larger layouts: the global slab)
 #define ESM_PLAT_PTS 48   // walk points per direction a warp's shared memory holds (beyond: the global slab)
 #define ESM_PLAT_ROOTS 32 // roots of either kind it holds (beyond: the global slab)
-#define ESM_PLAT_STAGE (100 << 10)  // a group's shared memory with the move's states in it (more: read from global memory)
+#define ESM_PLAT_LONG 256 // threads of a long-range task
+#define ESM_PLAT_STAGE (110 << 10)  // its shared memory with the year's states and terms in it (two blocks an SM)
 
 // a task's layout (reals): a thread's array or a warp's shared memory, and the warp's global slab for what
 // that does not hold
@@ -58,12 +63,16 @@ struct PlatLayout {
     int sb, pb;                          // [2U] end node balances, current / previous
     int w;                               // [2U * (K + 2)] an evaluation's terms, in the order of their sum
     int ys, ny;                          // [U * ny] the states at the block's positions (ny 0: not staged)
+    int tc, nt;                          // [6 * nt] a long-range move's terms: cost and size in the sum, injection
+                                         // and d of the two last points kept (nt 0: in the global slab)
+    int red;                             // [ESM_PLAT_LONG / 32] a long-range task's reductions
     int total;
-    int gp, gr, gl, gtotal;              // global slab: points, roots, masses
+    int gp, gr, gl, gc, gtotal;          // global slab: points, roots, masses, terms
 };
 
-// U units, K kinked units per node, ny staged positions; wide: of a warp
-__host__ __device__ inline PlatLayout plat_layout(int maxpts, int U, int K, int ny, bool wide) {
+// U units, K kinked units per node, ny staged positions; wide: of a warp or block; nt, ng: terms of a
+// long-range move kept in shared memory, in the global slab
+__host__ __device__ inline PlatLayout plat_layout(int maxpts, int U, int K, int ny, bool wide, int nt = 0, int ng = 0) {
     PlatLayout L;
     int o = 0;
     L.K = K;
@@ -96,15 +105,19 @@ __host__ __device__ inline PlatLayout plat_layout(int maxpts, int U, int K, int 
     L.sb = o; o += 2 * U;
     L.pb = o; o += 2 * U;
     L.ys = o; o += U * ny;
+    L.nt = nt;
+    L.tc = o; o += 6 * nt;
+    L.red = o; o += ESM_PLAT_LONG / 32;
     L.total = (o + 3) & ~3;
     L.gp = 0;
     L.gr = 6 * maxpts;
     L.gl = L.gr + 2 * ESM_PLAT_RB;
-    L.gtotal = (L.gl + 2 * maxpts + 1 + 3) & ~3;
+    L.gc = L.gl + 2 * maxpts + 1;
+    L.gtotal = (L.gc + 6 * ng + 3) & ~3;
     return L;
 }
 
-// One move at a time of a task of G lanes (1 or 32). The (unit, end) pair i = 2 u + s belongs to lane
+// One move at a time of a task of G lanes (a thread, a warp, or the ESM_PLAT_LONG threads of a block). The (unit, end) pair i = 2 u + s belongs to lane
 // i % G, which alone writes and reads its entries; what the walk needs of them goes through sums,
 // minima and the root buffers that every lane of the task receives.
 template <class real, int G>
@@ -120,28 +133,39 @@ struct PLane {
     bool dup = false;  // two units at one node
     const int *uj;  // the move's storage units
     mutable real nzs = 0;
+    mutable int buf = 0;  // the kept terms that the next evaluation writes (the other: those at the last point saved)
 
     __device__ PLane(const DevModel<real> &M_, const PlatLayout &LL_, real *sm_, int sstride_, real *gm_)
-        : M(M_), LL(LL_), sm(sm_), gm(gm_), sstride(sstride_), lane(G == 1 ? 0 : threadIdx.x & 31) {}
+        : M(M_), LL(LL_), sm(sm_), gm(gm_), sstride(sstride_), lane(G == 1 ? 0 : threadIdx.x) {}
     __device__ inline void sync() const {
         if constexpr (G == 32) __syncwarp();
+        if constexpr (G > 32) __syncthreads();
     }
-    __device__ inline real bcast(real v, int l) const { return G == 1 ? v : __shfl_sync(0xffffffffu, v, l); }
+    // within a warp
     __device__ inline real wsum(real v) const {
-        for (int o = G / 2; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        return bcast(v, 0);
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        return __shfl_sync(0xffffffffu, v, 0);
     }
     __device__ inline real wmin(real v) const {
-        for (int o = G / 2; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
+        for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
         return v;
     }
-    __device__ inline real wmax(real v) const {
-        for (int o = G / 2; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    __device__ inline real wmax(real v) const { return -wmin(-v); }
+    // over the task, on every lane
+    __device__ inline real tmin(real v) const {
+        if constexpr (G > 1) v = wmin(v);
+        if constexpr (G > 32) {
+            sync();
+            if (lane % 32 == 0) S(LL.red, lane / 32) = v;
+            sync();
+            for (int w = 0; w < G / 32; ++w) v = fmin(v, S(LL.red, w));
+        }
         return v;
     }
+    __device__ inline real tmax(real v) const { return -tmin(-v); }
 
     __device__ inline real &S(int off, int i) const {
-        return G == 32 ? sm[off + i] : sm[(size_t)(off + i) * sstride];
+        return G > 1 ? sm[off + i] : sm[(size_t)(off + i) * sstride];
     }
     // walk point i of array a (0 position, 1 cost, 2 round-off bound to the right; 3, 4, 5 to the left)
     __device__ inline real &pt(int a, int i) const {
@@ -152,17 +176,19 @@ struct PLane {
         return G == 1 || i < LL.nrt ? S(LL.ro, h * LL.nrt + i) : gm[LL.gr + h * ESM_PLAT_RB + i];
     }
     __device__ inline real &lm(int j) const { return G == 1 || j < 2 * LL.nrt ? S(LL.ro, j) : gm[LL.gl + j]; }
+    // kept term array a (0 cost, 1 size; 2, 3 injection and 4, 5 d of either buffer), term i
+    __device__ inline real &tc(int a, int i) const { return LL.nt ? sm[LL.tc + a * LL.nt + i] : gm[LL.gc + a * M.T + i]; }
     __device__ inline int &cnt(int h) const { return reinterpret_cast<int *>(sm + LL.cnt)[h]; }
     __device__ inline size_t ix(int x, int t) const { return sidx(x, t, rep, M.T, M.R); }
     // unit data: 0 capacity, 1 hours, 2 inflow, 3 and 4 efficiencies, 5 marginal cost (a thread's task reads
     // the model, at the same address as its warp's others)
     __device__ inline real par(int u, int k) const {
-        if constexpr (G == 32) return S(LL.par, 7 * u + k);
+        if constexpr (G > 1) return S(LL.par, 7 * u + k);
         const int j = uj[u];
         const real *const f[6] = {M.kc_s, M.s_hours, M.s_qt, M.s_etain, M.s_etaout, M.s_mc};
         return f[k][j];
     }
-    __device__ inline int node(int u) const { return G == 32 ? (int)S(LL.par, 7 * u + 6) : M.s_bus[uj[u]]; }
+    __device__ inline int node(int u) const { return G > 1 ? (int)S(LL.par, 7 * u + 6) : M.s_bus[uj[u]]; }
     // block positions: step b0 + q, cyclic (the long-range plateaus wrap); the interior terms (both
     // states raised) are q0() .. q0() + nq() - 1, the raised states q0() .. q0() + ns() - 1
     __device__ inline int cyc(int x) const { return x >= M.T ? x - M.T : x; }
@@ -172,9 +198,9 @@ struct PLane {
     __device__ inline int ns() const { return lvl ? M.T : L; }
     __device__ inline int tau_end(int s) const { return s == 0 ? stp(0) : stp(L); }
     // the state of unit u at position q, and at the one after it
-    __device__ inline real Y(int u, int q) const { return G == 32 && LL.ny ? S(LL.ys, u * LL.ny + q) : M.e[ix(uj[u], stp(q))]; }
+    __device__ inline real Y(int u, int q) const { return G > 1 && LL.ny ? S(LL.ys, u * LL.ny + q) : M.e[ix(uj[u], stp(q))]; }
     __device__ inline real Y1(int u, int q) const {
-        return G == 32 && LL.ny ? S(LL.ys, u * LL.ny + (lvl && q + 1 == M.T ? 0 : q + 1)) : M.e[ix(uj[u], cyc(stp(q) + 1))];
+        return G > 1 && LL.ny ? S(LL.ys, u * LL.ny + (lvl && q + 1 == M.T ? 0 : q + 1)) : M.e[ix(uj[u], cyc(stp(q) + 1))];
     }
     // an interior term whose two states stay strictly inside (0, 1) at t is exactly unchanged
     __device__ inline bool quiet(int u, int q, real t) const {
@@ -287,7 +313,8 @@ struct PLane {
     // interval, the other interior terms are exactly unchanged. A unit with more than NACT such
     // steps gets an empty interval (evaluated whole).
     __device__ __noinline__ void intervals() const {
-        for (int u = 0; u < U; ++u) {
+        constexpr int W = G > 1 ? 32 : 1;  // (a block's first warp)
+        for (int u = 0; u < (lane < W ? U : 0); ++u) {
             real mn = 2, mx = -1;
             int na = 0;
             bool over = false;
@@ -296,7 +323,7 @@ struct PLane {
                     if (S(LL.act, u * ESM_PLAT_NACT + i) == real(qt)) return;
                 if (na < ESM_PLAT_NACT) {
                     S(LL.act, u * ESM_PLAT_NACT + na++) = real(qt);  // (every lane writes the same value)
-                    sync();
+                    if constexpr (G > 1) __syncwarp();
                 } else {
                     over = true;
                 }
@@ -310,7 +337,7 @@ struct PLane {
                     if (q <= L - 1) list(q);
                 }
             };
-            for (int base = 0; base < ns(); base += G) {
+            for (int base = 0; base < ns(); base += W) {
                 int p = base + lane, qo = -1;
                 if (p < ns()) {
                     int q = q0() + p;
@@ -323,7 +350,7 @@ struct PLane {
                     }
                 }
                 // the states outside the box, in step order, listed alike on every lane
-                if constexpr (G == 32) {
+                if constexpr (G > 1) {
                     unsigned bal = over ? 0u : __ballot_sync(0xffffffffu, qo >= 0);
                     while (bal && !over) {
                         int l = __ffs(bal) - 1;
@@ -334,8 +361,10 @@ struct PLane {
                     out_state(qo);
                 }
             }
-            mn = wmin(mn);
-            mx = wmax(mx);
+            if constexpr (G > 1) {
+                mn = wmin(mn);
+                mx = wmax(mx);
+            }
             bool ok = !over && mn <= mx;
             if (lane == 0) {
                 if (!over && mn > mx) {  // every raised state outside the box: no interval, terms listed
@@ -380,32 +409,54 @@ struct PLane {
         const real dt = M.dt, cv = M.c_viol, k0 = M.kappa0;
         real D = 0, A = 0;
         // interior steps of a unit: storage term and node balance; the listed terms in order, the terms of
-        // a unit outside its interval by lanes, each on to its next term that changes
+        // a unit outside its interval by lanes of a warp, each on to its next term that changes. (The warps
+        // of a long-range task take every 8th round and keep the terms, which its first warp sums as if
+        // it had made them, and from which collect takes the secondaries.)
         auto inner = [&](int u) {
             const bool in = inside(u, t);
             const int nt = nterms(u, in);
             real Di = 0, Ai = 0;
-            auto term = [&](int q, real *v, real *a) {
-                real dj, d1;
-                real cs = sterm(u, q, t, &dj, &d1);
-                real cb = dt * phibal_diff<real>(M.r[ix(node(u), stp(q))], dj, M.c_shed, M.c_dump);
+            auto term = [&](int q, real *v, real *a, real *dj, real *d1) {
+                real cs = sterm(u, q, t, dj, d1);
+                real cb = dt * phibal_diff<real>(M.r[ix(node(u), stp(q))], *dj, M.c_shed, M.c_dump);
                 *v = cs + cb;
                 *a = fabs(cs) + fabs(cb);
             };
-            if (G == 32 && in) {
-                real v = 0, a = 0;
-                if (lane < nt) term(term_q(u, true, lane), &v, &a);
-                for (int l = 0; l < nt; ++l) {
-                    Di += bcast(v, l);
-                    Ai += bcast(a, l);
+            real v = 0, a = 0, dj, d1;
+            if (G > 1 && in) {
+                if (lane < nt) term(term_q(u, true, lane), &v, &a, &dj, &d1);
+                if (lane < 32)
+                    for (int l = 0; l < nt; ++l) {
+                        Di += __shfl_sync(0xffffffffu, v, l);
+                        Ai += __shfl_sync(0xffffffffu, a, l);
+                    }
+            } else if constexpr (G > 32) {
+                for (int i = lane; i < nt; i += G) {
+                    v = a = 0;
+                    if (!quiet(u, q0() + i, t)) {
+                        term(q0() + i, &v, &a, &dj, &d1);
+                        tc(2 + buf, i) = dj;
+                        tc(4 + buf, i) = d1;
+                    }
+                    tc(0, i) = v;
+                    tc(1, i) = a;
+                }
+                sync();
+                if (lane < 32) {
+#pragma unroll 8
+                    for (int i = lane; i < nt; i += 32) {
+                        Di += tc(0, i);
+                        Ai += tc(1, i);
+                    }
+                    Di = wsum(Di);
+                    Ai = wsum(Ai);
                 }
             } else {
                 int i = lane;
                 while (true) {
                     while (i < nt && !in && quiet(u, q0() + i, t)) i += G;
                     if (i >= nt) break;
-                    real v, a;
-                    term(term_q(u, in, i), &v, &a);
+                    term(term_q(u, in, i), &v, &a, &dj, &d1);
                     Di += v;
                     Ai += a;
                     i += G;
@@ -429,7 +480,7 @@ struct PLane {
             const int u = i >> 1, s = i & 1, q = s == 0 ? 0 : L;
             const int w = i * (LL.K + 2);
             auto add = [&](int h, real v) {  // a term of the sum
-                if constexpr (G == 32) {
+                if constexpr (G > 1) {
                     S(LL.w, w + h) = v;
                 } else {
                     D += v;
@@ -464,7 +515,7 @@ struct PLane {
             S(LL.sb, i) = r0 + dr;
             if (G == 1 && s == 1) inner(u);
         }
-        if constexpr (G == 32) {
+        if constexpr (G > 1) {
             for (int u = 0; u < U; ++u) inner(u);
             sync();
             for (int u = 0; u < U; ++u) {
@@ -486,6 +537,7 @@ struct PLane {
             for (int h = 0; h < 3; ++h) S(LL.p3, 3 * i + h) = S(LL.s3, 3 * i + h);
             S(LL.pb, i) = S(LL.sb, i);
         }
+        buf ^= 1;
     }
 
     __device__ static inline bool root_of(real a, real b, real lo, real hi, real sgn, real *x) {
@@ -508,7 +560,7 @@ struct PLane {
     // units whose states leave their interval in [lo, hi]
     __device__ __noinline__ void collect(real lo, real hi, real sgn, bool want_stor, int *nro, int *ngro) const {
         int n[2] = {0, 0};
-        if constexpr (G == 32) {
+        if constexpr (G > 1) {
             sync();
             if (lane < 2) cnt(lane) = 0;
             sync();
@@ -528,8 +580,18 @@ struct PLane {
             [&](int u, bool in, int q) {
                 if (!in && quiet(u, q, lo) && quiet(u, q, hi)) return;
                 real dja, d1a, djb, d1b;
-                sterm(u, q, lo, &dja, &d1a);
-                sterm(u, q, hi, &djb, &d1b);
+                if (G > 32 && !inside(u, lo) && !quiet(u, q, lo)) {  // (as the evaluation at lo kept it)
+                    dja = tc(2 + (buf ^ 1), q - q0());
+                    d1a = tc(4 + (buf ^ 1), q - q0());
+                } else {
+                    sterm(u, q, lo, &dja, &d1a);
+                }
+                if (G > 32 && !inside(u, hi) && !quiet(u, q, hi)) {
+                    djb = tc(2 + buf, q - q0());
+                    d1b = tc(4 + buf, q - q0());
+                } else {
+                    sterm(u, q, hi, &djb, &d1b);
+                }
                 if (want_stor) {
                     real a3[3], b3[3];
                     sec3(u, d1a, a3);
@@ -540,7 +602,7 @@ struct PLane {
                 real r0 = M.r[ix(node(u), stp(q))];
                 if (root_of(r0 + dja, r0 + djb, lo, hi, sgn, &x)) add_root(0, x, n);
             });
-        if constexpr (G == 32) {
+        if constexpr (G > 1) {
             sync();
             n[0] = cnt(0);
             n[1] = cnt(1);
@@ -626,7 +688,7 @@ struct PLane {
             i += G;
         }
         sync();
-        real key = wmin(have ? sgn * best : real(INFINITY));  // the nearest over the lanes (a sign flip is exact)
+        real key = tmin(have ? sgn * best : real(INFINITY));  // the nearest over the lanes (a sign flip is exact)
         have = key < real(INFINITY);
         *out = have ? sgn * key : real(0);
         return have;
@@ -821,7 +883,7 @@ struct PLane {
             mx = fmax(mx, m);
         }
         sync();
-        mx = wmax(mx);
+        mx = tmax(mx);
         for (int j = lane; j < nseg; j += G) lm(j) = exp(lm(j) - mx);
         sync();
         real tot = 0;
@@ -864,7 +926,7 @@ struct PLane {
                             (double)S(LL.kp, i)));
         };
         double *lw = reinterpret_cast<double *>(sm + LL.w);
-        if constexpr (G == 32) {
+        if constexpr (G > 1) {
             sync();
             for (int i = lane; i < (lvl ? 0 : 2 * U); i += G) lw[i] = lg(i);
             sync();
@@ -876,7 +938,7 @@ struct PLane {
                 const int i = 2 * u + s;
                 if (S(LL.kv, i) == 0) continue;
                 *any = true;
-                lj += (double)S(LL.knm, i) * (G == 32 ? lw[i] : lg(i));
+                lj += (double)S(LL.knm, i) * (G > 1 ? lw[i] : lg(i));
             }
         return lj;
     }
@@ -989,19 +1051,23 @@ __global__ void __launch_bounds__(32, 16) k_plateau(const __grid_constant__ DevM
     }
 }
 
-// The long-range storage sweep (storage_long_sweep!, src/storage_long.jl:245): warps take (unit,
-// replica) tasks and run the unit's moves in order -- the level move (every instant of the year
+// The long-range storage sweep (storage_long_sweep!, src/storage_long.jl:245): warps or blocks of G
+// threads take (unit, replica) tasks and run the unit's moves in order -- the level move (every instant of the year
 // rises) and the long-range plateaus (prep_slong!, :77: one unit, the cyclic instants a+1 .. a+L,
 // compensation at steps a and a+L). plan: per unit [stor index, moves, (L, a) per move]; L = T is the
 // level move. The moves of different units touch different nodes (one unit per node and carrier).
-// A move's points each go over up to T states, from shared memory where a year of them fits
-// (ESM_PLAT_STAGE); each lane goes on to its next state that a bound is near, not the warp.
-template <class real>
-__global__ void __launch_bounds__(32, 16) k_storage_long(const __grid_constant__ DevModel<real> M, const int *plan,
-                                                     const __grid_constant__ PlatLayout LL, int nunits, uint32_t sweep,
-                                                     real *scratch, unsigned long long *stats) {
+// A move's points each go over up to T states and evaluate those that a bound is near: the states and
+// the terms of the last two points stay in shared memory where a year of them fits (ESM_PLAT_STAGE;
+// else the terms in the global slab), so that the roots between two points need no second evaluation.
+// G is 256, or 32 for a year of
+// at most 256 steps, where 8 warps wait for one another longer than they share (T=120, 33 units, 33
+// replicas: 1.6 ms with 32, 2.1 with 256). 40 units, T=2920: 80 -> 25 ms at 16 replicas, 106 -> 47 at 64.
+template <class real, int G>
+__global__ void __launch_bounds__(G, 512 / G) k_storage_long(const __grid_constant__ DevModel<real> M, const int *plan,
+                                                          const __grid_constant__ PlatLayout LL, int nunits,
+                                                          uint32_t sweep, real *scratch, unsigned long long *stats) {
     extern __shared__ __align__(16) char plat_smem[];
-    PLane<real, 32> Ln(M, LL, reinterpret_cast<real *>(plat_smem), 1, scratch + (size_t)blockIdx.x * LL.gtotal);
+    PLane<real, G> Ln(M, LL, reinterpret_cast<real *>(plat_smem), 1, scratch + (size_t)blockIdx.x * LL.gtotal);
     unsigned long long tried = 0, moved = 0, guards = 0;
     const size_t ntask = (size_t)nunits * M.R;
     for (size_t task = blockIdx.x; task < ntask; task += gridDim.x) {
@@ -1048,48 +1114,64 @@ __global__ void __launch_bounds__(32, 16) k_storage_long(const __grid_constant__
 // the layout of a task of the multiscale sweep's pass: a thread for blocks below 32 steps, else a warp
 inline bool plat_wide(int L) { return L >= 32; }
 
-// tasks of the storage kernels that the global scratch holds at a time, and the reals of one: the warps'
-// slabs (32 warps an SM), or the threads' layouts if the largest is beyond their local arrays. The
-// kernels' shared memory limit is set here.
+inline bool long_block(int T) { return T > 256; }
+// the layout of a long-range task: states and terms in shared memory, the terms in the global slab, or both there
 template <class real>
-int plateau_slots(const DevModel<real> &M, int maxd) {
+PlatLayout long_layout(const DevModel<real> &M, int maxd) {
+    if (!long_block(M.T)) return plat_layout(M.maxpts, 1, maxd, M.T + 1, true);
+    PlatLayout LL = plat_layout(M.maxpts, 1, maxd, M.T + 1, true, M.T);
+    if (LL.total * sizeof(real) > ESM_PLAT_STAGE) LL = plat_layout(M.maxpts, 1, maxd, M.T + 1, true, 0, M.T);
+    if (LL.total * sizeof(real) > ESM_PLAT_STAGE) LL = plat_layout(M.maxpts, 1, maxd, 0, true, 0, M.T);
+    return LL;
+}
+
+// the reals of global scratch that the storage kernels use if they can have them: the slabs of 32 warps an
+// SM or 2 long-range tasks an SM, or the layouts of 512 threads an SM if the largest is beyond their
+// local arrays. The kernels' shared memory limit is set here.
+template <class real>
+size_t plateau_scratch_reals(const DevModel<real> &M, int maxd, size_t *least) {
     int dev = 0, nsm = 1, lim = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&lim, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaFuncSetAttribute(k_plateau<real, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(k_storage_long<real>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    return nsm * (plat_layout(M.maxpts, ESM_PLAT_MAXU, maxd, 0, false).total <= ESM_PLAT_LOCAL ? 32 : 512);
-}
-template <class real>
-size_t plateau_scratch_reals(const DevModel<real> &M, int maxd) {
-    const PlatLayout a = plat_layout(M.maxpts, ESM_PLAT_MAXU, maxd, 0, false), b = plat_layout(M.maxpts, 1, 1, 0, true);
-    return a.total > ESM_PLAT_LOCAL && a.total > b.gtotal ? a.total : b.gtotal;
+    cudaFuncSetAttribute(k_storage_long<real, ESM_PLAT_LONG>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    const size_t thread = plat_layout(M.maxpts, ESM_PLAT_MAXU, maxd, 0, false).total;
+    const size_t warp = plat_layout(M.maxpts, 1, 1, 0, true).gtotal, lng = long_layout(M, maxd).gtotal;
+    const size_t t = thread <= ESM_PLAT_LOCAL ? 0 : thread;
+    auto most = [](size_t a, size_t b, size_t c) { return a > b ? (a > c ? a : c) : (b > c ? b : c); };
+    *least = most(32 * t, warp, lng);  // one task each
+    return most((size_t)nsm * 512 * t, (size_t)nsm * 32 * warp, (size_t)nsm * 2 * lng);
 }
 template <class real>
 cudaError_t launch_storage_long(const DevModel<real> &M, int maxd, const int *plan, int nunits, uint32_t sweep,
-                                real *scratch, int slots, unsigned long long *stats, cudaStream_t s) {
-    PlatLayout LL = plat_layout(M.maxpts, 1, maxd, M.T + 1, true);
-    if (LL.total * sizeof(real) > ESM_PLAT_STAGE) LL = plat_layout(M.maxpts, 1, maxd, 0, true);
-    size_t ntask = (size_t)nunits * M.R;  // one warp per (unit, replica) task
-    int blocks = (int)(ntask < (size_t)slots ? ntask : (size_t)slots);
-    k_storage_long<real><<<blocks, 32, LL.total * sizeof(real), s>>>(M, plan, LL, nunits, sweep, scratch, stats);
+                                real *scratch, size_t reals, unsigned long long *stats, cudaStream_t s) {
+    const PlatLayout LL = long_layout(M, maxd);
+    const size_t ntask = (size_t)nunits * M.R, slots = reals / LL.gtotal;
+    const unsigned blocks = (unsigned)(ntask < slots ? ntask : slots);
+    const size_t smem = LL.total * sizeof(real);
+    if (long_block(M.T))
+        k_storage_long<real, ESM_PLAT_LONG><<<blocks, ESM_PLAT_LONG, smem, s>>>(M, plan, LL, nunits, sweep, scratch, stats);
+    else
+        k_storage_long<real, 32><<<blocks, 32, smem, s>>>(M, plan, LL, nunits, sweep, scratch, stats);
     return cudaGetLastError();
 }
 template <class real>
 cudaError_t launch_plateau(const DevModel<real> &M, int maxd, const PlatMoves &mv, uint32_t sweep, real *scratch,
-                           int slots, unsigned long long *stats, cudaStream_t s) {
+                           size_t reals, unsigned long long *stats, cudaStream_t s) {
     int U = 1;
     for (int m = 0; m < 8; ++m) U = mv.nu[m] > U ? mv.nu[m] : U;
     size_t ntask = (size_t)mv.nb * M.R;
     if (plat_wide(mv.L)) {
-        PlatLayout LL = plat_layout(M.maxpts, U, maxd, mv.L + 2, true);
-        int blocks = (int)(ntask < (size_t)slots ? ntask : (size_t)slots);
-        k_plateau<real, 32><<<blocks, 32, LL.total * sizeof(real), s>>>(M, mv, LL, sweep, scratch, stats);
+        const PlatLayout LL = plat_layout(M.maxpts, U, maxd, mv.L + 2, true);
+        const size_t slots = reals / LL.gtotal;
+        k_plateau<real, 32><<<(unsigned)(ntask < slots ? ntask : slots), 32, LL.total * sizeof(real), s>>>(
+            M, mv, LL, sweep, scratch, stats);
     } else {
-        PlatLayout LL = plat_layout(M.maxpts, U, maxd, 0, false);
-        size_t n = LL.total <= ESM_PLAT_LOCAL || ntask < (size_t)slots ? ntask : (size_t)slots;
-        k_plateau<real, 1><<<(int)((n + 31) / 32), 32, 0, s>>>(M, mv, LL, sweep, scratch, stats);
+        const PlatLayout LL = plat_layout(M.maxpts, U, maxd, 0, false);
+        const size_t warps = (ntask + 31) / 32, slots = reals / LL.total / 32;
+        k_plateau<real, 1><<<(unsigned)(LL.total <= ESM_PLAT_LOCAL || warps < slots ? warps : slots), 32, 0, s>>>(
+            M, mv, LL, sweep, scratch, stats);
     }
     return cudaGetLastError();
 }
