@@ -10,8 +10,8 @@
 // is one launch in which tasks (block, replica), replica fastest (neighbouring state access), run
 // the class's 8 moves in order. The move selections are state-independent and drawn on the host
 // from the class stream, as the local sweep's move list is. Blocks below 32 steps take one thread
-// a task: thousands of tasks, whose walks go through one state machine so that the threads of a
-// warp evaluate together. Longer blocks take one warp a task and the long-range moves one block of 8
+// a task where there are thousands of tasks, whose walks go through one state machine so that the threads of a
+// warp evaluate together. Longer blocks, and few tasks, take one warp a task and the long-range moves one block of 8
 // warps, with the move's states, units and ends in shared memory: the threads take one (unit, end),
 // one interior step or one segment each, the sums are formed in a fixed order, and what the walk
 // decides every thread decides alike. Bound by the latency and the instructions of the evaluations'
@@ -41,6 +41,7 @@ namespace esm {
 #define ESM_PLAT_LOCAL 4096  // reals of a thread's local array, if a task has one thread (larger layouts: the global slab)
 #define ESM_PLAT_PTS 48   // walk points per direction a warp's shared memory holds (beyond: the global slab)
 #define ESM_PLAT_ROOTS 32 // roots of either kind it holds (beyond: the global slab)
+#define ESM_PLAT_SHORT 32 // blocks below this length: at most a warp's interior steps, summed in order
 #define ESM_PLAT_LONG 256 // threads of a long-range task
 #define ESM_PLAT_STAGE (110 << 10)  // its shared memory with the year's states and terms in it (two blocks an SM)
 
@@ -131,6 +132,7 @@ struct PLane {
     int L, b0, rep, U;
     bool lvl = false;  // the level move of the long-range sweep: every instant of the year rises, no end steps
     bool dup = false;  // two units at one node
+    bool inorder = false;  // a short block's: interior sums in step order, whatever G
     const int *uj;  // the move's storage units
     mutable real nzs = 0;
     mutable int buf = 0;  // the kept terms that the next evaluation writes (the other: those at the last point saved)
@@ -408,8 +410,9 @@ struct PLane {
     __device__ __noinline__ real eval(real t) const {
         const real dt = M.dt, cv = M.c_viol, k0 = M.kappa0;
         real D = 0, A = 0;
-        // interior steps of a unit: storage term and node balance; the listed terms in order, the terms of
-        // a unit outside its interval by lanes of a warp, each on to its next term that changes. (The warps
+        // interior steps of a unit: storage term and node balance; the listed terms and those of a short
+        // block in order, the terms of a longer one outside the unit's interval by lanes of a warp, each
+        // on to its next term that changes. (The warps
         // of a long-range task take every 8th round and keep the terms, which its first warp sums as if
         // it had made them, and from which collect takes the secondaries.)
         auto inner = [&](int u) {
@@ -423,8 +426,9 @@ struct PLane {
                 *a = fabs(cs) + fabs(cb);
             };
             real v = 0, a = 0, dj, d1;
-            if (G > 1 && in) {
-                if (lane < nt) term(term_q(u, true, lane), &v, &a, &dj, &d1);
+            if (G > 1 && (in || (G == 32 && inorder))) {  // (no more than a warp's lanes)
+                const int q = lane < nt ? term_q(u, in, lane) : 0;
+                if (lane < nt && (in || !quiet(u, q, t))) term(q, &v, &a, &dj, &d1);
                 if (lane < 32)
                     for (int l = 0; l < nt; ++l) {
                         Di += __shfl_sync(0xffffffffu, v, l);
@@ -1006,6 +1010,7 @@ __global__ void __launch_bounds__(32, 16) k_plateau(const __grid_constant__ DevM
     real *lay = G == 32 ? reinterpret_cast<real *>(plat_smem) : loc ? local : scratch + slot;
     PLane<real, G> Ln(M, LL, lay, G == 32 || loc ? 1 : (int)n, scratch + (G == 32 ? slot * LL.gtotal : 0));
     Ln.L = mv.L;
+    Ln.inorder = mv.L < ESM_PLAT_SHORT;
     unsigned long long tried = 0, moved = 0, guards = 0;
     const size_t ntask = (size_t)mv.nb * M.R;
     const size_t wbase = (size_t)blockIdx.x * (32 / G);
@@ -1111,8 +1116,18 @@ __global__ void __launch_bounds__(G, 512 / G) k_storage_long(const __grid_consta
     }
 }
 
-// the layout of a task of the multiscale sweep's pass: a thread for blocks below 32 steps, else a warp
-inline bool plat_wide(int L) { return L >= 32; }
+// A class pass's tasks take a warp each if the blocks are long, whose interior steps the lanes share, or
+// if the tasks are no more than the warps that the device holds at 128 registers (16 an SM): by threads,
+// a pass takes as long as the longest walk of 32 however few they are. 40 nodes, T=584, 16 replicas (at
+// most 2336 tasks a pass): a sweep takes 61 ms by threads, 29 by warps; 12 nodes, T=24, 4 replicas: 22 and
+// 6.6. Beyond, the threads of a warp share its instructions: 40 nodes, T=2920, 64 replicas, 5824 tasks of 16
+// steps take 4.5 to 6.5 ms by threads, and half as many of 32 steps 4.8 to 5.4 by warps.
+inline bool plat_wide(int L, size_t ntask) {
+    int dev = 0, nsm = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    return L >= ESM_PLAT_SHORT || ntask <= (size_t)nsm * 16;
+}
 
 inline bool long_block(int T) { return T > 256; }
 // the layout of a long-range task: states and terms in shared memory, the terms in the global slab, or both there
@@ -1162,7 +1177,7 @@ cudaError_t launch_plateau(const DevModel<real> &M, int maxd, const PlatMoves &m
     int U = 1;
     for (int m = 0; m < 8; ++m) U = mv.nu[m] > U ? mv.nu[m] : U;
     size_t ntask = (size_t)mv.nb * M.R;
-    if (plat_wide(mv.L)) {
+    if (plat_wide(mv.L, ntask)) {
         const PlatLayout LL = plat_layout(M.maxpts, U, maxd, mv.L + 2, true);
         const size_t slots = reals / LL.gtotal;
         k_plateau<real, 32><<<(unsigned)(ntask < slots ? ntask : slots), 32, LL.total * sizeof(real), s>>>(
