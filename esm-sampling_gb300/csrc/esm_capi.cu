@@ -634,7 +634,7 @@ int class_pass_any(esm_ctx *c, uint32_t sweep, int cls, int limit = 0) {
     CK(cudaGetLastError());
     int nmoves = c->precision == 64 ? c->Md.natoms + c->Md.nextra : c->Mf.natoms + c->Mf.nextra;
     int nrun = limit > 0 && limit < nmoves ? limit : nmoves;
-    c->launches += 2 + (c->mblocks > 0 ? 2 : 1) * nrun;
+    c->launches += 3 + (c->mblocks > 0 ? 2 : 1) * nrun;
     if (limit > 0) return class_pass_launch(c, cls, limit);
     if (!c->graph[cls]) {
         cudaGraph_t g = nullptr;
@@ -1969,7 +1969,7 @@ int batch_sweep(esm_batch *b, uint32_t sweep) {
         BCK(e);
     }
     BCK(cudaGraphLaunch(b->graph, b->stream));
-    b->launches += 1 + b->n + b->bl.maxpass * (1 + (b->bl.bblocks > 0 ? 2 : 1) * b->bl.maxmoves);
+    b->launches += 1 + b->n + b->bl.maxpass * (2 + (b->bl.bblocks > 0 ? 2 : 1) * b->bl.maxmoves);
     return ESM_OK;
 }
 

@@ -4,7 +4,7 @@
 // Mapping. All (step, replica) tasks of a class run the same move list (the move selection reads
 // only capacities and static tables, src/local.jl:14 "selection uses only (k, x)"), so a move's
 // structure -- entries, lines, touched nodes, storage terms -- is the same for every task and is
-// built once per class pass (k_prep_moves). k_move then runs one move for every task: a warp owns
+// built once per class pass (k_prep_list, k_prep_moves). k_move then runs one move for every task: a warp owns
 // 32 tasks of a tile (span consecutive steps x replicas, replica fastest, so that every state
 // access of the warp is one coalesced 128-byte line of the (X, T, R) arrays), and each lane walks
 // its own piecewise-exponential line conditional (walk!, src/local.jl:1294) and draws t
@@ -973,15 +973,27 @@ struct Lane {
 // ---------------------------------------------------------------------------------------------
 // warp-uniform move construction
 // ---------------------------------------------------------------------------------------------
-struct Stream {  // the class stream (TAG_LIST), every lane holds the same copy
+// The class stream (TAG_LIST), read by a whole warp alike: a lane holds one of the 32 numbers from
+// `base` on, so that a warp makes 32 at a time (each number by itself took a Philox evaluation and its
+// FP64 scaling, some 400 cycles of every move's selection).
+struct Stream {
     uint64_t seed;
     uint32_t tile, cls, sweep, j;
-    __device__ double next() {
+    uint32_t base;  // (of the lanes' numbers; any other multiple of 32: none yet)
+    double u;
+    __device__ Stream(uint64_t seed_, uint32_t cls_, uint32_t sweep_, uint32_t j_)
+        : seed(seed_), tile(0u), cls(cls_), sweep(sweep_), j(j_), base((j_ & ~31u) + 32u), u(0) {}
+    __device__ void fill() {
+        if (base == (j & ~31u)) return;
+        base = j & ~31u;
         double u0, u1;
-        uniform2(seed, ESM_TAG_LIST, j >> 1, tile, cls, sweep, &u0, &u1);
-        double u = (j & 1) ? u1 : u0;
-        ++j;
-        return u;
+        const uint32_t i = base + (threadIdx.x & 31);
+        uniform2(seed, ESM_TAG_LIST, i >> 1, tile, cls, sweep, &u0, &u1);
+        u = (i & 1) ? u1 : u0;
+    }
+    __device__ double next() {
+        fill();
+        return __shfl_sync(0xffffffffu, u, j++ & 31);
     }
     __device__ int pick(int n) {
         int i = (int)floor(next() * n);
@@ -992,12 +1004,11 @@ struct Stream {  // the class stream (TAG_LIST), every lane holds the same copy
 // the move list of a tile (local_sweep!, src/local.jl:1964-1974): atoms, then nextra family draws,
 // shuffled (Fisher-Yates). Encoding: atom a -> a, family f -> -(f + 1).
 template <class real>
-__device__ __noinline__ void build_list(const DevModel<real> &M, Desc<real> &d, Stream &st, int lane) {
+__device__ __noinline__ void build_list(const DevModel<real> &M, int *moves, Stream &st, int lane) {
     int na = M.natoms, n = na + M.nextra;
     __syncwarp();
-    for (int i = lane; i < na; i += 32) d.moves[i] = i;
+    for (int i = lane; i < na; i += 32) moves[i] = i;
     __syncwarp();
-    // family draws: every lane draws the same numbers; lane 0 writes
     for (int i = 0; i < M.nextra; ++i) {
         double u = st.next();
         int kd = ESM_NFAM - 1;
@@ -1006,16 +1017,24 @@ __device__ __noinline__ void build_list(const DevModel<real> &M, Desc<real> &d, 
                 kd = q;
                 break;
             }
-        if (lane == 0) d.moves[na + i] = -(kd + 1);
+        if (lane == 0) moves[na + i] = -(kd + 1);
     }
     __syncwarp();
-    for (int i = n - 1; i >= 1; --i) {
-        int j = st.pick(i + 1);
-        if (lane == 0) {
-            int tmp = d.moves[i];
-            d.moves[i] = d.moves[j];
-            d.moves[j] = tmp;
+    for (int i = n - 1; i >= 1;) {  // (the picks of up to 32 exchanges at once, the exchanges in order)
+        st.fill();
+        const int k = (int)(st.j & 31), m = min(32 - k, i);
+        const int b = i - (lane - k) + 1;  // the number of lane k + q picks among i - q + 1
+        int pk = (int)floor(st.u * b);
+        if (pk >= b) pk = b - 1;
+        for (int q = 0; q < m; ++q, --i) {
+            const int j = __shfl_sync(0xffffffffu, pk, k + q);
+            if (lane == 0) {
+                int tmp = moves[i];
+                moves[i] = moves[j];
+                moves[j] = tmp;
+            }
         }
+        st.j += m;
     }
     __syncwarp();
 }
@@ -1038,6 +1057,101 @@ __device__ inline real kappa_d(const DevModel<real> &M, int j) {
     return M.d_avail[j] * M.kc_d[j];
 }
 
+// The selection of a move of family fam: every number it takes from the class stream, and the tests on
+// which later ones depend (units u1, u2 or groups of a cell; x: the pair, cell or storage unit).
+// False: rejected.
+struct Sel {
+    int n, m, u1, u2, x;
+};
+template <class real>
+__device__ __noinline__ bool select_move(const DevModel<real> &M, Stream &st, int fam, Sel *out) {
+    auto nun = [&](int n) { return M.up[n + 1] - M.up[n]; };
+    auto unit = [&](int n) { return M.ua[M.up[n] + st.pick(nun(n))]; };
+    Sel &s = *out;
+    switch (fam) {
+        case ESM_FAM_UNIT:
+            s.n = st.pick(M.N);
+            if (nun(s.n) == 0) return false;
+            s.u1 = unit(s.n);
+            return true;
+        case ESM_FAM_PAIR:
+        case ESM_FAM_XPAIR:
+            s.n = st.pick(M.N);
+            s.m = fam == ESM_FAM_PAIR ? s.n : st.pick(M.N);
+            if (fam == ESM_FAM_XPAIR && (s.m == s.n || M.comp[s.m] != M.comp[s.n])) return false;
+            if (nun(s.n) == 0 || nun(s.m) == 0) return false;
+            s.u1 = unit(s.n);
+            s.u2 = unit(s.m);
+            return s.u1 != s.u2;
+        case ESM_FAM_XLOC:
+        case ESM_FAM_XLOCC: {
+            s.n = st.pick(M.N);
+            int np = M.xpp[s.n + 1] - M.xpp[s.n];
+            if (np == 0) return false;
+            s.x = M.xpp[s.n] + st.pick(np);
+            s.m = M.xp[s.x];
+            if (nun(s.n) == 0 || nun(s.m) == 0) return false;
+            s.u1 = unit(s.n);
+            s.u2 = unit(s.m);
+            return true;
+        }
+        case ESM_FAM_POTENTIAL:
+        case ESM_FAM_TPOT:
+            s.n = st.pick(M.N);
+            return M.theta_nnz[s.n] != 0;
+        case ESM_FAM_CELLPAIR:
+        case ESM_FAM_CELL: {
+            double u = st.next();
+            int q = M.nlev - 1;
+            for (int l = 0; l < M.nlev; ++l)
+                if (M.qcum[l] >= u) {
+                    q = l;
+                    break;
+                }
+            int ncell = M.clp[q + 1] - M.clp[q];
+            s.x = M.clp[q] + st.pick(ncell);
+            // distinct injecting groups of the cell, ascending
+            int fl[8], nfl = 0;
+            for (int p = M.cp[s.x]; p < M.cp[s.x + 1]; ++p) {
+                int gg = M.d_group[M.cu[p]];
+                bool seen = false;
+                for (int i = 0; i < nfl; ++i) seen |= fl[i] == gg;
+                if (!seen && nfl < 8) fl[nfl++] = gg;
+            }
+            for (int i = 1; i < nfl; ++i)
+                for (int j = i; j > 0 && fl[j] < fl[j - 1]; --j) {
+                    int tmp = fl[j];
+                    fl[j] = fl[j - 1];
+                    fl[j - 1] = tmp;
+                }
+            if (nfl == 0) return false;
+            if (fam == ESM_FAM_CELL) {
+                s.u1 = fl[st.pick(nfl)];
+                return true;
+            }
+            if (nfl < 2) return false;
+            s.u1 = fl[st.pick(nfl)];
+            s.u2 = fl[st.pick(nfl)];
+            return s.u1 != s.u2;
+        }
+        case ESM_FAM_SPAIR:
+        case ESM_FAM_TSOC: {
+            s.n = st.pick(M.N);
+            int ns = M.sp[s.n + 1] - M.sp[s.n];
+            if (ns == 0 || (fam == ESM_FAM_SPAIR && nun(s.n) == 0)) return false;
+            s.x = M.sa[M.sp[s.n] + st.pick(ns)];
+            real ks = M.kc_s[s.x] * M.s_hours[s.x] / M.dt;
+            if (ks < M.kmin) return false;
+            if (fam == ESM_FAM_SPAIR) {
+                s.u1 = unit(s.n);
+                s.u2 = unit(s.n);
+            }
+            return true;
+        }
+    }
+    return true;
+}
+
 // Build the warp-uniform part of move `mv` (lane 0 writes shared memory). Returns the family
 // index for the statistics (ESM_NFAM for atoms) or -1 when the selection rejects the move.
 template <class real>
@@ -1054,7 +1168,6 @@ __device__ __noinline__ int prep_move(const DevModel<real> &M, Desc<real> &d, St
     int ng = 0, nse = 0, nth = 0, nk = 0, nku = 0, nga = 0;
     int nku0 = -1;  // kinked units of step tau (-1: all of them)
     real kmin = M.kmin;
-    auto nun = [&](int n) { return M.up[n + 1] - M.up[n]; };
     bool ok = true;
     if (mv >= 0) {  // prep_atom! (src/local.jl:1567)
         int f = 0;
@@ -1080,17 +1193,13 @@ __device__ __noinline__ int prep_move(const DevModel<real> &M, Desc<real> &d, St
             ng = cnt;
         else
             nse = cnt;
+    } else if (Sel sl; !select_move(M, st, fam, &sl)) {
+        ok = false;
     } else {
         switch (fam) {
             case ESM_FAM_UNIT: {
-                int n = st.pick(N);
-                if (nun(n) == 0) {
-                    ok = false;
-                    break;
-                }
-                int j = M.ua[M.up[n] + st.pick(nun(n))];
                 if (w0) {
-                    d.gi[0] = j;
+                    d.gi[0] = sl.u1;
                     d.ga[0] = 1;
                 }
                 ng = 1;
@@ -1098,22 +1207,7 @@ __device__ __noinline__ int prep_move(const DevModel<real> &M, Desc<real> &d, St
             }
             case ESM_FAM_PAIR:
             case ESM_FAM_XPAIR: {
-                int n = st.pick(N);
-                int m = fam == ESM_FAM_PAIR ? n : st.pick(N);
-                if (fam == ESM_FAM_XPAIR && (m == n || M.comp[m] != M.comp[n])) {
-                    ok = false;
-                    break;
-                }
-                if (nun(n) == 0 || nun(m) == 0) {
-                    ok = false;
-                    break;
-                }
-                int u1 = M.ua[M.up[n] + st.pick(nun(n))];
-                int u2 = M.ua[M.up[m] + st.pick(nun(m))];
-                if (u1 == u2) {
-                    ok = false;
-                    break;
-                }
+                const int n = sl.n, m = sl.m, u1 = sl.u1, u2 = sl.u2;
                 real k1 = kappa_d(M, u1), k2 = kappa_d(M, u2);
                 if (fabs(k1) < kmin || fabs(k2) < kmin) {
                     ok = false;
@@ -1144,20 +1238,7 @@ __device__ __noinline__ int prep_move(const DevModel<real> &M, Desc<real> &d, St
             }
             case ESM_FAM_XLOC:
             case ESM_FAM_XLOCC: {
-                int n = st.pick(N);
-                int np = M.xpp[n + 1] - M.xpp[n];
-                if (np == 0) {
-                    ok = false;
-                    break;
-                }
-                int pair = M.xpp[n] + st.pick(np);
-                int m = M.xp[pair];
-                if (nun(n) == 0 || nun(m) == 0) {
-                    ok = false;
-                    break;
-                }
-                int u1 = M.ua[M.up[n] + st.pick(nun(n))];
-                int u2 = M.ua[M.up[m] + st.pick(nun(m))];
+                const int u1 = sl.u1, u2 = sl.u2, pair = sl.x;
                 real k1 = kappa_d(M, u1), k2 = kappa_d(M, u2);
                 if (fabs(k1) < kmin || fabs(k2) < kmin) {
                     ok = false;
@@ -1201,13 +1282,8 @@ __device__ __noinline__ int prep_move(const DevModel<real> &M, Desc<real> &d, St
                 break;
             }
             case ESM_FAM_POTENTIAL: {
-                int n = st.pick(N);
-                if (M.theta_nnz[n] == 0) {
-                    ok = false;
-                    break;
-                }
                 if (w0) {
-                    d.thn[0] = n;
+                    d.thn[0] = sl.n;
                     d.tha[0] = 1;
                 }
                 nth = 1;
@@ -1215,35 +1291,9 @@ __device__ __noinline__ int prep_move(const DevModel<real> &M, Desc<real> &d, St
             }
             case ESM_FAM_CELLPAIR:
             case ESM_FAM_CELL: {
-                double u = st.next();
-                int q = M.nlev - 1;
-                for (int l = 0; l < M.nlev; ++l)
-                    if (M.qcum[l] >= u) {
-                        q = l;
-                        break;
-                    }
-                int ncell = M.clp[q + 1] - M.clp[q];
-                int cidx = M.clp[q] + st.pick(ncell);
-                // distinct injecting groups of the cell, ascending
-                int fl[8], nfl = 0;
-                for (int p = M.cp[cidx]; p < M.cp[cidx + 1]; ++p) {
-                    int gg = M.d_group[M.cu[p]];
-                    bool seen = false;
-                    for (int i = 0; i < nfl; ++i) seen |= fl[i] == gg;
-                    if (!seen && nfl < 8) fl[nfl++] = gg;
-                }
-                for (int i = 1; i < nfl; ++i)
-                    for (int j = i; j > 0 && fl[j] < fl[j - 1]; --j) {
-                        int tmp = fl[j];
-                        fl[j] = fl[j - 1];
-                        fl[j - 1] = tmp;
-                    }
-                if (nfl == 0) {
-                    ok = false;
-                    break;
-                }
+                const int cidx = sl.x;
                 if (fam == ESM_FAM_CELL) {
-                    int f = fl[st.pick(nfl)];
+                    const int f = sl.u1;
                     int c = 0;
                     for (int p = M.cp[cidx]; p < M.cp[cidx + 1]; ++p)
                         if (M.d_group[M.cu[p]] == f) {
@@ -1256,15 +1306,7 @@ __device__ __noinline__ int prep_move(const DevModel<real> &M, Desc<real> &d, St
                     ng = c;
                     break;
                 }
-                if (nfl < 2) {
-                    ok = false;
-                    break;
-                }
-                int f1 = fl[st.pick(nfl)], f2 = fl[st.pick(nfl)];
-                if (f1 == f2) {
-                    ok = false;
-                    break;
-                }
+                const int f1 = sl.u1, f2 = sl.u2;
                 real K1 = 0, K2 = 0;
                 for (int p = M.cp[cidx]; p < M.cp[cidx + 1]; ++p) {
                     int j = M.cu[p];
@@ -1296,20 +1338,8 @@ __device__ __noinline__ int prep_move(const DevModel<real> &M, Desc<real> &d, St
                 break;
             }
             case ESM_FAM_SPAIR: {
-                int n = st.pick(N);
-                int ns = M.sp[n + 1] - M.sp[n];
-                if (ns == 0 || nun(n) == 0) {
-                    ok = false;
-                    break;
-                }
-                int sj = M.sa[M.sp[n] + st.pick(ns)];
+                const int u1 = sl.u1, u2 = sl.u2, sj = sl.x;
                 real ks = M.kc_s[sj] * M.s_hours[sj] / M.dt;
-                if (ks < kmin) {
-                    ok = false;
-                    break;
-                }
-                int u1 = M.ua[M.up[n] + st.pick(nun(n))];
-                int u2 = M.ua[M.up[n] + st.pick(nun(n))];
                 real k1 = kappa_d(M, u1), k2 = kappa_d(M, u2);
                 if (fabs(k1) < kmin || fabs(k2) < kmin) {
                     ok = false;
@@ -1329,11 +1359,7 @@ __device__ __noinline__ int prep_move(const DevModel<real> &M, Desc<real> &d, St
                 break;
             }
             case ESM_FAM_TPOT: {  // prep_tpot! (src/local.jl:1741): the angle of node n rises by t
-                int n = st.pick(N);
-                if (M.theta_nnz[n] == 0) {
-                    ok = false;
-                    break;
-                }
+                const int n = sl.n;
                 if (w0) {
                     d.thn[0] = n;
                     d.tha[0] = 1;
@@ -1380,18 +1406,8 @@ __device__ __noinline__ int prep_move(const DevModel<real> &M, Desc<real> &d, St
                 break;
             }
             case ESM_FAM_TSOC: {  // prep_tsoc! (src/local.jl:1849): energy moved from step tau - 1 to tau
-                int n = st.pick(N);
-                int ns = M.sp[n + 1] - M.sp[n];
-                if (ns == 0) {
-                    ok = false;
-                    break;
-                }
-                int sj = M.sa[M.sp[n] + st.pick(ns)];
+                const int n = sl.n, sj = sl.x;
                 real ks = M.kc_s[sj] * M.s_hours[sj] / M.dt;
-                if (ks < kmin) {
-                    ok = false;
-                    break;
-                }
                 if (w0) {
                     d.si[0] = sj;
                     d.sa[0] = 1;
@@ -1602,15 +1618,41 @@ namespace esm {
 // The move list of a colour class and the descriptor of each of its moves. The list and the
 // selection draws come from one stream per (class, sweep) (TAG_LIST with tile word 0), shared by
 // every task of the class; the selection reads only capacities and static tables, so every
-// descriptor is the same for all tasks and is built once here, by one warp, in stream order.
-// Descriptor mi goes to descs + mi * stride; its header word 12 holds the family index (-1: no move).
-// The body of k_prep_moves for one model, run by one warp: smem is its descriptor workspace
-// (stride bytes), sd the shared Desc that carves it.
+// descriptor is the same for all tasks and is built once here. One warp makes the list and runs
+// through the selections, which fixes where in the stream each move's begins (list_class; header
+// words 13 and 14 of descriptor mi: that place, the move); then one warp per move builds its
+// descriptor (descs + mi * stride; header word 12: the family index, -1: no move), smem its workspace
+// of stride bytes, sd the shared Desc that carves it. Bound by the latency of the one warp's selections.
+// 40 nodes (319 moves): 2.2 ms with one warp for the descriptors too, 0.30 so; 128 nodes (1023): 0.96.
+// the header words of a descriptor
 template <class real>
-__device__ __forceinline__ void prep_class(const DevModel<real> &M, char *smem, Desc<real> &sd, uint32_t sweep, int cls,
-                                           int nrun, char *descs, size_t stride, int lane) {
-    int nmoves = M.natoms + M.nextra;
-    if (lane == 0) sd = carve_desc<real>(smem, M, nmoves);
+__device__ inline int *desc_hdr(char *desc, const DevModel<real> &M) {
+    Carve c(desc);
+    c.take<int>(M.natoms + M.nextra);
+    return c.take<int>(16);
+}
+
+template <class real>
+__device__ __forceinline__ void list_class(const DevModel<real> &M, int *moves, uint32_t sweep, int cls, int nrun,
+                                           char *descs, size_t stride, int lane) {
+    Stream st(M.seed, (uint32_t)cls, sweep, 0u);
+    build_list(M, moves, st, lane);
+    for (int mi = 0; mi < nrun; ++mi) {
+        const int mv = moves[mi];
+        if (lane == 0) {
+            int *h = desc_hdr<real>(descs + (size_t)mi * stride, M);
+            h[13] = (int)st.j;
+            h[14] = mv;
+        }
+        Sel sl;
+        if (mv < 0) select_move(M, st, -mv - 1, &sl);
+    }
+}
+
+template <class real>
+__device__ __forceinline__ void prep_desc(const DevModel<real> &M, char *smem, Desc<real> &sd, uint32_t sweep, int cls,
+                                          char *out, size_t stride, int lane) {
+    if (lane == 0) sd = carve_desc<real>(smem, M, M.natoms + M.nextra);
     __syncwarp();
     Desc<real> &d = sd;
     for (int i = lane; i < M.N; i += 32) {
@@ -1620,25 +1662,30 @@ __device__ __forceinline__ void prep_class(const DevModel<real> &M, char *smem, 
     }
     for (int i = lane; i < M.L; i += 32) d.lmark[i] = 0;
     __syncwarp();
-    Stream st{M.seed, 0u, (uint32_t)cls, sweep, 0u};
-    build_list(M, d, st, lane);
-    for (int mi = 0; mi < nrun; ++mi) {
-        int fi = prep_move(M, d, st, d.moves[mi], lane);
-        if (lane == 0) d.hdr[12] = fi;
-        __syncwarp();
-        const int4 *src = (const int4 *)smem;
-        int4 *dst = (int4 *)(descs + (size_t)mi * stride);
-        for (size_t i = lane; i < stride / 16; i += 32) dst[i] = src[i];
-        __syncwarp();
-    }
+    const int *h = desc_hdr<real>(out, M);
+    Stream st(M.seed, (uint32_t)cls, sweep, (uint32_t)h[13]);
+    int fi = prep_move(M, d, st, h[14], lane);
+    if (lane == 0) d.hdr[12] = fi;
+    __syncwarp();
+    const size_t from = (size_t)((char *)d.hdr - smem) / 16 * 16;  // (the list in front is of no use to a move)
+    const int4 *src = (const int4 *)(smem + from);
+    int4 *dst = (int4 *)(out + from);
+    for (size_t i = lane; i < (stride - from) / 16; i += 32) dst[i] = src[i];
+}
+
+template <class real>
+__global__ void __launch_bounds__(32) k_prep_list(const __grid_constant__ DevModel<real> M, const uint32_t *sweep_p, int cls,
+                                                 int nrun, char *descs, size_t stride) {
+    extern __shared__ __align__(16) char smem[];
+    list_class<real>(M, (int *)smem, *sweep_p, cls, nrun, descs, stride, threadIdx.x);
 }
 
 template <class real>
 __global__ void __launch_bounds__(32) k_prep_moves(const __grid_constant__ DevModel<real> M, const uint32_t *sweep_p, int cls,
-                                                  int nrun, char *descs, size_t stride) {
+                                                  char *descs, size_t stride) {
     extern __shared__ __align__(16) char smem[];
     __shared__ Desc<real> sd;
-    prep_class<real>(M, smem, sd, *sweep_p, cls, nrun, descs, stride, threadIdx.x);
+    prep_desc<real>(M, smem, sd, *sweep_p, cls, descs + (size_t)blockIdx.x * stride, stride, threadIdx.x);
 }
 
 // Move mi of the class (its descriptor built by k_prep_moves) for every (step, replica) task. One
@@ -1970,6 +2017,7 @@ int linemove_blocks_per_sm(const DevModel<real> &M, int wpb) {
     size_t stride = linemove_smem_per_warp(M);
     // (the dynamic shared memory limits are set here, at context creation, so that no later call --
     // possibly under stream capture -- has to)
+    cudaFuncSetAttribute(k_prep_list<real>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(k_prep_moves<real>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaError_t e;
     if (wpb == 4) {
@@ -2029,7 +2077,9 @@ cudaError_t launch_class_pass(const DevModel<real> &M, const int *steps, int nst
     size_t stride = linemove_smem_per_warp(M);
     cudaError_t e = cudaMemsetAsync(counters, 0, sizeof(unsigned int) * nrun, s);
     if (e != cudaSuccess) return e;
-    k_prep_moves<real><<<1, 32, stride, s>>>(M, sweep, cls, nrun, descs, stride);
+    k_prep_list<real><<<1, 32, sizeof(int) * nmoves, s>>>(M, sweep, cls, nrun, descs, stride);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    k_prep_moves<real><<<nrun, 32, stride, s>>>(M, sweep, cls, descs, stride);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     int ntile = (nsteps + M.span - 1) / M.span;
     int wpt = (M.span * M.R + 31) / 32;
@@ -2079,15 +2129,14 @@ cudaError_t launch_class_pass(const DevModel<real> &M, const int *steps, int nst
 // a batch of models
 // ---------------------------------------------------------------------------------------------
 #define ESM_CHUNK 64  // tasks that a block of k_move_blocks_batch takes at a time
-// Pass p of every model of a batch: block b builds the descriptors of the class that model b runs
-// in pass p of the sweep (its own class order, class_order_of), exactly as k_prep_moves does for
+// Pass p of every model of a batch: block b makes the move list of the class that model b runs
+// in pass p of the sweep (its own class order, class_order_of), exactly as k_prep_list does for
 // the model alone; block 0 also writes every model's class of the pass and the pass's item prefix
 // over the models (items: the model's tiles of its class x the warps of a tile).
 template <class real>
-__global__ void __launch_bounds__(32) k_prep_batch(const BatchModel<real> *bm, int nm, const uint32_t *sweep_p, int p,
+__global__ void __launch_bounds__(32) k_list_batch(const BatchModel<real> *bm, int nm, const uint32_t *sweep_p, int p,
                                                    int *pass_cls, unsigned int *off, unsigned int *choff) {
     extern __shared__ __align__(16) char smem[];
-    __shared__ Desc<real> sd;
     int b = blockIdx.x, lane = threadIdx.x;
     uint32_t sweep = *sweep_p;
     const BatchModel<real> &B = bm[b];
@@ -2114,7 +2163,18 @@ __global__ void __launch_bounds__(32) k_prep_batch(const BatchModel<real> *bm, i
         }
     }
     if (p >= ncls || B.nsteps[order[p]] == 0) return;
-    prep_class<real>(B.M, smem, sd, sweep, order[p], B.nmoves, B.descs, B.stride, lane);
+    list_class<real>(B.M, (int *)smem, sweep, order[p], B.nmoves, B.descs, B.stride, lane);
+}
+
+// the descriptor of move blockIdx.x of model blockIdx.y
+template <class real>
+__global__ void __launch_bounds__(32) k_prep_batch(const BatchModel<real> *bm, const uint32_t *sweep_p, const int *pass_cls) {
+    extern __shared__ __align__(16) char smem[];
+    __shared__ Desc<real> sd;
+    const BatchModel<real> &B = bm[blockIdx.y];
+    const int cls = pass_cls[blockIdx.y];
+    if (cls < 0 || B.nsteps[cls] == 0 || (int)blockIdx.x >= B.nmoves) return;
+    prep_desc<real>(B.M, smem, sd, *sweep_p, cls, B.descs + (size_t)blockIdx.x * B.stride, B.stride, threadIdx.x);
 }
 
 // Move mi of the current pass for every task of the first nact models of the batch. A warp takes
@@ -2302,6 +2362,7 @@ template <class real>
 int batch_warps_per_sm(int wpb) {
     int nb = 0;
     cudaError_t e;
+    cudaFuncSetAttribute(k_list_batch<real>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(k_prep_batch<real>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (wpb == 2)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_move_batch<real, 2>, 64, 0);
@@ -2321,7 +2382,9 @@ cudaError_t launch_batch_passes(const BatchModel<real> *bm, const BatchLaunch &b
         int *pc = bl.pass_cls + (size_t)p * bl.nm;
         unsigned int *off = bl.off + (size_t)p * (bl.nm + 1);
         unsigned int *choff = bl.choff + (size_t)p * (bl.nm + 1);
-        k_prep_batch<real><<<bl.nm, 32, bl.prep_smem, s>>>(bm, bl.nm, sweep, p, pc, off, choff);
+        k_list_batch<real><<<bl.nm, 32, sizeof(int) * bl.maxmoves, s>>>(bm, bl.nm, sweep, p, pc, off, choff);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        k_prep_batch<real><<<dim3(bl.nmove, bl.nm), 32, bl.prep_smem, s>>>(bm, sweep, pc);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         for (int mi = 0; mi < bl.nmove; ++mi) {
             unsigned int *ctr = bl.counters + (size_t)p * bl.maxmoves + mi;
