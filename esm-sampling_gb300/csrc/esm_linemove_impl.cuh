@@ -1840,8 +1840,10 @@ __device__ __forceinline__ int scan_warp(int *slot) {
 
 // Move mi of the class for every (step, replica) task when sep_run (a separable move of at least sepmin
 // units; sepmin 0: none) or walk_run walks it (else nothing: k_move does).
+// Registers: four blocks an SM in FP32 (128 a thread); two in FP64, whose walks spill at 128 (a sweep of 40
+// nodes, T = 1460, 4 replicas: 231 ms with four, 251 with three, 192 with two; T = 120, 32 replicas: 153 and 156).
 template <class real>
-__global__ void __launch_bounds__(32 * ESM_SEP_WARPS, 4)
+__global__ void __launch_bounds__(32 * ESM_SEP_WARPS, sizeof(real) == 8 ? 2 : 4)
     k_move_blocks(const __grid_constant__ DevModel<real> M, const int *steps, int nsteps, const uint32_t *sweep_p,
                   int mi, const char *descs, size_t stride, int sepmin, int region, int walk_region, char *tmp,
                   int tmp_warp, real *scratch, size_t scratch_per_warp, unsigned long long *stats,
@@ -2188,7 +2190,7 @@ __global__ void __launch_bounds__(32) k_prep_batch(const BatchModel<real> *bm, c
 // Move mi of the current pass for the models whose move sep_run or walk_run walks: blocks take chunks of
 // ESM_CHUNK tasks of one model from the launch's counter (choff: the chunk prefix over the models).
 template <class real>
-__global__ void __launch_bounds__(32 * ESM_SEP_WARPS, 4)
+__global__ void __launch_bounds__(32 * ESM_SEP_WARPS, sizeof(real) == 8 ? 2 : 4)
     k_move_blocks_batch(const BatchModel<real> *bm, int nact, const int *pass_cls, const unsigned int *choff,
                         const uint32_t *sweep_p, int mi, int region, char *tmp, int tmp_warp, real *scratch,
                         size_t scratch_per_warp, unsigned int *next_chunk) {
