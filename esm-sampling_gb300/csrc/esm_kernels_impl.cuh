@@ -98,6 +98,7 @@ __global__ void k_rebuild(DevModel<real> M) {
 // ---------------------------------------------------------------------------------------------
 #define ESM_SCORE_NSLOT 8
 #define ESM_SCORE_MAXU 8
+#define ESM_SCORE_MAXL 12  // lines of a node kept in shared memory (k_scores_f32; more: read each step)
 #define ESM_U64 1.1102230246251565e-16  // 2^-53
 #define ESM_U32 5.9604645e-8f           // 2^-24
 
@@ -292,7 +293,10 @@ __global__ void __launch_bounds__(32 * ESM_SCORE_NSLOT)
     }
 }
 
-// The FP32 build of the pass (see above). Bounds are summed in units of 2^-24 beside the terms:
+// The FP32 build of the pass (see above). Bound by the latency of a step's loads at 16 warps per SM: the
+// node's lines and units lie in shared memory, so that a state's address needs no chain of table reads, and
+// the units' states are read together once, not in both loops (40 nodes, T = 2920, 64 replicas: 0.76 ms; the
+// capacity step at T = 8760: 6.20 -> 5.96 ms). Bounds are summed in units of 2^-24 beside the terms:
 // a product or quotient of rounded inputs contributes a few units of its magnitude; the logistic
 // availability contributes its weather value's rounding (the sum of the magnitudes of its two
 // parts) on top; a storage term contributes the rounding of its flow d (4|Q| + |qt| + 2|d|, Q the
@@ -301,6 +305,10 @@ static __global__ void __launch_bounds__(32 * ESM_SCORE_NSLOT)
     k_scores_f32(const __grid_constant__ DevModel<float> M, const __grid_constant__ DevModel<double> Md, int tchunk,
                  double *partial) {
     __shared__ double sp[ESM_SCORE_NSLOT][32][10];
+    __shared__ int sl_o[ESM_SCORE_NSLOT][ESM_SCORE_MAXL];    // other end; -1 - it where the node is the line's second
+    __shared__ float sl_b[ESM_SCORE_NSLOT][ESM_SCORE_MAXL], sl_s[ESM_SCORE_NSLOT][ESM_SCORE_MAXL];
+    __shared__ int su_k[ESM_SCORE_NSLOT][ESM_SCORE_MAXU], su_x[ESM_SCORE_NSLOT][ESM_SCORE_MAXU];  // kind, state row or series
+    __shared__ float su_p[ESM_SCORE_NSLOT][ESM_SCORE_MAXU][7];
     int lane = threadIdx.x, slot = threadIdx.y;
     int rep = blockIdx.x * 32 + lane;
     int n = blockIdx.y * ESM_SCORE_NSLOT + slot;
@@ -309,12 +317,45 @@ static __global__ void __launch_bounds__(32 * ESM_SCORE_NSLOT)
     size_t nrk = (size_t)R * K, half = (size_t)nchunk * (nrk + (size_t)ng * R * 5);
     NSum part[5];
     float pe[5] = {0, 0, 0, 0, 0};
+    // the node's lines and units (n is the warp's: all its lanes stage them)
+    const bool have = n < M.N;
+    const int l0 = have ? M.nlp[n] : 0, nl = have ? M.nlp[n + 1] - l0 : 0;
+    const int p0 = have ? M.nu_ptr[n] : 0, p1 = have ? M.nu_ptr[n + 1] : 0;
+    const int nu = min(p1 - p0, ESM_SCORE_MAXU);
+    auto end = [&](int i, int *o, float *lb, float *ls) {
+        const int e = M.nl[l0 + i], fa = M.bus0[e], fb = M.bus1[e];
+        *o = fa == n ? fb : -1 - fa;
+        *lb = M.lb[e];
+        *ls = M.ls[e];
+    };
+    for (int i = lane; i < min(nl, ESM_SCORE_MAXL); i += 32) end(i, &sl_o[slot][i], &sl_b[slot][i], &sl_s[slot][i]);
+    if (lane < nu) {
+        const int j = M.u_loc[M.nu_unit[p0 + lane]], kd = M.u_kind[M.nu_unit[p0 + lane]];
+        float *q = su_p[slot][lane];
+        su_k[slot][lane] = kd;
+        su_x[slot][lane] = j;
+        if (kd == ESM_UNIT_REN) {
+            su_x[slot][lane] = M.r_series[j];
+            q[0] = M.kc_r[j];
+            q[1] = M.r_mc[j];
+        } else if (kd == ESM_UNIT_DISP) {
+            q[0] = M.kc_d[j];
+            q[1] = M.d_mc[j];
+            q[2] = M.d_avail[j];
+        } else {
+            q[0] = M.kc_s[j];
+            q[1] = M.s_mc[j];
+            q[2] = M.s_hours[j];
+            q[3] = M.s_qt[j];
+            q[4] = M.s_etain[j];
+            q[5] = M.s_etaout[j];
+        }
+    }
+    __syncwarp();
     if (rep < R && n < M.N) {
         int t0 = c * tchunk, t1 = min(T, t0 + tchunk);
         const float dt = M.dt, cv = M.c_viol, k0 = M.kappa0, csh = M.c_shed, cdu = M.c_dump;
         const float *th = M.theta, *gv = M.g, *ev = M.e, *zv = M.z;
-        int p0 = M.nu_ptr[n], p1 = M.nu_ptr[n + 1];
-        int nu = min(p1 - p0, ESM_SCORE_MAXU);
         NSum dk[ESM_SCORE_MAXU];
         float de[ESM_SCORE_MAXU];
 #pragma unroll
@@ -332,17 +373,25 @@ static __global__ void __launch_bounds__(32 * ESM_SCORE_NSLOT)
             float rr = x > 0 ? x : 0.f;
             float ab = rr, br = bx;
             int nt = 1;
-            for (int p = M.nlp[n]; p < M.nlp[n + 1]; ++p) {
-                int e = M.nl[p];
-                int a = M.bus0[e], b = M.bus1[e];
-                float fl = M.lb[e] * (th[sidx(a, t, rep, T, R)] - th[sidx(b, t, rep, T, R)]);
+            const float tn = th[sidx(n, t, rep, T, R)];
+            for (int i = 0; i < nl; ++i) {
+                int o;
+                float lb, ls;
+                if (i < ESM_SCORE_MAXL) {
+                    o = sl_o[slot][i];
+                    lb = sl_b[slot][i];
+                    ls = sl_s[slot][i];
+                } else {
+                    end(i, &o, &lb, &ls);
+                }
+                const float to = th[sidx(o >= 0 ? o : -1 - o, t, rep, T, R)];
+                float fl = lb * (o >= 0 ? tn - to : to - tn);
                 float afl = fabsf(fl);
                 ab += afl;
                 br += 2.f * afl;
                 ++nt;
-                if (a == n) {
+                if (o >= 0) {
                     rr += fl;
-                    float ls = M.ls[e];
                     float pen = cv * dt * (ls * fmaxf(afl / ls - 1.f, 0.f));
                     part[4].add(pen);
                     pe[4] += 6.f * pen + (afl >= 0.999f * ls ? 3.f * cv * dt * afl : 0.f);
@@ -350,7 +399,54 @@ static __global__ void __launch_bounds__(32 * ESM_SCORE_NSLOT)
                     rr -= fl;
                 }
             }
-            for (int p = p0; p < p1; ++p) {
+            // the units' states: availability and its bound, dispatch, or the two states of charge
+            float x0[ESM_SCORE_MAXU], x1[ESM_SCORE_MAXU];
+#pragma unroll
+            for (int q = 0; q < ESM_SCORE_MAXU; ++q) {
+                if (q >= nu) break;
+                const int kd = su_k[slot][q], j = su_x[slot][q];
+                if (kd == ESM_UNIT_REN)
+                    x0[q] = wr(j, &x1[q]);
+                else if (kd == ESM_UNIT_DISP)
+                    x0[q] = gv[sidx(j, t, rep, T, R)];
+                else {
+                    x0[q] = ev[sidx(j, t, rep, T, R)];
+                    x1[q] = ev[sidx(j, t + 1 < T ? t + 1 : 0, rep, T, R)];
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < ESM_SCORE_MAXU; ++q) {
+                if (q >= nu) break;
+                const int kd = su_k[slot][q];
+                const float *P = su_p[slot][q];
+                float v = 0, bv = 0;
+                if (kd == ESM_UNIT_REN) {
+                    x0[q] = avail_map<float>(x0[q]);
+                    v = -(x0[q] * P[0]);
+                    bv = (8.f + x1[q]) * fabsf(v);
+                } else if (kd == ESM_UNIT_DISP) {
+                    v = -(P[2] * P[0] * clampr<float>(x0[q], 0, 1));
+                    bv = 4.f * fabsf(v);
+                } else {
+                    float ec = clampr<float>(x0[q], 0, 1);
+                    float ec1 = clampr<float>(x1[q], 0, 1);
+                    float Q = P[2] * (ec1 - ec) / dt, d = Q - P[3];
+                    float ein = P[4], eout = P[5];
+                    float pc = 0, mcx = 0;
+                    if (d >= 0)
+                        pc = ein > 0 ? d / ein : 0.f;
+                    else
+                        mcx = fminf(-d * eout, 1.f);
+                    v = P[0] * (pc - mcx);
+                    float sd = fmaxf(ein > 0 ? 1.f / ein : 0.f, eout);
+                    bv = P[0] * sd * (4.f * fabsf(Q) + fabsf(P[3]) + 4.f * fabsf(d)) + 3.f * fabsf(v);
+                }
+                rr += v;
+                ab += fabsf(v);
+                br += bv;
+                ++nt;
+            }
+            for (int p = p0 + ESM_SCORE_MAXU; p < p1; ++p) {  // (a node of more units)
                 int u = M.nu_unit[p], j = M.u_loc[u];
                 int kd = M.u_kind[u];
                 float v = 0, bv = 0;
@@ -402,23 +498,22 @@ static __global__ void __launch_bounds__(32 * ESM_SCORE_NSLOT)
 #pragma unroll
             for (int q = 0; q < ESM_SCORE_MAXU; ++q) {
                 if (q >= nu) break;
-                int u = M.nu_unit[p0 + q], j = M.u_loc[u];
-                int kd = M.u_kind[u];
+                const int kd = su_k[slot][q];
+                const float *P = su_p[slot][q];
                 if (kd == ESM_UNIT_REN) {
-                    float bs;
-                    float A = avail_map<float>(wr(M.r_series[j], &bs));
-                    float wA = 8.f + bs;  // A's bound relative to A
-                    float g0 = dt * (M.r_mc[j] * (A * M.kc_r[j]));
+                    float A = x0[q];
+                    float wA = 8.f + x1[q];  // A's bound relative to A
+                    float g0 = dt * (P[1] * (A * P[0]));
                     part[0].add(g0);
                     pe[0] += (wA + 4.f) * fabsf(g0);
-                    float a1 = dt * (M.r_mc[j] * A), a2 = A * Gn;
+                    float a1 = dt * (P[1] * A), a2 = A * Gn;
                     dk[q].add(a1 - a2);
                     de[q] += (wA + 4.f) * (fabsf(a1) + fabsf(a2)) + A * gb;
                 } else if (kd == ESM_UNIT_DISP) {
-                    float A = M.d_avail[j], kv = M.kc_d[j];
-                    float Y = gv[sidx(j, t, rep, T, R)];
+                    float A = P[2], kv = P[0];
+                    float Y = x0[q];
                     float Yc = clampr<float>(Y, 0, 1);
-                    float g0 = dt * (M.d_mc[j] * (A * kv * Yc));
+                    float g0 = dt * (P[1] * (A * kv * Yc));
                     part[0].add(g0);
                     pe[0] += 6.f * fabsf(g0);
                     float exs = fabsf(Y - Yc);
@@ -432,13 +527,13 @@ static __global__ void __launch_bounds__(32 * ESM_SCORE_NSLOT)
                         dk[q].add(a0);
                         de[q] += 5.f * a0;
                     }
-                    float a1 = dt * (M.d_mc[j] * A * Yc), a2 = A * Yc * Gn;
+                    float a1 = dt * (P[1] * A * Yc), a2 = A * Yc * Gn;
                     dk[q].add(a1 - a2);
                     de[q] += 6.f * (fabsf(a1) + fabsf(a2)) + A * Yc * gb;
                 } else {
-                    float kv = M.kc_s[j], h = M.s_hours[j], qt = M.s_qt[j], ein = M.s_etain[j], eout = M.s_etaout[j];
-                    float mc = M.s_mc[j];
-                    float ye = ev[sidx(j, t, rep, T, R)], ye1 = ev[sidx(j, (t + 1) % T, rep, T, R)];
+                    float kv = P[0], h = P[2], qt = P[3], ein = P[4], eout = P[5];
+                    float mc = P[1];
+                    float ye = x0[q], ye1 = x1[q];
                     float dd, jj;
                     float cc = soc_cost<float>(h, qt, ein, eout, mc, kv, kv + k0, dt, cv, ye, ye1, &dd, &jj);
                     float Ec = clampr<float>(ye, 0, 1), Ec1 = clampr<float>(ye1, 0, 1);
@@ -594,12 +689,17 @@ template <class real>
 __global__ void k_follow_disp(DevModel<real> M, const int *disp, const double *kold, const double *knew,
                               const double *u_lo, const double *u_hi) {
     const unsigned tr = blockIdx.x * blockDim.x + threadIdx.x;
-    if (tr >= (unsigned)M.T * M.R) return;
     const int j = blockIdx.y;
+    __shared__ double ssc;  // (once a block: its FP64 division took longer than the pass; 221 -> 68 us)
+    if (threadIdx.x == 0) {
+        int u = disp[j];
+        double kc0 = fmin(fmax(kold[u], u_lo[u]), u_hi[u]), kc1 = fmin(fmax(knew[u], u_lo[u]), u_hi[u]);
+        ssc = kc0 == kc1 ? 1.0 : kc0 / kc1;  // kc_ratio (src/local.jl:2119)
+    }
+    __syncthreads();
+    if (tr >= (unsigned)M.T * M.R) return;
     const size_t i = (size_t)j * M.T * M.R + tr;
-    int u = disp[j];
-    double kc0 = fmin(fmax(kold[u], u_lo[u]), u_hi[u]), kc1 = fmin(fmax(knew[u], u_lo[u]), u_hi[u]);
-    double sc = kc0 == kc1 ? 1.0 : kc0 / kc1;  // kc_ratio (src/local.jl:2119)
+    const double sc = ssc;
     if (sc == 1.0) return;
     real y = M.g[i];
     M.g[i] = y + y * (real)(sc - 1);
@@ -608,12 +708,28 @@ __global__ void k_follow_disp(DevModel<real> M, const int *disp, const double *k
 // kop curve of the renewable and storage units of one node (kop_term / kop_eval with commit,
 // src/kop.jl:79-160; follow_capacities! src/replicas.jl:456-470), per (node, step, replica), units in
 // flat order. kold/knew raw capacities (FP64); kc of the dispatchable units already updated.
+#define ESM_KOP_UNITS 32  // units of a node whose capacity change a block keeps (more: made by each thread)
 template <class real>
 __global__ void k_kop(DevModel<real> M, const double *kold, const double *k1v, const double *u_lo,
                       const double *u_hi, double kmin) {
     const unsigned tr = blockIdx.x * blockDim.x + threadIdx.x;  // (step, replica) of node blockIdx.y
+    const int n = blockIdx.y, u0 = M.nu_ptr[n], nun = M.nu_ptr[n + 1] - u0;
+    // the capacity change of every unit of the node, in FP64, once a block: an FP64 instruction holds its
+    // unit for 16 cycles of the SM whatever its lanes hold, and a thread of its own took six per unit
+    // (40 nodes, T = 2920, 64 replicas: 456 us, 310 so)
+    __shared__ real sdk[ESM_KOP_UNITS];
+    __shared__ bool sfo[ESM_KOP_UNITS];  // at or above kmin: dispatch follows
+    auto change = [&](int u, bool *follow) {
+        double k0raw = kold[u];
+        double kc0 = fmin(fmax(k0raw, u_lo[u]), u_hi[u]);
+        double kc1 = fmin(fmax(k1v[u], u_lo[u]), u_hi[u]);
+        *follow = k0raw >= kmin;
+        return (real)(kc1 - kc0);
+    };
+    if (threadIdx.x < min(nun, ESM_KOP_UNITS)) sdk[threadIdx.x] = change(M.nu_unit[u0 + threadIdx.x], &sfo[threadIdx.x]);
+    __syncthreads();
     if (tr >= (unsigned)M.T * M.R) return;
-    const int n = blockIdx.y;
+    const real km = (real)kmin;
     const size_t i = (size_t)n * M.T * M.R + tr;
     const int t = (int)(tr / (unsigned)M.R), rep = (int)(tr - (unsigned)t * M.R);
     int T = M.T, R = M.R;
@@ -621,9 +737,14 @@ __global__ void k_kop(DevModel<real> M, const double *kold, const double *k1v, c
         int u = M.nu_unit[p], j = M.u_loc[u];
         int kd = M.u_kind[u];
         if (kd == ESM_UNIT_DISP) continue;
-        double k0raw = kold[u];
-        double kc0 = fmin(fmax(k0raw, u_lo[u]), u_hi[u]);
-        double kc1 = fmin(fmax(k1v[u], u_lo[u]), u_hi[u]);
+        bool follow;
+        real dkc;
+        if (p - u0 < ESM_KOP_UNITS) {
+            dkc = sdk[p - u0];
+            follow = sfo[p - u0];
+        } else {
+            dkc = change(u, &follow);
+        }
         real jinj;
         if (kd == ESM_UNIT_REN) {
             jinj = avail_map<real>(wraw(M, M.r_series[j], t, rep));
@@ -641,16 +762,15 @@ __global__ void k_kop(DevModel<real> M, const double *kold, const double *k1v, c
             }
             jinj = mcx - pc;
         }
-        real dkc = (real)(kc1 - kc0);
         real dinj = jinj * dkc;
         real dS = -dinj;
-        if (k0raw >= kmin) {  // below kmin: the capacity alone, no following (src/replicas.jl:461)
+        if (follow) {  // below kmin: the capacity alone, no following (src/replicas.jl:461)
             real Pt = 0, Qs = 0;
             int nu = 0;
             for (int q = M.up[n]; q < M.up[n + 1]; ++q) {
                 int jd = M.ua[q];
                 real kap = M.d_avail[jd] * M.kc_d[jd];
-                if (!(fabs(kap) >= (real)kmin)) continue;
+                if (!(fabs(kap) >= km)) continue;
                 real om = M.g[sidx(jd, t, rep, T, R)];
                 Pt += kap * om;
                 Qs += kap * clampr<real>(om, 0, 1);
@@ -663,7 +783,7 @@ __global__ void k_kop(DevModel<real> M, const double *kold, const double *k1v, c
                 for (int q = M.up[n]; q < M.up[n + 1]; ++q) {
                     int jd = M.ua[q];
                     real kap = M.d_avail[jd] * M.kc_d[jd];
-                    if (!(fabs(kap) >= (real)kmin)) continue;
+                    if (!(fabs(kap) >= km)) continue;
                     size_t gi = sidx(jd, t, rep, T, R);
                     real y0 = M.g[gi];
                     real sigma = kap * y0 / Pt;
@@ -809,11 +929,8 @@ cudaError_t launch_rebuild(const DevModel<real> &M, cudaStream_t s) {
 }
 
 
-// step chunks of the fused score pass: one per 64 steps, fewer where the partials (and the R*(K+8)
-// final sums) would not fit the static score scratch of 2^20 doubles, so that both score entry
-// points sum in the same order
 // step chunks of the score pass: 64 steps a chunk, fewer chunks where the partials (values and
-// bounds) and the sums would not fit 2^20 doubles (the static scratch). Two blocks of the pass are resident
+// bounds) and the sums would not fit 2^20 doubles (the static scratch), so that both score entry points sum in the same order. Two blocks of the pass are resident
 // per SM, 304 in all: a grid of a little more runs a second wave nearly empty, so it takes the fewer chunks
 // that fill whole waves (40 nodes, T = 8760, 64 replicas: 30 chunks of 10 blocks and not 33).
 __host__ inline int score_chunks(int T, int R, int K, int N) {
