@@ -23,55 +23,89 @@ __device__ inline real avail_map(real x) {  // logistic availability map (builde
 // LocalCost rebuild (src/local.jl:313, rebuild_step! :332): residual per node, flows per line.
 // Accumulation order per node as the reference: load, lines, generators, storage.
 // ---------------------------------------------------------------------------------------------
-template <class real>
-__global__ void k_rebuild(DevModel<real> M) {
-    const unsigned tr = blockIdx.x * blockDim.x + threadIdx.x;  // (step, replica) of node blockIdx.y
-    if (tr >= (unsigned)M.T * M.R) return;
+#define ESM_REBUILD_BLOCKS 1216  // 8 blocks of 256 threads on each of 152 SMs
+// A thread takes Q (step, replica) pairs of a node, 256 apart: the node's tables are read once for all of
+// them, and their states' loads are under way together. Q is 4 where that still fills the device, else 1
+// (40 nodes, T = 2920, 64 replicas: 216 us with 1, 178 with 4).
+template <class real, int Q>
+__global__ void __launch_bounds__(256) k_rebuild(DevModel<real> M) {
+    const unsigned TR = (unsigned)M.T * M.R, tr0 = blockIdx.x * 256u * Q + threadIdx.x;  // of node blockIdx.y
+    if (tr0 >= TR) return;
     const int n = blockIdx.y;
-    const size_t i = (size_t)n * M.T * M.R + tr;
-    const int t = (int)(tr / (unsigned)M.R), rep = (int)(tr - (unsigned)t * M.R);
-    int T = M.T, R = M.R;
-    real x = wraw(M, n, t, rep);
-    real r = x > 0 ? x : real(0);
+    const size_t row = (size_t)M.T * M.R;
+    unsigned tr[Q], tx[Q];  // the pair (past the end: the first again), the same replica a step on
+    int t[Q];
+    real r[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        tr[q] = tr0 + 256u * q < TR ? tr0 + 256u * q : tr0;
+        t[q] = (int)(tr[q] / (unsigned)M.R);
+        tx[q] = t[q] + 1 < M.T ? tr[q] + M.R : tr[q] + M.R - TR;
+    }
+    auto weather = [&](int s, int q) { return M.xbar[(size_t)s * M.T + t[q]] + M.wscale[s] * M.z[s * row + tr[q]]; };
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        real x = weather(n, q);
+        r[q] = x > 0 ? x : real(0);
+    }
     for (int p = M.nlp[n]; p < M.nlp[n + 1]; ++p) {
         int e = M.nl[p];
         int a = M.bus0[e], b = M.bus1[e];
-        real fl = M.lb[e] * (M.theta[sidx(a, t, rep, T, R)] - M.theta[sidx(b, t, rep, T, R)]);
-        if (a == n) {
-            M.F[sidx(e, t, rep, T, R)] = fl;
-            r += fl + real(0.5) * real(0);
-        } else {
-            r += -fl + real(0.5) * real(0);
+        const real lb = M.lb[e];
+        const real *ta = M.theta + a * row, *tb = M.theta + b * row;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            real fl = lb * (ta[tr[q]] - tb[tr[q]]);
+            if (a == n) {
+                M.F[e * row + tr[q]] = fl;
+                r[q] += fl + real(0.5) * real(0);
+            } else {
+                r[q] += -fl + real(0.5) * real(0);
+            }
         }
     }
     for (int p = M.nu_ptr[n]; p < M.nu_ptr[n + 1]; ++p) {
         int u = M.nu_unit[p], j = M.u_loc[u];
         int kd = M.u_kind[u];
         if (kd == ESM_UNIT_REN) {
-            real A = avail_map<real>(wraw(M, M.r_series[j], t, rep));
-            r -= A * M.kc_r[j] * real(1);
+            const int s = M.r_series[j];
+            const real kc = M.kc_r[j];
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                real A = avail_map<real>(weather(s, q));
+                r[q] -= A * kc * real(1);
+            }
         } else if (kd == ESM_UNIT_DISP) {
-            real y = clampr<real>(M.g[sidx(j, t, rep, T, R)], 0, 1);
-            r -= M.d_avail[j] * M.kc_d[j] * y;
+            const real av = M.d_avail[j], kc = M.kc_d[j];
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                real y = clampr<real>(M.g[j * row + tr[q]], 0, 1);
+                r[q] -= av * kc * y;
+            }
         }
     }
     for (int p = M.nu_ptr[n]; p < M.nu_ptr[n + 1]; ++p) {
         int u = M.nu_unit[p], j = M.u_loc[u];
         if (M.u_kind[u] != ESM_UNIT_STOR) continue;
-        real ec = clampr<real>(M.e[sidx(j, t, rep, T, R)], 0, 1);
-        real ec1 = clampr<real>(M.e[sidx(j, (t + 1) % T, rep, T, R)], 0, 1);
-        real d = M.s_hours[j] * (ec1 - ec) / M.dt - M.s_qt[j];
-        real pc, mcx;
-        if (d >= 0) {
-            pc = M.s_etain[j] > 0 ? d / M.s_etain[j] : real(0);
-            mcx = 0;
-        } else {
-            pc = 0;
-            mcx = fmin(-d * M.s_etaout[j], real(1));
+        const real h = M.s_hours[j], qt = M.s_qt[j], ein = M.s_etain[j], eout = M.s_etaout[j], kc = M.kc_s[j];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            real ec = clampr<real>(M.e[j * row + tr[q]], 0, 1);
+            real ec1 = clampr<real>(M.e[j * row + tx[q]], 0, 1);
+            real d = h * (ec1 - ec) / M.dt - qt;
+            real pc, mcx;
+            if (d >= 0) {
+                pc = ein > 0 ? d / ein : real(0);
+                mcx = 0;
+            } else {
+                pc = 0;
+                mcx = fmin(-d * eout, real(1));
+            }
+            r[q] += kc * (pc - mcx);
         }
-        r += M.kc_s[j] * (pc - mcx);
     }
-    M.r[i] = r;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) M.r[n * row + tr[q]] = r[q];
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -924,7 +958,11 @@ inline dim3 row_grid(const DevModel<real> &M, int n) {
 }
 template <class real>
 cudaError_t launch_rebuild(const DevModel<real> &M, cudaStream_t s) {
-    k_rebuild<real><<<row_grid(M, M.N), 256, 0, s>>>(M);
+    const dim3 g = row_grid(M, M.N);
+    if ((size_t)g.x * g.y >= 4 * ESM_REBUILD_BLOCKS)
+        k_rebuild<real, 4><<<dim3((g.x + 3) / 4, g.y), 256, 0, s>>>(M);
+    else
+        k_rebuild<real, 1><<<g, 256, 0, s>>>(M);
     return cudaGetLastError();
 }
 
