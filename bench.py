@@ -765,8 +765,8 @@ def main():
     ap.add_argument("--cpu-moves", type=int, default=64, help="--case n256: moves of the oracle's sample")
     ap.add_argument("--arms", default="", help="the arms measured: --case ess (default plain,learned,da), "
                     "--case learned (default plain,plain4,sur1,surinf)")
-    ap.add_argument("--sep", type=int, default=0, help="--case small: cooperative walk of separable moves of "
-                                                     "at least this many units (0: off)")
+    ap.add_argument("--sep", type=int, default=0, help="--case small: block walk of separable moves of "
+                                                     "at least this many units (0: all)")
     ap.add_argument("--case", default="full", choices=["full", "small", "batch", "storage", "n256", "ess", "mlp", "learned"],
                     help="small: the reduced profiling case (sweeps only, no JSON contract line)")
     args = ap.parse_args()
@@ -857,8 +857,8 @@ def main():
     ess = ess_arms(d, m, ctl, it0 + args.warmup + 2 * args.steps + 1, args.ess_steps) if args.ess_steps > 0 else None
     if rank != 0:
         return
-    # roofline of the dominant kernels (one colour class: k_prep_moves and one k_move launch per
-    # move, timed together as one span): algorithmic bytes of one class pass = the compulsory FP32
+    # roofline of the dominant kernels (one colour class: the descriptors' launches and a k_move and a
+    # k_move_blocks launch per move, timed together as one span): algorithmic bytes of one class pass = the compulsory FP32
     # state traffic of one colour class, 4 (11 N + 2 L) (T/2) R bytes
     N, L, T = m.N, m.L, m.T
     cls_ms, cls_n = kt["class_pass"]
@@ -880,10 +880,10 @@ def main():
             "config": config_dict(),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "peak_kind": kind,
-                         "kernel": "k_prep_moves + k_move (the line moves of one colour class, one span)",
-                         "note": ("the exact line sampler is latency-bound (per-lane walk scratch, divergent walks): "
-                                  "the HBM bytes are the compulsory state; `traffic` is the measured DRAM traffic, "
-                                  "mostly walk scratch")},
+                         "kernel": "k_prep_moves + k_move + k_move_blocks (the line moves of one colour class, one span)",
+                         "note": ("the exact line sampler is latency-bound (dependent chains of the walks): "
+                                  "the HBM bytes are the compulsory state; `traffic` is the DRAM traffic of the "
+                                  "one-lane walks (profiles/linemove_traffic.json), mostly walk scratch")},
             "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},
             "gpu_launches": int(launches), "clocks": clocks,
             "move_grid": {"warps_per_block": grid[0], "warps_per_sm": grid[1], "schedule": d.move_schedule(),

@@ -33,8 +33,8 @@ template <class real>
 int walk_region_bytes(const DevModel<real> &M);
 template <class real>
 int move_blocks(const DevModel<real> &M, int nsm, int smem, int max_warps);
-// one colour class: the descriptors of its moves into descs ((natoms + nextra) descriptors), then
-// per move one k_move launch (and one k_move_sep launch; the kernel that does not take the move
+// one colour class: the list and the descriptors of its moves into descs ((natoms + nextra) descriptors),
+// then per move one k_move launch and one k_move_blocks launch (the kernel that does not take the move
 // returns at once); the sweep index is read on the device from *sweep (graph-capturable)
 template <class real>
 cudaError_t launch_class_pass(const DevModel<real> &M, const int *steps, int nsteps, const uint32_t *sweep, int cls,

@@ -27,8 +27,8 @@
 // unit in registers, and the lists stay in shared memory. What bounds it now: the latency of the
 // events' dependent arithmetic and of the scan, at 16 warps per SM (four blocks by registers and by
 // shared memory). Measured for one move at T = 2920, 64 replicas (93440 tasks), FP32, one-lane walk
-// and block walk: 40 units 16.4 and 3.7 ms, 20 units 5.7 and 2.1 ms, 10 units 2.1 and 1.3 ms, 7 units
-// 1.4 and 0.7 ms; an operation sweep at 40 nodes, T = 8760, 64 replicas 1.47 and 0.91 s.
+// and block walk: 40 units 16.4 and 3.2 ms, 20 units 5.7 and 1.8 ms, 10 units 2.1 and 1.2 ms, 7 units
+// 1.4 and 0.7 ms.
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>

@@ -326,7 +326,8 @@ class DeviceChain:
         return out.reshape(nunits, 5, self._mlog_nrep)
 
     def set_sep_walk(self, min_units):
-        """The cooperative walk for separable moves of at least min_units units (0: off)."""
+        """The block walk for separable moves of at least min_units units (0: of all; the others keep the
+        one-lane walk)."""
         self._check(self.L.esm_set_sep_walk(self.h, int(min_units)), "esm_set_sep_walk")
 
     def sep_walk(self):

@@ -286,8 +286,8 @@ int esm_move_log(esm_ctx *ctx, int32_t cls, double *out);
    nothing else (the state-of-charge atoms, walk!, src/local.jl:1294, on a potential that is a sum of
    per-unit functions) with at least min_units units is walked by blocks of warps, a batch of (step,
    replica) tasks at a time: lanes make the units' breakpoints, the breakpoints of a window are sorted
-   in shared memory, and the sums over them are taken in order. Smaller and other moves keep one task
-   per lane (k_move). min_units 0 (the default): every separable move that fits a block's shared memory.
+   in shared memory, and the sums over them are taken in order. Smaller ones keep one task per lane
+   (k_move). min_units 0 (the default): every separable move that fits a block's shared memory.
    The same draws and points as the one-lane walk, to the last bit. esm_set_sep_walk drops the
    captured class graphs; esm_sep_walk reads the setting and the kernel's warps. No reference
    counterpart. */
