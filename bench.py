@@ -371,7 +371,7 @@ def profile_case(args):
         d.set_move_grid(*(int(x) for x in args.grid.lower().split("x")))
     elif args.autotune:
         grid = d.autotune_moves(sweep=0)[0]
-    if args.sep:
+    if args.sep is not None:
         d.set_sep_walk(args.sep)
     d.sweeps(args.warmup, 0, stats=False)
     d.set_timing(True)
@@ -379,7 +379,7 @@ def profile_case(args):
     d.scores()
     kt = d.timing()
     print(json.dumps({"case": "small", "N": w["N"], "T": w["T"], "R": w["R"], "sweeps": args.steps,
-                      "grid": list(d.move_grid()[:2]), "schedule": d.move_schedule(), "sep_walk_min_units": args.sep,
+                      "grid": list(d.move_grid()[:2]), "schedule": d.move_schedule(), "sep_walk_min_units": d.sep_walk()[0],
                       "kernel_ms": {k: v[0] for k, v in kt.items()}, "launches": {k: v[1] for k, v in kt.items()},
                       "moves_tried": int(st[:-1:2].sum()), "guards": int(st[-1])}), flush=True)
 
@@ -765,8 +765,8 @@ def main():
     ap.add_argument("--cpu-moves", type=int, default=64, help="--case n256: moves of the oracle's sample")
     ap.add_argument("--arms", default="", help="the arms measured: --case ess (default plain,learned,da), "
                     "--case learned (default plain,plain4,sur1,surinf)")
-    ap.add_argument("--sep", type=int, default=0, help="--case small: block walk of separable moves of "
-                                                     "at least this many units (0: all)")
+    ap.add_argument("--sep", type=int, default=None, help="--case small: block walk of separable moves of "
+                                                        "at least this many units (0: none)")
     ap.add_argument("--case", default="full", choices=["full", "small", "batch", "storage", "n256", "ess", "mlp", "learned"],
                     help="small: the reduced profiling case (sweeps only, no JSON contract line)")
     args = ap.parse_args()

@@ -52,8 +52,9 @@ struct esm_ctx {
     bool has_state = false, has_scores = false;
     int move_wpb = 1;           // k_move block shape: warps per block (1, 2 or 4)
     int max_warps = 0;          // k_move warps launched per move: the resident limit or a tuned count
-    // the moves walked by blocks (k_move_blocks): separable moves with at least sep_min units (0: all);
+    // the moves walked by blocks (k_move_blocks): separable moves with at least sep_min units (0: none);
     // the grid (0: not used), its shared memory, that of either kind of move, the buffer of long sorts
+    bool sep_asked = false;  // sep_min was set by a call
     int sep_min = ESM_SEP_MIN_DEFAULT, mblocks = 0, mblocks_smem = 0, sep_region = 0, walk_region = 0, sep_tmp_warp = 0;
     char *d_sep_tmp = nullptr;
     int sl_nunits = 0;  // eligible units of the last long-range storage sweep (its move log)
@@ -598,7 +599,9 @@ int class_pass_launch(esm_ctx *c, int cls, int limit) {
     int ns = c->class_len[cls];
     esm::SepLaunch sep{c->sep_min, c->mblocks, c->mblocks_smem, c->sep_region, c->sep_tmp_warp, c->walk_region,
                        c->d_sep_tmp};
-    esm::WaveLaunch wave{c->move_schedule == ESM_MOVES_PER_CLASS, c->d_wave_done, c->d_wave_err, c->wave_items};
+    // (the whole-class launch walks every move one task per lane: not where a block walk was asked for)
+    bool on = c->move_schedule == ESM_MOVES_PER_CLASS && !(c->sep_asked && c->sep_min > 0);
+    esm::WaveLaunch wave{on, c->d_wave_done, c->d_wave_err, c->wave_items};
     if (c->precision == 64)
         CK(esm::launch_class_pass<double>(c->Md, c->d_steps[cls], ns, c->d_sweep, cls, limit, (double *)c->d_scratch,
                                           c->move_wpb, c->max_warps, c->d_stats, c->d_descs, c->d_item_ctr, sep,
@@ -1657,7 +1660,7 @@ int esm_move_log(esm_ctx *c, int32_t cls, double *out) {
 int esm_set_sep_walk(esm_ctx *c, int32_t min_units) {
     if (!c) return ESM_EINVAL;
     if (min_units < 0) return fail(c, ESM_EINVAL, "min_units must be >= 0");
-    if (min_units == c->sep_min) return ESM_OK;
+    if (min_units == c->sep_min && c->sep_asked) return ESM_OK;
     int rc = esm_sync(c, 600.0);  // the captured class passes hold the old choice: drop them
     if (rc) return rc;
     for (auto &g : c->graph)
@@ -1666,6 +1669,7 @@ int esm_set_sep_walk(esm_ctx *c, int32_t min_units) {
             g = nullptr;
         }
     c->sep_min = min_units;
+    c->sep_asked = true;
     if (c->probe) return esm_set_sep_walk(c->probe, min_units);
     return ESM_OK;
 }

@@ -11,13 +11,13 @@ size_t linemove_scratch_reals(const DevModel<real> &M);  // per warp
 template <class real>
 size_t linemove_smem_per_warp(const DevModel<real> &M);  // bytes of one move descriptor
 // the moves walked by blocks (k_move_blocks) on `blocks` blocks (0: none, k_move walks every move) with
-// smem bytes of shared memory: the separable moves of at least min_units units (0: all) with `region`
+// smem bytes of shared memory: the separable moves of at least min_units units (0: none) with `region`
 // bytes (0: none) and tmp_warp bytes of tmp a warp, and the other moves with walk_region bytes (0: none)
 struct SepLaunch {
     int min_units, blocks, smem, region, tmp_warp, walk_region;
     char *tmp;
 };
-// the whole class pass in one k_move_wave launch (on = 1; not with the cooperative walk): done
+// the whole class pass in one k_move_wave launch (on = 1), every move one task per lane: done
 // holds the moves completed per work item (max_items), err is set when a bounded wait runs out
 struct WaveLaunch {
     int on;

@@ -2088,7 +2088,7 @@ cudaError_t launch_class_pass(const DevModel<real> &M, const int *steps, int nst
     int items = ntile * wpt;
     int warps = items < max_warps ? items : max_warps;
     int blocks = (warps + wpb - 1) / wpb;
-    if (wave.on && sep.min_units == 0 && (size_t)items <= wave.max_items &&
+    if (wave.on && (size_t)items <= wave.max_items &&
         (unsigned long long)items * nrun < (1ull << 32)) {
         if ((e = cudaMemsetAsync(wave.done, 0, sizeof(unsigned int) * items, s)) != cudaSuccess) return e;
         if (wpb == 4)
@@ -2102,8 +2102,7 @@ cudaError_t launch_class_pass(const DevModel<real> &M, const int *steps, int nst
                                                       scratch, stats, counters, wave.done, wave.err);
         return cudaGetLastError();
     }
-    // (min_units 0: every separable move goes to the block walk)
-    int sepmin = sep.region > 0 ? (sep.min_units > 0 ? sep.min_units : 1) : 0;
+    int sepmin = sep.region > 0 ? sep.min_units : 0;
     int ntask = nsteps * M.R;
     int bblocks = ntask < sep.blocks ? ntask : sep.blocks;
     for (int mi = 0; mi < nrun; ++mi) {

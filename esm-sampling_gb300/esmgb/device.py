@@ -326,12 +326,12 @@ class DeviceChain:
         return out.reshape(nunits, 5, self._mlog_nrep)
 
     def set_sep_walk(self, min_units):
-        """The block walk for separable moves of at least min_units units (0: of all; the others keep the
-        one-lane walk)."""
+        """The block walk for separable moves of at least min_units units (1, the default: all; 0: none; the
+        others keep the one-lane walk)."""
         self._check(self.L.esm_set_sep_walk(self.h, int(min_units)), "esm_set_sep_walk")
 
     def sep_walk(self):
-        """(min_units, warps of the cooperative walk kernel)."""
+        """(min_units, warps of the block walks' kernel)."""
         a, b = np.zeros(1, np.int32), np.zeros(1, np.int32)
         self._check(self.L.esm_sep_walk(self.h, _p(a, P_i32), _p(b, P_i32)), "esm_sep_walk")
         return int(a[0]), int(b[0])

@@ -286,12 +286,15 @@ int esm_move_log(esm_ctx *ctx, int32_t cls, double *out);
    nothing else (the state-of-charge atoms, walk!, src/local.jl:1294, on a potential that is a sum of
    per-unit functions) with at least min_units units is walked by blocks of warps, a batch of (step,
    replica) tasks at a time: lanes make the units' breakpoints, the breakpoints of a window are sorted
-   in shared memory, and the sums over them are taken in order. Smaller ones keep one task per lane
-   (k_move). min_units 0 (the default): every separable move that fits a block's shared memory.
-   The same draws and points as the one-lane walk, to the last bit. esm_set_sep_walk drops the
-   captured class graphs; esm_sep_walk reads the setting and the kernel's warps. No reference
-   counterpart. */
-#define ESM_SEP_MIN_DEFAULT 0
+   in shared memory, and the sums over them are taken in order. Smaller ones, and those that do not fit
+   a block's shared memory, keep one task per lane (k_move). min_units 1 (the default): every separable
+   move; 0: none.
+   The same draws and points as the one-lane walk, to the last bit, with one exception: in FP32 the two
+   walks may take events of one time in different orders, so where the point cap falls inside such a
+   group one of them may reach its end and the other the cap (a guard event). In FP64 the order is fixed.
+   esm_set_sep_walk drops the captured class graphs; esm_sep_walk reads the setting and the kernel's
+   warps. No reference counterpart. */
+#define ESM_SEP_MIN_DEFAULT 1
 int esm_set_sep_walk(esm_ctx *ctx, int32_t min_units);
 int esm_sep_walk(const esm_ctx *ctx, int32_t *min_units, int32_t *warps);
 
@@ -302,7 +305,8 @@ int esm_sep_walk(const esm_ctx *ctx, int32_t *min_units, int32_t *warps);
    independent, so a task's moves and their results are the same: bit-identical states), without
    the idle tail each per-move launch ends with; each of its waits for an item's previous move is
    bounded, and one that runs out makes the next esm_sync or statistics read return ESM_ETIMEOUT.
-   It walks every move one task per lane; esm_set_sep_walk > 0 keeps the per-move launches. No
+   It walks every move one task per lane; after a call of esm_set_sep_walk with a value above 0 (the
+   default's own value as well) the launches stay per move. No
    reference counterpart. */
 enum { ESM_MOVES_PER_MOVE = 0, ESM_MOVES_PER_CLASS = 1 };
 int esm_set_move_schedule(esm_ctx *ctx, int32_t schedule);

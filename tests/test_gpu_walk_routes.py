@@ -1,0 +1,64 @@
+"""Which walk a line move takes (esm_set_sep_walk, esm_set_move_schedule), seen where the walks
+differ: in FP32 the walks of one move take events of one time in their own orders, so a point cap inside
+such a group ends them differently; everywhere else every route gives the same bits."""
+import numpy as np
+import pytest
+
+from esmgb.device import DeviceChain
+from esmgb.model import initial_state, make_model
+
+pytestmark = pytest.mark.gpu
+
+
+def _state(m, R, seed, edge):
+    st = initial_state(m, R, seed=seed)
+    rng = np.random.Generator(np.random.PCG64(seed))
+    st.g = st.g + 0.02 * rng.standard_normal(st.g.shape)
+    st.theta = 5.0 * rng.standard_normal(st.theta.shape)
+    st.e = rng.uniform(-0.02, 1.02, st.e.shape)
+    if edge:                                            # many clamps at one time
+        st.e = np.round(4.0 * st.e) / 4.0
+    return st
+
+
+def _chain(m, R, st, precision=32, sep=None, schedule="move", **kw):
+    d = DeviceChain(m, R, precision=precision, seed=9, **kw)
+    d.upload(st)
+    if sep is not None:
+        d.set_sep_walk(sep)
+    d.set_move_schedule(schedule)
+    return d
+
+
+def _run(*a, **kw):
+    d = _chain(*a, **kw)
+    counts = d.sweeps(1, 0)
+    out = d.download()
+    d.close()
+    return counts, out
+
+
+def _same(x, y):
+    return np.array_equal(x[0], y[0]) and all(np.array_equal(x[1][k], y[1][k]) for k in ("theta", "g", "e"))
+
+
+def _ties():
+    """A model and state on which the block walk and the one-lane walk end differently in FP32."""
+    m = make_model(40, 60, 24, seed=3)
+    return m, 8, _state(m, 8, 7, True), {"max_points": 8}
+
+
+def test_sep_walk_zero_is_off():
+    """0 keeps the one-lane walk (the walk of the whole-class launch); the default is 1."""
+    m, R, st, kw = _ties()
+    one_lane = _run(m, R, st, schedule="class", **kw)
+    assert _same(_run(m, R, st, sep=0, **kw), one_lane)
+    block = _run(m, R, st, sep=1, **kw)
+    assert not _same(block, one_lane)                   # (else the model shows nothing)
+    assert _same(_run(m, R, st, **kw), block)
+    # a setting above 0 that was asked for keeps the launches per move, the default does not
+    assert _same(_run(m, R, st, sep=1, schedule="class", **kw), block)
+    assert _same(_run(m, R, st, sep=0, schedule="class", **kw), one_lane)
+    d = DeviceChain(m, R, seed=9)
+    assert d.sep_walk()[0] == 1
+    d.close()
