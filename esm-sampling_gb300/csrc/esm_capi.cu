@@ -1825,6 +1825,7 @@ struct esm_batch {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev = nullptr, t0 = nullptr, t1 = nullptr;
     std::vector<int> nact;        // per move index: the models that have it
+    std::vector<int> sep_on;      // per model: its sep_on on the device
     esm::BatchLaunch bl{};
     void *d_models = nullptr;     // BatchModel<real>[n]
     uint32_t *d_sweep = nullptr;
@@ -1872,6 +1873,9 @@ const esm::DevModel<float> &ctx_model<float>(const esm_ctx *c) { return c->Mf; }
 template <>
 const esm::DevModel<double> &ctx_model<double>(const esm_ctx *c) { return c->Md; }
 
+// separable moves of a chain that go to the block walk: those of at least this many units (0: none)
+int sep_units(const esm_ctx *c) { return c->sep_region > 0 ? c->sep_min : 0; }
+
 // the batch's device tables, grid limits and walk slabs
 template <class real>
 int batch_setup(esm_batch *b) {
@@ -1893,7 +1897,8 @@ int batch_setup(esm_batch *b) {
         m.descs = c->d_descs;
         m.stride = esm::linemove_smem_per_warp<real>(m.M);
         m.stats = c->d_stats;
-        m.sep_on = c->sep_region > 0 ? 1 : 0;
+        m.sep_on = sep_units(c);
+        b->sep_on.push_back(m.sep_on);
         m.walk_region = c->walk_region;
         b->bl.region = std::max(b->bl.region, std::max(c->sep_region, c->walk_region));
         b->bl.tmp_warp = std::max(b->bl.tmp_warp, c->sep_tmp_warp);
@@ -1939,6 +1944,19 @@ int batch_setup(esm_batch *b) {
     if ((rc = balloc(b, &b->bl.off, (size_t)b->bl.maxpass * (n + 1)))) return rc;
     if ((rc = balloc(b, &b->bl.counters, 2 * (size_t)b->bl.maxpass * b->bl.maxmoves))) return rc;
     if ((rc = balloc(b, &b->d_sweep, 1))) return rc;
+    return ESM_OK;
+}
+
+// the chains' settings as they are now (the captured sweep reads them on the device)
+template <class real>
+int batch_settings(esm_batch *b) {
+    esm::BatchModel<real> *dev = (esm::BatchModel<real> *)b->d_models;
+    for (int i = 0; i < b->n; ++i) {
+        int v = sep_units(b->ctx[i]);
+        if (v == b->sep_on[i]) continue;
+        BCK(cudaMemcpyAsync(&dev[i].sep_on, &v, sizeof v, cudaMemcpyHostToDevice, b->stream));
+        b->sep_on[i] = v;
+    }
     return ESM_OK;
 }
 
@@ -2065,6 +2083,7 @@ int esm_batch_sweeps(esm_batch *b, int32_t n, int64_t sweep0, int64_t *stats) {
         if (!c->has_state) return bfail(b, ESM_ESTATE, "a context has no state uploaded");
     int rc;
     if ((rc = batch_join_in(b))) return rc;
+    if ((rc = b->precision == 64 ? batch_settings<double>(b) : batch_settings<float>(b))) return rc;
     const size_t ns = 2 * (ESM_NFAM + 1) + 1;
     for (esm_ctx *c : b->ctx) BCK(cudaMemsetAsync(c->d_stats, 0, sizeof(unsigned long long) * ns, b->stream));
     BCK(cudaEventRecord(b->t0, b->stream));
@@ -2142,6 +2161,7 @@ int esm_batch_autotune(esm_batch *b, int64_t sweep, int32_t *best, int32_t *cand
     for (esm_ctx *c : b->ctx)
         if ((rc = esm_state_save(c))) return bfail(b, rc, "state save: %s", c->err.c_str());
     if ((rc = batch_join_in(b))) return rc;
+    if ((rc = b->precision == 64 ? batch_settings<double>(b) : batch_settings<float>(b))) return rc;
     int bw = b->bl.wpb, bs = (b->bl.warps + b->nsm - 1) / b->nsm;
     int nmove = std::min(b->bl.maxmoves, ESM_BATCH_TUNE_MOVES);
     double tbest = 1e300;

@@ -57,7 +57,7 @@ struct BatchModel {
     char *descs;                // its descriptor buffer: nmoves descriptors of stride bytes
     size_t stride;
     unsigned long long *stats;  // its move counts, laid out as a context's
-    int sep_on, walk_region;    // as in its own passes: separable moves from this many units; walk_run's bytes
+    int sep_on, walk_region;    // as in its own passes: separable moves from this many units (0: none); walk_run's bytes
 };
 struct BatchLaunch {
     int nm;                  // models

@@ -382,8 +382,9 @@ int64_t esm_launch_count(const esm_ctx *ctx);
  * CUDA graph captured at the batch's first sweep: the caching rebuild of every model, then per
  * colour-class pass one launch that builds every model's move descriptors and one line-move launch
  * per move index, whose work items are the tasks of every model that has that move. Each task
- * runs the arithmetic of the model's own class pass, so every model's state after
- * esm_batch_sweeps equals the state esm_operation_sweeps gives it on its own context.
+ * runs the arithmetic of the model's own class pass, by the walk that esm_set_sep_walk asks for at
+ * the time of the call, so every model's state after esm_batch_sweeps equals the state
+ * esm_operation_sweeps gives it on its own context (its launches per move).
  * ------------------------------------------------------------------------------------------ */
 typedef struct esm_batch esm_batch;
 /* ctxs [n]: contexts created by esm_create with the same precision, states uploaded, the storage

@@ -1,10 +1,10 @@
-"""Which walk a line move takes (esm_set_sep_walk, esm_set_move_schedule), seen where the walks
+"""Which walk a line move takes (esm_set_sep_walk, esm_set_move_schedule, a batch), seen where the walks
 differ: in FP32 the walks of one move take events of one time in their own orders, so a point cap inside
 such a group ends them differently; everywhere else every route gives the same bits."""
 import numpy as np
 import pytest
 
-from esmgb.device import DeviceChain
+from esmgb.device import DeviceBatch, DeviceChain
 from esmgb.model import initial_state, make_model
 
 pytestmark = pytest.mark.gpu
@@ -62,3 +62,23 @@ def test_sep_walk_zero_is_off():
     d = DeviceChain(m, R, seed=9)
     assert d.sep_walk()[0] == 1
     d.close()
+
+
+def test_batch_takes_the_chains_walk():
+    """A batch walks a chain's separable moves as the chain's own sweeps do, also when the setting changes
+    after the batch was made."""
+    m, R, st, kw = _ties()
+    m2 = make_model(12, 18, 73, seed=5)
+    st2 = _state(m2, 4, 8, False)
+    a, b = _chain(m, R, st, **kw), _chain(m2, 4, st2)
+    batch = DeviceBatch([a, b])
+    for sep in (0, 41):                                 # (no move has 41 units)
+        a.set_sep_walk(sep)
+        a.upload(st)
+        b.upload(st2)
+        counts = batch.sweeps(1, sweep0=0)
+        assert _same((counts[0], a.download()), _run(m, R, st, sep=sep, **kw)), sep
+        assert _same((counts[1], b.download()), _run(m2, 4, st2)), sep
+    batch.close()
+    a.close()
+    b.close()
