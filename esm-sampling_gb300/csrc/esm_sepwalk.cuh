@@ -1034,13 +1034,16 @@ struct SepWalk {
     }
 };
 
-// Whether move descriptor d is separable with at least sepmin units (the moves of sep_run).
+// Whether a move's header is that of a separable move; whether descriptor d is such a move with at least
+// sepmin units (the moves of sep_run).
+__device__ inline bool sep_header(const int *h) {
+    return h[1] > 0 && h[0] == 0 && h[2] == 0 && h[3] == 0 && h[4] == 0 && h[6] == 0 && h[8] == 0 && h[5] == h[1] &&
+           h[7] == h[1];
+}
 template <class real>
 __device__ inline bool sep_move(const Desc<real> &d, int sepmin) {
     const int *h = d.hdr;
-    bool sep = h[1] > 0 && h[0] == 0 && h[2] == 0 && h[3] == 0 && h[4] == 0 && h[6] == 0 && h[8] == 0 &&
-               h[5] == h[1] && h[7] == h[1];
-    return sepmin > 0 && h[12] >= 0 && sep && h[1] >= sepmin;
+    return sepmin > 0 && h[12] >= 0 && sep_header(h) && h[1] >= sepmin;
 }
 
 // The walks of separable move mi of one model over a block's tasks, in batches of as many as its shared

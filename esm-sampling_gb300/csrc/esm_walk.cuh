@@ -454,11 +454,13 @@ struct LineWalk {
     }
 };
 
-// Whether the walk of descriptor d is this file's, in a block with `region` bytes.
+// Whether the walk of descriptor d is this file's, in a block with `region` bytes. A separable move that the
+// block walk does not take (its units below the threshold, or no room) is not, whatever its units: the
+// one-lane walk advances its potential along the units' slopes, which rounds otherwise than evaluations do.
 template <class real>
 __device__ inline bool walk_move(const Desc<real> &d, int region, WalkLayout *w) {
     const int *h = d.hdr;
-    if (region == 0 || h[12] < 0 || h[3] > 0 || h[4] > 0 || h[1] > 1) return false;
+    if (region == 0 || h[12] < 0 || h[3] > 0 || h[4] > 0 || h[1] > 1 || sep_header(h)) return false;
     *w = walk_layout<real>(h[0], h[6], h[2], h[1], h[5], h[7]);
     return walk_const_bytes<real>(*w) + walk_warp_bytes<real>(*w) <= region;
 }

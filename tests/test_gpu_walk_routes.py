@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from esmgb.device import DeviceBatch, DeviceChain
-from esmgb.model import initial_state, make_model
+from esmgb.model import ROLE_SE, Atoms, initial_state, make_model
 
 pytestmark = pytest.mark.gpu
 
@@ -82,3 +82,17 @@ def test_batch_takes_the_chains_walk():
     batch.close()
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+def test_single_unit_below_the_threshold(precision):
+    """Atoms of one storage unit, below the set number of units, keep the one-lane walk's bits."""
+    m = make_model(12, 18, 73, seed=3)
+    for f, a in enumerate(m.atoms):
+        if a.role == ROLE_SE:
+            idx = np.unique(a.idx).astype(np.int32)
+            m.atoms[f] = Atoms(ROLE_SE, np.arange(len(idx) + 1, dtype=np.int32), idx, np.ones(len(idx)))
+    st = _state(m, 8, 7, False)
+    one_lane = _run(m, 8, st, precision, schedule="class")
+    for sep in (0, 1, 2):
+        assert _same(_run(m, 8, st, precision, sep=sep), one_lane), sep
