@@ -197,6 +197,7 @@ struct LineWalk {
         real xs = 0, cs = 0, zs = 0;                   // a storage root's point
         real pdcs = 0, pdca = 0, dcs = 0, dca = 0;     // the storage term's d, before and now
         int np = 0, nx = 0, nro = 0, ri = 0, ngo = 0, gi = 0;
+        int nlast = 0;  // roots of the segment taken at `last`
         bool more = false;
         auto push = [&](real x, real v, real z) {
             if (np >= maxpts) {
@@ -216,15 +217,17 @@ struct LineWalk {
             pdcs = dcs;
             pdca = dca;
         };
-        // the sign changes of the node balances between lo and hi beyond the last root taken, in walking
-        // order; as many as the buffer takes
+        // the sign changes of the node balances between lo and hi in walking order, as many as the buffer
+        // takes; beyond: those after the roots already taken, of which nlast lie at `last`
         auto roots = [&](bool beyond) {
+            int skip = beyond ? nlast : 0;
+            if (!beyond) nlast = 0;
             nro = 0;
             more = false;
             for (int q = 0; q < m; ++q) {
                 real x, b = add_rn(T(W.tr + q), L(W.cur + q));
                 if (!sep_root<real>(L(W.prev + q), b, lo, hi, sgn, &x)) continue;
-                if (beyond && !(sgn * (x - last) > 0)) continue;
+                if (beyond && !(sgn * (x - last) > 0) && (x != last || skip-- > 0)) continue;
                 int j = nro;
                 if (j == ESM_WALK_ROOTS) {
                     more = true;
@@ -347,6 +350,7 @@ struct LineWalk {
                     piece = true;
                 } else {  // ROOT
                     push(te, v, z);
+                    nlast = nlast > 0 && te == last ? nlast + 1 : 1;
                     last = te;
                     if (st != DONE && ++ri == nro) {
                         if (more)

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from esmgb.device import DeviceBatch, DeviceChain
-from esmgb.model import ROLE_SE, Atoms, initial_state, make_model
+from esmgb.model import ROLE_GEN, ROLE_SE, Atoms, initial_state, make_model
 
 pytestmark = pytest.mark.gpu
 
@@ -96,3 +96,29 @@ def test_single_unit_below_the_threshold(precision):
     one_lane = _run(m, 8, st, precision, schedule="class")
     for sep in (0, 1, 2):
         assert _same(_run(m, 8, st, precision, sep=sep), one_lane), sep
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("cap", [10, 13, 0])
+def test_equal_roots_beyond_the_buffer(precision, cap):
+    """More node-balance roots at one time than the walk takes at once are all points of the walk: with a
+    cap between the buffer and their number it ends in a guard event."""
+    m = make_model(12, 18, 24, seed=3)
+    for a in m.atoms:                                   # the one generator atom of all nodes, no other move
+        n = np.diff(a.ptr)
+        keep = int(np.flatnonzero(n == 12)[0]) if a.role == ROLE_GEN else 0
+        s = slice(a.ptr[keep], a.ptr[keep + 1] if a.role == ROLE_GEN else a.ptr[keep])
+        a.idx, a.val = a.idx[s].copy(), a.val[s].copy()
+        a.ptr = np.array([0, len(a.idx)] if len(a.idx) else [0], np.int32)
+    m.xbar[:m.N] = 2000.0                               # nodes alike: their balances vanish at one t
+    m.wscale[:] = 0.0
+    m.unit_mc[:] = 40.0
+    st = initial_state(m, 4, seed=7)
+    st.z[:] = 0.0
+    st.g[:] = 0.3
+    st.k[:] = 0.0
+    st.k[m.disp] = 5000.0
+    out = [_run(m, 4, st, precision, schedule=s, extra=0.0, max_points=cap) for s in ("move", "class")]
+    assert out[1][0][:-1:2].sum() == m.T * 4
+    assert out[1][0][-1] == (m.T * 4 if 0 < cap < 13 else 0)
+    assert _same(*out)
