@@ -1621,8 +1621,9 @@ namespace esm {
 // descriptor is the same for all tasks and is built once here. One warp makes the list and runs
 // through the selections, which fixes where in the stream each move's begins (list_class; header
 // words 13 and 14 of descriptor mi: that place, the move); then one warp per move builds its
-// descriptor (descs + mi * stride; header word 12: the family index, -1: no move), smem its workspace
-// of stride bytes, sd the shared Desc that carves it. Bound by the latency of the one warp's selections.
+// descriptor (descs + mi * stride), smem its workspace of stride bytes, sd the shared Desc that carves it.
+// Its header says which kernel walks the move, so that the other's launch is over after one read: word 12 the
+// family index (-1: no move), word 13 walk_bytes, word 15 sep_units. Bound by the latency of the one warp's selections.
 // 40 nodes (319 moves): 2.2 ms with one warp for the descriptors too, 0.30 so; 128 nodes (1023): 0.96.
 // the header words of a descriptor
 template <class real>
@@ -1665,7 +1666,11 @@ __device__ __forceinline__ void prep_desc(const DevModel<real> &M, char *smem, D
     const int *h = desc_hdr<real>(out, M);
     Stream st(M.seed, (uint32_t)cls, sweep, (uint32_t)h[13]);
     int fi = prep_move(M, d, st, h[14], lane);
-    if (lane == 0) d.hdr[12] = fi;
+    if (lane == 0) {
+        d.hdr[12] = fi;
+        d.hdr[13] = fi < 0 ? 0x7fffffff : walk_bytes<real>(d.hdr);
+        d.hdr[15] = fi < 0 ? 0 : sep_units(d.hdr);
+    }
     __syncwarp();
     const size_t from = (size_t)((char *)d.hdr - smem) / 16 * 16;  // (the list in front is of no use to a move)
     const int4 *src = (const int4 *)(smem + from);
@@ -1748,8 +1753,8 @@ __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
     int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     {  // not a valid move, or one that k_move_blocks walks: nothing to do (grid-uniform)
         const Desc<real> g = carve_desc<real>((char *)(descs + (size_t)mi * stride), M, M.natoms + M.nextra);
-        WalkLayout w;
-        if (g.hdr[12] < 0 || sep_move<real>(g, sepmin) || walk_move<real>(g, walk_region, &w)) return;
+        const bool none = g.hdr[12] < 0, sep = sep_move<real>(g, sepmin), walk = walk_move<real>(g, walk_region);
+        if (none || sep || walk) return;
     }
     {  // the block's warps share one copy of the descriptor
         const int4 *src = (const int4 *)(descs + (size_t)mi * stride);
@@ -1859,9 +1864,8 @@ __global__ void __launch_bounds__(32 * ESM_SEP_WARPS, sizeof(real) == 8 ? 2 : 4)
                       tmp + ((size_t)blockIdx.x * ESM_SEP_WARPS + wib) * tmp_warp, steps, nsteps, *sweep_p, mi, ntask,
                       tried, moved, guards, [&](int n) { return (int)atomicAdd(next_item, 1u) * n; });
     } else {
-        WalkLayout w;
-        if (!walk_move<real>(d, walk_region, &w)) return;  // (grid-uniform)
-        if (threadIdx.x == 0) sW = w;
+        if (!walk_move<real>(d, walk_region)) return;  // (grid-uniform)
+        if (threadIdx.x == 0) sW = desc_walk<real>(d);
         __syncthreads();
         walk_run<real>(M, d, sW, smem, walk_region,
                        scratch + ((size_t)blockIdx.x * ESM_WALK_WARPS + wib) * scratch_per_warp, steps, nsteps, *sweep_p,
@@ -2250,9 +2254,8 @@ __global__ void __launch_bounds__(32 * ESM_SEP_WARPS, sizeof(real) == 8 ? 2 : 4)
                               return x;
                           });
         } else {
-            WalkLayout w;
-            if (!walk_move<real>(d, bm[b].walk_region, &w)) continue;  // (block-uniform)
-            if (threadIdx.x == 0) sW = w;
+            if (!walk_move<real>(d, bm[b].walk_region)) continue;  // (block-uniform)
+            if (threadIdx.x == 0) sW = desc_walk<real>(d);
             __syncthreads();
             int at = t0 + 16 * wib;
             walk_run<real>(M, d, sW, smem, bm[b].walk_region, scratch, steps, nsteps, sweep, mi, end, tried, moved, guards,
@@ -2322,8 +2325,8 @@ __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
             __syncwarp();
             cur = b;
             fi = sd[wib].hdr[12];
-            WalkLayout w;  // (k_move_blocks_batch's moves: nothing to do)
-            if (fi >= 0 && (sep_move<real>(sd[wib], bm[b].sep_on) || walk_move<real>(sd[wib], bm[b].walk_region, &w))) fi = -1;
+            // (k_move_blocks_batch's moves: nothing to do)
+            if (sep_move<real>(sd[wib], bm[b].sep_on) || walk_move<real>(sd[wib], bm[b].walk_region)) fi = -1;
             cls = pass_cls[b];
             nsteps = cls >= 0 ? bm[b].nsteps[cls] : 0;
             steps = cls >= 0 ? bm[b].steps[cls] : nullptr;

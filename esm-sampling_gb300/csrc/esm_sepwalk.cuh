@@ -1034,16 +1034,15 @@ struct SepWalk {
     }
 };
 
-// Whether a move's header is that of a separable move; whether descriptor d is such a move with at least
-// sepmin units (the moves of sep_run).
-__device__ inline bool sep_header(const int *h) {
-    return h[1] > 0 && h[0] == 0 && h[2] == 0 && h[3] == 0 && h[4] == 0 && h[6] == 0 && h[8] == 0 && h[5] == h[1] &&
-           h[7] == h[1];
+// The units of a separable move by its header (0: not separable); whether descriptor d is such a move with at
+// least sepmin units (the moves of sep_run).
+__device__ inline int sep_units(const int *h) {
+    bool sep = h[0] == 0 && h[2] == 0 && h[3] == 0 && h[4] == 0 && h[6] == 0 && h[8] == 0 && h[5] == h[1] && h[7] == h[1];
+    return sep ? h[1] : 0;
 }
 template <class real>
 __device__ inline bool sep_move(const Desc<real> &d, int sepmin) {
-    const int *h = d.hdr;
-    return sepmin > 0 && h[12] >= 0 && sep_header(h) && h[1] >= sepmin;
+    return sepmin > 0 && d.hdr[15] >= sepmin;
 }
 
 // The walks of separable move mi of one model over a block's tasks, in batches of as many as its shared

@@ -458,15 +458,24 @@ struct LineWalk {
     }
 };
 
-// Whether the walk of descriptor d is this file's, in a block with `region` bytes. A separable move that the
-// block walk does not take (its units below the threshold, or no room) is not, whatever its units: the
-// one-lane walk advances its potential along the units' slopes, which rounds otherwise than evaluations do.
+// The shared memory of a move's walk in a block with one warp, by its header; more than any block has where
+// the walk is not this file's: kinks, several storage units, or a separable move (one that the block walk does
+// not take keeps the one-lane walk, which advances its potential along the units' slopes: other roundings).
 template <class real>
-__device__ inline bool walk_move(const Desc<real> &d, int region, WalkLayout *w) {
+__device__ inline int walk_bytes(const int *h) {
+    if (h[3] > 0 || h[4] > 0 || h[1] > 1 || sep_units(h) > 0) return 0x7fffffff;
+    const WalkLayout w = walk_layout<real>(h[0], h[6], h[2], h[1], h[5], h[7]);
+    return walk_const_bytes<real>(w) + walk_warp_bytes<real>(w);
+}
+// whether descriptor d is walked so in a block with `region` bytes
+template <class real>
+__device__ inline bool walk_move(const Desc<real> &d, int region) {
+    return d.hdr[13] <= region;
+}
+template <class real>
+__device__ inline WalkLayout desc_walk(const Desc<real> &d) {
     const int *h = d.hdr;
-    if (region == 0 || h[12] < 0 || h[3] > 0 || h[4] > 0 || h[1] > 1 || sep_header(h)) return false;
-    *w = walk_layout<real>(h[0], h[6], h[2], h[1], h[5], h[7]);
-    return walk_const_bytes<real>(*w) + walk_warp_bytes<real>(*w) <= region;
+    return walk_layout<real>(h[0], h[6], h[2], h[1], h[5], h[7]);
 }
 
 // The walks of move mi of one model by the warps of a block, as many as its shared memory (region bytes
