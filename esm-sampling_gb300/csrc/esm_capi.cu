@@ -57,6 +57,7 @@ struct esm_ctx {
     bool sep_asked = false;  // sep_min was set by a call
     int sep_min = ESM_SEP_MIN_DEFAULT, mblocks = 0, mblocks_smem = 0, sep_region = 0, walk_region = 0, sep_tmp_warp = 0;
     char *d_sep_tmp = nullptr;
+    int *d_redo = nullptr;   // FP32: tasks of a move that the block walk leaves to the one-lane walk
     int sl_nunits = 0;  // eligible units of the last long-range storage sweep (its move log)
     int device = -1;                   // the device the context was created on
     double *score_scratch = nullptr;   // device address of the static score scratch on that device
@@ -503,12 +504,13 @@ int alloc_state(esm_ctx *c) {
     if (c->mblocks_smem > 0) c->mblocks = esm::move_blocks<real>(M, nsm, c->mblocks_smem, (int)wscr);
     c->sep_tmp_warp = esm::sep_tmp_bytes<real>(M);
     if ((rc = dalloc(c, &c->d_sep_tmp, (size_t)4 * c->sep_tmp_warp * c->mblocks))) return rc;
+    if (sizeof(real) == 4 && (rc = dalloc(c, &c->d_redo, (size_t)((M.T + 1) / 2) * M.R))) return rc;
     // the move descriptors of a class pass
     char *dp;
     if ((rc = dalloc(c, &dp, esm::linemove_smem_per_warp<real>(M) * (size_t)(M.natoms + M.nextra)))) return rc;
     c->d_descs = dp;
     unsigned int *ctr;
-    if ((rc = dalloc(c, &ctr, (size_t)(M.natoms + M.nextra)))) return rc;
+    if ((rc = dalloc(c, &ctr, 2 * (size_t)(M.natoms + M.nextra)))) return rc;
     c->d_item_ctr = ctr;
     if ((rc = dalloc(c, &c->d_sweep, 1))) return rc;
     if ((rc = dalloc(c, &c->d_sms_stats, 3))) return rc;
@@ -598,7 +600,7 @@ __global__ void k_set_word(uint32_t *p, uint32_t v) { *p = v; }
 int class_pass_launch(esm_ctx *c, int cls, int limit) {
     int ns = c->class_len[cls];
     esm::SepLaunch sep{c->sep_min, c->mblocks, c->mblocks_smem, c->sep_region, c->sep_tmp_warp, c->walk_region,
-                       c->d_sep_tmp};
+                       c->d_sep_tmp, c->d_redo};
     // (the whole-class launch walks every move one task per lane: not where a block walk was asked for)
     bool on = c->move_schedule == ESM_MOVES_PER_CLASS && !(c->sep_asked && c->sep_min > 0);
     esm::WaveLaunch wave{on, c->d_wave_done, c->d_wave_err, c->wave_items};
@@ -1881,7 +1883,7 @@ template <class real>
 int batch_setup(esm_batch *b) {
     int n = b->n, rc;
     std::vector<esm::BatchModel<real>> hm(n);
-    size_t maxstride = 0, maxlane = 0;
+    size_t maxstride = 0, maxlane = 0, tasks = 0;
     b->bl.maxpass = 0;
     for (int i = 0; i < n; ++i) {
         esm_ctx *c = b->ctx[i];
@@ -1905,6 +1907,7 @@ int batch_setup(esm_batch *b) {
         maxstride = std::max(maxstride, m.stride);
         maxlane = std::max(maxlane, esm::linemove_scratch_reals<real>(m.M));
         b->bl.maxpass = std::max(b->bl.maxpass, c->ncls);
+        tasks += (size_t)((m.M.T + 1) / 2) * m.M.R;
     }
     if ((rc = balloc(b, (esm::BatchModel<real> **)&b->d_models, (size_t)n))) return rc;
     BCK(cudaMemcpy(b->d_models, hm.data(), sizeof(esm::BatchModel<real>) * n, cudaMemcpyHostToDevice));
@@ -1942,7 +1945,8 @@ int batch_setup(esm_batch *b) {
     if ((rc = balloc(b, &b->bl.pass_cls, (size_t)b->bl.maxpass * n))) return rc;
     if ((rc = balloc(b, &b->bl.choff, (size_t)b->bl.maxpass * (n + 1)))) return rc;
     if ((rc = balloc(b, &b->bl.off, (size_t)b->bl.maxpass * (n + 1)))) return rc;
-    if ((rc = balloc(b, &b->bl.counters, 2 * (size_t)b->bl.maxpass * b->bl.maxmoves))) return rc;
+    if ((rc = balloc(b, &b->bl.counters, 3 * (size_t)b->bl.maxpass * b->bl.maxmoves))) return rc;
+    if (sizeof(real) == 4 && (rc = balloc(b, &b->bl.redo, tasks))) return rc;
     if ((rc = balloc(b, &b->d_sweep, 1))) return rc;
     return ESM_OK;
 }

@@ -16,6 +16,7 @@ size_t linemove_smem_per_warp(const DevModel<real> &M);  // bytes of one move de
 struct SepLaunch {
     int min_units, blocks, smem, region, tmp_warp, walk_region;
     char *tmp;
+    int *redo;  // [tasks of a class] FP32: those of a move that the block walk leaves to k_move
 };
 // the whole class pass in one k_move_wave launch (on = 1), every move one task per lane: done
 // holds the moves completed per work item (max_items), err is set when a bounded wait runs out
@@ -72,7 +73,8 @@ struct BatchLaunch {
     int *pass_cls;           // device [maxpass * nm]: the class model b runs in pass p (-1: none)
     unsigned int *off;       // device [maxpass * (nm + 1)]: the item prefix over the models of pass p
     unsigned int *choff;     // device [maxpass * (nm + 1)]: the chunk prefix (k_move_blocks_batch)
-    unsigned int *counters;  // device [2 * maxpass * maxmoves]: the item and chunk counters of the launches
+    unsigned int *counters;  // device [3 * maxpass * maxmoves]: the item, chunk and redo counters of the launches
+    unsigned long long *redo;  // device [tasks of a pass] FP32: chunk (high word) and task left to k_move_batch
     int bblocks, region, tmp_warp;  // k_move_blocks_batch: blocks (0: not used), shared memory, sort buffer
     char *tmp;
 };

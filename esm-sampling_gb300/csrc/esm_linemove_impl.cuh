@@ -1626,10 +1626,9 @@ namespace esm {
 // family index (-1: no move), word 13 walk_bytes, word 15 sep_units. Bound by the latency of the one warp's selections.
 // 40 nodes (319 moves): 2.2 ms with one warp for the descriptors too, 0.30 so; 128 nodes (1023): 0.96.
 // the header words of a descriptor
-template <class real>
-__device__ inline int *desc_hdr(char *desc, const DevModel<real> &M) {
+__device__ inline int *desc_hdr(char *desc, int nmoves) {
     Carve c(desc);
-    c.take<int>(M.natoms + M.nextra);
+    c.take<int>(nmoves);
     return c.take<int>(16);
 }
 
@@ -1641,7 +1640,7 @@ __device__ __forceinline__ void list_class(const DevModel<real> &M, int *moves, 
     for (int mi = 0; mi < nrun; ++mi) {
         const int mv = moves[mi];
         if (lane == 0) {
-            int *h = desc_hdr<real>(descs + (size_t)mi * stride, M);
+            int *h = desc_hdr(descs + (size_t)mi * stride, M.natoms + M.nextra);
             h[13] = (int)st.j;
             h[14] = mv;
         }
@@ -1663,7 +1662,7 @@ __device__ __forceinline__ void prep_desc(const DevModel<real> &M, char *smem, D
     }
     for (int i = lane; i < M.L; i += 32) d.lmark[i] = 0;
     __syncwarp();
-    const int *h = desc_hdr<real>(out, M);
+    const int *h = desc_hdr(out, M.natoms + M.nextra);
     Stream st(M.seed, (uint32_t)cls, sweep, (uint32_t)h[13]);
     int fi = prep_move(M, d, st, h[14], lane);
     if (lane == 0) {
@@ -1746,15 +1745,19 @@ template <class real, int WPB>
 __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
     k_move(const __grid_constant__ DevModel<real> M, const int *steps, int nsteps, int ntile, int wpt,
            const uint32_t *sweep_p, int mi, const char *descs, size_t stride, real *scratch,
-           unsigned long long *stats, unsigned int *next_item, int sepmin, int walk_region) {
+           unsigned long long *stats, unsigned int *next_item, int sepmin, int walk_region, const int *redo,
+           const unsigned int *nredo) {
     extern __shared__ __align__(16) char smem[];
     __shared__ Desc<real> sd;
     __shared__ LaneLayout sLL;
     int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    {  // not a valid move, or one that k_move_blocks walks: nothing to do (grid-uniform)
-        const Desc<real> g = carve_desc<real>((char *)(descs + (size_t)mi * stride), M, M.natoms + M.nextra);
-        const bool none = g.hdr[12] < 0, sep = sep_move<real>(g, sepmin), walk = walk_move<real>(g, walk_region);
-        if (none || sep || walk) return;
+    // of a move that k_move_blocks walked, the tasks it left (redo; read with the header, not after it)
+    int left = sizeof(real) == 4 ? (int)*nredo : 0;
+    {  // not a valid move, or one of k_move_blocks that left none: nothing to do (grid-uniform)
+        const int *g = desc_hdr((char *)(descs + (size_t)mi * stride), M.natoms + M.nextra);
+        const bool none = g[12] < 0, sep = sep_move(g, sepmin), walk = walk_move(g, walk_region);
+        if (none || walk || (sep && left == 0)) return;
+        if (left == 0) left = -1;
     }
     {  // the block's warps share one copy of the descriptor
         const int4 *src = (const int4 *)(descs + (size_t)mi * stride);
@@ -1780,18 +1783,30 @@ __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
     Lane<real> Ln(M, d, slab, loc ? 1 : 32, lane, LL);
     uint32_t sweep = *sweep_p;
     unsigned long long tried = 0, moved = 0, guards = 0;
-    int nitems = ntile * wpt;
+    const int nitems = left >= 0 ? (left + 31) / 32 : ntile * wpt;
+    int at = blockIdx.x * WPB + wib;
     while (true) {
-        unsigned int it = 0;
-        if (lane == 0) it = atomicAdd(next_item, 1u);
-        int item = (int)__shfl_sync(0xffffffffu, it, 0);
+        int item = at, q, task;
+        if (left >= 0) {
+            at += gridDim.x * WPB;
+        } else {
+            unsigned int it = 0;
+            if (lane == 0) it = atomicAdd(next_item, 1u);
+            item = (int)__shfl_sync(0xffffffffu, it, 0);
+        }
         if (item >= nitems) break;
-        int tile = item / wpt, grp = item % wpt;
-        int task = grp * 32 + lane;
-        int sit = task / M.R;
+        if (left >= 0) {
+            if (item * 32 + lane >= left) continue;
+            task = redo[item * 32 + lane];
+            q = task / M.R;
+        } else {
+            int tile = item / wpt, grp = item % wpt;
+            task = grp * 32 + lane;
+            int sit = task / M.R;
+            q = tile * M.span + sit;
+            if (!(sit < M.span && q < nsteps)) continue;
+        }
         Ln.rep = task % M.R;
-        int q = tile * M.span + sit;
-        if (!(sit < M.span && q < nsteps)) continue;
         bool guard;
         real t = move_task<real>(Ln, M, d, LL, fi, mi, steps[q], sweep, &guard);
         if (guard) ++guards;
@@ -1844,7 +1859,8 @@ __device__ __forceinline__ int scan_warp(int *slot) {
 }
 
 // Move mi of the class for every (step, replica) task when sep_run (a separable move of at least sepmin
-// units; sepmin 0: none) or walk_run walks it (else nothing: k_move does).
+// units; sepmin 0: none) or walk_run walks it (else nothing: k_move does, which is launched after this kernel
+// and also takes the tasks that it lists in redo).
 // Registers: four blocks an SM in FP32 (128 a thread); two in FP64, whose walks spill at 128 (a sweep of 40
 // nodes, T = 1460, 4 replicas: 231 ms with four, 251 with three, 192 with two; T = 120, 32 replicas: 153 and 156).
 template <class real>
@@ -1852,19 +1868,20 @@ __global__ void __launch_bounds__(32 * ESM_SEP_WARPS, sizeof(real) == 8 ? 2 : 4)
     k_move_blocks(const __grid_constant__ DevModel<real> M, const int *steps, int nsteps, const uint32_t *sweep_p,
                   int mi, const char *descs, size_t stride, int sepmin, int region, int walk_region, char *tmp,
                   int tmp_warp, real *scratch, size_t scratch_per_warp, unsigned long long *stats,
-                  unsigned int *next_item) {
+                  unsigned int *next_item, int *redo, unsigned int *nredo) {
     extern __shared__ __align__(16) char smem[];
     __shared__ SepBlock<real> B;
     __shared__ WalkLayout sW;
     const Desc<real> d = carve_desc<real>((char *)(descs + (size_t)mi * stride), M, M.natoms + M.nextra);
     const int ntask = nsteps * M.R, wib = threadIdx.x >> 5;
     unsigned int tried = 0, moved = 0, guards = 0;
-    if (sep_move<real>(d, sepmin)) {
+    if (sep_move(d.hdr, sepmin)) {
         sep_run<real>(M, d, B, smem, region, (ntask + gridDim.x - 1) / gridDim.x, scan_warp(&B.batch),
                       tmp + ((size_t)blockIdx.x * ESM_SEP_WARPS + wib) * tmp_warp, steps, nsteps, *sweep_p, mi, ntask,
-                      tried, moved, guards, [&](int n) { return (int)atomicAdd(next_item, 1u) * n; });
+                      tried, moved, guards, [&](int n) { return (int)atomicAdd(next_item, 1u) * n; },
+                      [&](int task) { redo[atomicAdd(nredo, 1u)] = task; });
     } else {
-        if (!walk_move<real>(d, walk_region)) return;  // (grid-uniform)
+        if (!walk_move(d.hdr, walk_region)) return;  // (grid-uniform)
         if (threadIdx.x == 0) sW = desc_walk<real>(d);
         __syncthreads();
         walk_run<real>(M, d, sW, smem, walk_region,
@@ -2081,7 +2098,8 @@ cudaError_t launch_class_pass(const DevModel<real> &M, const int *steps, int nst
     int nmoves = M.natoms + M.nextra;
     int nrun = limit > 0 && limit < nmoves ? limit : nmoves;
     size_t stride = linemove_smem_per_warp(M);
-    cudaError_t e = cudaMemsetAsync(counters, 0, sizeof(unsigned int) * nrun, s);
+    unsigned int *nredo = counters + nmoves;
+    cudaError_t e = cudaMemsetAsync(counters, 0, sizeof(unsigned int) * 2 * nmoves, s);
     if (e != cudaSuccess) return e;
     k_prep_list<real><<<1, 32, sizeof(int) * nmoves, s>>>(M, sweep, cls, nrun, descs, stride);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -2110,22 +2128,22 @@ cudaError_t launch_class_pass(const DevModel<real> &M, const int *steps, int nst
     int ntask = nsteps * M.R;
     int bblocks = ntask < sep.blocks ? ntask : sep.blocks;
     for (int mi = 0; mi < nrun; ++mi) {
-        if (wpb == 4)
-            k_move<real, 4><<<blocks, 128, stride, s>>>(M, steps, nsteps, ntile, wpt, sweep, mi, descs, stride, scratch,
-                                                       stats, counters + mi, sepmin, sep.walk_region);
-        else if (wpb == 2)
-            k_move<real, 2><<<blocks, 64, stride, s>>>(M, steps, nsteps, ntile, wpt, sweep, mi, descs, stride, scratch,
-                                                      stats, counters + mi, sepmin, sep.walk_region);
-        else
-            k_move<real, 1><<<blocks, 32, stride, s>>>(M, steps, nsteps, ntile, wpt, sweep, mi, descs, stride, scratch,
-                                                      stats, counters + mi, sepmin, sep.walk_region);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
         if (sep.blocks > 0) {
             k_move_blocks<real><<<bblocks, 32 * ESM_SEP_WARPS, sep.smem, s>>>(
                 M, steps, nsteps, sweep, mi, descs, stride, sepmin, sep.region, sep.walk_region, sep.tmp, sep.tmp_warp,
-                scratch, linemove_scratch_reals(M), stats, counters + mi);
+                scratch, linemove_scratch_reals(M), stats, counters + mi, sep.redo, nredo + mi);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
+        if (wpb == 4)
+            k_move<real, 4><<<blocks, 128, stride, s>>>(M, steps, nsteps, ntile, wpt, sweep, mi, descs, stride, scratch,
+                                                       stats, counters + mi, sepmin, sep.walk_region, sep.redo, nredo + mi);
+        else if (wpb == 2)
+            k_move<real, 2><<<blocks, 64, stride, s>>>(M, steps, nsteps, ntile, wpt, sweep, mi, descs, stride, scratch,
+                                                      stats, counters + mi, sepmin, sep.walk_region, sep.redo, nredo + mi);
+        else
+            k_move<real, 1><<<blocks, 32, stride, s>>>(M, steps, nsteps, ntile, wpt, sweep, mi, descs, stride, scratch,
+                                                      stats, counters + mi, sepmin, sep.walk_region, sep.redo, nredo + mi);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
@@ -2182,21 +2200,27 @@ __global__ void __launch_bounds__(32) k_prep_batch(const BatchModel<real> *bm, c
     prep_desc<real>(B.M, smem, sd, *sweep_p, cls, B.descs + (size_t)blockIdx.x * B.stride, B.stride, threadIdx.x);
 }
 
-// Move mi of the current pass for every task of the first nact models of the batch. A warp takes
-// items from the launch's counter; an item (32 tasks of one model's tile, as in k_move) belongs to
-// the model b with off[b] <= item < off[b + 1]. When a warp's item comes from another model than
-// its last one, the warp copies that model's tables and layout into its shared memory and points
-// its descriptor at the model's descriptor mi in global memory (read-only during the move), after
-// adding its counts so far to the previous model's statistics. Each task then runs exactly the
-// arithmetic of k_move (move_task), so a model's state after a batch pass is the state its own
-// class pass gives. The cooperative walk of separable moves is not used in a batch.
+// the last of n models whose prefix is <= x
+__device__ __forceinline__ int prefix_at(const unsigned int *off, int n, unsigned int x) {
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        int mid = (lo + hi + 1) >> 1;
+        if (off[mid] <= x)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    return lo;
+}
+
 // Move mi of the current pass for the models whose move sep_run or walk_run walks: blocks take chunks of
 // ESM_CHUNK tasks of one model from the launch's counter (choff: the chunk prefix over the models).
 template <class real>
 __global__ void __launch_bounds__(32 * ESM_SEP_WARPS, sizeof(real) == 8 ? 2 : 4)
     k_move_blocks_batch(const BatchModel<real> *bm, int nact, const int *pass_cls, const unsigned int *choff,
                         const uint32_t *sweep_p, int mi, int region, char *tmp, int tmp_warp, real *scratch,
-                        size_t scratch_per_warp, unsigned int *next_chunk) {
+                        size_t scratch_per_warp, unsigned int *next_chunk, unsigned long long *redo,
+                        unsigned int *nredo) {
     extern __shared__ __align__(16) char smem[];
     __shared__ SepBlock<real> B;
     __shared__ DevModel<real> M;
@@ -2217,18 +2241,7 @@ __global__ void __launch_bounds__(32 * ESM_SEP_WARPS, sizeof(real) == 8 ? 2 : 4)
         __syncthreads();
         const unsigned int it = sit;
         const bool done = it >= total;
-        int b = cur;
-        if (!done) {  // the last model whose prefix is <= it
-            int lo = 0, hi = nact - 1;
-            while (lo < hi) {
-                int mid = (lo + hi + 1) >> 1;
-                if (choff[mid] <= it)
-                    lo = mid;
-                else
-                    hi = mid - 1;
-            }
-            b = lo;
-        }
+        const int b = done ? cur : prefix_at(choff, nact, it);
         if (done || b != cur) {  // block-uniform
             if (cur >= 0 && fi >= 0) block_counts(bm[cur].stats, fi, tried, moved, guards);
             tried = moved = guards = 0;
@@ -2245,16 +2258,17 @@ __global__ void __launch_bounds__(32 * ESM_SEP_WARPS, sizeof(real) == 8 ? 2 : 4)
         fi = d.hdr[12];
         const int t0 = (int)(it - choff[b]) * ESM_CHUNK;
         const int end = min(nsteps * M.R, t0 + ESM_CHUNK);
-        if (sep_move<real>(d, bm[b].sep_on)) {
+        if (sep_move(d.hdr, bm[b].sep_on)) {
             int at = t0;
             sep_run<real>(M, d, B, smem, region, ESM_CHUNK, rot, tmp, steps, nsteps, sweep, mi, end, tried, moved, guards,
                           [&](int n) {
                               int x = at;
                               at += n;
                               return x;
-                          });
+                          },
+                          [&](int task) { redo[atomicAdd(nredo, 1u)] = (unsigned long long)sit << 32 | (unsigned)task; });
         } else {
-            if (!walk_move<real>(d, bm[b].walk_region)) continue;  // (block-uniform)
+            if (!walk_move(d.hdr, bm[b].walk_region)) continue;  // (block-uniform)
             if (threadIdx.x == 0) sW = desc_walk<real>(d);
             __syncthreads();
             int at = t0 + 16 * wib;
@@ -2268,89 +2282,117 @@ __global__ void __launch_bounds__(32 * ESM_SEP_WARPS, sizeof(real) == 8 ? 2 : 4)
     }
 }
 
+// Move mi of the current pass for every task of the first nact models of the batch. A warp takes
+// items from the launch's counter; an item (32 tasks of one model's tile, as in k_move) belongs to
+// the model b with off[b] <= item < off[b + 1]. When a warp's item comes from another model than
+// its last one, the warp copies that model's tables and layout into its shared memory and points
+// its descriptor at the model's descriptor mi in global memory (read-only during the move), after
+// adding its counts so far to the previous model's statistics. Each task then runs exactly the
+// arithmetic of k_move (move_task), so a model's state after a batch pass is the state its own
+// class pass gives. The moves of k_move_blocks_batch, which is launched before it, are left out, but for the
+// tasks that that kernel lists in redo (chunk, task): a warp takes 32 of them, model by model.
 template <class real, int WPB>
 __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
     k_move_batch(const BatchModel<real> *bm, int nact, const int *pass_cls, const unsigned int *off,
-                 const uint32_t *sweep_p, int mi, real *scratch, size_t scratch_per_warp, unsigned int *next_item) {
+                 const unsigned int *choff, const uint32_t *sweep_p, int mi, real *scratch, size_t scratch_per_warp, unsigned int *next_item,
+                 const unsigned long long *redo, const unsigned int *nredo) {
     __shared__ DevModel<real> sM[WPB];
     __shared__ Desc<real> sd[WPB];
     __shared__ LaneLayout sLL[WPB];
     int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     uint32_t sweep = *sweep_p;
     unsigned int total = off[nact];
+    const unsigned int left = *nredo;
     real local[ESM_LANE_LOCAL];
     int cur = -1, fi = -1, cls = 0, nsteps = 0;
     const int *steps = nullptr;
     unsigned long long tried = 0, moved = 0, guards = 0;
+    auto leave = [&]() {  // the counts so far to the model in hand (by the whole warp)
+        for (int o = 16; o > 0; o >>= 1) {
+            tried += __shfl_xor_sync(0xffffffffu, tried, o);
+            moved += __shfl_xor_sync(0xffffffffu, moved, o);
+            guards += __shfl_xor_sync(0xffffffffu, guards, o);
+        }
+        if (lane == 0 && cur >= 0 && fi >= 0) {
+            unsigned long long *st = bm[cur].stats;
+            if (tried) atomicAdd(&st[2 * fi], tried);
+            if (moved) atomicAdd(&st[2 * fi + 1], moved);
+            if (guards) atomicAdd(&st[2 * (ESM_NFAM + 1)], guards);
+        }
+        tried = moved = guards = 0;
+    };
+    auto enter = [&](int b) {  // model b's tables and move mi, once the counts of the model before are added
+        leave();
+        const unsigned int *src = (const unsigned int *)&bm[b].M;
+        unsigned int *dst = (unsigned int *)&sM[wib];
+        for (int i = lane; i < (int)(sizeof(DevModel<real>) / 4); i += 32) dst[i] = src[i];
+        __syncwarp();
+        if (lane == 0) {
+            sd[wib] = carve_desc<real>(bm[b].descs + (size_t)mi * bm[b].stride, sM[wib], bm[b].nmoves);
+            const DevModel<real> &Mb = sM[wib];
+            sLL[wib] = lane_layout(Mb.maxpts, Mb.maxn, Mb.maxstu, linemove_maxroots(Mb), Mb.maxk, Mb.maxku);
+        }
+        __syncwarp();
+        cur = b;
+        fi = sd[wib].hdr[12];
+        cls = pass_cls[b];
+        nsteps = cls >= 0 ? bm[b].nsteps[cls] : 0;
+        steps = cls >= 0 ? bm[b].steps[cls] : nullptr;
+    };
+    auto walk = [&](int q, int rep) {  // the lane's task: the class's step q
+        const DevModel<real> &M = sM[wib];
+        const LaneLayout &LL = sLL[wib];
+        bool loc = LL.total <= ESM_LANE_LOCAL;
+        real *slab = loc ? local : scratch + ((size_t)blockIdx.x * WPB + wib) * scratch_per_warp + lane;
+        Lane<real> Ln(M, sd[wib], slab, loc ? 1 : 32, lane, LL);
+        Ln.rep = rep;
+        bool guard;
+        real t = move_task<real>(Ln, M, sd[wib], LL, fi, mi, steps[q], sweep, &guard);
+        if (guard) ++guards;
+        ++tried;
+        if (t != 0) ++moved;
+    };
+    // the items
+    int seen = -1;
+    bool none = false;  // nothing to do for model `seen`: no valid move, or one of k_move_blocks_batch
     while (true) {
         unsigned int it = 0;
         if (lane == 0) it = atomicAdd(next_item, 1u);
-        unsigned int item = __shfl_sync(0xffffffffu, it, 0);
-        bool done = item >= total;
-        int b = cur;
-        if (!done) {  // the last model whose prefix is <= item
-            int lo = 0, hi = nact - 1;
-            while (lo < hi) {
-                int mid = (lo + hi + 1) >> 1;
-                if (off[mid] <= item)
-                    lo = mid;
-                else
-                    hi = mid - 1;
-            }
-            b = lo;
+        const unsigned int item = __shfl_sync(0xffffffffu, it, 0);
+        if (item >= total) break;
+        const int b = prefix_at(off, nact, item);
+        if (b != seen) {
+            const int *h = desc_hdr(bm[b].descs + (size_t)mi * bm[b].stride, bm[b].nmoves);
+            none = h[12] < 0 || sep_move(h, bm[b].sep_on) || walk_move(h, bm[b].walk_region);
+            seen = b;
         }
-        if (done || b != cur) {  // warp-uniform
-            for (int o = 16; o > 0; o >>= 1) {
-                tried += __shfl_xor_sync(0xffffffffu, tried, o);
-                moved += __shfl_xor_sync(0xffffffffu, moved, o);
-                guards += __shfl_xor_sync(0xffffffffu, guards, o);
-            }
-            if (lane == 0 && cur >= 0 && fi >= 0) {
-                unsigned long long *st = bm[cur].stats;
-                if (tried) atomicAdd(&st[2 * fi], tried);
-                if (moved) atomicAdd(&st[2 * fi + 1], moved);
-                if (guards) atomicAdd(&st[2 * (ESM_NFAM + 1)], guards);
-            }
-            tried = moved = guards = 0;
-            if (done) break;
-            const unsigned int *src = (const unsigned int *)&bm[b].M;
-            unsigned int *dst = (unsigned int *)&sM[wib];
-            for (int i = lane; i < (int)(sizeof(DevModel<real>) / 4); i += 32) dst[i] = src[i];
-            __syncwarp();
-            if (lane == 0) {
-                sd[wib] = carve_desc<real>(bm[b].descs + (size_t)mi * bm[b].stride, sM[wib], bm[b].nmoves);
-                const DevModel<real> &Mb = sM[wib];
-                sLL[wib] = lane_layout(Mb.maxpts, Mb.maxn, Mb.maxstu, linemove_maxroots(Mb), Mb.maxk, Mb.maxku);
-            }
-            __syncwarp();
-            cur = b;
-            fi = sd[wib].hdr[12];
-            // (k_move_blocks_batch's moves: nothing to do)
-            if (sep_move<real>(sd[wib], bm[b].sep_on) || walk_move<real>(sd[wib], bm[b].walk_region)) fi = -1;
-            cls = pass_cls[b];
-            nsteps = cls >= 0 ? bm[b].nsteps[cls] : 0;
-            steps = cls >= 0 ? bm[b].steps[cls] : nullptr;
-        }
-        if (fi < 0) continue;  // the model's move mi is not a valid move: its tasks do nothing
+        if (none) continue;
+        if (b != cur) enter(b);
         const DevModel<real> &M = sM[wib];
-        const LaneLayout &LL = sLL[wib];
         unsigned int li = item - off[b];
         int wpt = (M.span * M.R + 31) / 32;
         int tile = (int)(li / wpt), grp = (int)(li % wpt);
         int task = grp * 32 + lane;
         int sit = task / M.R;
         int q = tile * M.span + sit;
-        if (!(sit < M.span && q < nsteps)) continue;
-        bool loc = LL.total <= ESM_LANE_LOCAL;
-        real *slab = loc ? local : scratch + ((size_t)blockIdx.x * WPB + wib) * scratch_per_warp + lane;
-        Lane<real> Ln(M, sd[wib], slab, loc ? 1 : 32, lane, LL);
-        Ln.rep = task % M.R;
-        bool guard;
-        real t = move_task<real>(Ln, M, sd[wib], LL, fi, mi, steps[q], sweep, &guard);
-        if (guard) ++guards;
-        ++tried;
-        if (t != 0) ++moved;
+        if (sit < M.span && q < nsteps) walk(q, task % M.R);
+        __syncwarp();
     }
+    // the tasks of redo
+    for (unsigned int base = (blockIdx.x * WPB + wib) * 32; base < left; base += gridDim.x * WPB * 32) {
+        const unsigned long long mine = base + lane < left ? redo[base + lane] : 0;
+        const int model = prefix_at(choff, nact, (unsigned)(mine >> 32)), task = (int)(unsigned)mine;
+        unsigned int todo = __ballot_sync(0xffffffffu, base + lane < left);
+        while (todo) {
+            const int b = __shfl_sync(0xffffffffu, model, __ffs(todo) - 1);
+            const bool act = ((todo >> lane) & 1) && model == b;
+            todo &= ~__ballot_sync(0xffffffffu, act);
+            if (b != cur) enter(b);
+            if (act) walk(task / sM[wib].R, task % sM[wib].R);
+            __syncwarp();
+        }
+    }
+    leave();
 }
 
 // resident blocks of k_move_blocks_batch per SM with `region` bytes of shared memory
@@ -2379,7 +2421,7 @@ int batch_warps_per_sm(int wpb) {
 template <class real>
 cudaError_t launch_batch_passes(const BatchModel<real> *bm, const BatchLaunch &bl, const uint32_t *sweep,
                                 cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(bl.counters, 0, sizeof(unsigned int) * 2 * bl.maxpass * bl.maxmoves, s);
+    cudaError_t e = cudaMemsetAsync(bl.counters, 0, sizeof(unsigned int) * 3 * bl.maxpass * bl.maxmoves, s);
     if (e != cudaSuccess) return e;
     int blocks = (bl.warps + bl.wpb - 1) / bl.wpb;
     for (int p = 0; p < bl.npass; ++p) {
@@ -2392,19 +2434,20 @@ cudaError_t launch_batch_passes(const BatchModel<real> *bm, const BatchLaunch &b
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         for (int mi = 0; mi < bl.nmove; ++mi) {
             unsigned int *ctr = bl.counters + (size_t)p * bl.maxmoves + mi;
-            if (bl.wpb == 2)
-                k_move_batch<real, 2><<<blocks, 64, 0, s>>>(bm, bl.nact[mi], pc, off, sweep, mi, (real *)bl.scratch,
-                                                           bl.scratch_per_warp, ctr);
-            else
-                k_move_batch<real, 1><<<blocks, 32, 0, s>>>(bm, bl.nact[mi], pc, off, sweep, mi, (real *)bl.scratch,
-                                                           bl.scratch_per_warp, ctr);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            unsigned int *nredo = ctr + 2 * (size_t)bl.maxpass * bl.maxmoves;
             if (bl.bblocks > 0) {
                 k_move_blocks_batch<real><<<bl.bblocks, 32 * ESM_SEP_WARPS, bl.region, s>>>(
                     bm, bl.nact[mi], pc, choff, sweep, mi, bl.region, bl.tmp, bl.tmp_warp, (real *)bl.scratch,
-                    bl.scratch_per_warp, ctr + (size_t)bl.maxpass * bl.maxmoves);
+                    bl.scratch_per_warp, ctr + (size_t)bl.maxpass * bl.maxmoves, bl.redo, nredo);
                 if ((e = cudaGetLastError()) != cudaSuccess) return e;
             }
+            if (bl.wpb == 2)
+                k_move_batch<real, 2><<<blocks, 64, 0, s>>>(bm, bl.nact[mi], pc, off, choff, sweep, mi, (real *)bl.scratch,
+                                                           bl.scratch_per_warp, ctr, bl.redo, nredo);
+            else
+                k_move_batch<real, 1><<<blocks, 32, 0, s>>>(bm, bl.nact[mi], pc, off, choff, sweep, mi, (real *)bl.scratch,
+                                                           bl.scratch_per_warp, ctr, bl.redo, nredo);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
     }
     return cudaSuccess;

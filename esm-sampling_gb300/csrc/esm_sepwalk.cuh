@@ -105,6 +105,14 @@ __device__ __noinline__ real sep_pick(real p0, real p1, real g, real L, real uof
                                           : p1 - Lane<real>::trexp_offset(uoff, -g, L, flat);
 }
 
+// Whether the potential change x of a segment lies where the order of a group's events decides on which side of
+// the segment's round-off scale it is: the scale of the group's last point lies between that of its potential
+// alone (c) and that with the slopes behind the group (zo more), `rest` the other terms.
+static __device__ __noinline__ bool sep_unsure(float x, float flat, float c, float zo, float rest) {
+    float lo = 4.8e-7f * c + rest;
+    return x < 1.0001f * fmaxf(flat, lo + zo) && x >= 0.9999f * fmaxf(flat, lo);
+}
+
 // How a list is laid out: the entries of a batch's list, those of a small move's, and those of a task
 // that runs alone, with room for the events beyond the last clamp (two a unit) and for every ray point.
 enum { SEP_BATCH = 0, SEP_SMALL = 1, SEP_SOLE = 2 };
@@ -199,7 +207,12 @@ __device__ __forceinline__ double sep_get(const SepPair<real> &p) {
         return p.x;
 }
 
-enum { SEP_OPEN = 2, SEP_PROPER = 1, SEP_IMPROPER = 0, SEP_GUARD = -1, SEP_ALONE = -2 };
+// SEP_REDO: left to the one-lane walk. In FP32 a list's events of one time stand in an order of the list's
+// own, which depends on the lists beside it; the one-lane walk's comes from its heap. Neither the points'
+// times and potentials nor the stop tests depend on it, but two things do: which of the group's events come
+// before a point cap that cuts it, and the round-off scale of the group's last point. A walk that they
+// decide is walked again by k_move.
+enum { SEP_OPEN = 2, SEP_PROPER = 1, SEP_IMPROPER = 0, SEP_GUARD = -1, SEP_ALONE = -2, SEP_REDO = -3 };
 
 // One storage term of a unit (its step tau or its step tau - 1) at the start: d0, its piece, the
 // linear coefficients there and its parts.
@@ -569,7 +582,7 @@ struct SepWalk {
     // The first n <= 32 E entries of a list in order, by the warp, E consecutive entries a lane in
     // registers: a bitonic network whose comparisons all point upward (each merge starts with mirrored
     // pairs); strides below E stay in the lane.
-    // (FP32 entries of one time keep the order that the network gives them, the same in every run.)
+    // (FP32 entries of one time keep the order that the network gives them: SEP_REDO.)
     __device__ __forceinline__ static bool after(real ka, unsigned pa, real kb, unsigned pb) {
         if constexpr (sizeof(real) == 8) return ka > kb || (ka == kb && pa > pb);
         return ka > kb;
@@ -779,6 +792,8 @@ struct SepWalk {
             }
         }
         if (st == SEP_OPEN && i < n) st = SEP_GUARD;  // more points than the cap
+        // the cap cuts the group of events that the walk ends in
+        if (sizeof(real) == 4 && n > M.maxpts && st != SEP_OPEN && kc == fabs(A.key[M.maxpts])) st = SEP_REDO;
         B.np[l] = i;
         B.ab[l] = abf;
         B.st[l] = st;
@@ -880,6 +895,9 @@ struct SepWalk {
                 if (c - cmin > maxnats) st = SEP_PROPER;
             }
         }
+        // (as in scan; no event ends a walk in the ray phase)
+        if (sizeof(real) == 4 && n > maxpts && ray == 0x7fffffff && (st == SEP_PROPER || st == SEP_GUARD))
+            if (A.key[np - 1] == A.key[maxpts]) st = SEP_REDO;
         B.np[l] = np;
         B.ray[l] = ray;
         B.st[l] = st;
@@ -933,8 +951,9 @@ struct SepWalk {
     }
 
     // the draw over the segments of task k; the sums in segment order: the left walk's from its last
-    // point inward, then the right walk's. *again: the round-off scales decide, which a batch has not.
-    __device__ __forceinline__ real draw(int k, real ucat, real uoff, bool *again) const {
+    // point inward, then the right walk's. *st: SEP_ALONE where the round-off scales decide, which a batch
+    // has not, SEP_REDO where the order of events of one time does.
+    __device__ __forceinline__ real draw(int k, real ucat, real uoff, int *st) const {
         const Points R = points(2 * k), Lf = points(2 * k + 1);
         const int nr = B.np[2 * k], nl = B.np[2 * k + 1];
         // masses j of a list, in its order: eight loads, then the sums one after the other
@@ -1001,8 +1020,18 @@ struct SepWalk {
             real gl = slope(m0 - 1), gm = slope(m0), gr = slope(m0 + 1);
             if (full) {
                 auto Z = [&](int m) -> real { return m < 0 ? Lf.z(-m - 1) : R.z(m - 1); };
-                real z0 = Z(m0) + real(2.4e-7) * fabs(p0) * fmax(gl, gm);
-                real z1 = Z(m0 + 1) + real(2.4e-7) * fabs(p1) * fmax(gm, gr);
+                real x0 = real(2.4e-7) * fabs(p0) * fmax(gl, gm), x1 = real(2.4e-7) * fabs(p1) * fmax(gm, gr);
+                real z0 = Z(m0) + x0;
+                real z1 = Z(m0 + 1) + x1;
+                // the segment's inner end, where it is one of a group
+                const bool left = m0 < 0;
+                if (left ? m0 <= -3 && p1 == P(m0 + 2) : m0 >= 2 && p0 == P(m0 - 1)) {
+                    real zi = left ? fabs(c1) : fabs(c0), zo = left ? Z(m0) * fabs(p1 / p0) : Z(m0 + 1) * fabs(p0 / p1);
+                    if (sep_unsure(fabs(g * L), flat, zi, zo, left ? z0 + x1 : z1 + x0)) {
+                        *st = SEP_REDO;
+                        return 0;
+                    }
+                }
                 flat = fmax(flat, z0 + z1);
             } else {
                 // an upper bound of the two scales: where it leaves no doubt they are not needed
@@ -1010,7 +1039,7 @@ struct SepWalk {
                 real most = real(4.9e-7) * (fabs(c0) + a0 * fabs(p0) + fabs(c1) + a1 * fabs(p1)) +
                             real(2.5e-7) * (fabs(p0) * fmax(gl, gm) + fabs(p1) * fmax(gm, gr));
                 if (!(fabs(g * L) > most && fabs(g * L) > flat)) {
-                    *again = true;
+                    *st = SEP_ALONE;
                     return 0;
                 }
             }
@@ -1034,27 +1063,25 @@ struct SepWalk {
     }
 };
 
-// The units of a separable move by its header (0: not separable); whether descriptor d is such a move with at
-// least sepmin units (the moves of sep_run).
+// The units of a separable move by its header (0: not separable); whether a descriptor's header is of such a
+// move with at least sepmin units (the moves of sep_run).
 __device__ inline int sep_units(const int *h) {
     bool sep = h[0] == 0 && h[2] == 0 && h[3] == 0 && h[4] == 0 && h[6] == 0 && h[8] == 0 && h[5] == h[1] && h[7] == h[1];
     return sep ? h[1] : 0;
 }
-template <class real>
-__device__ inline bool sep_move(const Desc<real> &d, int sepmin) {
-    return sepmin > 0 && d.hdr[15] >= sepmin;
-}
+__device__ inline bool sep_move(const int *hdr, int sepmin) { return sepmin > 0 && hdr[15] >= sepmin; }
 
 // The walks of separable move mi of one model over a block's tasks, in batches of as many as its shared
 // memory (region bytes at smem) holds lists for, but no more than `share`; next(n), called by thread 0,
 // gives the first task of a batch of n (none from `end` on). A task whose walk passes every clamp, or
-// whose draw needs the round-off scales of its points, runs again, alone, with room for both. rot: the
-// warp that the scans start at; tmp: the warp's buffer for long sorts.
-template <class real, class Next>
+// whose draw needs the round-off scales of its points, runs again, alone, with room for both; redo(task)
+// takes those left to the one-lane walk. rot: the warp that the scans start at; tmp: the warp's buffer for
+// long sorts.
+template <class real, class Next, class Redo>
 __device__ __forceinline__ void sep_run(const DevModel<real> &M, const Desc<real> &d, SepBlock<real> &B, char *smem,
                                         int region, int share, int rot, char *tmp, const int *steps, int nsteps,
                                         uint32_t sweep, int mi, int end, unsigned int &tried, unsigned int &moved,
-                                        unsigned int &guards, Next next) {
+                                        unsigned int &guards, Next next, Redo redo) {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int nu = d.hdr[1], T = M.T;
     SepUnits<real> U(smem, nu);
@@ -1180,14 +1207,15 @@ __device__ __forceinline__ void sep_run(const DevModel<real> &M, const Desc<real
                 int a = B.st[2 * k], b = B.st[2 * k + 1];
                 // the right walk's outcome counts first, as in the one-lane walk
                 int w = a != SEP_PROPER ? a : b;
-                bool again = w == SEP_ALONE;
                 if (w == SEP_PROPER) {
                     double uc, uo;
                     uniform2(M.seed, ESM_TAG_LANE, 2 * (uint32_t)mi, (uint32_t)ts, (uint32_t)r, sweep, &uc, &uo);
-                    t = S.draw(k, unit_uniform<real>(uc), unit_uniform<real>(uo), &again);
+                    t = S.draw(k, unit_uniform<real>(uc), unit_uniform<real>(uo), &w);
                 }
-                if (again) {
+                if (w == SEP_ALONE) {
                     B.alone[atomicAdd(&B.nalone, 1)] = tk;
+                } else if (sizeof(real) == 4 && w == SEP_REDO) {
+                    redo(tk);
                 } else {
                     ++tried;
                     if (w == SEP_GUARD) ++guards;

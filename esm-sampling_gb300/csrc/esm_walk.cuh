@@ -467,11 +467,8 @@ __device__ inline int walk_bytes(const int *h) {
     const WalkLayout w = walk_layout<real>(h[0], h[6], h[2], h[1], h[5], h[7]);
     return walk_const_bytes<real>(w) + walk_warp_bytes<real>(w);
 }
-// whether descriptor d is walked so in a block with `region` bytes
-template <class real>
-__device__ inline bool walk_move(const Desc<real> &d, int region) {
-    return d.hdr[13] <= region;
-}
+// whether the move of a descriptor's header is walked so in a block with `region` bytes
+__device__ inline bool walk_move(const int *hdr, int region) { return hdr[13] <= region; }
 template <class real>
 __device__ inline WalkLayout desc_walk(const Desc<real> &d) {
     const int *h = d.hdr;

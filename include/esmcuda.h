@@ -289,9 +289,9 @@ int esm_move_log(esm_ctx *ctx, int32_t cls, double *out);
    in shared memory, and the sums over them are taken in order. Smaller ones, and those that do not fit
    a block's shared memory, keep one task per lane (k_move). min_units 1 (the default): every separable
    move; 0: none.
-   The same draws and points as the one-lane walk, to the last bit, with one exception: in FP32 the two
-   walks may take events of one time in different orders, so where the point cap falls inside such a
-   group one of them may reach its end and the other the cap (a guard event). In FP64 the order is fixed.
+   The same draws and points as the one-lane walk, to the last bit: breakpoints at one t come in unit order
+   in FP64, and in FP32 the few walks whose end or draw depends on their order (the point cap cuts the
+   group, or the round-off scale of its last point decides a draw) are left to the one-lane walk.
    esm_set_sep_walk drops the captured class graphs; esm_sep_walk reads the setting and the kernel's
    warps. No reference counterpart. */
 #define ESM_SEP_MIN_DEFAULT 1

@@ -1,6 +1,7 @@
-"""Which walk a line move takes (esm_set_sep_walk, esm_set_move_schedule, a batch), seen where the walks
-differ: in FP32 the walks of one move take events of one time in their own orders, so a point cap inside
-such a group ends them differently; everywhere else every route gives the same bits."""
+"""Which walk a line move takes (esm_set_sep_walk, esm_set_move_schedule, a batch): every route gives the
+same states and counts, bit for bit, also where a point cap cuts a group of breakpoints at one t. (Before the
+block walk left such walks to the one-lane walk, the two ended them differently in FP32, and these tests
+showed by it which walk had run.)"""
 import numpy as np
 import pytest
 
@@ -43,7 +44,7 @@ def _same(x, y):
 
 
 def _ties():
-    """A model and state on which the block walk and the one-lane walk end differently in FP32."""
+    """A model and state whose walks the cap cuts inside groups of events of one time."""
     m = make_model(40, 60, 24, seed=3)
     return m, 8, _state(m, 8, 7, True), {"max_points": 8}
 
@@ -52,15 +53,15 @@ def test_sep_walk_zero_is_off():
     """0 keeps the one-lane walk (the walk of the whole-class launch); the default is 1."""
     m, R, st, kw = _ties()
     one_lane = _run(m, R, st, schedule="class", **kw)
-    assert _same(_run(m, R, st, sep=0, **kw), one_lane)
-    block = _run(m, R, st, sep=1, **kw)
-    assert not _same(block, one_lane)                   # (else the model shows nothing)
-    assert _same(_run(m, R, st, **kw), block)
+    for sep in (0, 1, None):
+        assert _same(_run(m, R, st, sep=sep, **kw), one_lane), sep
     # a setting above 0 that was asked for keeps the launches per move, the default does not
-    assert _same(_run(m, R, st, sep=1, schedule="class", **kw), block)
-    assert _same(_run(m, R, st, sep=0, schedule="class", **kw), one_lane)
+    for sep in (0, 1):
+        assert _same(_run(m, R, st, sep=sep, schedule="class", **kw), one_lane), sep
     d = DeviceChain(m, R, seed=9)
     assert d.sep_walk()[0] == 1
+    d.set_sep_walk(0)
+    assert d.sep_walk()[0] == 0
     d.close()
 
 
@@ -72,7 +73,7 @@ def test_batch_takes_the_chains_walk():
     st2 = _state(m2, 4, 8, False)
     a, b = _chain(m, R, st, **kw), _chain(m2, 4, st2)
     batch = DeviceBatch([a, b])
-    for sep in (0, 41):                                 # (no move has 41 units)
+    for sep in (0, 41, 1, 13):                          # (no move has 41 units)
         a.set_sep_walk(sep)
         a.upload(st)
         b.upload(st2)
@@ -122,3 +123,26 @@ def test_equal_roots_beyond_the_buffer(precision, cap):
     assert out[1][0][:-1:2].sum() == m.T * 4
     assert out[1][0][-1] == (m.T * 4 if 0 < cap < 13 else 0)
     assert _same(*out)
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("cap", [8, 20, 45, 0])
+@pytest.mark.parametrize("N,T,R", [(40, 24, 8), (12, 73, 3)])
+def test_equal_times_at_the_cap(N, T, R, cap, precision):
+    """States of charge at quarters, and all at one half: many events of one time, which the cap cuts."""
+    m = make_model(N, (3 * N) // 2, T, seed=3)
+    for seed, steps in ((7, 4.0), (11, 4.0), (13, 2.0)):
+        st = _state(m, R, seed, True)
+        if steps == 2.0:
+            st.e[:] = 0.5
+        one_lane = _run(m, R, st, precision, schedule="class", max_points=cap)
+        assert _same(_run(m, R, st, precision, max_points=cap), one_lane), seed
+        other = make_model(20, 30, 24, seed=5)          # (another split of the block's lists)
+        a = _chain(m, R, st, precision, max_points=cap)
+        b = _chain(other, 16, _state(other, 16, 8, False), precision)
+        batch = DeviceBatch([a, b])
+        counts = batch.sweeps(1, sweep0=0)
+        assert _same((counts[0], a.download()), one_lane), seed
+        batch.close()
+        a.close()
+        b.close()
