@@ -38,9 +38,9 @@ struct Carve {
 
 template <class real>
 struct Desc {
-    int *moves;
-    int *hdr;  // [0] ng, [1] nse, [2] nl, [3] nk, [4] nku, [5] nns, [6] nga, [7] nna, [8] nth, [9] valid, [10] fam,
-               // [11] nku0 (the kinked units of step tau; those of step tau - 1 follow)
+    int *hdr;  // (first) [0] ng, [1] nse, [2] nl, [3] nk, [4] nku, [5] nns, [6] nga, [7] nna, [8] nth, [9] valid,
+               // [10] fam, [11] nku0 (the kinked units of step tau; those of step tau - 1 follow), [12] to [15]
+               // which kernel walks the move (prep_desc)
     int *gi, *gpos;
     real *ga;
     int *si, *spos, *sposa;
@@ -64,10 +64,9 @@ struct Desc {
 };
 
 template <class real>
-__host__ __device__ inline Desc<real> carve_desc(char *base, const DevModel<real> &M, int nmoves) {
+__host__ __device__ inline Desc<real> carve_desc(char *base, const DevModel<real> &M) {
     Carve c(base);
     Desc<real> d;
-    d.moves = c.take<int>(nmoves);
     d.hdr = c.take<int>(16);
     d.gi = c.take<int>(M.maxe);
     d.gpos = c.take<int>(M.maxe);
@@ -105,11 +104,10 @@ __host__ __device__ inline Desc<real> carve_desc(char *base, const DevModel<real
 }
 
 template <class real>
-size_t desc_bytes(const DevModel<real> &M, int nmoves) {
+size_t desc_bytes(const DevModel<real> &M) {
     // size by carving from an aligned base
     char *base = (char *)(uintptr_t)4096;
     Carve c(base);
-    c.take<int>(nmoves);
     c.take<int>(16);
     c.take<int>(M.maxe);
     c.take<int>(M.maxe);
@@ -1625,13 +1623,6 @@ namespace esm {
 // Its header says which kernel walks the move, so that the other's launch is over after one read: word 12 the
 // family index (-1: no move), word 13 walk_bytes, word 15 sep_units. Bound by the latency of the one warp's selections.
 // 40 nodes (319 moves): 2.2 ms with one warp for the descriptors too, 0.30 so; 128 nodes (1023): 0.96.
-// the header words of a descriptor
-__device__ inline int *desc_hdr(char *desc, int nmoves) {
-    Carve c(desc);
-    c.take<int>(nmoves);
-    return c.take<int>(16);
-}
-
 template <class real>
 __device__ __forceinline__ void list_class(const DevModel<real> &M, int *moves, uint32_t sweep, int cls, int nrun,
                                            char *descs, size_t stride, int lane) {
@@ -1640,7 +1631,7 @@ __device__ __forceinline__ void list_class(const DevModel<real> &M, int *moves, 
     for (int mi = 0; mi < nrun; ++mi) {
         const int mv = moves[mi];
         if (lane == 0) {
-            int *h = desc_hdr(descs + (size_t)mi * stride, M.natoms + M.nextra);
+            int *h = (int *)(descs + (size_t)mi * stride);
             h[13] = (int)st.j;
             h[14] = mv;
         }
@@ -1652,7 +1643,7 @@ __device__ __forceinline__ void list_class(const DevModel<real> &M, int *moves, 
 template <class real>
 __device__ __forceinline__ void prep_desc(const DevModel<real> &M, char *smem, Desc<real> &sd, uint32_t sweep, int cls,
                                           char *out, size_t stride, int lane) {
-    if (lane == 0) sd = carve_desc<real>(smem, M, M.natoms + M.nextra);
+    if (lane == 0) sd = carve_desc<real>(smem, M);
     __syncwarp();
     Desc<real> &d = sd;
     for (int i = lane; i < M.N; i += 32) {
@@ -1662,7 +1653,7 @@ __device__ __forceinline__ void prep_desc(const DevModel<real> &M, char *smem, D
     }
     for (int i = lane; i < M.L; i += 32) d.lmark[i] = 0;
     __syncwarp();
-    const int *h = desc_hdr(out, M.natoms + M.nextra);
+    const int *h = (const int *)out;
     Stream st(M.seed, (uint32_t)cls, sweep, (uint32_t)h[13]);
     int fi = prep_move(M, d, st, h[14], lane);
     if (lane == 0) {
@@ -1671,10 +1662,9 @@ __device__ __forceinline__ void prep_desc(const DevModel<real> &M, char *smem, D
         d.hdr[15] = fi < 0 ? 0 : sep_units(d.hdr);
     }
     __syncwarp();
-    const size_t from = (size_t)((char *)d.hdr - smem) / 16 * 16;  // (the list in front is of no use to a move)
-    const int4 *src = (const int4 *)(smem + from);
-    int4 *dst = (int4 *)(out + from);
-    for (size_t i = lane; i < (stride - from) / 16; i += 32) dst[i] = src[i];
+    const int4 *src = (const int4 *)smem;
+    int4 *dst = (int4 *)out;
+    for (size_t i = lane; i < stride / 16; i += 32) dst[i] = src[i];
 }
 
 template <class real>
@@ -1754,7 +1744,7 @@ __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
     // of a move that k_move_blocks walked, the tasks it left (redo; read with the header, not after it)
     int left = sizeof(real) == 4 ? (int)*nredo : 0;
     {  // not a valid move, or one of k_move_blocks that left none: nothing to do (grid-uniform)
-        const int *g = desc_hdr((char *)(descs + (size_t)mi * stride), M.natoms + M.nextra);
+        const int *g = (const int *)(descs + (size_t)mi * stride);
         const bool none = g[12] < 0, sep = sep_move(g, sepmin), walk = walk_move(g, walk_region);
         if (none || walk || (sep && left == 0)) return;
         if (left == 0) left = -1;
@@ -1765,7 +1755,7 @@ __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
         for (size_t i = threadIdx.x; i < stride / 16; i += 32 * WPB) dst[i] = src[i];
     }
     if (threadIdx.x == 0) {
-        sd = carve_desc<real>(smem, M, M.natoms + M.nextra);
+        sd = carve_desc<real>(smem, M);
         sLL = lane_layout(M.maxpts, M.maxn, M.maxstu, linemove_maxroots(M), M.maxk, M.maxku);
     }
     if (WPB == 1)
@@ -1872,7 +1862,7 @@ __global__ void __launch_bounds__(32 * ESM_SEP_WARPS, sizeof(real) == 8 ? 2 : 4)
     extern __shared__ __align__(16) char smem[];
     __shared__ SepBlock<real> B;
     __shared__ WalkLayout sW;
-    const Desc<real> d = carve_desc<real>((char *)(descs + (size_t)mi * stride), M, M.natoms + M.nextra);
+    const Desc<real> d = carve_desc<real>((char *)(descs + (size_t)mi * stride), M);
     const int ntask = nsteps * M.R, wib = threadIdx.x >> 5;
     unsigned int tried = 0, moved = 0, guards = 0;
     if (sep_move(d.hdr, sepmin)) {
@@ -1943,7 +1933,6 @@ __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
     uint32_t sweep = *sweep_p;
     const unsigned int nitems = (unsigned int)(ntile * wpt);
     const unsigned int total = nitems * (unsigned int)nrun;  // (the host keeps it below 2^32)
-    const int nmoves = M.natoms + M.nextra;
     int cur = -1, fi = -1;
     unsigned long long tried = 0, moved = 0, guards = 0;
     while (true) {
@@ -1965,7 +1954,7 @@ __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
             }
             tried = moved = guards = 0;
             if (stop) break;
-            if (lane == 0) sd[wib] = carve_desc<real>((char *)descs + (size_t)mi * stride, M, nmoves);
+            if (lane == 0) sd[wib] = carve_desc<real>((char *)descs + (size_t)mi * stride, M);
             __syncwarp();
             cur = mi;
             fi = sd[wib].hdr[12];
@@ -2029,7 +2018,7 @@ size_t linemove_scratch_reals(const DevModel<real> &M) {
 // bytes of one move descriptor (the per-move buffer stride and the dynamic shared memory of k_move)
 template <class real>
 size_t linemove_smem_per_warp(const DevModel<real> &M) {
-    return (desc_bytes(M, M.natoms + M.nextra) + 15) & ~(size_t)15;
+    return (desc_bytes(M) + 15) & ~(size_t)15;
 }
 
 // warps of k_move resident per SM with blocks of wpb warps (1, 2 or 4), for the grid and scratch
@@ -2254,7 +2243,7 @@ __global__ void __launch_bounds__(32 * ESM_SEP_WARPS, sizeof(real) == 8 ? 2 : 4)
             steps = cls >= 0 ? bm[b].steps[cls] : nullptr;
             __syncthreads();
         }
-        const Desc<real> d = carve_desc<real>(bm[b].descs + (size_t)mi * bm[b].stride, M, bm[b].nmoves);
+        const Desc<real> d = carve_desc<real>(bm[b].descs + (size_t)mi * bm[b].stride, M);
         fi = d.hdr[12];
         const int t0 = (int)(it - choff[b]) * ESM_CHUNK;
         const int end = min(nsteps * M.R, t0 + ESM_CHUNK);
@@ -2328,7 +2317,7 @@ __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
         for (int i = lane; i < (int)(sizeof(DevModel<real>) / 4); i += 32) dst[i] = src[i];
         __syncwarp();
         if (lane == 0) {
-            sd[wib] = carve_desc<real>(bm[b].descs + (size_t)mi * bm[b].stride, sM[wib], bm[b].nmoves);
+            sd[wib] = carve_desc<real>(bm[b].descs + (size_t)mi * bm[b].stride, sM[wib]);
             const DevModel<real> &Mb = sM[wib];
             sLL[wib] = lane_layout(Mb.maxpts, Mb.maxn, Mb.maxstu, linemove_maxroots(Mb), Mb.maxk, Mb.maxku);
         }
@@ -2362,7 +2351,7 @@ __global__ void __launch_bounds__(32 * WPB, MoveBounds<WPB>::min_blocks)
         if (item >= total) break;
         const int b = prefix_at(off, nact, item);
         if (b != seen) {
-            const int *h = desc_hdr(bm[b].descs + (size_t)mi * bm[b].stride, bm[b].nmoves);
+            const int *h = (const int *)(bm[b].descs + (size_t)mi * bm[b].stride);
             none = h[12] < 0 || sep_move(h, bm[b].sep_on) || walk_move(h, bm[b].walk_region);
             seen = b;
         }
