@@ -25,8 +25,9 @@
 // in different units and pieces, and its unit and heap state, several KB a lane, goes through L2.
 // Here the events, which are nearly all of the arithmetic, are made by lanes in step, with the
 // unit in registers, and the lists stay in shared memory. What bounds it now: the latency of the
-// events' dependent arithmetic and of the scan, at 16 warps per SM (four blocks by registers and by
-// shared memory). Measured for one move at T = 2920, 64 replicas (93440 tasks), FP32, one-lane walk
+// events' dependent arithmetic and of the scan, at 16 warps per SM in FP32 (four blocks by registers and
+// by shared memory) and 8 in FP64 (two, by registers); the warps of a batch of few long lists wait for its
+// scan. Measured for one move at T = 2920, 64 replicas (93440 tasks), FP32, one-lane walk
 // and block walk: 40 units 16.4 and 3.2 ms, 20 units 5.7 and 1.8 ms, 10 units 2.1 and 1.2 ms, 7 units
 // 1.4 and 0.7 ms.
 #pragma once
@@ -103,14 +104,6 @@ template <class real>
 __device__ __noinline__ real sep_pick(real p0, real p1, real g, real L, real uoff, real flat) {
     return (g >= 0 || fabs(g * L) < flat) ? p0 + Lane<real>::trexp_offset(uoff, g, L, flat)
                                           : p1 - Lane<real>::trexp_offset(uoff, -g, L, flat);
-}
-
-// Whether the potential change x of a segment lies where the order of a group's events decides on which side of
-// the segment's round-off scale it is: the scale of the group's last point lies between that of its potential
-// alone (c) and that with the slopes behind the group (zo more), `rest` the other terms.
-static __device__ __noinline__ bool sep_unsure(float x, float flat, float c, float zo, float rest) {
-    float lo = 4.8e-7f * c + rest;
-    return x < 1.0001f * fmaxf(flat, lo + zo) && x >= 0.9999f * fmaxf(flat, lo);
 }
 
 // How a list is laid out: the entries of a batch's list, those of a small move's, and those of a task
@@ -1020,18 +1013,17 @@ struct SepWalk {
             real gl = slope(m0 - 1), gm = slope(m0), gr = slope(m0 + 1);
             if (full) {
                 auto Z = [&](int m) -> real { return m < 0 ? Lf.z(-m - 1) : R.z(m - 1); };
-                real x0 = real(2.4e-7) * fabs(p0) * fmax(gl, gm), x1 = real(2.4e-7) * fabs(p1) * fmax(gm, gr);
-                real z0 = Z(m0) + x0;
-                real z1 = Z(m0 + 1) + x1;
-                // the segment's inner end, where it is one of a group
-                const bool left = m0 < 0;
-                if (left ? m0 <= -3 && p1 == P(m0 + 2) : m0 >= 2 && p0 == P(m0 - 1)) {
-                    real zi = left ? fabs(c1) : fabs(c0), zo = left ? Z(m0) * fabs(p1 / p0) : Z(m0 + 1) * fabs(p0 / p1);
-                    if (sep_unsure(fabs(g * L), flat, zi, zo, left ? z0 + x1 : z1 + x0)) {
+                real z0 = Z(m0) + real(2.4e-7) * fabs(p0) * fmax(gl, gm);
+                real z1 = Z(m0 + 1) + real(2.4e-7) * fabs(p1) * fmax(gm, gr);
+                // Where the segment's inner end is one of a group, its scale depends on the group's order, by no
+                // more than the outer end's (whose slopes are those behind the group): below twice the sum of
+                // both, the order decides. Below `flat` alone the draw is uniform in any order.
+                const real x = fabs(g * L);
+                if (x < real(2.001) * (z0 + z1) && x >= real(0.9999) * flat)
+                    if (m0 < 0 ? m0 <= -3 && p1 == P(m0 + 2) : m0 >= 2 && p0 == P(m0 - 1)) {
                         *st = SEP_REDO;
                         return 0;
                     }
-                }
                 flat = fmax(flat, z0 + z1);
             } else {
                 // an upper bound of the two scales: where it leaves no doubt they are not needed
