@@ -882,8 +882,8 @@ def main():
                          "frac": achieved / peak, "traffic": traffic, "peak_kind": kind,
                          "kernel": "k_prep_moves + k_move + k_move_blocks (the line moves of one colour class, one span)",
                          "note": ("the exact line sampler is latency-bound (dependent chains of the walks): "
-                                  "the HBM bytes are the compulsory state; `traffic` is the DRAM traffic of the "
-                                  "one-lane walks (profiles/linemove_traffic.json), mostly walk scratch")},
+                                  "the HBM bytes are the compulsory state; `traffic` is the DRAM traffic of one "
+                                  "class, scaled from sampled launches (profiles/linemove_traffic.json)")},
             "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},
             "gpu_launches": int(launches), "clocks": clocks,
             "move_grid": {"warps_per_block": grid[0], "warps_per_sm": grid[1], "schedule": d.move_schedule(),

@@ -23,7 +23,7 @@ __device__ inline real avail_map(real x) {  // logistic availability map (builde
 // LocalCost rebuild (src/local.jl:313, rebuild_step! :332): residual per node, flows per line.
 // Accumulation order per node as the reference: load, lines, generators, storage.
 // ---------------------------------------------------------------------------------------------
-#define ESM_REBUILD_BLOCKS 1216  // 8 blocks of 256 threads on each of 152 SMs
+#define ESM_REBUILD_BLOCKS 1216  // 8 blocks of 256 threads on each of the chip's 152 SMs
 // A thread takes Q (step, replica) pairs of a node, 256 apart: the node's tables are read once for all of
 // them, and their states' loads are under way together. Q is 4 where that still fills the device, else 1
 // (40 nodes, T = 2920, 64 replicas: 216 us with 1, 178 with 4).
@@ -967,10 +967,13 @@ cudaError_t launch_rebuild(const DevModel<real> &M, cudaStream_t s) {
 }
 
 
-// step chunks of the score pass: 64 steps a chunk, fewer chunks where the partials (values and
-// bounds) and the sums would not fit 2^20 doubles (the static scratch), so that both score entry points sum in the same order. Two blocks of the pass are resident
-// per SM, 304 in all: a grid of a little more runs a second wave nearly empty, so it takes the fewer chunks
-// that fill whole waves (40 nodes, T = 8760, 64 replicas: 30 chunks of 10 blocks and not 33).
+// Step chunks of the score pass: 64 steps a chunk, fewer chunks where the partials (values and bounds) and the
+// sums would not fit 2^20 doubles (the static scratch), so that both score entry points sum in the same order.
+// Two blocks of either pass (k_scores_f32, k_scores_fused in FP64; by registers) are resident on each of the
+// chip's 152 SMs, 304 in all: a grid of a little more runs a second wave nearly empty, so it takes the fewer
+// chunks that fill whole waves (40 nodes, T = 8760, 64 replicas: 30 chunks of 10 blocks and not 33). 304 is a
+// constant and not asked of the device: the chunks fix the order of the sums, and with it the last bits of
+// the scores.
 __host__ inline int score_chunks(int T, int R, int K, int N) {
     int ng = (N + ESM_SCORE_NSLOT - 1) / ESM_SCORE_NSLOT;
     long long room = (1LL << 20) - 2LL * R * (K + 8);

@@ -1852,7 +1852,8 @@ __device__ __forceinline__ int scan_warp(int *slot) {
 // units; sepmin 0: none) or walk_run walks it (else nothing: k_move does, which is launched after this kernel
 // and also takes the tasks that it lists in redo).
 // Registers: four blocks an SM in FP32 (128 a thread); two in FP64, whose walks spill at 128 (a sweep of 40
-// nodes, T = 1460, 4 replicas: 231 ms with four, 251 with three, 192 with two; T = 120, 32 replicas: 153 and 156).
+// nodes, T = 1460, 4 replicas: 231 ms with four, 251 with three, 192 with two, and 203 while each of the two
+// walks had a kernel of its own; T = 120, 32 replicas: 153 with four, 156 with two).
 template <class real>
 __global__ void __launch_bounds__(32 * ESM_SEP_WARPS, sizeof(real) == 8 ? 2 : 4)
     k_move_blocks(const __grid_constant__ DevModel<real> M, const int *steps, int nsteps, const uint32_t *sweep_p,

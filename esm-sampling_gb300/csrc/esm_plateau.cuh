@@ -704,9 +704,9 @@ struct PLane {
     // whose walks differ in length and in roots, stay together over the evaluation; the secondaries at a
     // point are saved before the roots of its segment are evaluated, so that none is evaluated again only to
     // restore them. The roots of both kinds come from one pass over the segment; those of the node balances
-    // are taken again, piece by piece, only where the segment has storage roots. Two storage
-    // sweeps of 40 nodes, T=2920, 16 replicas: 193 ms with the evaluation called from nine places of two
-    // walks, 64 ms so.
+    // are taken again, piece by piece, only where the segment has storage roots. One
+    // multiscale and one long-range sweep of 40 nodes, T=2920, 16 replicas: 193 ms with the evaluation called
+    // from nine places of two walks; with this walk and the kernels below 53 to 74 ms, by the state.
     __device__ __noinline__ int walks(int *nr, int *nl) const {
         // the point evaluated next: 0; a breakpoint (chosen first); the slope probe of a ray step; the
         // segment's end; a storage root; the segment's end again; a node-balance root

@@ -298,16 +298,15 @@ int esm_move_log(esm_ctx *ctx, int32_t cls, double *out);
 int esm_set_sep_walk(esm_ctx *ctx, int32_t min_units);
 int esm_sep_walk(const esm_ctx *ctx, int32_t *min_units, int32_t *warps);
 
-/* How the line moves of a class pass are launched. ESM_MOVES_PER_MOVE (the default): one k_move
-   launch per move, all tasks of move mi before any task of move mi + 1. ESM_MOVES_PER_CLASS: the
+/* How the line moves of a class pass are launched. ESM_MOVES_PER_MOVE (the default): one launch of
+   k_move_blocks and one of k_move per move, all tasks of move mi before any task of move mi + 1. ESM_MOVES_PER_CLASS: the
    whole class pass in one launch, whose warps take (move, 32-task item) pairs in move-major order
    and run an item's move mi + 1 as soon as its move mi is done (the tasks of a colour class are
    independent, so a task's moves and their results are the same: bit-identical states), without
    the idle tail each per-move launch ends with; each of its waits for an item's previous move is
    bounded, and one that runs out makes the next esm_sync or statistics read return ESM_ETIMEOUT.
    It walks every move one task per lane; after a call of esm_set_sep_walk with a value above 0 (the
-   default's own value as well) the launches stay per move. No
-   reference counterpart. */
+   default's own value as well) the launches stay per move. No reference counterpart. */
 enum { ESM_MOVES_PER_MOVE = 0, ESM_MOVES_PER_CLASS = 1 };
 int esm_set_move_schedule(esm_ctx *ctx, int32_t schedule);
 int esm_move_schedule(const esm_ctx *ctx, int32_t *schedule);
@@ -380,8 +379,9 @@ int64_t esm_launch_count(const esm_ctx *ctx);
  * in one program, device/src/replica_run.jl:84-108) over the local sweep (local_sweep!,
  * src/local.jl:1927, as esm_operation_sweeps runs it without the storage sweeps). A sweep is one
  * CUDA graph captured at the batch's first sweep: the caching rebuild of every model, then per
- * colour-class pass one launch that builds every model's move descriptors and one line-move launch
- * per move index, whose work items are the tasks of every model that has that move. Each task
+ * colour-class pass one launch that makes every model's move list, one that builds the descriptors, and
+ * two line-move launches per move index (block walks and one-lane walks), whose work items are the tasks
+ * of every model that has that move. Each task
  * runs the arithmetic of the model's own class pass, by the walk that esm_set_sep_walk asks for at
  * the time of the call, so every model's state after esm_batch_sweeps equals the state
  * esm_operation_sweeps gives it on its own context (its launches per move).
